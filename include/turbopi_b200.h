@@ -227,6 +227,33 @@ int tpb200_nvfp4_quantize_act_pieces(const void* x, int x_dtype, int ldx, void* 
                                      int piece_rows, tpb200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------
+ * 4-bit weights x bf16 activations on the tensor cores, weights dequantised into tensor memory:
+ *   out[M, N] = act(alpha * sum_k x[m, k] * w[n, k] + bias[n]) + beta * out
+ * NVFP4 weights in either operand form of tpb200_nvfp4_gemm_ex (row-major codes with row pitch w_pitch + swizzled scale
+ * atoms, or the tiled image), dequantised exactly; INT4 weights in the layouts of tpb200_w4a16_gemm.  The activations
+ * stay bf16: no residual pieces, no quantiser launch.  x [M, K] with row stride ldx (elements, a multiple of 8).
+ * NVFP4: K % 16 == 0; INT4: K % 128 == 0.  N % 8 == 0, ldo % 8 == 0.
+ *   gated != 0 (NVFP4): W = [gate; up] stacked, out[m, j] = bf16(act(bf16(gate_j))) * bf16(up_j), N / 2 columns
+ *          (GemmaMLP, openpi/src/openpi/models_pytorch/transformers_replace/models/gemma/modeling_gemma.py:212-230);
+ *          `activation` GELU or SILU, N % 128 == 0.
+ *   qkv_k_rows != NULL (NVFP4): the fused QKV + RoPE + cache append of tpb200_nvfp4_gemm_ex (same row permutation); q goes to
+ *          `out` with row stride ldo.
+ * No workspace: K is split over the CTAs of a cluster, which sum through distributed shared memory in a fixed order.
+ * ------------------------------------------------------------------------------------------- */
+enum { TPB200_W4_NVFP4_ROWMAJOR = 0, TPB200_W4_NVFP4_TILED = 1, TPB200_W4_INT4_KBLOCK = 2, TPB200_W4_INT4_PLUGIN = 3 };
+typedef struct {
+    const void* x; int ldx;
+    int format; const void* w; int w_pitch; const void* w_scales; const void* w_zeros;
+    float alpha; float beta; const void* bias; int bias_dtype; int activation; int gated;
+    void* out; int out_dtype; int ldo;
+    int M, N, K;
+    int qkv_q_dim; void* qkv_k_rows; void* qkv_v_rows;
+    const int* qkv_positions; const void* qkv_rope_cos; const void* qkv_rope_sin;
+    int flags;
+} tpb200_w4_gemm_args;
+int tpb200_w4_gemm(const tpb200_w4_gemm_args* args, tpb200_stream_t stream);
+
+/* ---------------------------------------------------------------------------------------------
  * NVFP4 weight-only GEMV for decode shapes (M <= 16) on the tensor cores: same result as
  * tpb200_nvfp4_gemv (E4M3 block-16 scales + global scale), no per-weight work on the SM.
  * w_image is the tensor-core GEMM's tiled B image (tpb200_nvfp4_tile_weights; blocks

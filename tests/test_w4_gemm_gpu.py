@@ -1,0 +1,115 @@
+"""The GEMM that dequantises 4-bit weights into tensor memory, against float64 on the dequantised weights."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _nvfp4(N, K, device, seed):
+    """(codes [N, pitch], scale atoms, dequantised float64 [N, K])"""
+    from turbopi_b200 import ops
+    from turbopi_b200.nvfp4_packed import unpack_nvfp4
+    g = torch.Generator().manual_seed(seed)
+    codes = torch.randint(0, 256, (N, K // 2), generator=g, dtype=torch.uint8)
+    scales = torch.randint(0, 0x7F, (N, K // 16), generator=g, dtype=torch.uint8)      # every finite UE4M3 value
+    w = unpack_nvfp4(codes, N, K).double() * scales.view(torch.float8_e4m3fn).double().repeat_interleave(16, 1)
+    b = torch.zeros((N, ops.packed_pitch(K)), dtype=torch.uint8)
+    b[:, :K // 2] = codes
+    return b.to(device), ops.swizzle_scales(scales).to(device), w.to(device)
+
+
+def _check(y, ref, mag, out_eps):
+    """|y - ref| <= half an ulp of the output type + fp32 accumulation (mag = sum |x w|, K terms in any order)"""
+    err = (y.double() - ref).abs()
+    assert bool((err <= out_eps * ref.abs() + 2e-6 * mag + 1e-30).all()), float((err / (ref.abs() + mag)).max())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (17, 128, 64), (50, 1024, 4096), (50, 2560, 1024), (64, 136, 272),
+                                   (128, 1152, 592), (129, 4304, 1152), (256, 264, 4304), (257, 128, 2048), (712, 2048, 2048)])
+@pytest.mark.parametrize("tiled", [False, True])
+def test_nvfp4(cuda_device, M, N, K, tiled):
+    from turbopi_b200 import _lib, ops
+    b, sf, w = _nvfp4(N, K, cuda_device, M + N + K)
+    x = torch.randn((M, K + 8), generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(cuda_device)[:, :K]
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(N)).to(cuda_device)
+    ref, mag = x.double() @ w.t(), x.double().abs() @ w.abs().t()
+    weight = (ops.tile_weights(b, sf, N, K), N, _lib.W4_NVFP4_TILED) if tiled else (b, N, _lib.W4_NVFP4_ROWMAJOR, sf)
+    y = ops.w4_gemm(x, *weight, alpha=0.25, out_dtype=torch.float32)
+    _check(y, 0.25 * ref, mag, 2.0 ** -22)
+    y = ops.w4_gemm(x, *weight, alpha=0.25, bias=bias)
+    _check(y, 0.25 * ref + bias.double(), mag, 2.0 ** -8)
+    out = torch.randn((M, N + 8), device=cuda_device).to(torch.float16)
+    old = out.clone()
+    ops.w4_gemm(x, *weight, alpha=2.0 ** -8, beta=0.5, out=out[:, :N])
+    _check(out[:, :N], 2.0 ** -8 * ref + 0.5 * old[:, :N].double(), 2.0 ** -8 * mag + old[:, :N].double().abs(), 2.0 ** -10)
+    assert torch.equal(out[:, N:], old[:, N:])
+    assert _lib.load().tpb200_device_error(0) == 0
+
+
+@pytest.mark.parametrize("M,I,K", [(1, 64, 64), (50, 4096, 1024), (130, 192, 304), (300, 448, 1024)])
+@pytest.mark.parametrize("tiled", [False, True])
+def test_gated(cuda_device, M, I, K, tiled):
+    from turbopi_b200 import _lib, ops
+    b, sf, w = _nvfp4(2 * I, K, cuda_device, M + I + K)
+    x = torch.randn((M, K), generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(cuda_device)
+    a = 1.0 / float((x.double() @ w.t()).std())
+    weight = (ops.tile_weights(b, sf, 2 * I, K), 2 * I, _lib.W4_NVFP4_TILED) if tiled else (b, 2 * I, _lib.W4_NVFP4_ROWMAJOR, sf)
+    gu = ops.w4_gemm(x, *weight, alpha=a)                                  # checked above
+    for act, fn in ((_lib.ACT_GELU, lambda v: torch.nn.functional.gelu(v, approximate="tanh")),
+                    (_lib.ACT_SILU, torch.nn.functional.silu)):
+        y = ops.w4_gemm(x, *weight, alpha=a, activation=act, gated=True).double()
+        g = fn(gu[:, :I].double())
+        ref = g.to(torch.bfloat16).double() * gu[:, I:].double()
+        # the activation may round to the neighbouring bf16 (2^-8 of it), the product rounds once more (2^-9)
+        assert bool(((y - ref).abs() <= 1.6 * 2.0 ** -8 * ref.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("M", [1, 50, 177])
+def test_qkv_epilogue_equals_the_piecewise_gemm(cuda_device, M):
+    """Same projection, rotation and cache rows as the e2m1-piece GEMM's epilogue, up to its activation rounding."""
+    from turbopi_b200 import _lib, ops
+    K, q_dim, N = 1024, 2048, 2560
+    b, sf, _ = _nvfp4(N, K, cuda_device, 3)
+    x = torch.randn((M, K), generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(cuda_device)
+    cos, sin = ops.rope_tables(1024, device=cuda_device)
+    pos = torch.randperm(1024, generator=torch.Generator().manual_seed(1))[:M].to(torch.int32).to(cuda_device)
+    kv = torch.zeros((4, M + 2, 256), dtype=torch.bfloat16, device=cuda_device)
+    ref = ops.fused_qkv_rope_append(x, b, sf, q_dim, kv[0], kv[1], pos, cos, sin, 2.0 ** -9, 4)
+    q = torch.empty_like(ref)
+    p = ops._ptr
+    ops._w4_gemm(_lib.W4GemmArgs(x=p(x), ldx=K, format=_lib.W4_NVFP4_ROWMAJOR, w=p(b), w_pitch=b.stride(0), w_scales=p(sf),
+                                 alpha=2.0 ** -9, out=p(q), out_dtype=_lib.BF16, ldo=q_dim, M=M, N=N, K=K, qkv_q_dim=q_dim,
+                                 qkv_k_rows=p(kv[2]), qkv_v_rows=p(kv[3]), qkv_positions=p(pos), qkv_rope_cos=p(cos),
+                                 qkv_rope_sin=p(sin)), cuda_device)
+    for a, c in ((q, ref), (kv[2], kv[0]), (kv[3], kv[1])):
+        # four pieces leave 3e-3 of a row's largest entry; two more bf16 roundings
+        assert float((a.double() - c.double()).abs().max()) <= 8e-3 * float(c.double().abs().max())
+    assert float((kv[2:, M:]).abs().max()) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 8, 128), (50, 1032, 1024), (200, 136, 384), (257, 512, 2048), (712, 2048, 1024)])
+@pytest.mark.parametrize("plugin", [False, True])
+def test_int4(cuda_device, M, N, K, plugin):
+    from turbopi_b200 import _lib, ops
+    from turbopi_b200.w4a16 import _codes_to_words
+    g = torch.Generator().manual_seed(M + N + K)
+    codes = torch.randint(0, 16, (N, K), generator=g, dtype=torch.uint8)
+    x = torch.randn((M, K), generator=g).to(torch.bfloat16)
+    q = codes.double() - 8
+    words = _codes_to_words(codes)
+    if plugin:
+        sc = (torch.rand((N, K // 128), generator=g) * 0.1).to(torch.bfloat16)
+        zp = (torch.randn((N, K // 128), generator=g) * 0.1).to(torch.bfloat16)
+        w = (q * sc.double().repeat_interleave(128, 1) + zp.double().repeat_interleave(128, 1)).float().to(torch.bfloat16)
+        packed = (words.view(torch.uint8).reshape(N, K // 2) ^ 0x88).to(cuda_device)      # two's-complement nibbles
+        args = (packed, N, _lib.W4_INT4_PLUGIN, sc.to(cuda_device), zp.to(cuda_device))
+    else:
+        sc = (torch.rand((N, K // 32), generator=g) * 0.1).half()
+        w = (q * sc.double().repeat_interleave(32, 1)).float().to(torch.bfloat16)         # exact in fp32, one rounding
+        packed = words.reshape(N, K // 32, 4).permute(1, 0, 2).contiguous().to(cuda_device)
+        args = (packed, N, _lib.W4_INT4_KBLOCK, sc.t().contiguous().to(cuda_device))
+    xd, wd = x.to(cuda_device), w.double().to(cuda_device)
+    y = ops.w4_gemm(xd, *args, out_dtype=torch.float32)
+    _check(y, xd.double() @ wd.t(), xd.double().abs() @ wd.abs().t(), 2.0 ** -22)
+    assert _lib.load().tpb200_device_error(0) == 0

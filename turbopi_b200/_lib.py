@@ -14,6 +14,7 @@ F32, F16, BF16 = 0, 1, 2
 ACT_NONE, ACT_GELU, ACT_SILU, ACT_GEGLU = 0, 1, 2, 3
 SCALE_F32, SCALE_E4M3, SCALE_F16, SCALE_BF16 = 0, 1, 2, 3
 INT4_KBLOCK, INT4_ROWMAJOR, INT4_PLUGIN = 0, 1, 2
+W4_NVFP4_ROWMAJOR, W4_NVFP4_TILED, W4_INT4_KBLOCK, W4_INT4_PLUGIN = 0, 1, 2, 3
 FLAG_NONE, FLAG_PDL = 0, 1
 MAX_GROUP = 64
 
@@ -40,6 +41,16 @@ class GemmArgs(ctypes.Structure):
                 ("qkv_k_rows", c_void_p), ("qkv_v_rows", c_void_p),
                 ("qkv_positions", c_void_p), ("qkv_rope_cos", c_void_p), ("qkv_rope_sin", c_void_p),
                 ("workspace", c_void_p), ("workspace_bytes", c_size_t), ("layout", c_int), ("flags", c_int)]
+
+
+class W4GemmArgs(ctypes.Structure):
+    _fields_ = [("x", c_void_p), ("ldx", c_int),
+                ("format", c_int), ("w", c_void_p), ("w_pitch", c_int), ("w_scales", c_void_p), ("w_zeros", c_void_p),
+                ("alpha", c_float), ("beta", c_float), ("bias", c_void_p), ("bias_dtype", c_int), ("activation", c_int),
+                ("gated", c_int), ("out", c_void_p), ("out_dtype", c_int), ("ldo", c_int),
+                ("M", c_int), ("N", c_int), ("K", c_int),
+                ("qkv_q_dim", c_int), ("qkv_k_rows", c_void_p), ("qkv_v_rows", c_void_p),
+                ("qkv_positions", c_void_p), ("qkv_rope_cos", c_void_p), ("qkv_rope_sin", c_void_p), ("flags", c_int)]
 
 
 class GemvTcProblem(ctypes.Structure):
@@ -106,6 +117,7 @@ SIGNATURES = {
     "tpb200_nvfp4_quantize_act": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]),
     "tpb200_nvfp4_gemm": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int,
                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "tpb200_w4_gemm": (c_int, [ctypes.POINTER(W4GemmArgs), c_void_p]),
     "tpb200_nvfp4_gemm_ex": (c_int, [ctypes.POINTER(GemmArgs), c_void_p]),
     "tpb200_nvfp4_quantize_act_pieces": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                                  c_int, c_int, c_int, c_void_p]),

@@ -1233,6 +1233,20 @@ bool make_tensor_map_bytes_sw128(CUtensorMap* map, const void* base, uint64_t ro
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// 2-D tensor [dim1, dim0] (dim0 contiguous) of any element type, zero fill past the edges, 128-byte swizzle or none.
+bool make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t dim0, uint64_t dim1,
+                        uint64_t pitch_bytes, uint32_t box0, uint32_t box1, bool swizzle128) {
+    EncodeFn fn = get_encode_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[2] = {dim0, dim1};
+    const cuuint64_t strides[1] = {pitch_bytes};
+    const cuuint32_t box[2] = {box0, box1};
+    const cuuint32_t elem_strides[2] = {1, 1};
+    return fn(map, type, 2, const_cast<void*>(base), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // bf16 tensor of `rank` (2..5) dimensions, dims[0] contiguous, strides_bytes[i] = byte stride of dims[i + 1];
 // box[0] <= 64 elements (one 128-byte swizzle row), elements past the end of a dimension read as zero.
 bool make_tensor_map_bf16_nd_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,

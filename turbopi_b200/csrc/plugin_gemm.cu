@@ -8,9 +8,7 @@
 #include "common.cuh"
 
 namespace tpb {
-int w4a16_gemm_tc_launch(int format, const void* x, const void* w, const void* scale, const void* zero, const void* bias,
-                         int bias_dtype, void* out, int out_dtype, int M, int N, int K, int ldo, float alpha, float beta,
-                         int flags, cudaStream_t stream);
+int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream);
 }
 
 namespace tpb {
@@ -72,8 +70,22 @@ extern "C" void w4a16GemmForward(const void* activation, const void* weight_pack
     if (M < 1 || N < 1 || K < tpb::kW4A16Group || K % tpb::kW4A16Group != 0) return tpb::set_last_error(TPB200_ERR_SHAPE);
     if (M > 16) {
         // prefill-sized: one tensor-core launch (zero points, alpha and beta in its epilogue; no workspace)
-        const int st = tpb::w4a16_gemm_tc_launch(0, activation, weight_packed, weight_scale, weight_zero, nullptr, TPB200_F32,
-                                                 output, TPB200_BF16, M, N, K, N, alpha, beta, TPB200_FLAG_NONE, stream);
+        tpb200_w4_gemm_args a = {};
+        a.x = activation;
+        a.ldx = K;
+        a.format = TPB200_W4_INT4_PLUGIN;
+        a.w = weight_packed;
+        a.w_scales = weight_scale;
+        a.w_zeros = weight_zero;
+        a.alpha = alpha;
+        a.beta = beta;
+        a.out = output;
+        a.out_dtype = TPB200_BF16;
+        a.ldo = N;
+        a.M = M;
+        a.N = N;
+        a.K = K;
+        const int st = tpb::w4_gemm_launch(&a, stream);
         tpb::set_last_error(st);
         return;
     }

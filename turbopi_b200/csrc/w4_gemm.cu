@@ -1,0 +1,794 @@
+// 4-bit weights x bf16 activations on the 5th-generation tensor cores, weights dequantised into TENSOR MEMORY:
+//   out[M, N] = act(alpha * sum_k x[m, k] * w[n, k] + bias[n]) + beta * out
+//
+// A tile is 128 weight rows x NT tokens (NT a multiple of 16, up to 256).  The weight rows are the M side of
+// tcgen05.mma kind::f16 and come from tensor memory, the tokens are the N side and come from shared memory, so a
+// few tokens cost a few columns instead of a padded 128-row tile.  Two groups of four warps turn codes into bf16
+// in registers (thread = weight row) and store them with tcgen05.st; nothing dequantised passes through shared
+// memory, whose port the activation tiles and the MMAs need.  What a weight becomes:
+//   NVFP4        e2m1 x UE4M3 has six significant bits: the product is EXACT in bf16, and so is the result up to the
+//                fp32 accumulation -- activations need no residual pieces and no quantiser launch in front
+//   INT4 k-block (q - 8) * scale with an 11-bit fp16 scale, rounded once to bf16: the scale is split into two bf16
+//                parts, q * low part is exact, so one fused multiply-add rounds like the fp32 product would
+//   INT4 plugin  q * scale + zero, one fused multiply-add
+//
+// Split K: the CTAs of a thread-block cluster take K ranges of one tile; each parks its partial sums in its own
+// shared memory, and every CTA finishes its share of the tokens from all of them through distributed shared
+// memory, summed in rank order (deterministic; no workspace, no counters, no waiting on other clusters).
+//
+// What bounds it: four 128 x NT x 16 MMAs with A in tensor memory take exactly 2 NT cycles (measured, NT 32..256), the
+// dequantisation of their 128 x 64 weights ~320 ALU cycles of an SM, and the token tiles are re-read once per 128 weight
+// rows (8-9 TB/s from L2 at 712 x 16384 x 2048).  B200, in a chain of programmatic dependent launches: INT4
+// 712 x 16384 x 2048 49 us (975 TFLOP/s; 85 us with weights dequantised through shared memory), 397 x 2048 x 16384 33 us
+// with four K ranges (265 us without split K).  Pairs of CTAs sharing the token tile (cta_group::2) halve those reads
+// but were slower (147 against 103 us at 712 x 32768 x 2048): the barrier round trips between the two SMs sit on the
+// issuing warp's path.
+//
+// Roles (352 threads): warp 0 activation tiles (TMA), warp 1 tensor memory + MMA issue, warps 2..9 dequantisation
+// and epilogue, warp 10 weight blocks (256 K values of 128 rows: 16 KB of codes + scales).  Weight blocks are
+// requested and dequantised BEFORE griddepcontrol.wait: under programmatic dependent launch a launch's weights are
+// already in tensor memory when its predecessor's activations arrive.  Every wait is bounded.
+#include <algorithm>
+#include <atomic>
+
+#include "tcgen05.cuh"
+
+namespace tpb {
+
+bool make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t dim0, uint64_t dim1,
+                        uint64_t pitch_bytes, uint32_t box0, uint32_t box1, bool swizzle128);
+
+namespace {
+
+constexpr int kRows = 128;                       // weight rows per tile
+constexpr int kBlkK = 256;                       // K values of one weight block
+constexpr int kStepK = 64;                       // K values of one MMA step: a 128-byte row of bf16
+constexpr int kSlabBytes = 2048;                 // scales of 128 rows x 256 K
+constexpr int kCodeBytes = kRows * kBlkK / 2;    // 16 KB
+constexpr int kWSlot = kCodeBytes + 2 * kSlabBytes;
+constexpr int kMaxW = 4, kMaxS = 14;
+constexpr int kXWarp = 0, kMmaWarp = 1, kWWarp = 2, kDqWarp0 = 3;
+constexpr int kDqWarpsPerSm = 16;                // 16 dequantisation warps with an SM of its own, 8 with two CTAs per SM
+constexpr long long kWaitG = 400000000LL;        // ~0.2 s
+
+enum { kFmtNvfp4 = 0, kFmtKblock = 1, kFmtPlugin = 2 };
+enum { kEpiPlain = 0, kEpiQkv = 1, kEpiGated = 2 };
+
+struct W4gParams {
+    CUtensorMap map_x;                           // bf16 [M, K], box 64 x NT, 128-byte swizzle
+    CUtensorMap map_w;                           // codes (unused with a tiled image)
+    CUtensorMap map_s;                           // k-block scales
+    const uint8_t* image;                        // tiled NVFP4 image or null
+    const uint8_t* sf;                           // row-major NVFP4: scale atoms
+    const __half* kb_scale;                      // k-block scales that TMA cannot fetch (base not 16-byte aligned), else null
+    const __nv_bfloat16* pl_scale;               // plugin: [N, K / 128]
+    const __nv_bfloat16* pl_zero;
+    const void* bias;
+    void* out;
+    int bias_dtype, out_dtype, ldo, activation;
+    float alpha, beta;
+    int M, N, K;
+    int nt;                                      // tokens per tile
+    int splits;                                  // CTAs (cluster size) per tile, each with a K range
+    int k_blocks, k_steps;
+    int n_w, n_s;                                // ring depths: weight blocks, operand steps
+    int tmem_cols, a_col;
+    int epilogue;
+    int gated_rows;                              // kEpiGated: rows of one half (I), W = [gate; up]
+    int img_kblocks;                             // K blocks per 256-row block of the image / atoms per row tile / 4
+    int q_dim, ldq;
+    __nv_bfloat16* k_rows;
+    __nv_bfloat16* v_rows;
+    const int* positions;
+    const __nv_bfloat16* rope_cos;
+    const __nv_bfloat16* rope_sin;
+};
+
+struct W4gControl {
+    uint64_t w_full[kMaxW], w_empty[kMaxW];      // raw weight blocks
+    uint64_t full[kMaxS], empty[kMaxS];          // operand steps: weights in tensor memory + activations in shared memory
+    uint64_t acc_full;
+    uint32_t tmem_base;
+};
+
+__device__ __forceinline__ uint32_t idesc_bf16(int n) {
+    // D = f32, A = B = bf16, both K-major, N >> 3 at [17,23), M = 128
+    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+// D[tmem] (+)= A[tmem] * B[smem]^T
+__device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n"
+        " .reg .pred p;\n"
+        " setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) { return __byte_perm(a, b, s); }
+__device__ __forceinline__ uint32_t bits(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
+
+// prmt with selector bit 3 live (replicate the selected byte's sign), which __byte_perm masks off
+__device__ __forceinline__ uint32_t prmt_raw(uint32_t a, uint32_t b, uint32_t s) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s));
+    return d;
+}
+
+// Eight e2m1 codes (code i at bits 4 i) -> bf16 pairs in K order, times the block scale (exact).  The three magnitude
+// bits select the high and the low byte of the bf16 value from two byte tables; a code's own bit 3, used as prmt's
+// "replicate the sign" flag on a table of 0x80, marks the negative ones.
+__device__ __forceinline__ void dequant_e2m1x8(uint32_t w, __nv_bfloat162 s, uint32_t* out) {
+    const uint32_t m = w & 0x77777777u;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t mm = h ? m >> 16 : m, ww = h ? w >> 16 : w;
+        const uint32_t lo = prmt_raw(0xC0800000u, 0xC0804000u, mm);
+        uint32_t hi = prmt_raw(0x3F3F3F00u, 0x40404040u, mm);
+        const uint32_t neg = prmt_raw(0x80808080u, 0x80808080u, ww);   // 0x80 or, for a negative code, 0xFF
+        hi |= (neg << 7) & 0x80808080u;
+        out[2 * h] = bits(__hmul2(as_bf162(prmt_raw(lo, hi, 0x5140)), s));
+        out[2 * h + 1] = bits(__hmul2(as_bf162(prmt_raw(lo, hi, 0x7362)), s));
+    }
+}
+
+// Eight unsigned nibbles (zero point 8) -> q - 8 as exact bf16 pairs in K order
+__device__ __forceinline__ void nibbles_minus8(uint32_t w, __nv_bfloat162* q) {
+    const __nv_bfloat162 k136 = as_bf162(0x43084308u);
+    uint32_t h[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = bits(__hsub2(as_bf162(((w >> (4 * j)) & 0x000F000Fu) | 0x43004300u), k136));
+    q[0] = as_bf162(prmt(h[0], h[1], 0x5410));
+    q[1] = as_bf162(prmt(h[2], h[3], 0x5410));
+    q[2] = as_bf162(prmt(h[0], h[1], 0x7632));
+    q[3] = as_bf162(prmt(h[2], h[3], 0x7632));
+}
+
+__device__ __forceinline__ float act_fast(float x, int act) {
+    if (act == TPB200_ACT_GELU) {   // 0.5 x (1 + tanh z) == x * sigmoid(2 z), without cancellation for negative x
+        const float z2 = 1.5957691216057308f * (x + 0.044715f * x * x * x);
+        return __fdividef(x, 1.0f + __expf(-z2));
+    }
+    if (act == TPB200_ACT_SILU) return __fdividef(x, 1.0f + __expf(-x));
+    return x;
+}
+__device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+    return make_uint4(bits(__floats2bfloat162_rn(v[0], v[1])), bits(__floats2bfloat162_rn(v[2], v[3])),
+                      bits(__floats2bfloat162_rn(v[4], v[5])), bits(__floats2bfloat162_rn(v[6], v[7])));
+}
+
+template <int kFmt>
+__global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__ W4gParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sW = smem;                                              // [n_w][16 KB codes | 2 scale slabs]
+    uint8_t* sB = sW + P.n_w * kWSlot;                               // [n_b][nt rows of 128 bytes]
+    const int b_bytes = P.nt * 128;
+    __shared__ W4gControl ctl;
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform, and known to be
+    const int splits = P.splits;
+    const int tile = blockIdx.x / splits;
+    const int rank = blockIdx.x - tile * splits;                     // K range
+    const int groups = ((blockDim.x >> 5) - kDqWarp0) >> 2;          // of four dequantisation warps
+    const int t0 = blockIdx.y * P.nt;                                // first token
+    const int blk0 = rank * P.k_blocks / splits, blk1 = (rank + 1) * P.k_blocks / splits;
+    const int nblk = blk1 - blk0;
+    const int steps = min(blk1 * 4, P.k_steps) - blk0 * 4;
+    // weight rows of the tile: rows 0..63 start at row_a, 64..127 at row_b (apart only in the gated form)
+    const int row_a = P.epilogue == kEpiGated ? tile * 64 : tile * kRows;
+    const int row_b = P.epilogue == kEpiGated ? P.gated_rows + row_a : row_a + 64;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < P.n_w; ++s) {
+            mbar_init(&ctl.w_full[s], 1);
+            mbar_init(&ctl.w_empty[s], 16);                          // 4 steps x 4 warps
+        }
+        for (int s = 0; s < P.n_s; ++s) {
+            mbar_init(&ctl.full[s], 5);                              // the activation tile and four dequantising warps
+            mbar_init(&ctl.empty[s], 1);
+        }
+        mbar_init(&ctl.acc_full, 1);
+        fence_mbar_init();
+    }
+    if (warp == kMmaWarp) {
+        __syncwarp();
+        tc::tmem_alloc(&ctl.tmem_base, P.tmem_cols);
+        tc::tmem_relinquish();
+    }
+    if (warp == kXWarp && lane == 0) tc::prefetch_tensormap(&P.map_x);
+    if (warp == kWWarp && lane == 0 && P.image == nullptr) tc::prefetch_tensormap(&P.map_w);
+    tc::fence_before_thread_sync();
+    __syncthreads();
+    tc::fence_after_thread_sync();
+    const uint32_t tmem = ctl.tmem_base;
+    pdl_launch_dependents();
+
+    if (warp == kXWarp) {
+        // ------------------------------------------------------------ activation tiles
+        if (lane == 0) {
+            pdl_wait_prior_grids();
+            int s = 0, ph = 1;
+            for (int i = 0; i < steps; ++i) {
+                if (i >= P.n_s && !mbar_wait_bounded(&ctl.empty[s], ph, kWaitG)) {
+                    record_error(kErrGemmEmptyBarrierTimeout);
+                    break;
+                }
+                mbar_expect_tx(&ctl.full[s], b_bytes);
+                tc::tma_load_2d(sB + s * b_bytes, &P.map_x, (blk0 * 4 + i) * kStepK, t0, &ctl.full[s]);
+                if (++s == P.n_s) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == kWWarp) {
+        // ------------------------------------------------------------ weight blocks
+        const uint64_t policy = l2_policy_evict_first();
+        const bool gated = P.epilogue == kEpiGated;
+        const uint32_t bytes = kFmt == kFmtNvfp4 ? (gated ? kCodeBytes + 2 * kSlabBytes : kCodeBytes + kSlabBytes)
+                               : kFmt == kFmtKblock && P.kb_scale == nullptr ? kCodeBytes + kSlabBytes : kCodeBytes;
+        for (int j = 0; j < nblk; ++j) {
+            const int s = j % P.n_w, kb = blk0 + j;
+            uint8_t* slot = sW + s * kWSlot;
+            if (lane == 0) {
+                if (j >= P.n_w && !mbar_wait_bounded(&ctl.w_empty[s], ((j / P.n_w) - 1) & 1, kWaitG)) {
+                    record_error(kErrGemmEmptyBarrierTimeout);
+                }
+                mbar_expect_tx(&ctl.w_full[s], bytes);
+            }
+            __syncwarp();
+            // the requests of a block leave from different lanes: one lane needs ~0.3 us per request
+            if (kFmt == kFmtNvfp4) {
+                const int half = lane & 1, row = half ? row_b : row_a;
+                if (lane < 2) {
+                    if (P.image != nullptr) {
+                        const uint8_t* b = P.image + (static_cast<size_t>(row >> 8) * P.img_kblocks + kb) * 36864;
+                        bulk_copy_g2s_hint(slot + half * 8192, b + (row & 255) * 128, 8192, &ctl.w_full[s], policy);
+                    } else {
+                        tc::tma_load_2d(slot + half * 8192, &P.map_w, kb * 128, row, &ctl.w_full[s]);
+                    }
+                } else if (lane < (gated ? 4 : 3)) {
+                    const uint8_t* src = P.image != nullptr
+                                             ? P.image + (static_cast<size_t>(row >> 8) * P.img_kblocks + kb) * 36864 + 32768 +
+                                                   ((row >> 7) & 1) * kSlabBytes
+                                             : P.sf + (static_cast<size_t>(row >> 7) * P.img_kblocks + kb) * kSlabBytes;
+                    bulk_copy_g2s_hint(slot + kCodeBytes + half * kSlabBytes, src, kSlabBytes, &ctl.w_full[s], policy);
+                }
+            } else if (kFmt == kFmtKblock) {
+                if (lane == 0) tc::tma_load_2d(slot, &P.map_w, row_a * 2, kb * 8, &ctl.w_full[s]);
+                if (lane == 1 && P.kb_scale == nullptr) tc::tma_load_2d(slot + kCodeBytes, &P.map_s, row_a, kb * 8, &ctl.w_full[s]);
+            } else {
+                if (lane < 2) tc::tma_load_2d(slot + lane * 8192, &P.map_w, kb * 128, lane ? row_b : row_a, &ctl.w_full[s]);
+            }
+            __syncwarp();
+        }
+    } else if (warp == kMmaWarp) {
+        // ------------------------------------------------------------ MMA issue
+        // The whole warp walks the loop and one elected lane issues: with warp-uniform control flow the operands of
+        // tcgen05.mma stay in uniform registers.  Under `if (lane == 0)` every MMA and commit took ~70 cycles to issue
+        // and this one thread was the kernel's critical path (750 cycles per 64-K step for 128-480 cycles of MMA).
+        {
+            const uint32_t idesc = idesc_bf16(P.nt);
+            const uint32_t b16 = smem_u32(sB) >> 4;
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            int s = 0, ph = 0;
+            for (int i = 0; i < steps; ++i) {
+                if (!mbar_wait_bounded(&ctl.full[s], ph, kWaitG)) {
+                    if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
+                    break;
+                }
+                tc::fence_after_thread_sync();
+                const uint32_t a_col = tm + P.a_col + s * 32, b_lo = b16 + ((s * b_bytes) >> 4);
+                if (tc::elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) {
+                        mma_bf16_ts(tm, a_col + kk * 8, tc::desc_from_words(b_lo + kk * 2, tc::kDescHiKmajorSw128), idesc,
+                                    (i > 0 || kk > 0) ? 1u : 0u);
+                    }
+                    tc::commit(&ctl.empty[s]);
+                }
+                __syncwarp();
+                if (++s == P.n_s) { s = 0; ph ^= 1; }
+            }
+            if (tc::elect_one()) tc::commit(&ctl.acc_full);
+        }
+    } else {
+        // ------------------------------------------------------------ codes -> bf16 -> tensor memory; thread = weight row
+        const int grp = (warp - kDqWarp0) >> 2;                      // takes every groups-th K step
+        const int r = (warp & 3) * 32 + lane;                        // the lanes of tensor memory this warp can reach
+        const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        const int row = r < 64 ? row_a + r : row_b + r - 64;
+        const int sf_off = (r >= 64 && P.epilogue == kEpiGated ? kSlabBytes : 0) + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+        bool ok = true;
+        float psc[2] = {0.0f, 0.0f}, pzp[2] = {0.0f, 0.0f};
+        for (int i = grp; i < steps; i += groups) {
+            const int j = i >> 2, kk = i & 3;
+            const int sw = j % P.n_w, sa = i % P.n_s;
+            if (kFmt == kFmtPlugin && row < P.N) {                   // two scales per 256 K, straight from global memory
+                const size_t g = static_cast<size_t>(row) * (P.K / 128) + (blk0 + j) * 2 + (kk >> 1);
+                psc[0] = __bfloat162float(__ldg(P.pl_scale + g));
+                pzp[0] = P.pl_zero != nullptr ? __bfloat162float(__ldg(P.pl_zero + g)) : 0.0f;
+            }
+            if (!mbar_wait_bounded(&ctl.w_full[sw], (j / P.n_w) & 1, kWaitG)) ok = false;
+            const uint8_t* slot = sW + sw * kWSlot;
+            uint32_t out[32];
+            uint4 c[2];
+            if (kFmt == kFmtKblock) {
+                c[0] = *reinterpret_cast<const uint4*>(slot + (2 * kk) * 2048 + r * 16);
+                c[1] = *reinterpret_cast<const uint4*>(slot + (2 * kk + 1) * 2048 + r * 16);
+            } else {
+                c[0] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk) ^ (r & 7)) << 4));
+                c[1] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk + 1) ^ (r & 7)) << 4));
+            }
+            uint32_t sc = 0;
+            if (kFmt == kFmtNvfp4) sc = *reinterpret_cast<const uint32_t*>(slot + kCodeBytes + kk * 512 + sf_off);
+            if (kFmt == kFmtKblock) {
+                if (P.kb_scale == nullptr) {
+                    const __half* sp = reinterpret_cast<const __half*>(slot + kCodeBytes) + (2 * kk) * kRows + r;
+                    psc[0] = __half2float(sp[0]);
+                    psc[1] = __half2float(sp[kRows]);
+                } else if (row < P.N) {
+                    const __half* sp = P.kb_scale + static_cast<size_t>((blk0 + j) * 8 + 2 * kk) * P.N + row;
+                    psc[0] = __half2float(__ldg(sp));
+                    psc[1] = __half2float(__ldg(sp + P.N));
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl.w_empty[sw]);            // every lane's codes are in registers
+            const uint32_t w[8] = {c[0].x, c[0].y, c[0].z, c[0].w, c[1].x, c[1].y, c[1].z, c[1].w};
+            if (kFmt == kFmtNvfp4) {
+                const float2 f0 = decode_e4m3x2(static_cast<uint16_t>(sc)), f1 = decode_e4m3x2(static_cast<uint16_t>(sc >> 16));
+                const float f[4] = {f0.x, f0.y, f1.x, f1.y};
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const __nv_bfloat162 s2 = __float2bfloat162_rn(f[b]);
+                    dequant_e2m1x8(w[2 * b], s2, out + 8 * b);
+                    dequant_e2m1x8(w[2 * b + 1], s2, out + 8 * b + 4);
+                }
+            } else {
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const float s = kFmt == kFmtKblock ? psc[b] : psc[0];
+                    const __nv_bfloat162 s_hi = __float2bfloat162_rn(s);
+                    const __nv_bfloat162 s_lo = __float2bfloat162_rn(s - __low2float(s_hi));
+                    const __nv_bfloat162 zp = __float2bfloat162_rn(pzp[0]);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        __nv_bfloat162 q[4];
+                        nibbles_minus8(w[4 * b + u] ^ (kFmt == kFmtPlugin ? 0x88888888u : 0u), q);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            out[16 * b + 4 * u + e] = kFmt == kFmtKblock ? bits(__hfma2(q[e], s_hi, __hmul2(q[e], s_lo)))
+                                                                         : bits(__hfma2(q[e], s_hi, zp));
+                        }
+                    }
+                }
+            }
+            if (i >= P.n_s && !mbar_wait_bounded(&ctl.empty[sa], ((i / P.n_s) - 1) & 1, kWaitG)) ok = false;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+                if (lane == 0) record_error(kErrGemmEmptyBarrierTimeout);
+                break;
+            }
+            tc::fence_after_thread_sync();
+            tmem_st_32x32b_x32(lane_addr + P.a_col + sa * 32, out);
+            tmem_st_wait();
+            tc::fence_before_thread_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl.full[sa]);
+        }
+        // ------------------------------------------------------------ accumulator -> shared memory, [token][128 rows]
+        if (ok && !mbar_wait_bounded(&ctl.acc_full, 0, kWaitG)) {
+            record_error(kErrGemmMmaBarrierTimeout);
+            ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            tc::fence_after_thread_sync();
+            float* st = reinterpret_cast<float*>(smem);              // every ring slot has been consumed
+            const int valid = min(P.nt, P.M - t0);
+            for (int c0 = grp * 16; c0 < valid; c0 += groups * 16) {
+                uint32_t v[16];
+                tmem_ld_32x32b_x16(lane_addr + c0, v);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    if (c0 + e < valid) st[(c0 + e) * kRows + r] = __uint_as_float(v[e]);
+                }
+            }
+        }
+        tc::fence_before_thread_sync();
+    }
+
+    if (splits > 1) {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
+    if (warp == kMmaWarp) {
+        __syncwarp();
+        tc::fence_after_thread_sync();
+        tc::tmem_dealloc(tmem, P.tmem_cols);
+    }
+
+    // ---------------------------------------------------------------- this CTA's share of the tokens, all 128 rows
+    {
+        pdl_wait_prior_grids();                                      // a no-op by now; orders reads of `out` (beta)
+        const int valid = min(P.nt, P.M - t0);
+        const int tb = rank * valid / splits, te = (rank + 1) * valid / splits;
+        const uint32_t base = smem_u32(smem);
+        uint32_t peer[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) peer[p] = p < splits && splits > 1 ? map_to_rank(base, p) : base;
+        auto sum8 = [&](int t, int c, float (&v)[8]) {
+            const uint32_t off = static_cast<uint32_t>((t * kRows + c) * 4);
+            float4 a, b;
+            if (splits == 1) {
+                a = *reinterpret_cast<const float4*>(smem + off);
+                b = *reinterpret_cast<const float4*>(smem + off + 16);
+            } else {
+                a = ld_cluster_f4(peer[0] + off);
+                b = ld_cluster_f4(peer[0] + off + 16);
+#pragma unroll
+                for (int p = 1; p < 8; ++p) {
+                    if (p < splits) {
+                        const float4 x = ld_cluster_f4(peer[p] + off), y = ld_cluster_f4(peer[p] + off + 16);
+                        a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+                        b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+                    }
+                }
+            }
+            v[0] = a.x * P.alpha; v[1] = a.y * P.alpha; v[2] = a.z * P.alpha; v[3] = a.w * P.alpha;
+            v[4] = b.x * P.alpha; v[5] = b.y * P.alpha; v[6] = b.z * P.alpha; v[7] = b.w * P.alpha;
+        };
+        if (P.epilogue == kEpiPlain) {
+            for (int u = tb * 16 + threadIdx.x; u < te * 16; u += static_cast<int>(blockDim.x)) {
+                const int t = u >> 4, c = (u & 15) * 8, n = row_a + c;
+                if (n >= P.N) continue;                              // N is a multiple of 8
+                float v[8];
+                sum8(t, c, v);
+                if (P.bias != nullptr) {
+                    if (P.bias_dtype == TPB200_F32 && (reinterpret_cast<uintptr_t>(P.bias) & 15) == 0) {
+                        const float4* bp = reinterpret_cast<const float4*>(static_cast<const float*>(P.bias) + n);
+                        const float4 b0 = __ldg(bp), b1 = __ldg(bp + 1);
+                        v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
+                        v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] += load_as_float(P.bias, P.bias_dtype, n + e);
+                    }
+                }
+                if (P.activation != TPB200_ACT_NONE) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = act_fast(v[e], P.activation);
+                }
+                const size_t o = static_cast<size_t>(t0 + t) * P.ldo + n;
+                if (P.beta != 0.0f) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = fmaf(P.beta, load_as_float(P.out, P.out_dtype, o + e), v[e]);
+                }
+                if (P.out_dtype == TPB200_BF16) {
+                    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.out) + o) = pack8(v);
+                } else if (P.out_dtype == TPB200_F32) {
+                    float4* op = reinterpret_cast<float4*>(static_cast<float*>(P.out) + o);
+                    op[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    op[1] = make_float4(v[4], v[5], v[6], v[7]);
+                } else {
+                    uint32_t h[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const __half2 h2 = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+                        h[e] = *reinterpret_cast<const uint32_t*>(&h2);
+                    }
+                    *reinterpret_cast<uint4*>(static_cast<__half*>(P.out) + o) = make_uint4(h[0], h[1], h[2], h[3]);
+                }
+            }
+        } else if (P.epilogue == kEpiGated) {
+            // gate rows 0..63, up rows 64..127 of the tile; the roundings of the module: both projections, the
+            // activation and the product go to bf16
+            for (int u = tb * 8 + threadIdx.x; u < te * 8; u += static_cast<int>(blockDim.x)) {
+                const int t = u >> 3, c = (u & 7) * 8;
+                float g[8], up[8];
+                sum8(t, c, g);
+                sum8(t, c + 64, up);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) g[e] = bf16r(act_fast(bf16r(g[e]), P.activation)) * bf16r(up[e]);
+                *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.out) + static_cast<size_t>(t0 + t) * P.ldo + row_a + c) =
+                    pack8(g);
+            }
+        } else {
+            // rows 0..63 of the tile are head offsets i, rows 64..127 their rotate-half partners i + 128; the rotation
+            // in bf16, each product and the sum rounded, as torch does it.  V heads pass through.
+            const int head = tile >> 1, i0 = (tile & 1) * 64, heads = P.q_dim >> 8;
+            for (int u = tb * 8 + threadIdx.x; u < te * 8; u += static_cast<int>(blockDim.x)) {
+                const int t = u >> 3, c = (u & 7) * 8, m = t0 + t;
+                float lo[8], hi[8];
+                sum8(t, c, lo);
+                sum8(t, c + 64, hi);
+                uint32_t olo[4], ohi[4];
+                uint4 cv = make_uint4(0, 0, 0, 0), sv = cv;
+                if (head <= heads) {
+                    const size_t p = static_cast<size_t>(__ldg(P.positions + m)) * 128 + i0 + c;
+                    cv = __ldg(reinterpret_cast<const uint4*>(P.rope_cos + p));
+                    sv = __ldg(reinterpret_cast<const uint4*>(P.rope_sin + p));
+                }
+                const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w}, sw[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    __nv_bfloat162 a = __floats2bfloat162_rn(lo[2 * e], lo[2 * e + 1]);
+                    __nv_bfloat162 b = __floats2bfloat162_rn(hi[2 * e], hi[2 * e + 1]);
+                    if (head <= heads) {
+                        const __nv_bfloat162 co = as_bf162(cw[e]), si = as_bf162(sw[e]);
+                        const __nv_bfloat162 ra = __hadd2(__hmul2(a, co), __hmul2(__hneg2(b), si));
+                        const __nv_bfloat162 rb = __hadd2(__hmul2(b, co), __hmul2(a, si));
+                        a = ra;
+                        b = rb;
+                    }
+                    olo[e] = bits(a);
+                    ohi[e] = bits(b);
+                }
+                __nv_bfloat16* dst = head < heads ? static_cast<__nv_bfloat16*>(P.out) + static_cast<size_t>(m) * P.ldq + head * 256
+                                     : (head == heads ? P.k_rows : P.v_rows) + static_cast<size_t>(m) * 256;
+                *reinterpret_cast<uint4*>(dst + i0 + c) = make_uint4(olo[0], olo[1], olo[2], olo[3]);
+                *reinterpret_cast<uint4*>(dst + i0 + c + 128) = make_uint4(ohi[0], ohi[1], ohi[2], ohi[3]);
+            }
+        }
+    }
+    if (splits > 1) {                                                // nobody leaves while a peer still reads its sums
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
+}
+
+// ---------------------------------------------------------------- launch plan
+// Tokens per tile, K ranges per tile, and whether two CTAs share an SM (8 dequantising warps each) or one has it
+// to itself (16 warps).  Measured (B200, us per launch; 50 tokens, K = 1024 / 2048 / 1024 / 4096): qkv 5.4, o 5.3, gate_up
+// 6.2, down 6.8, where the e2m1-piece GEMM takes 7.8, 7.9, 8.5 and 8.8 behind a quantiser.
+struct W4gPlan { int nt, splits; bool half; };
+
+W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
+    // Microseconds on a B200, fitted to launches chained by programmatic dependent launch (50 to 712 tokens, 1024 to
+    // 32768 rows, K 1024 to 16384); it only has to rank the candidates.
+    W4gPlan best{256, 1, false};
+    float best_cost = 1e30f;
+    for (int nt = 16; nt <= 256; nt += 16) {
+        const int tt = (M + nt - 1) / nt;
+        if (tt > 65535 || (nt > 16 && (M + nt - 17) / (nt - 16) == tt)) continue;      // a narrower tile does the same
+        for (int s = 1, l = 0; s <= 8 && s <= k_blocks; s *= 2, ++l) {
+            const long long ctas = static_cast<long long>(tiles) * tt * s;
+            const bool half = nt <= 128 && ctas > sms;
+            const int steps = (k_blocks + s - 1) / s * 4;
+            const float split = l == 0 ? 0.0f : l == 1 ? 0.9f : l == 2 ? 1.5f : 3.2f;
+            // A K step: 0.25 us with 16 dequantising warps, 0.37 with 8; two CTAs on one SM share it.
+            const float step = half ? (ctas > sms ? 0.74f : 0.37f) : 0.25f + 0.0003f * nt;
+            const long long waves = (ctas + (half ? 2 * sms : sms) - 1) / (half ? 2 * sms : sms);
+            // a grid of more than half the SMs leaves the next launch no room to start its weight loads
+            const float crowd = half || 2 * ctas > sms ? 1.6f : 0.0f;
+            const float cost = waves * (1.9f + steps * step + 0.008f * nt) + split + crowd + 0.004f * std::min(ctas, 150LL);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = {nt, s, half};
+            }
+        }
+    }
+    return best;
+}
+
+}  // namespace
+
+int device_error_w4_gemm(int clear) { return read_device_error(clear); }
+
+int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
+    TPB_REQUIRE(a != nullptr && a->x != nullptr && a->w != nullptr && a->out != nullptr, TPB200_ERR_NULL);
+    TPB_REQUIRE(a->format >= TPB200_W4_NVFP4_ROWMAJOR && a->format <= TPB200_W4_INT4_PLUGIN, TPB200_ERR_ENUM);
+    TPB_REQUIRE((a->flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
+    TPB_REQUIRE(a->activation >= TPB200_ACT_NONE && a->activation <= TPB200_ACT_SILU, TPB200_ERR_ENUM);
+    const int M = a->M, N = a->N, K = a->K;
+    const bool nv = a->format == TPB200_W4_NVFP4_ROWMAJOR || a->format == TPB200_W4_NVFP4_TILED;
+    const bool qkv = a->qkv_k_rows != nullptr;
+    const bool gated = a->gated != 0;
+    TPB_REQUIRE(M >= 1 && M <= 65535 * 256 && N >= 8 && N % 8 == 0 && K >= 16, TPB200_ERR_SHAPE);
+    TPB_REQUIRE(nv ? K % 16 == 0 : K % 128 == 0, TPB200_ERR_SHAPE);
+    TPB_REQUIRE(a->ldx >= K && a->ldx % 8 == 0 && tpb_aligned16(a->x) && tpb_aligned16(a->w) && tpb_aligned16(a->out),
+                TPB200_ERR_ALIGN);
+    TPB_REQUIRE(a->format != TPB200_W4_NVFP4_ROWMAJOR || tpb_aligned16(a->w_scales), TPB200_ERR_ALIGN);
+    TPB_REQUIRE(a->format == TPB200_W4_NVFP4_TILED || a->w_scales != nullptr, TPB200_ERR_NULL);
+    TPB_REQUIRE(a->w_zeros == nullptr || a->format == TPB200_W4_INT4_PLUGIN, TPB200_ERR_ENUM);
+    TPB_REQUIRE(!(qkv && gated) && (nv || (!qkv && !gated)), TPB200_ERR_ENUM);
+    if (qkv) {
+        TPB_REQUIRE(a->qkv_v_rows && a->qkv_positions && a->qkv_rope_cos && a->qkv_rope_sin, TPB200_ERR_NULL);
+        TPB_REQUIRE(a->qkv_q_dim >= 256 && a->qkv_q_dim % 256 == 0 && N == a->qkv_q_dim + 512 && a->ldo >= a->qkv_q_dim &&
+                        a->ldo % 8 == 0,
+                    TPB200_ERR_SHAPE);
+        TPB_REQUIRE(tpb_aligned16(a->qkv_k_rows) && tpb_aligned16(a->qkv_v_rows) && tpb_aligned16(a->qkv_rope_cos) &&
+                        tpb_aligned16(a->qkv_rope_sin),
+                    TPB200_ERR_ALIGN);
+        TPB_REQUIRE(a->out_dtype == TPB200_BF16 && a->bias == nullptr && a->beta == 0.0f && a->activation == TPB200_ACT_NONE,
+                    TPB200_ERR_ENUM);
+    } else if (gated) {
+        TPB_REQUIRE(N % 128 == 0 && a->ldo >= N / 2 && a->ldo % 8 == 0, TPB200_ERR_SHAPE);
+        TPB_REQUIRE(a->out_dtype == TPB200_BF16 && a->bias == nullptr && a->beta == 0.0f && a->activation != TPB200_ACT_NONE,
+                    TPB200_ERR_ENUM);
+    } else {
+        TPB_REQUIRE(tpb_valid_dtype(a->out_dtype) && (a->bias == nullptr || tpb_valid_dtype(a->bias_dtype)), TPB200_ERR_ENUM);
+        TPB_REQUIRE(a->ldo >= N, TPB200_ERR_SHAPE);
+        TPB_REQUIRE(static_cast<long long>(a->ldo) * tpb_dtype_size(a->out_dtype) % 16 == 0, TPB200_ERR_ALIGN);
+    }
+    W4gParams P = {};
+    const int fmt = nv ? kFmtNvfp4 : a->format == TPB200_W4_INT4_KBLOCK ? kFmtKblock : kFmtPlugin;
+    const int tiles = (N + kRows - 1) / kRows;
+    P.k_blocks = (K + kBlkK - 1) / kBlkK;
+    P.k_steps = (K + kStepK - 1) / kStepK;
+    P.img_kblocks = P.k_blocks;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const W4gPlan plan = plan_w4_gemm(tiles, M, P.k_blocks, sms);
+    P.nt = plan.nt;
+    P.splits = plan.splits;
+    bool ok = make_tensor_map_2d(&P.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a->x, K, M, static_cast<uint64_t>(a->ldx) * 2, 64,
+                                 P.nt, true);
+    if (a->format == TPB200_W4_NVFP4_TILED) {
+        P.image = static_cast<const uint8_t*>(a->w);
+    } else if (a->format == TPB200_W4_INT4_KBLOCK) {
+        ok = ok && make_tensor_map_2d(&P.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT64, a->w, 2ull * N, K / 32, 16ull * N, 256, 8, false);
+        if (tpb_aligned16(a->w_scales)) {
+            ok = ok && make_tensor_map_2d(&P.map_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, a->w_scales, N, K / 32, 2ull * N, 128, 8, false);
+        } else {
+            P.kb_scale = static_cast<const __half*>(a->w_scales);
+        }
+    } else {
+        const int pitch = a->format == TPB200_W4_INT4_PLUGIN ? K / 2 : a->w_pitch;
+        TPB_REQUIRE(pitch >= K / 2 && pitch % 16 == 0, TPB200_ERR_ALIGN);
+        ok = ok && make_tensor_map_2d(&P.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, a->w, K / 2, N, pitch, 128, 64, true);
+    }
+    if (!ok) return TPB200_ERR_CUDA;
+    P.sf = static_cast<const uint8_t*>(a->w_scales);
+    P.pl_scale = static_cast<const __nv_bfloat16*>(a->w_scales);
+    P.pl_zero = static_cast<const __nv_bfloat16*>(a->w_zeros);
+    P.bias = a->bias;
+    P.bias_dtype = a->bias_dtype;
+    P.out = a->out;
+    P.out_dtype = a->out_dtype;
+    P.ldo = a->ldo;
+    P.activation = a->activation;
+    P.alpha = a->alpha;
+    P.beta = a->beta;
+    P.M = M;
+    P.N = N;
+    P.K = K;
+    P.epilogue = qkv ? kEpiQkv : gated ? kEpiGated : kEpiPlain;
+    P.gated_rows = N / 2;
+    P.q_dim = a->qkv_q_dim;
+    P.ldq = a->ldo;
+    P.k_rows = static_cast<__nv_bfloat16*>(a->qkv_k_rows);
+    P.v_rows = static_cast<__nv_bfloat16*>(a->qkv_v_rows);
+    P.positions = a->qkv_positions;
+    P.rope_cos = static_cast<const __nv_bfloat16*>(a->qkv_rope_cos);
+    P.rope_sin = static_cast<const __nv_bfloat16*>(a->qkv_rope_sin);
+
+    // Ring depths.  Up to 128 tokens: half an SM's shared and tensor memory, so that two CTAs (of this launch or of the
+    // next one in the stream) share an SM; more tokens: one CTA per SM.
+    const bool half = plan.half;
+    P.tmem_cols = half ? 256 : 512;
+    P.a_col = (P.nt + 31) / 32 * 32;
+    const int blocks_per = (P.k_blocks + P.splits - 1) / P.splits, steps_per = std::min(blocks_per * 4, P.k_steps);
+    const int budget = (half ? 112 : 225) * 1024 - 1024;
+    const int b_bytes = P.nt * 128;
+    P.n_w = std::min(half ? (P.nt <= 64 ? 3 : 2) : 3, blocks_per);
+    P.n_s = std::min(std::min(std::min(kMaxS, (P.tmem_cols - P.a_col) / 32), steps_per), (budget - P.n_w * kWSlot) / b_bytes);
+    int smem = P.n_w * kWSlot + P.n_s * b_bytes;
+    smem = std::max(smem, P.nt * kRows * 4) + 1024;
+
+    static void (*const kernels[3])(const W4gParams) = {w4_gemm_kernel<kFmtNvfp4>, w4_gemm_kernel<kFmtKblock>,
+                                                        w4_gemm_kernel<kFmtPlugin>};
+    auto kernel = kernels[fmt];
+    static std::atomic<uint64_t> configured[3] = {};
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(configured[fmt].load(std::memory_order_relaxed) & bit)) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) {
+            return TPB200_ERR_CUDA;
+        }
+        configured[fmt].fetch_or(bit, std::memory_order_relaxed);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles * P.splits, (M + P.nt - 1) / P.nt, 1);
+    cfg.blockDim = dim3((kDqWarp0 + kDqWarpsPerSm / (half ? 2 : 1)) * 32, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (P.splits > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = P.splits;
+        attr[na].val.clusterDim.y = 1;
+        attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
+    if (a->flags & TPB200_FLAG_PDL) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na].val.programmaticStreamSerializationAllowed = 1;
+        ++na;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    return cudaLaunchKernelEx(&cfg, kernel, P) == cudaSuccess ? TPB200_OK : TPB200_ERR_CUDA;
+}
+
+}  // namespace tpb
+
+extern "C" int tpb200_w4_gemm(const tpb200_w4_gemm_args* a, tpb200_stream_t stream) {
+    return tpb::w4_gemm_launch(a, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int tpb200_w4a16_gemm(const void* x, const void* weight, const void* scales, const void* zeros,
+                                 const void* bias, int bias_dtype, void* out, int out_dtype, int M, int N, int K, int ldo,
+                                 int layout, float alpha, float beta, int flags, tpb200_stream_t stream) {
+    TPB_REQUIRE((flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
+    TPB_REQUIRE(layout == TPB200_INT4_KBLOCK || layout == TPB200_INT4_PLUGIN, TPB200_ERR_ENUM);
+    TPB_REQUIRE(tpb_valid_dtype(out_dtype) && tpb_valid_dtype(bias_dtype), TPB200_ERR_ENUM);
+    tpb200_w4_gemm_args a = {};
+    a.x = x;
+    a.ldx = K;
+    a.format = layout == TPB200_INT4_KBLOCK ? TPB200_W4_INT4_KBLOCK : TPB200_W4_INT4_PLUGIN;
+    a.w = weight;
+    a.w_scales = scales;
+    a.w_zeros = zeros;
+    a.alpha = alpha;
+    a.beta = beta;
+    a.bias = bias;
+    a.bias_dtype = bias_dtype;
+    a.out = out;
+    a.out_dtype = out_dtype;
+    a.ldo = ldo == 0 ? N : ldo;
+    a.M = M;
+    a.N = N;
+    a.K = K;
+    a.flags = flags;
+    return tpb::w4_gemm_launch(&a, reinterpret_cast<cudaStream_t>(stream));
+}

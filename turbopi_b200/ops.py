@@ -381,6 +381,34 @@ def nvfp4_gemm_w4a16(x, b_packed, b_sf, N, alpha=1.0, bias=None, activation=ACT_
     return out
 
 
+def w4_gemm(x, w, N, format, w_scales=None, w_zeros=None, alpha=1.0, beta=0.0, bias=None, activation=ACT_NONE,
+            gated=False, out=None, out_dtype=torch.bfloat16):
+    """out[M, N] = act(alpha * x @ dequant(W)^T + bias) + beta * out with bf16 activations and 4-bit weights dequantised
+    inside the kernel (tpb200_w4_gemm).  `format`: _lib.W4_NVFP4_ROWMAJOR (w = codes [N, pitch], w_scales = swizzled
+    atoms), W4_NVFP4_TILED (w = the tiled image), W4_INT4_KBLOCK, W4_INT4_PLUGIN.  `gated`: W = [gate; up], the result
+    is act(gate) * up with N / 2 columns.  x [M, K] bf16, unit last stride, row stride a multiple of 8."""
+    _cuda(x, w, w_scales, w_zeros, bias, out)
+    M, K = x.shape
+    if x.dtype != torch.bfloat16 or x.stride(1) != 1:
+        raise TurboPiError("w4_gemm: bf16 activations with a contiguous last dimension")
+    if out is None:
+        out = torch.empty((M, N // 2 if gated else N), dtype=out_dtype, device=x.device)
+    args = _lib.W4GemmArgs(x=_ptr(x), ldx=x.stride(0) if M > 1 else K, format=int(format), w=_ptr(w),
+                           w_pitch=w.stride(0) if format == _lib.W4_NVFP4_ROWMAJOR else 0, w_scales=_ptr(w_scales),
+                           w_zeros=_ptr(w_zeros), alpha=float(alpha), beta=float(beta), bias=_ptr(bias),
+                           bias_dtype=_dt(bias) if bias is not None else F32, activation=int(activation), gated=int(gated),
+                           out=_ptr(out), out_dtype=_dt(out), ldo=out.stride(0) if M > 1 else out.shape[1], M=M, N=N, K=K)
+    _w4_gemm(args, x.device)
+    return out
+
+
+def _w4_gemm(args, device):
+    args.flags = _launch_flags
+    with torch.cuda.device(device):
+        st = _lib.load().tpb200_w4_gemm(ctypes.byref(args), torch.cuda.current_stream(device).cuda_stream)
+    _lib.check(st, "tpb200_w4_gemm")
+
+
 def qkv_tile_permutation(q_dim, head_dim=256):
     """Row order of the stacked [Wq; Wk; Wv] the fused-QKV kernel expects: every 128-row tile holds 64
     rows of one head's first half followed by their rotate-half partners (+ head_dim / 2)."""
