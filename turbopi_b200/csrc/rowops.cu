@@ -340,8 +340,9 @@ extern "C" int tpb200_row_transform_quantize(const tpb200_rowop_args* a, tpb200_
     P.kb_pad = (a->K + 255) / 256 * 16;
     P.tiled = a->layout == TPB200_OPERANDS_TILED;
     // rows of up to 4096 elements: two threads per 16-element block (the three residual pieces are a dependent
-    // chain per block; halving it is what a latency-bound launch gains from); longer rows: one or two blocks per thread
-    const bool halves = a->packed != nullptr && P.kb_pad <= tpb::kThreads / 2;
+    // chain per block; halving it is what a latency-bound launch gains from -- and a launch without a quantiser has twice
+    // the loads in flight); longer rows: one or two blocks per thread
+    const bool halves = P.kb_pad <= tpb::kThreads / 2;
     const int threads = halves ? 2 * P.kb_pad : std::min(tpb::kThreads, (P.kb_pad + 31) / 32 * 32);
     TPB_REQUIRE((a->flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
     cudaLaunchConfig_t cfg = {};

@@ -6,10 +6,12 @@ cache (`PI0Pytorch.sample_actions`, openpi/src/openpi/models_pytorch/pi0_pytorch
 cached denoise step :524-654; adaptive RMSNorm / gated residual / MLP,
 transformers_replace/models/gemma/modeling_gemma.py:49-129,212-230).
 
-Every linear layer runs as NVFP4 weights x bf16 activations on the tcgen05 GEMM (activations
-carried as residual e2m1 pieces); norms, residuals and GELU*up are the fused row kernels that
-write the next GEMM's operand directly; Q/K/V + RoPE + KV-cache append is the GEMM's fused
-epilogue; attention is the tensor-core kernel of csrc/attention.cu (`ops.attention`).  All buffers are
+Every linear layer runs as NVFP4 weights x bf16 activations on the tensor cores.  The two large prefix MLP
+matrices take the block-scaled e2m1 GEMM (activations as residual e2m1 pieces, written by the row kernels);
+every other linear takes the GEMM that dequantises its weights into tensor memory and reads the bf16
+activations as they are (csrc/w4_gemm.cu): no quantiser in front of it, GELU(gate) * up and Q/K/V + RoPE +
+KV-cache append in its epilogue.  Norms and residuals are the fused row kernels; attention is the
+tensor-core kernel of csrc/attention.cu (`ops.attention`).  All buffers are
 allocated once, so the whole inference (or just the denoise loop) replays as ONE CUDA graph.
 
 Weights come from a reference-named state dict (`Pi05.from_state_dict`, tensor names of
@@ -81,9 +83,8 @@ class TcLinear:
     an fp32 global scale), the global scale, an optional fp32 bias, in one of the GEMM's two operand forms:
     the tiled image (`sf is None`; 128 x 256 output tiles, one contiguous block per K stage: the form for the
     large prefix MLP matrices), or
-    row-major codes [N, pitch] + swizzled scale atoms (128 x 128 tiles, a three-stage ring: ~2 us less per launch
-    on the small, latency-bound linears of the vision tower and the action expert).  The activation operand
-    (`QuantBuf`) must be in the same form.  `raw` keeps the reference-layout codes / scale bytes for
+    row-major codes [N, pitch] + swizzled scale atoms.  A call with a `QuantBuf` (in the weight's form) runs the
+    block-scaled GEMM; `dense` / `dense_qkv` take bf16 activations and dequantise the weights inside the kernel.  `raw` keeps the reference-layout codes / scale bytes for
     dequantisation in tests."""
 
     def __init__(self, image, g, N, K, bias=None, raw=None, sf=None):
@@ -139,6 +140,30 @@ class TcLinear:
         args.qkv_k_rows, args.qkv_v_rows, args.qkv_positions = p(k_rows), p(v_rows), p(positions)
         args.qkv_rope_cos, args.qkv_rope_sin = p(cos), p(sin)
         ops._gemm_ex(args, q_out.device, self.ws)
+        return q_out
+
+    def _w4_args(self, x, M, out, ldo):
+        p = ops._ptr
+        return _lib.W4GemmArgs(x=p(x), ldx=x.stride(0), format=_lib.W4_NVFP4_ROWMAJOR if self.rowmajor else _lib.W4_NVFP4_TILED,
+                               w=p(self.b), w_pitch=self.b.stride(0) if self.rowmajor else 0, w_scales=p(self.sf),
+                               alpha=float(self.g), out=p(out), out_dtype=ops._dt(out), ldo=ldo, M=M, N=self.N, K=self.K)
+
+    def dense(self, x, out, activation=ACT_NONE, gated=False):
+        """out = act(x W^T + bias) for bf16 x [M, >= K]; `gated`: W = [gate; up], out = act(gate) * up."""
+        args = self._w4_args(x, x.shape[0], out, out.stride(0))
+        args.bias, args.activation, args.gated = ops._ptr(self.bias), int(activation), int(gated)
+        ops._w4_gemm(args, out.device)
+        return out
+
+    def dense_qkv(self, x, q_out, k_rows, v_rows, positions, cos, sin, q_dim):
+        M = x.shape[0]
+        if k_rows.shape[0] < M or v_rows.shape[0] < M or positions.numel() < M:
+            raise TurboPiError("fused QKV: cache rows / positions shorter than the token count")
+        p = ops._ptr
+        args = self._w4_args(x, M, q_out, q_out.stride(0))
+        args.qkv_q_dim, args.qkv_k_rows, args.qkv_v_rows, args.qkv_positions = q_dim, p(k_rows), p(v_rows), p(positions)
+        args.qkv_rope_cos, args.qkv_rope_sin = p(cos), p(sin)
+        ops._w4_gemm(args, q_out.device)
         return q_out
 
 
@@ -232,7 +257,8 @@ class Pi05:
         PG = "paligemma_with_expert.paligemma.model."
         EX = "paligemma_with_expert.gemma_expert.model."
 
-        # Operand form per linear: the tiled image for the large prefix MLP matrices (gate_up, down), row-major
+        # Operand form per linear: the tiled image for the large prefix MLP matrices (gate_up, down: 712 x 32768 x 2048 in
+        # 71 us + 27 us of row kernel against 114 us on the dequantising GEMM, 712 x 2048 x 16384 in 40 against 49), row-major
         # for everything else (the vision tower, the attention projections, the action expert, the small projections).
         def lin(wname, bias=True, perm=None, rm=True):
             return TcLinear.from_weight(get(wname + ".weight"), get(wname + ".bias") if bias else None, perm, kr, rm)
@@ -372,23 +398,24 @@ class Pi05:
         self.cache = torch.zeros((c.prefix_layers, 2, c.max_seq, c.head_dim), dtype=bf, device=d)
         self.b = dict(
             # vision
-            patches=torch.zeros((T, self.patch_k), dtype=bf, device=d), q_patch=QuantBuf(T, self.patch_k, P, d, tiled=False),
+            patches=torch.zeros((T, self.patch_k), dtype=bf, device=d),
             vh=torch.empty((T, vw), dtype=bf, device=d), vy=torch.empty((T, vw), dtype=bf, device=d),
-            q_v=QuantBuf(T, vw, P, d, tiled=False), v_qkv=torch.empty((T, 3 * vw), dtype=bf, device=d),
+            vx=torch.empty((T, vw), dtype=bf, device=d), v_qkv=torch.empty((T, 3 * vw), dtype=bf, device=d),
             v_attn=torch.empty((T, vw), dtype=bf, device=d),
-            v_fc1=torch.empty((T, c.vision_mlp), dtype=bf, device=d), q_vmlp=QuantBuf(T, c.vision_mlp, P, d, tiled=False),
+            v_fc1=torch.empty((T, c.vision_mlp), dtype=bf, device=d),
             # prefix
             ph=torch.empty((S, c.width), dtype=bf, device=d), py=torch.empty((S, c.width), dtype=bf, device=d),
-            q_p=QuantBuf(S, c.width, P, d), q_pqkv=QuantBuf(S, c.width, P, d, tiled=False), p_q=torch.empty((S, c.q_dim), dtype=bf, device=d),
-            q_pattn=QuantBuf(S, c.q_dim, P, d, tiled=False), p_gu=torch.empty((S, 2 * c.mlp), dtype=bf, device=d),
+            q_p=QuantBuf(S, c.width, P, d), px=torch.empty((S, c.width), dtype=bf, device=d),
+            p_q=torch.empty((S, c.q_dim), dtype=bf, device=d), p_attn=torch.empty((S, c.q_dim), dtype=bf, device=d), p_gu=torch.empty((S, 2 * c.mlp), dtype=bf, device=d),
             q_pmlp=QuantBuf(S, c.mlp, P, d), pos_prefix=torch.arange(S, dtype=torch.int32, device=d),
             # expert
             x_t=torch.zeros((A, c.action_dim), dtype=torch.float32, device=d),
-            x_bf=torch.zeros((A, c.action_dim), dtype=bf, device=d), q_act=QuantBuf(A, c.action_dim, P, d, tiled=False),
+            x_bf=torch.zeros((A, c.action_dim), dtype=bf, device=d),
             eh=torch.empty((A, ew), dtype=bf, device=d), ey=torch.empty((A, ew), dtype=bf, device=d),
-            q_e=QuantBuf(A, ew, P, d, tiled=False), e_q=torch.empty((A, c.q_dim), dtype=bf, device=d),
-            q_eattn=QuantBuf(A, c.q_dim, P, d, tiled=False), e_gu=torch.empty((A, 2 * c.expert_mlp), dtype=bf, device=d),
-            q_emlp=QuantBuf(A, c.expert_mlp, P, d, tiled=False), v_out=torch.empty((A, c.action_dim), dtype=torch.float32, device=d),
+            ex=torch.empty((A, ew), dtype=bf, device=d), e_q=torch.empty((A, c.q_dim), dtype=bf, device=d),
+            e_attn=torch.empty((A, c.q_dim), dtype=bf, device=d), e_mlp=torch.empty((A, c.expert_mlp), dtype=bf, device=d),
+            e_gu=torch.empty((A if c.expert_mlp % 64 else 0, 2 * c.expert_mlp), dtype=bf, device=d),
+            v_out=torch.empty((A, c.action_dim), dtype=torch.float32, device=d),
             pos_suffix=torch.arange(S, S + A, dtype=torch.int32, device=d),
         )
         for _, obj in self._named_parts():
@@ -444,14 +471,6 @@ class Pi05:
         ops.attention(q.view(L * c.heads, c.head_dim), k, v, out.view(L * c.heads, c.head_dim), c.head_dim ** -0.5,
                       self.key_bias, self.attn_ws)
 
-    def _attention_to_operand(self, q, k, v, quant):
-        """The same attention, its result written only as the operand of the output projection that follows
-        (the merge kernel quantises each token's H * D row itself: no bf16 round trip, no row-kernel launch)."""
-        c = self.cfg
-        L = q.shape[0]
-        ops.attention(q.view(L * c.heads, c.head_dim), k, v, None, c.head_dim ** -0.5, self.key_bias, self.attn_ws,
-                      quant=quant, rows_per_token=c.heads)
-
     def vision_tower(self):
         c, b = self.cfg, self.b
         T, vw = c.num_images * c.image_tokens, c.vision_width
@@ -459,33 +478,30 @@ class Pi05:
         img = self.images.float().div_(127.5).sub_(1.0)                               # [-1, 1]
         pt = img.view(c.num_images, n, c.patch, n, c.patch, 3).permute(0, 1, 3, 5, 2, 4).reshape(T, -1)   # (c, i, j)
         b["patches"][:, :pt.shape[1]].copy_(pt)
-        rowop(_lib.ROW_NONE, b["patches"], self.patch_k, b["q_patch"])
-        self.patch_embed(b["q_patch"], b["vh"])
+        self.patch_embed.dense(b["patches"], b["vh"])
         b["vh"].view(c.num_images, c.image_tokens, vw).add_(self.pos_emb)
         hd = vw // c.vision_heads
         first = True
         for L in self.vision:
             if first:
-                rowop(_lib.ROW_LAYERNORM, b["vh"], vw, b["q_v"], w0=L["ln1_w"], w1=L["ln1_b"], eps=c.eps)
+                rowop(_lib.ROW_LAYERNORM, b["vh"], vw, y_out=b["vx"], w0=L["ln1_w"], w1=L["ln1_b"], eps=c.eps)
                 first = False
             else:
-                rowop(_lib.ROW_LAYERNORM, b["vy"], vw, b["q_v"], res_in=b["vh"], h_out=b["vh"], w0=L["ln1_w"],
+                rowop(_lib.ROW_LAYERNORM, b["vy"], vw, y_out=b["vx"], res_in=b["vh"], h_out=b["vh"], w0=L["ln1_w"],
                       w1=L["ln1_b"], eps=c.eps)
-            L["qkv"](b["q_v"], b["v_qkv"])
+            L["qkv"].dense(b["vx"], b["v_qkv"])
             qkv = b["v_qkv"].view(c.num_images, c.image_tokens, 3, c.vision_heads, hd).permute(2, 0, 3, 1, 4)
             ops.attention(qkv[0], qkv[1], qkv[2],
                           b["v_attn"].view(c.num_images, c.image_tokens, c.vision_heads, hd).permute(0, 2, 1, 3),
                           hd ** -0.5, None, self.attn_ws)
-            rowop(_lib.ROW_NONE, b["v_attn"], vw, b["q_v"])
-            L["out"](b["q_v"], b["vy"])
-            rowop(_lib.ROW_LAYERNORM, b["vy"], vw, b["q_v"], res_in=b["vh"], h_out=b["vh"], w0=L["ln2_w"], w1=L["ln2_b"],
+            L["out"].dense(b["v_attn"], b["vy"])
+            rowop(_lib.ROW_LAYERNORM, b["vy"], vw, y_out=b["vx"], res_in=b["vh"], h_out=b["vh"], w0=L["ln2_w"], w1=L["ln2_b"],
                   eps=c.eps)
-            L["fc1"](b["q_v"], b["v_fc1"], ACT_GELU)
-            rowop(_lib.ROW_NONE, b["v_fc1"], c.vision_mlp, b["q_vmlp"])
-            L["fc2"](b["q_vmlp"], b["vy"])
-        rowop(_lib.ROW_LAYERNORM, b["vy"], vw, b["q_v"], res_in=b["vh"], h_out=b["vh"], w0=self.post_ln_w,
+            L["fc1"].dense(b["vx"], b["v_fc1"], ACT_GELU)
+            L["fc2"].dense(b["v_fc1"], b["vy"])
+        rowop(_lib.ROW_LAYERNORM, b["vy"], vw, y_out=b["vx"], res_in=b["vh"], h_out=b["vh"], w0=self.post_ln_w,
               w1=self.post_ln_b, eps=c.eps)
-        self.projector(b["q_v"], b["ph"][:T])                                          # image tokens of the prefix
+        self.projector.dense(b["vx"], b["ph"][:T])                                          # image tokens of the prefix
 
     def prefix_pass(self):
         c, b = self.cfg, self.b
@@ -494,15 +510,15 @@ class Pi05:
         first = True
         for l, L in enumerate(self.prefix):
             if first:
-                rowop(_lib.ROW_RMSNORM, b["ph"], c.width, b["q_pqkv"], w0=L["in_norm"], eps=c.eps)
+                rowop(_lib.ROW_RMSNORM, b["ph"], c.width, y_out=b["px"], w0=L["in_norm"], eps=c.eps)
                 first = False
             else:
-                rowop(_lib.ROW_RMSNORM, b["py"], c.width, b["q_pqkv"], res_in=b["ph"], h_out=b["ph"], w0=L["in_norm"],
+                rowop(_lib.ROW_RMSNORM, b["py"], c.width, y_out=b["px"], res_in=b["ph"], h_out=b["ph"], w0=L["in_norm"],
                       eps=c.eps)
-            L["qkv"].qkv(b["q_pqkv"], b["p_q"], self.cache[l, 0], self.cache[l, 1], b["pos_prefix"], self.cos, self.sin,
-                         c.q_dim)
-            self._attention_to_operand(b["p_q"], self.cache[l, 0, :S], self.cache[l, 1, :S], b["q_pattn"])
-            L["o"](b["q_pattn"], b["py"])
+            L["qkv"].dense_qkv(b["px"], b["p_q"], self.cache[l, 0], self.cache[l, 1], b["pos_prefix"], self.cos, self.sin,
+                               c.q_dim)
+            self._attention(b["p_q"], self.cache[l, 0, :S], self.cache[l, 1, :S], b["p_attn"])
+            L["o"].dense(b["p_attn"], b["py"])
             rowop(_lib.ROW_RMSNORM, b["py"], c.width, b["q_p"], res_in=b["ph"], h_out=b["ph"], w0=L["post_norm"],
                   eps=c.eps)
             # GELU(gate) * up rides in the row kernel: in the GEMM's epilogue (ACT_GEGLU) it would sit between
@@ -521,15 +537,11 @@ class Pi05:
             ts = torch.tensor([1.0 + i * dt for i in range(num_steps)], dtype=torch.float32)
             self._time_emb[num_steps] = sinusoidal_time_embedding(ts, ew).to(torch.bfloat16).to(d)
         emb = self._time_emb[num_steps]
-        qb = QuantBuf(num_steps, ew, c.pieces, d, tiled=False)
-        t1 = torch.empty((num_steps, ew), dtype=torch.bfloat16, device=d)
-        rowop(_lib.ROW_NONE, emb, ew, qb)
-        self.time_mlp_in(qb, t1, ACT_SILU)
-        rowop(_lib.ROW_NONE, t1, ew, qb)
-        self.time_mlp_out(qb, t1, ACT_SILU)
-        rowop(_lib.ROW_NONE, t1, ew, qb)
+        t1 = torch.empty((2, num_steps, ew), dtype=torch.bfloat16, device=d)
+        self.time_mlp_in.dense(emb, t1[0], ACT_SILU)
+        self.time_mlp_out.dense(t1[0], t1[1], ACT_SILU)
         mod = torch.empty((num_steps, self.n_norms * 3 * ew), dtype=torch.bfloat16, device=d)
-        self.ada_dense(qb, mod)
+        self.ada_dense.dense(t1[1], mod)
         return mod.view(num_steps, self.n_norms, 3, ew)
 
     def denoise_step(self, mod, dt):
@@ -537,30 +549,32 @@ class Pi05:
         c, b = self.cfg, self.b
         S, A, ew = c.prefix_len, c.action_horizon, c.expert_width
         b["x_bf"].copy_(b["x_t"])
-        rowop(_lib.ROW_NONE, b["x_bf"], c.action_dim, b["q_act"])
-        self.action_in(b["q_act"], b["eh"])
+        self.action_in.dense(b["x_bf"], b["eh"])
         prev_gate = None
         for l, L in enumerate(self.expert):
             m_in, m_post = mod[2 * l], mod[2 * l + 1]
             if prev_gate is None:
-                rowop(_lib.ROW_ADARMS, b["eh"], ew, b["q_e"], w0=m_in[0], w1=m_in[1], eps=c.eps)
+                rowop(_lib.ROW_ADARMS, b["eh"], ew, y_out=b["ex"], w0=m_in[0], w1=m_in[1], eps=c.eps)
             else:
-                rowop(_lib.ROW_ADARMS, b["ey"], ew, b["q_e"], res_in=b["eh"], gate=prev_gate, h_out=b["eh"], w0=m_in[0],
+                rowop(_lib.ROW_ADARMS, b["ey"], ew, y_out=b["ex"], res_in=b["eh"], gate=prev_gate, h_out=b["eh"], w0=m_in[0],
                       w1=m_in[1], eps=c.eps)
-            L["qkv"].qkv(b["q_e"], b["e_q"], self.cache[l, 0, S:], self.cache[l, 1, S:], b["pos_suffix"], self.cos,
-                         self.sin, c.q_dim)
-            self._attention_to_operand(b["e_q"], self.cache[l, 0, :S + A], self.cache[l, 1, :S + A], b["q_eattn"])
-            L["o"](b["q_eattn"], b["ey"])
-            rowop(_lib.ROW_ADARMS, b["ey"], ew, b["q_e"], res_in=b["eh"], gate=m_in[2], h_out=b["eh"], w0=m_post[0],
+            L["qkv"].dense_qkv(b["ex"], b["e_q"], self.cache[l, 0, S:], self.cache[l, 1, S:], b["pos_suffix"], self.cos,
+                               self.sin, c.q_dim)
+            self._attention(b["e_q"], self.cache[l, 0, :S + A], self.cache[l, 1, :S + A], b["e_attn"])
+            L["o"].dense(b["e_attn"], b["ey"])
+            rowop(_lib.ROW_ADARMS, b["ey"], ew, y_out=b["ex"], res_in=b["eh"], gate=m_in[2], h_out=b["eh"], w0=m_post[0],
                   w1=m_post[1], eps=c.eps)
-            L["gate_up"](b["q_e"], b["e_gu"])
-            rowop(_lib.ROW_GELU_MUL, b["e_gu"], c.expert_mlp, b["q_emlp"])
-            L["down"](b["q_emlp"], b["ey"])
+            if c.expert_mlp % 64 == 0:
+                L["gate_up"].dense(b["ex"], b["e_mlp"], ACT_GELU, gated=True)
+            else:                       # the gated epilogue pairs 64 gate rows with 64 up rows
+                L["gate_up"].dense(b["ex"], b["e_gu"])
+                rowop(_lib.ROW_GELU_MUL, b["e_gu"], c.expert_mlp, y_out=b["e_mlp"])
+            L["down"].dense(b["e_mlp"], b["ey"])
             prev_gate = m_post[2]
         m_f = mod[2 * c.expert_layers]
-        rowop(_lib.ROW_ADARMS, b["ey"], ew, b["q_e"], res_in=b["eh"], gate=prev_gate, h_out=b["eh"], w0=m_f[0], w1=m_f[1],
+        rowop(_lib.ROW_ADARMS, b["ey"], ew, y_out=b["ex"], res_in=b["eh"], gate=prev_gate, h_out=b["eh"], w0=m_f[0], w1=m_f[1],
               eps=c.eps)
-        self.action_out(b["q_e"], b["v_out"])
+        self.action_out.dense(b["ex"], b["v_out"])
         b["x_t"].add_(b["v_out"], alpha=dt)
 
     def _modulation(self, num_steps):
