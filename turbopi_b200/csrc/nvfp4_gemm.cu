@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
     uint8_t* out_stage = smem + nstages * stage_sz;                       // 2 x 16 KB, 1024-byte aligned
     SharedControl* ctl = reinterpret_cast<SharedControl*>(out_stage + 2 * kOutBuf);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);        // warp-uniform, and known to be
     const int lane = threadIdx.x & 31;
     const int splits = P.splits;
     const int total_items = P.m_blocks * P.n_blocks * splits;
@@ -414,7 +414,10 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // The whole warp walks the loop and one elected lane issues: with warp-uniform control flow the operands of the
+        // tcgen05 instructions stay in uniform registers.  Under `if (lane == 0)` each of the 33 instructions of a
+        // three-piece stage took ~70 cycles, 1.2 us per stage for 0.78 us of MMAs.
+        {
             constexpr uint32_t idesc = tc::make_idesc_mxf4nvf4(kBN);
             // descriptor words: (stage base >> 4) + compile-time offsets; see tcgen05.cuh
             const uint32_t stage16 = static_cast<uint32_t>(stage_sz) >> 4;
@@ -422,64 +425,69 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
             const uint32_t off_sfb16 = static_cast<uint32_t>(off_sfb) >> 4;
             const uint32_t off_sfa16 = static_cast<uint32_t>(off_sfa) >> 4;
             const uint32_t base16 = smem_u32(smem) >> 4;
-            const uint32_t t_sfa = tmem_base + kSfaCol;
-            const uint32_t t_sfb = tmem_base + kSfbCol;
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint32_t t_sfa = tm + kSfaCol;
+            const uint32_t t_sfb = tm + kSfbCol;
             int s = 0;
             uint32_t full_phase = 0;
             uint32_t lo0 = base16;                 // descriptor word of the current stage's first byte
             int tile_iter = 0;
-            for (int w = blockIdx.x; w < total_items && !*abort_flag; w += gridDim.x, ++tile_iter) {
+            for (int w = blockIdx.x; w < total_items; w += gridDim.x, ++tile_iter) {
+                if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
                 const int ks0 = (w % splits) * P.stages_per_split;
                 const int ks1 = min(P.k_stages, ks0 + P.stages_per_split);
                 const int buf = tile_iter % kAccBufs;
                 const int use = tile_iter / kAccBufs;
-                if (use >= 1 && !mbar_wait_bounded(&ctl->acc_empty[buf], (use - 1) & 1)) {
-                    record_error(kErrGemmEpilogueBarrierTimeout);
+                if (use >= 1 && !__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->acc_empty[buf], (use - 1) & 1))) {
+                    if (lane == 0) record_error(kErrGemmEpilogueBarrierTimeout);
                     *abort_flag = 1;
                     break;
                 }
                 tc::fence_after_thread_sync();
-                const uint32_t tmem_acc = tmem_base + buf * 128;
+                const uint32_t tmem_acc = tm + buf * 128;
                 uint32_t accumulate = 0;           // the first MMA of the item overwrites the accumulator
                 for (int ks = ks0; ks < ks1; ++ks) {
-                    if (!mbar_wait_bounded(&ctl->full[s], full_phase)) {
-                        record_error(kErrGemmTmaBarrierTimeout);
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], full_phase))) {
+                        if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
                         *abort_flag = 1;
                         break;
                     }
                     tc::fence_after_thread_sync();
-                    if (tile_iter == 0 && ks == ks0) TL(4);
-                    // B scales of K atom a sit in kSubTiles * 4 consecutive columns (4 per 128 rows)
-#pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-#pragma unroll
-                        for (int h = 0; h < kSubTiles; ++h) {
-                            tc::cp_sf_32x128b(t_sfb + 4 * (kSubTiles * a + h),
-                                              tc::desc_from_words(lo0 + off_sfb16 + ((h * kSfSlab + a * 512) >> 4),
-                                                                  tc::kDescHiSfAtom));
-                        }
-                    }
-                    uint32_t lo_a = lo0 + off_a16;         // piece p's code tile
-                    uint32_t lo_sfa = lo0 + off_sfa16;     // piece p's scale slab
-                    uint32_t t_sfa_p = t_sfa;
-                    for (int p = 0; p < pieces; ++p) {
+                    if (tile_iter == 0 && ks == ks0 && lane == 0) TL(4);
+                    if (tc::elect_one()) {
+                        // B scales of K atom a sit in kSubTiles * 4 consecutive columns (4 per 128 rows)
 #pragma unroll
                         for (int a = 0; a < 4; ++a) {
-                            tc::cp_sf_32x128b(t_sfa_p + 4 * a,
-                                              tc::desc_from_words(lo_sfa + ((a * 512) >> 4), tc::kDescHiSfAtom));
-                        }
 #pragma unroll
-                        for (int a = 0; a < 4; ++a) {
-                            tc::mma_mxf4nvf4(tmem_acc, tc::desc_from_words(lo_a + ((a * 32) >> 4), tc::kDescHiKmajorSw128),
-                                             tc::desc_from_words(lo0 + ((a * 32) >> 4), tc::kDescHiKmajorSw128), idesc,
-                                             t_sfa_p + 4 * a, t_sfb + 4 * kSubTiles * a, accumulate);
-                            accumulate = 1;
+                            for (int h = 0; h < kSubTiles; ++h) {
+                                tc::cp_sf_32x128b(t_sfb + 4 * (kSubTiles * a + h),
+                                                  tc::desc_from_words(lo0 + off_sfb16 + ((h * kSfSlab + a * 512) >> 4),
+                                                                      tc::kDescHiSfAtom));
+                            }
                         }
-                        lo_a += kTile >> 4;
-                        lo_sfa += kSfSlab >> 4;
-                        t_sfa_p += 16;
+                        uint32_t lo_a = lo0 + off_a16;         // piece p's code tile
+                        uint32_t lo_sfa = lo0 + off_sfa16;     // piece p's scale slab
+                        uint32_t t_sfa_p = t_sfa;
+                        for (int p = 0; p < pieces; ++p) {
+#pragma unroll
+                            for (int a = 0; a < 4; ++a) {
+                                tc::cp_sf_32x128b(t_sfa_p + 4 * a,
+                                                  tc::desc_from_words(lo_sfa + ((a * 512) >> 4), tc::kDescHiSfAtom));
+                            }
+#pragma unroll
+                            for (int a = 0; a < 4; ++a) {
+                                tc::mma_mxf4nvf4(tmem_acc, tc::desc_from_words(lo_a + ((a * 32) >> 4), tc::kDescHiKmajorSw128),
+                                                 tc::desc_from_words(lo0 + ((a * 32) >> 4), tc::kDescHiKmajorSw128), idesc,
+                                                 t_sfa_p + 4 * a, t_sfb + 4 * kSubTiles * a, (accumulate | p | a) ? 1u : 0u);
+                            }
+                            lo_a += kTile >> 4;
+                            lo_sfa += kSfSlab >> 4;
+                            t_sfa_p += 16;
+                        }
+                        tc::commit(&ctl->empty[s]);   // stage s may be refilled once these MMAs have read it
                     }
-                    tc::commit(&ctl->empty[s]);   // stage s may be refilled once these MMAs have read it
+                    __syncwarp();
+                    accumulate = 1;
                     if (++s == nstages) {
                         s = 0;
                         full_phase ^= 1;
@@ -488,8 +496,9 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
                         lo0 += stage16;
                     }
                 }
-                tc::commit(&ctl->acc_full[buf]);  // accumulator complete
-                if (tile_iter == 0) TL(5);
+                if (tc::elect_one()) tc::commit(&ctl->acc_full[buf]);  // accumulator complete
+                __syncwarp();
+                if (tile_iter == 0 && lane == 0) TL(5);
             }
         }
     } else {

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             int s = 0, ph = 0;
             for (int i = 0; i < steps; ++i) {
-                if (!mbar_wait_bounded(&ctl.full[s], ph, kWaitG)) {
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[s], ph, kWaitG))) {
                     if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
                     break;
                 }
