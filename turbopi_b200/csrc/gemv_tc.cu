@@ -164,6 +164,7 @@ __device__ __forceinline__ void unpack16(const uint4 (&raw)[4], int dtype, float
 // Unit i of this CTA's list, once the producer has published it.  False at the end of the list, after an
 // abort, or when the (bounded) wait runs out.
 __device__ __forceinline__ bool fetch_unit(SharedControl* ctl, int i, TcUnit& un) {
+    if (ctl->abort_flag) return false;
     if (ctl->units_published <= i) {
         const long long start = clock64();
         while (ctl->units_published <= i) {
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemv_tc_kernel(const __grid
     const int kStageBytes = stage_bytes(P.pieces);
     SharedControl* ctl = reinterpret_cast<SharedControl*>(smem + kStages * kStageBytes);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform, and known to be
     const int lane = threadIdx.x & 31;
     const int NB = 16 * P.pieces;
     const int u_lo = P.cta_begin[blockIdx.x];        // this CTA's fixed units; more may come from the shared pool
@@ -402,60 +403,61 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemv_tc_kernel(const __grid
         }
         publish(end_mark);
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // ------------------------------------------------------------ MMA issuer.  The whole warp walks the loop and one
+        // elected lane issues: with warp-uniform control flow the operands of the tcgen05 instructions stay in uniform
+        // registers (under `if (lane == 0)` each took ~70 cycles to issue).
+        {
             const uint32_t idesc = tc::make_idesc_mxf4nvf4(NB);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
             // descriptor words: (stage address >> 4) + constants; see tcgen05.cuh
             const uint32_t base16 = smem_u32(smem) >> 4;
             const uint32_t stage16 = static_cast<uint32_t>(kStageBytes) >> 4;
-            const uint32_t t_sfa = tmem_base + kSfaCol;
-            const uint32_t t_sfb = tmem_base + kSfbCol;
+            const uint32_t t_sfa = tm + kSfaCol;
+            const uint32_t t_sfb = tm + kSfbCol;
             int s = 0;
             uint32_t full_phase = 0;
             uint32_t lo0 = base16;
             uint32_t g = 0;                        // stages issued so far; stage g uses scale set g & 1
             TcUnit un;
-            for (int i = 0; !ctl->abort_flag && fetch_unit(ctl, i, un); ++i) {
+            for (int i = 0; fetch_unit_warp(ctl, i, lane, un); ++i) {
                 const int buf = i & 1;
-                if (i >= 2 && !mbar_wait_bounded(&ctl->acc_empty[buf], ((i >> 1) - 1) & 1)) {
-                    record_error(kErrGemmEpilogueBarrierTimeout);
+                if (i >= 2 && !__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->acc_empty[buf], ((i >> 1) - 1) & 1))) {
+                    if (lane == 0) record_error(kErrGemmEpilogueBarrierTimeout);
                     ctl->abort_flag = 1;
                     break;
                 }
                 tc::fence_after_thread_sync();
-                const uint32_t tmem_acc = tmem_base + buf * 128;
+                const uint32_t tmem_acc = tm + buf * 128;
                 uint32_t accumulate = 0;
                 for (int ks = un.ks0; ks < un.ks1; ++ks) {
-                    if (!mbar_wait_bounded(&ctl->full[s], full_phase)) {
-                        record_error(kErrGemmTmaBarrierTimeout);
-                        ctl->abort_flag = 1;
-                        break;
-                    }
-                    tc::fence_after_thread_sync();
-                    if (g == 0) TL(4);
-                    // the scale copier (warp 6) has moved this stage's scales into set g & 1
+                    // the scale copier (warp 6) has moved this stage's scales into set g & 1, after the stage itself landed
                     const uint32_t set = g & 1u;
-                    if (!mbar_wait_bounded(&ctl->sf_full[set], (g >> 1) & 1u)) {
-                        record_error(kErrGemmTmaBarrierTimeout);
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], full_phase) &&
+                                                     mbar_wait_bounded(&ctl->sf_full[set], (g >> 1) & 1u))) {
+                        if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
                         ctl->abort_flag = 1;
                         break;
                     }
+                    if (g == 0 && lane == 0) TL(4);
                     tc::fence_after_thread_sync();
                     const uint32_t sfa = t_sfa + set * kSfSetCols;
                     const uint32_t sfb = t_sfb + set * kSfSetCols;
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        const uint64_t xdesc = tc::desc_from_words(lo0 + ((kWBlock + a * 32) >> 4), tc::kDescHiKmajorSw128);
+                        for (int a = 0; a < 4; ++a) {
+                            const uint64_t xdesc = tc::desc_from_words(lo0 + ((kWBlock + a * 32) >> 4), tc::kDescHiKmajorSw128);
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            tc::mma_mxf4nvf4(tmem_acc + h * kMaxNB,
-                                             tc::desc_from_words(lo0 + ((h * kWTile + a * 32) >> 4), tc::kDescHiKmajorSw128),
-                                             xdesc, idesc, sfa + 16 * h + 4 * a, sfb + 4 * a, a == 0 ? accumulate : 1u);
+                            for (int h = 0; h < 2; ++h) {
+                                tc::mma_mxf4nvf4(tmem_acc + h * kMaxNB,
+                                                 tc::desc_from_words(lo0 + ((h * kWTile + a * 32) >> 4), tc::kDescHiKmajorSw128),
+                                                 xdesc, idesc, sfa + 16 * h + 4 * a, sfb + 4 * a, a == 0 ? accumulate : 1u);
+                            }
                         }
+                        tc::commit(&ctl->empty[s]);
+                        tc::commit(&ctl->sf_empty[set]);
                     }
+                    __syncwarp();
                     accumulate = 1;
-                    tc::commit(&ctl->empty[s]);
-                    tc::commit(&ctl->sf_empty[set]);
                     ++g;
                     if (++s == kStages) {
                         s = 0;
@@ -465,9 +467,10 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemv_tc_kernel(const __grid
                         lo0 += stage16;
                     }
                 }
-                tc::commit(&ctl->acc_full[buf]);
+                if (tc::elect_one()) tc::commit(&ctl->acc_full[buf]);
+                __syncwarp();
             }
-            TL(5);
+            if (lane == 0) TL(5);
         }
     } else if (warp == 6) {
         // ------------------------------------------------------------ scale copier.
@@ -475,8 +478,9 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemv_tc_kernel(const __grid
         // copies of a stage on the MMA thread that thread, not the weight stream, set the pace.  Here they
         // run one stage ahead into the other set of scale columns.  The copies do not depend on the tile, so
         // this lane only needs the number of stages of each unit.
-        if (lane == 0) {
+        {
             const uint32_t base16 = smem_u32(smem) >> 4;
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint32_t stage16 = static_cast<uint32_t>(kStageBytes) >> 4;
             const uint32_t off_sfb16 = static_cast<uint32_t>(kWBlock + NB * 128) >> 4;
             int s = 0;
@@ -484,28 +488,31 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemv_tc_kernel(const __grid
             int g = 0;
             TcUnit un;
             bool stop = false;
-            for (int i = 0; !stop && !ctl->abort_flag && fetch_unit(ctl, i, un); ++i) {
+            for (int i = 0; !stop && fetch_unit_warp(ctl, i, lane, un); ++i) {
                 for (int ks = un.ks0; ks < un.ks1; ++ks, ++g) {
                     const uint32_t set = g & 1;
-                    if (!mbar_wait_bounded(&ctl->full[s], full_phase) ||
-                        (g >= 2 && !mbar_wait_bounded(&ctl->sf_empty[set], ((g >> 1) - 1) & 1))) {
-                        record_error(kErrGemmTmaBarrierTimeout);
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], full_phase) &&
+                                                     (g < 2 || mbar_wait_bounded(&ctl->sf_empty[set], ((g >> 1) - 1) & 1)))) {
+                        if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
                         ctl->abort_flag = 1;
                         stop = true;
                         break;
                     }
                     tc::fence_after_thread_sync();
-                    const uint32_t sfa = tmem_base + kSfaCol + set * kSfSetCols;
-                    const uint32_t sfb = tmem_base + kSfbCol + set * kSfSetCols;
+                    const uint32_t sfa = tm + kSfaCol + set * kSfSetCols;
+                    const uint32_t sfb = tm + kSfbCol + set * kSfSetCols;
                     // stage: [codes rows 0..127][codes rows 128..255][slab 0..127][slab 128..255][x codes][x slab]
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        tc::cp_sf_32x128b(sfa + 4 * a, tc::desc_from_words(lo0 + ((2 * kWTile + a * 512) >> 4), tc::kDescHiSfAtom));
-                        tc::cp_sf_32x128b(sfa + 16 + 4 * a,
-                                          tc::desc_from_words(lo0 + ((2 * kWTile + kSfSlab + a * 512) >> 4), tc::kDescHiSfAtom));
-                        tc::cp_sf_32x128b(sfb + 4 * a, tc::desc_from_words(lo0 + off_sfb16 + ((a * 512) >> 4), tc::kDescHiSfAtom));
+                        for (int a = 0; a < 4; ++a) {
+                            tc::cp_sf_32x128b(sfa + 4 * a, tc::desc_from_words(lo0 + ((2 * kWTile + a * 512) >> 4), tc::kDescHiSfAtom));
+                            tc::cp_sf_32x128b(sfa + 16 + 4 * a,
+                                              tc::desc_from_words(lo0 + ((2 * kWTile + kSfSlab + a * 512) >> 4), tc::kDescHiSfAtom));
+                            tc::cp_sf_32x128b(sfb + 4 * a, tc::desc_from_words(lo0 + off_sfb16 + ((a * 512) >> 4), tc::kDescHiSfAtom));
+                        }
+                        tc::commit(&ctl->sf_full[set]);
                     }
-                    tc::commit(&ctl->sf_full[set]);
+                    __syncwarp();
                     if (++s == kStages) {
                         s = 0;
                         full_phase ^= 1;
