@@ -14,13 +14,17 @@
 // softmax of its 128 x 256 block relative to the block's own row maxima (base-2 exponentials, 256 threads:
 // two per row), and O = P V (16 MMAs), and leaves O, the row maxima and the row sums in scratch; a second
 // small kernel combines the key tiles' partial results (the usual log-sum-exp merge).  With a single key
-// tile the first kernel writes the final rows itself.
+// tile the first kernel writes the final rows itself.  (The key tiles of a row tile as one thread-block cluster that
+// merges through distributed shared memory, without the second kernel, was slower in a chain of launches: 15.7 against
+// 12.6 us for 400 rows on 762 keys, 19.5 against 17.6 for 5696 on 712 -- each CTA reads 128 KB from its peers, where
+// the second kernel reads L2 from every SM.)
 //
 // Operands in shared memory, all in the 128-byte-swizzle image (rows of 128 B = 64 bf16, 16-byte chunk c of
 // row r at c ^ (r & 7), 8-row groups 1024 B apart, one 16 KB block per 64 columns of head_dim):
 //   Q [128 rows][D], K [2 x 128 keys][D]  K-major operands of S = Q K^T
 //   P [128 rows][256 keys]                K-major A operand of O = P V, written by the softmax threads over Q
-//   V [2 x 128 keys][D]                   loaded where K was once the S MMAs are done; the SAME image is read as an
+//   V [2 x 128 keys][D]                   loaded where K was once the S MMAs are done (with 128 keys per CTA: beside it,
+//                                         at once); the SAME image is read as an
 //                                         MN-major B operand (the 128-byte direction is head_dim = N, the rows
 //                                         are keys = K): no transposed copy of V.
 // Loads are TMA tile copies through 4-dimensional tensor maps (head_dim, rows, groups; zero fill past the end
@@ -81,7 +85,8 @@ struct AttnParams {
 };
 
 struct AttnControl {
-    uint64_t bar_k0, bar_k1, bar_s, bar_v, bar_o;
+    uint64_t bar_k[2][4];                       // per S tile and 64-column block of head_dim: K (and, for tile 0, Q) has landed
+    uint64_t bar_s, bar_v, bar_o;
     uint32_t tmem_base;
     float bias2[kKeysCta];
     float half_max[2][kRows];                   // row maxima / row sums of the two column halves
@@ -108,8 +113,9 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint6
         : "memory");
 }
 
-// 128 rows starting at `row0` of group (ga, gb): one 64-column box per 16 KB block of the swizzled image
-__device__ __forceinline__ void load_rows(uint8_t* dst, const AttnOperand& op, int row0, int ga, int gb, int nchunk,
+// 128 rows starting at `row0` of group (ga, gb), 64-column blocks [c_lo, c_hi): one box per 16 KB block of the
+// swizzled image
+__device__ __forceinline__ void load_rows(uint8_t* dst, const AttnOperand& op, int row0, int ga, int gb, int c_lo, int c_hi,
                                           uint64_t* bar) {
     const int v[3] = {row0 * op.mul[0], gb * op.mul[1], ga * op.mul[2]};
     int c1 = 0, c2 = 0, c3 = 0;
@@ -119,7 +125,7 @@ __device__ __forceinline__ void load_rows(uint8_t* dst, const AttnOperand& op, i
         c2 = op.slot[i] == 2 ? v[i] : c2;
         c3 = op.slot[i] == 3 ? v[i] : c3;
     }
-    for (int c = 0; c < nchunk; ++c) tc::tma_load_4d(dst + c * kChunkBytes, &op.map, c * 64, c1, c2, c3, bar);
+    for (int c = c_lo; c < c_hi; ++c) tc::tma_load_4d(dst + c * kChunkBytes, &op.map, c * 64, c1, c2, c3, bar);
 }
 
 __device__ __forceinline__ void bulk_store_s2g(void* gdst, const void* smem_src, uint32_t bytes) {
@@ -145,13 +151,12 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
 
     const int rt = blockIdx.x, kt = blockIdx.y, g = blockIdx.z;
     const int ga = g / P.groups_inner, gb = g - ga * P.groups_inner;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform, and known to be
     const int key0 = kt * P.keys_per_cta;
     const int nt = (P.keys_per_cta > kKeyTile && P.n_keys - key0 > kKeyTile) ? 2 : 1;  // S tiles of this CTA
 
     if (threadIdx.x == 0) {
-        mbar_init(&ctl->bar_k0, 1);
-        mbar_init(&ctl->bar_k1, 1);
+        for (int i = 0; i < 8; ++i) mbar_init(&ctl->bar_k[i >> 2][i & 3], 1);
         mbar_init(&ctl->bar_s, 1);
         mbar_init(&ctl->bar_v, 1);
         mbar_init(&ctl->bar_o, 1);
@@ -184,33 +189,56 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     }
 
     // ---------------------------------------------------------------- loads, S = Q K^T (two key tiles)
-    if (threadIdx.x == 0) {
-        mbar_expect_tx(&ctl->bar_k0, 2 * tile_bytes);
-        load_rows(sQ, P.q, rt * kRows, ga, gb, nchunk, &ctl->bar_k0);
-        load_rows(sKV, P.k, key0, ga, gb, nchunk, &ctl->bar_k0);
-        if (nt == 2) {
-            mbar_expect_tx(&ctl->bar_k1, tile_bytes);
-            load_rows(sKV + tile_bytes, P.k, key0 + kKeyTile, ga, gb, nchunk, &ctl->bar_k1);
+    // One key tile leaves the second tile's room to V, whose load then needs no wait for the S MMAs.
+    uint8_t* sV = sKV + (nt == 1 && P.keys_per_cta == kKeyTile ? tile_bytes : 0);
+    if (warp == 0) {
+        if (tc::elect_one()) {
+            // Q and K block by block, so that the first MMAs start when 32 KB have landed and not 128
+            for (int c = 0; c < nchunk; ++c) {
+                mbar_expect_tx(&ctl->bar_k[0][c], 2 * kChunkBytes);
+                load_rows(sQ, P.q, rt * kRows, ga, gb, c, c + 1, &ctl->bar_k[0][c]);
+                load_rows(sKV, P.k, key0, ga, gb, c, c + 1, &ctl->bar_k[0][c]);
+            }
+            if (nt == 2) {
+                for (int c = 0; c < nchunk; ++c) {
+                    mbar_expect_tx(&ctl->bar_k[1][c], kChunkBytes);
+                    load_rows(sKV + tile_bytes, P.k, key0 + kKeyTile, ga, gb, c, c + 1, &ctl->bar_k[1][c]);
+                }
+            }
+            if (sV != sKV) {
+                mbar_expect_tx(&ctl->bar_v, tile_bytes);
+                load_rows(sV, P.v, key0, ga, gb, 0, nchunk, &ctl->bar_v);
+            }
         }
+        __syncwarp();
+        // The whole warp walks the loop and one elected lane issues (operands in uniform registers).
         const uint32_t idesc = make_idesc_bf16(kKeyTile, 0);
-        const uint32_t q16 = smem_u32(sQ) >> 4;
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint32_t q16 = (smem_u32(sQ) & 0x3FFFFu) >> 4;
         const int ksteps = (P.head_dim + 15) >> 4;        // 16 columns of head_dim per MMA
         bool loaded = true;
         for (int t = 0; t < nt && loaded; ++t) {
-            loaded = mbar_wait_bounded(t == 0 ? &ctl->bar_k0 : &ctl->bar_k1, 0, kWaitCycles);
-            if (!loaded) {
-                record_error(kErrAttnBarrierTimeout);
-                break;
-            }
-            tc::fence_after_thread_sync();
-            const uint32_t k16 = (smem_u32(sKV) + t * tile_bytes) >> 4;
-            for (int kk = 0; kk < ksteps; ++kk) {
-                const uint32_t off = static_cast<uint32_t>((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4;
-                mma_bf16(tmem + kColS + t * kKeyTile, tc::desc_from_words(q16 + off, tc::kDescHiKmajorSw128),
-                         tc::desc_from_words(k16 + off, tc::kDescHiKmajorSw128), idesc, kk > 0 ? 1u : 0u);
+            const uint32_t k16 = ((smem_u32(sKV) + t * tile_bytes) & 0x3FFFFu) >> 4;
+            for (int c = 0; c < nchunk && loaded; ++c) {
+                loaded = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->bar_k[t][c], 0, kWaitCycles));
+                if (!loaded) {
+                    if (threadIdx.x == 0) record_error(kErrAttnBarrierTimeout);
+                    break;
+                }
+                tc::fence_after_thread_sync();
+                if (tc::elect_one()) {
+                    const int kk1 = min(ksteps, 4 * c + 4);
+                    for (int kk = 4 * c; kk < kk1; ++kk) {
+                        const uint32_t off = static_cast<uint32_t>((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4;
+                        mma_bf16(tm + kColS + t * kKeyTile, tc::desc_from_words(q16 + off, tc::kDescHiKmajorSw128),
+                                 tc::desc_from_words(k16 + off, tc::kDescHiKmajorSw128), idesc, kk > 0 ? 1u : 0u);
+                    }
+                }
+                __syncwarp();
             }
         }
-        if (loaded) tc::commit(&ctl->bar_s);              // otherwise the wait below runs out for the whole CTA
+        if (loaded && tc::elect_one()) tc::commit(&ctl->bar_s);   // otherwise the wait below runs out for the whole CTA
+        __syncwarp();
     }
     // every wait is short (the work behind it takes microseconds) and its outcome is made uniform over the CTA:
     // the tensor-memory loads below are warp-collective
@@ -218,12 +246,13 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     if (!ok) record_error(kErrAttnBarrierTimeout);
     ok = __syncthreads_and(ok);
     tc::fence_after_thread_sync();
+    if (!ok && sV != sKV && threadIdx.x == 0) mbar_wait_bounded(&ctl->bar_v, 0, kWaitCycles);   // V's copy is in flight
 
     // the S MMAs have read K: V takes its place while the softmax runs
-    if (threadIdx.x == 0 && ok) {
+    if (threadIdx.x == 0 && ok && sV == sKV) {
         mbar_expect_tx(&ctl->bar_v, nt * tile_bytes);
-        load_rows(sKV, P.v, key0, ga, gb, nchunk, &ctl->bar_v);
-        if (nt == 2) load_rows(sKV + tile_bytes, P.v, key0 + kKeyTile, ga, gb, nchunk, &ctl->bar_v);
+        load_rows(sKV, P.v, key0, ga, gb, 0, nchunk, &ctl->bar_v);
+        if (nt == 2) load_rows(sKV + tile_bytes, P.v, key0 + kKeyTile, ga, gb, 0, nchunk, &ctl->bar_v);
     }
 
     // ---------------------------------------------------------------- softmax of this block, P -> shared memory
@@ -291,23 +320,27 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     if (ok) l += ctl->half_sum[half ^ 1][row];
 
     // ---------------------------------------------------------------- O = P V
-    if (threadIdx.x == 0 && ok) {
-        if (mbar_wait_bounded(&ctl->bar_v, 0, kWaitCycles)) {
+    if (warp == 0 && ok) {
+        if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->bar_v, 0, kWaitCycles))) {
             tc::fence_after_thread_sync();
             const uint32_t idesc = make_idesc_bf16(P.dv, 1);  // B = V read MN-major
-            const uint32_t p16 = smem_u32(sQ) >> 4;
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint32_t p16 = (smem_u32(sQ) & 0x3FFFFu) >> 4, v16 = (smem_u32(sV) & 0x3FFFFu) >> 4;
             // MN-major, 128-byte swizzle: 64 columns of head_dim are contiguous, 8-key groups 1024 B apart
             // (stride offset), the next 64 columns one 16 KB block further (leading offset)
             constexpr uint32_t kDescHiMnSw128 = (1024u >> 4) | (1u << 14) | (static_cast<uint32_t>(tc::kSwizzle128B) << 29);
             constexpr uint32_t kLboField = (static_cast<uint32_t>(kChunkBytes) >> 4) << 16;
-            for (int kk = 0; kk < nt * (kKeyTile / 16); ++kk) {
-                const uint32_t a_off = static_cast<uint32_t>((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4;
-                const uint32_t v16 = (smem_u32(sKV) + (kk >> 3) * tile_bytes + (kk & 7) * 2048) >> 4;
-                mma_bf16(tmem + kColO, tc::desc_from_words(p16 + a_off, tc::kDescHiKmajorSw128),
-                         tc::desc_from_words(v16 | kLboField, kDescHiMnSw128), idesc, kk > 0 ? 1u : 0u);
+            if (tc::elect_one()) {
+                for (int kk = 0; kk < nt * (kKeyTile / 16); ++kk) {
+                    const uint32_t a_off = static_cast<uint32_t>((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4;
+                    const uint32_t v_off = ((kk >> 3) * tile_bytes + (kk & 7) * 2048) >> 4;
+                    mma_bf16(tm + kColO, tc::desc_from_words(p16 + a_off, tc::kDescHiKmajorSw128),
+                             tc::desc_from_words((v16 + v_off) | kLboField, kDescHiMnSw128), idesc, kk > 0 ? 1u : 0u);
+                }
+                tc::commit(&ctl->bar_o);
             }
-            tc::commit(&ctl->bar_o);
-        } else {
+            __syncwarp();
+        } else if (threadIdx.x == 0) {
             record_error(kErrAttnBarrierTimeout);         // the wait below runs out for the whole CTA
         }
     }
