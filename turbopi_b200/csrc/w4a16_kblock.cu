@@ -5,16 +5,25 @@
 // In this layout consecutive outputs are contiguous for a fixed K block, so a lane
 // owns an OUTPUT (no shuffle reduction): a CTA takes 64 outputs, streams their K
 // blocks through a 4-stage shared-memory ring (16 K-blocks x 64 outputs x 16 B per
-// stage, one bulk async copy per K-block row), and four thread groups split each
-// stage's K blocks; their partial sums meet in shared memory in a fixed order.
+// stage: ONE tiled TMA request for the codes and one for the scales), and four thread
+// groups split each stage's K blocks; their partial sums meet in shared memory in a
+// fixed order.  With a bulk copy per K-block row, 32 requests a stage from one thread,
+// the requests and not the bytes set the pace (16384 x 2048: 13.0 us, now 9.9; in a chain of
+// programmatic dependent launches 11.0 and 7.9).  Few output tiles with a long K are cut
+// along K over the CTAs of a cluster, whose first CTA adds the partial sums in rank order
+// (2048 x 16384: 85.7 us, 37.1 with one request per stage on 32 CTAs, 13.6 cut in eight).
 // Activations are staged once per CTA in shared memory as fp16 pairs in the order
 // the int4 decoder emits (k, k+4) and are read as warp-wide broadcasts.
 #include <algorithm>
 #include <atomic>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace tpb {
+
+bool make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t dim0, uint64_t dim1,
+                        uint64_t pitch_bytes, uint32_t box0, uint32_t box1, bool swizzle128);
+
 namespace {
 
 constexpr int kThreads = 256;
@@ -26,6 +35,8 @@ constexpr int kWStage = kQT * kNT * 16;
 constexpr int kSStage = kQT * kNT * 2;
 
 struct KBlockParams {
+    CUtensorMap map_w;        // [K / 32, 2 N] 64-bit words, box 16 x 128: 16 K blocks of 64 outputs, zeros past the edges
+    CUtensorMap map_s;        // [K / 32, N] fp16, box 16 x 64
     const uint8_t* w;
     const __half* scales;
     const void* x;
@@ -34,7 +45,21 @@ struct KBlockParams {
     int M, N, K;
     int x_dtype, bias_dtype, out_dtype;
     int scales_by_tma;
+    int splits;               // CTAs of a cluster per output tile, each with a range of K stages
 };
+
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(const float* p, int rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
 
 template <int M_TILE>
 __global__ void __launch_bounds__(kThreads, 2) w4a16_kblock_kernel(const __grid_constant__ KBlockParams P) {
@@ -55,9 +80,12 @@ __global__ void __launch_bounds__(kThreads, 2) w4a16_kblock_kernel(const __grid_
     const int ntiles = (N + kNT - 1) / kNT;
     const int m0 = blockIdx.y * M_TILE;
     // this CTA's work list: (tile, step) pairs in order, numbered `it`
-    const int my_tiles = (ntiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
-                         static_cast<int>(gridDim.x);
-    const int my_its = my_tiles * steps;
+    const int splits = P.splits;
+    const int rank = splits > 1 ? static_cast<int>(blockIdx.x) % splits : 0;
+    const int step0 = rank * steps / splits, nsteps = (rank + 1) * steps / splits - step0;
+    const int tile0 = splits > 1 ? static_cast<int>(blockIdx.x) / splits : static_cast<int>(blockIdx.x);
+    const int my_tiles = splits > 1 ? 1 : (ntiles - tile0 + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+    const int my_its = my_tiles * nsteps;
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
@@ -68,41 +96,51 @@ __global__ void __launch_bounds__(kThreads, 2) w4a16_kblock_kernel(const __grid_
 
     auto issue = [&](int it) {
         if (it >= my_its) return;
-        const int tile = blockIdx.x + (it / steps) * gridDim.x;
-        const int step = it % steps;
+        const int tile = tile0 + (it / nsteps) * gridDim.x;
+        const int step = step0 + it % nsteps;
         const int n0 = tile * kNT;
-        const int nv = min(kNT, N - n0);
         const int q0 = step * kQT;
-        const int qv = min(kQT, nqb - q0);
         const int s = it % kStages;
-        const uint32_t wb = static_cast<uint32_t>(nv) * 16u;
-        const uint32_t sb = P.scales_by_tma ? static_cast<uint32_t>(nv) * 2u : 0u;
-        mbar_expect_tx(&full[s], static_cast<uint32_t>(qv) * (wb + sb));
-        for (int q = 0; q < qv; ++q) {
-            const size_t e = static_cast<size_t>(q0 + q) * N + n0;
-            bulk_copy_g2s_hint(wst + s * kWStage + q * (kNT * 16), P.w + e * 16, wb, &full[s], l2_policy_evict_first());
-            if (sb) bulk_copy_g2s(sst + s * kSStage + q * (kNT * 2), P.scales + e, sb, &full[s]);
-        }
+        mbar_expect_tx(&full[s], kWStage + (P.scales_by_tma ? kSStage : 0));
+        tc::tma_load_2d(wst + s * kWStage, &P.map_w, n0 * 2, q0, &full[s]);
+        if (P.scales_by_tma) tc::tma_load_2d(sst + s * kSStage, &P.map_s, n0, q0, &full[s]);
     };
     if (tid == 0) {
+        tc::prefetch_tensormap(&P.map_w);
         for (int it = 0; it < kStages; ++it) issue(it);
     }
     pdl_launch_dependents();
     pdl_wait_prior_grids();
 
     // stage activations: xs[m][qb*16 + wd*4 + p] = (x[32qb + 8wd + p], x[32qb + 8wd + p + 4])
-    for (int i = tid; i < M_TILE * (K >> 1); i += kThreads) {
-        const int m = i / (K >> 1);
-        const int e = i - m * (K >> 1);
-        const int k = (e >> 2) * 8 + (e & 3);
-        float a = 0.0f, b = 0.0f;
+    for (int i = tid; i < M_TILE * (K >> 3); i += kThreads) {      // eight consecutive k: one 16- or two 16-byte loads
+        const int m = i / (K >> 3);
+        const int k8 = i - m * (K >> 3);
+        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (m0 + m < P.M) {
-            a = load_as_float(P.x, P.x_dtype, static_cast<size_t>(m0 + m) * K + k);
-            b = load_as_float(P.x, P.x_dtype, static_cast<size_t>(m0 + m) * K + k + 4);
+            const size_t e = static_cast<size_t>(m0 + m) * K + k8 * 8;
+            if (P.x_dtype == TPB200_F32) {
+                const float4* q = reinterpret_cast<const float4*>(static_cast<const float*>(P.x) + e);
+                const float4 a = __ldg(q), b = __ldg(q + 1);
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            } else {
+                const uint4 u = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(P.x) + e));
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = P.x_dtype == TPB200_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j]))
+                                                             : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+                    v[2 * j] = f.x;
+                    v[2 * j + 1] = f.y;
+                }
+            }
         }
-        a = fminf(fmaxf(a, -65504.0f), 65504.0f);
-        b = fminf(fmaxf(b, -65504.0f), 65504.0f);
-        xs[i] = __floats2half2_rn(a, b);
+        __half2 h[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            h[p] = __floats2half2_rn(fminf(fmaxf(v[p], -65504.0f), 65504.0f), fminf(fmaxf(v[p + 4], -65504.0f), 65504.0f));
+        }
+        *reinterpret_cast<uint4*>(xs + m * (K >> 1) + k8 * 4) = *reinterpret_cast<const uint4*>(h);
     }
     __syncthreads();
 
@@ -111,8 +149,8 @@ __global__ void __launch_bounds__(kThreads, 2) w4a16_kblock_kernel(const __grid_
     for (int m = 0; m < M_TILE; ++m) acc[m] = 0.0f;
 
     for (int it = 0; it < my_its; ++it) {
-        const int tile = blockIdx.x + (it / steps) * gridDim.x;
-        const int step = it % steps;
+        const int tile = tile0 + (it / nsteps) * gridDim.x;
+        const int step = step0 + it % nsteps;
         const int n0 = tile * kNT;
         const int nv = min(kNT, N - n0);
         const int q0 = step * kQT;
@@ -155,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 2) w4a16_kblock_kernel(const __grid_
                 }
             }
         }
-        const bool last_step = (step == steps - 1);
+        const bool last_step = (step == step0 + nsteps - 1);
         if (last_step) {
 #pragma unroll
             for (int m = 0; m < M_TILE; ++m) {
@@ -174,12 +212,27 @@ __global__ void __launch_bounds__(kThreads, 2) w4a16_kblock_kernel(const __grid_
                     float v = 0.0f;
 #pragma unroll
                     for (int q = 0; q < kParts; ++q) v += part[(q * M_TILE + m) * kNT + n];
-                    if (P.bias != nullptr) v += load_as_float(P.bias, P.bias_dtype, n0 + n);
-                    store_from_float(P.out, P.out_dtype, static_cast<size_t>(m0 + m) * N + n0 + n, v);
+                    if (splits > 1) {
+                        part[m * kNT + n] = v;                   // this K range's sum, read by the cluster's first CTA
+                    } else {
+                        if (P.bias != nullptr) v += load_as_float(P.bias, P.bias_dtype, n0 + n);
+                        store_from_float(P.out, P.out_dtype, static_cast<size_t>(m0 + m) * N + n0 + n, v);
+                    }
                 }
             }
             __syncthreads();  // `part` is rewritten by the next tile's last step
         }
+    }
+    if (splits > 1) {
+        cluster_barrier();
+        const int m = tid / kNT, n = tid % kNT, col = tile0 * kNT + n;
+        if (rank == 0 && m < M_TILE && col < N && m0 + m < P.M && !*abort_flag) {
+            float v = 0.0f;
+            for (int r = 0; r < splits; ++r) v += ld_cluster(part + m * kNT + n, r);
+            if (P.bias != nullptr) v += load_as_float(P.bias, P.bias_dtype, col);
+            store_from_float(P.out, P.out_dtype, static_cast<size_t>(m0 + m) * N + col, v);
+        }
+        cluster_barrier();                                       // nobody leaves while its sums are being read
     }
 }
 
@@ -205,12 +258,19 @@ int launch(const KBlockParams& P, int grid_x, int grid_y, int flags, cudaStream_
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
     if (flags & TPB200_FLAG_PDL) {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
         cfg.numAttrs = 1;
+    }
+    if (P.splits > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = P.splits;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
     }
     if (cudaLaunchKernelEx(&cfg, kernel, P) != cudaSuccess) return TPB200_ERR_CUDA;
     return TPB200_OK;
@@ -259,7 +319,7 @@ extern "C" int tpb200_w4a16_gemv(const void* x, int x_dtype, const void* weight_
     TPB_REQUIRE((flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
     TPB_REQUIRE(tpb_aligned16(x) && tpb_aligned16(weight_packed) && tpb_aligned16(scales) && tpb_aligned16(out),
                 TPB200_ERR_ALIGN);
-    tpb::KBlockParams P;
+    tpb::KBlockParams P = {};
     P.w = static_cast<const uint8_t*>(weight_packed);
     P.scales = static_cast<const __half*>(scales);
     P.x = x;
@@ -268,15 +328,25 @@ extern "C" int tpb200_w4a16_gemv(const void* x, int x_dtype, const void* weight_
     P.M = M; P.N = N; P.K = K;
     P.x_dtype = x_dtype; P.bias_dtype = bias_dtype; P.out_dtype = out_dtype;
     P.scales_by_tma = (N % 8 == 0) ? 1 : 0;
+    if (!tpb::make_tensor_map_2d(&P.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT64, weight_packed, 2ull * N, K / 32, 16ull * N,
+                                 2 * tpb::kNT, tpb::kQT, false) ||
+        (P.scales_by_tma && !tpb::make_tensor_map_2d(&P.map_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, scales, N, K / 32, 2ull * N,
+                                                     tpb::kNT, tpb::kQT, false))) {
+        return TPB200_ERR_CUDA;
+    }
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         return TPB200_ERR_CUDA;
     }
     const int ntiles = (N + tpb::kNT - 1) / tpb::kNT;
-    const int grid_x = std::min(ntiles, 2 * sms);
     const int m_tile = M >= 3 ? 4 : M;
     const int grid_y = (M + m_tile - 1) / m_tile;
+    // K is cut while that still fits two CTAs on every SM and leaves each at least one stage
+    const int stages = (K / 32 + tpb::kQT - 1) / tpb::kQT;
+    P.splits = 1;
+    while (P.splits < 8 && 2 * P.splits <= stages && static_cast<long long>(ntiles) * grid_y * P.splits * 2 <= 2 * sms) P.splits *= 2;
+    const int grid_x = P.splits > 1 ? ntiles * P.splits : std::min(ntiles, 2 * sms);
     if (m_tile == 1) return tpb::launch<1>(P, grid_x, grid_y, flags, stream);
     if (m_tile == 2) return tpb::launch<2>(P, grid_x, grid_y, flags, stream);
     return tpb::launch<4>(P, grid_x, grid_y, flags, stream);
