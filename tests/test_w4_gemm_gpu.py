@@ -113,3 +113,25 @@ def test_int4(cuda_device, M, N, K, plugin):
     y = ops.w4_gemm(xd, *args, out_dtype=torch.float32)
     _check(y, xd.double() @ wd.t(), xd.double().abs() @ wd.abs().t(), 2.0 ** -22)
     assert _lib.load().tpb200_device_error(0) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 512), (1, 72, 1024), (2, 136, 8192), (5, 1000, 4096), (1, 2048, 16384), (16, 8, 2080),
+                                   (3, 61, 1056)])
+def test_kblock_gemv_with_k_cut_over_a_cluster(cuda_device, M, N, K):
+    """Few output tiles, K ranges of unequal length, ragged N (scales by TMA or not)."""
+    from turbopi_b200 import _lib, ops
+    from turbopi_b200.w4a16 import _codes_to_words
+    g = torch.Generator().manual_seed(M + N + K)
+    codes = torch.randint(0, 16, (N, K), generator=g, dtype=torch.uint8)
+    sc = (torch.rand((N, K // 32), generator=g) * 0.1).half()
+    x = torch.randn((M, K), generator=g).half()
+    bias = torch.randn(N, generator=g)
+    w = (codes.double() - 8) * sc.double().repeat_interleave(32, 1)
+    words = _codes_to_words(codes).reshape(N, K // 32, 4).permute(1, 0, 2).contiguous().to(cuda_device)
+    out = torch.empty((M, N), dtype=torch.float32, device=cuda_device)
+    ops.w4a16_gemv_out(x.to(cuda_device), words, sc.t().contiguous().to(cuda_device), out, bias.to(cuda_device))
+    ref = x.double() @ w.t() + bias.double()
+    # chains of four fp16 products (2^-11 each of their magnitude), then fp32
+    mag = x.double().abs() @ w.abs().t() + bias.double().abs()
+    assert bool(((out.cpu().double() - ref).abs() <= 2.0 ** -10 * mag).all())
+    assert _lib.load().tpb200_device_error(0) == 0

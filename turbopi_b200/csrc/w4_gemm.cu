@@ -42,7 +42,7 @@ namespace {
 
 constexpr int kRows = 128;                       // weight rows per tile
 constexpr int kBlkK = 256;                       // K values of one weight block
-constexpr int kStepK = 64;                       // K values of one MMA step: a 128-byte row of bf16
+constexpr int kPartK = 64;                       // K values of one part of a step: a 128-byte row of bf16
 constexpr int kSlabBytes = 2048;                 // scales of 128 rows x 256 K
 constexpr int kCodeBytes = kRows * kBlkK / 2;    // 16 KB
 constexpr int kWSlot = kCodeBytes + 2 * kSlabBytes;
@@ -71,6 +71,7 @@ struct W4gParams {
     int nt;                                      // tokens per tile
     int splits;                                  // CTAs (cluster size) per tile, each with a K range
     int k_blocks, k_steps;
+    int parts;                                   // 64-K parts per operand step: 1, or 2 for narrow token tiles
     int n_w, n_s;                                // ring depths: weight blocks, operand steps
     int tmem_cols, a_col;
     int epilogue;
@@ -147,31 +148,28 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
     return v;
 }
 
+// two E4M3 bytes -> fp16 pair (exact)
+__device__ __forceinline__ __half2 decode_e4m3x2_h(uint16_t v) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"(v));
+    return *reinterpret_cast<__half2*>(&r);
+}
+
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) { return __byte_perm(a, b, s); }
 __device__ __forceinline__ uint32_t bits(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 __device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
 
-// prmt with selector bit 3 live (replicate the selected byte's sign), which __byte_perm masks off
-__device__ __forceinline__ uint32_t prmt_raw(uint32_t a, uint32_t b, uint32_t s) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s));
-    return d;
-}
-
-// Eight e2m1 codes (code i at bits 4 i) -> bf16 pairs in K order, times the block scale (exact).  The three magnitude
-// bits select the high and the low byte of the bf16 value from two byte tables; a code's own bit 3, used as prmt's
-// "replicate the sign" flag on a table of 0x80, marks the negative ones.
-__device__ __forceinline__ void dequant_e2m1x8(uint32_t w, __nv_bfloat162 s, uint32_t* out) {
-    const uint32_t m = w & 0x77777777u;
+// Eight e2m1 codes (code i at bits 4 i) -> bf16 pairs in K order, times the block scale.  The product is formed in fp16,
+// where it is exact (six significant bits, 2^-10 .. 2688), and stays exact through fp32 to bf16.  Half the cycles of
+// assembling bf16 from byte tables with prmt (729 against 1243 per 64-K step with 16 warps on the SM): the integer pipe
+// runs at half rate, the converter and the FMA pipe share this form's work.
+__device__ __forceinline__ void dequant_e2m1x8(uint32_t w, __half2 s, uint32_t* out) {
+    __half2 h[4];
+    decode_e2m1x8(w, h);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t mm = h ? m >> 16 : m, ww = h ? w >> 16 : w;
-        const uint32_t lo = prmt_raw(0xC0800000u, 0xC0804000u, mm);
-        uint32_t hi = prmt_raw(0x3F3F3F00u, 0x40404040u, mm);
-        const uint32_t neg = prmt_raw(0x80808080u, 0x80808080u, ww);   // 0x80 or, for a negative code, 0xFF
-        hi |= (neg << 7) & 0x80808080u;
-        out[2 * h] = bits(__hmul2(as_bf162(prmt_raw(lo, hi, 0x5140)), s));
-        out[2 * h + 1] = bits(__hmul2(as_bf162(prmt_raw(lo, hi, 0x7362)), s));
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(__hmul2(h[i], s));
+        out[i] = bits(__floats2bfloat162_rn(f.x, f.y));
     }
 }
 
@@ -208,7 +206,7 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sW = smem;                                              // [n_w][16 KB codes | 2 scale slabs]
     uint8_t* sB = sW + P.n_w * kWSlot;                               // [n_b][nt rows of 128 bytes]
-    const int b_bytes = P.nt * 128;
+    const int part_bytes = P.nt * 128, b_bytes = part_bytes * P.parts;
     __shared__ W4gControl ctl;
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform, and known to be
@@ -219,7 +217,8 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
     const int t0 = blockIdx.y * P.nt;                                // first token
     const int blk0 = rank * P.k_blocks / splits, blk1 = (rank + 1) * P.k_blocks / splits;
     const int nblk = blk1 - blk0;
-    const int steps = min(blk1 * 4, P.k_steps) - blk0 * 4;
+    const int parts = P.parts;                                       // a step past the end of K multiplies zeros
+    const int steps = (min(blk1 * 4, P.k_steps) - blk0 * 4 + parts - 1) / parts;
     // weight rows of the tile: rows 0..63 start at row_a, 64..127 at row_b (apart only in the gated form)
     const int row_a = P.epilogue == kEpiGated ? tile * 64 : tile * kRows;
     const int row_b = P.epilogue == kEpiGated ? P.gated_rows + row_a : row_a + 64;
@@ -227,7 +226,7 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.n_w; ++s) {
             mbar_init(&ctl.w_full[s], 1);
-            mbar_init(&ctl.w_empty[s], 16);                          // 4 steps x 4 warps
+            mbar_init(&ctl.w_empty[s], 16 / P.parts);                // 4 or 2 steps x 4 warps
         }
         for (int s = 0; s < P.n_s; ++s) {
             mbar_init(&ctl.full[s], 5);                              // the activation tile and four dequantising warps
@@ -260,7 +259,9 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
                     break;
                 }
                 mbar_expect_tx(&ctl.full[s], b_bytes);
-                tc::tma_load_2d(sB + s * b_bytes, &P.map_x, (blk0 * 4 + i) * kStepK, t0, &ctl.full[s]);
+                for (int u = 0; u < parts; ++u) {
+                    tc::tma_load_2d(sB + s * b_bytes + u * part_bytes, &P.map_x, (blk0 * 4 + i * parts + u) * kPartK, t0, &ctl.full[s]);
+                }
                 if (++s == P.n_s) { s = 0; ph ^= 1; }
             }
         }
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
         // and this one thread was the kernel's critical path (750 cycles per 64-K step for 128-480 cycles of MMA).
         {
             const uint32_t idesc = idesc_bf16(P.nt);
-            const uint32_t b16 = smem_u32(sB) >> 4;
+            const uint32_t b16 = (smem_u32(sB) & 0x3FFFFu) >> 4;      // without the bits that name the CTA in its cluster
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             int s = 0, ph = 0;
             for (int i = 0; i < steps; ++i) {
@@ -321,12 +322,19 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
                     break;
                 }
                 tc::fence_after_thread_sync();
-                const uint32_t a_col = tm + P.a_col + s * 32, b_lo = b16 + ((s * b_bytes) >> 4);
+                const uint32_t a_col = tm + P.a_col + s * 32 * parts, b_lo = b16 + ((s * b_bytes) >> 4);
                 if (tc::elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
                         mma_bf16_ts(tm, a_col + kk * 8, tc::desc_from_words(b_lo + kk * 2, tc::kDescHiKmajorSw128), idesc,
                                     (i > 0 || kk > 0) ? 1u : 0u);
+                    }
+                    if (parts == 2) {
+                        const uint32_t b_lo2 = b_lo + (part_bytes >> 4);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) {
+                            mma_bf16_ts(tm, a_col + 32 + kk * 8, tc::desc_from_words(b_lo2 + kk * 2, tc::kDescHiKmajorSw128), idesc, 1u);
+                        }
                     }
                     tc::commit(&ctl.empty[s]);
                 }
@@ -344,81 +352,97 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
         const int sf_off = (r >= 64 && P.epilogue == kEpiGated ? kSlabBytes : 0) + (row & 31) * 16 + ((row >> 5) & 3) * 4;
         bool ok = true;
         float psc[2] = {0.0f, 0.0f}, pzp[2] = {0.0f, 0.0f};
+        // ring positions and phases of this group's steps (kept by counting: four integer divisions a step would cost a
+        // third of the dequantisation's instructions)
+        int sw = 0, wph = 0, last_j = 0, sa = grp, sph = 1;
+        while (sa >= P.n_s) { sa -= P.n_s; sph ^= 1; }
         for (int i = grp; i < steps; i += groups) {
-            const int j = i >> 2, kk = i & 3;
-            const int sw = j % P.n_w, sa = i % P.n_s;
-            if (kFmt == kFmtPlugin && row < P.N) {                   // two scales per 256 K, straight from global memory
-                const size_t g = static_cast<size_t>(row) * (P.K / 128) + (blk0 + j) * 2 + (kk >> 1);
-                psc[0] = __bfloat162float(__ldg(P.pl_scale + g));
-                pzp[0] = P.pl_zero != nullptr ? __bfloat162float(__ldg(P.pl_zero + g)) : 0.0f;
+            const int j = i * parts >> 2;
+            while (last_j < j) {
+                ++last_j;
+                if (++sw == P.n_w) { sw = 0; wph ^= 1; }
             }
-            if (!mbar_wait_bounded(&ctl.w_full[sw], (j / P.n_w) & 1, kWaitG)) ok = false;
-            const uint8_t* slot = sW + sw * kWSlot;
-            uint32_t out[32];
-            uint4 c[2];
-            if (kFmt == kFmtKblock) {
-                c[0] = *reinterpret_cast<const uint4*>(slot + (2 * kk) * 2048 + r * 16);
-                c[1] = *reinterpret_cast<const uint4*>(slot + (2 * kk + 1) * 2048 + r * 16);
-            } else {
-                c[0] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk) ^ (r & 7)) << 4));
-                c[1] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk + 1) ^ (r & 7)) << 4));
-            }
-            uint32_t sc = 0;
-            if (kFmt == kFmtNvfp4) sc = *reinterpret_cast<const uint32_t*>(slot + kCodeBytes + kk * 512 + sf_off);
-            if (kFmt == kFmtKblock) {
-                if (P.kb_scale == nullptr) {
-                    const __half* sp = reinterpret_cast<const __half*>(slot + kCodeBytes) + (2 * kk) * kRows + r;
-                    psc[0] = __half2float(sp[0]);
-                    psc[1] = __half2float(sp[kRows]);
-                } else if (row < P.N) {
-                    const __half* sp = P.kb_scale + static_cast<size_t>((blk0 + j) * 8 + 2 * kk) * P.N + row;
-                    psc[0] = __half2float(__ldg(sp));
-                    psc[1] = __half2float(__ldg(sp + P.N));
+            if (!mbar_wait_bounded(&ctl.w_full[sw], wph, kWaitG)) ok = false;
+            for (int u = 0; u < parts; ++u) {
+                const int kk = (i * parts + u) & 3;
+                if (kFmt == kFmtPlugin && row < P.N) {                   // two scales per 256 K, straight from global memory
+                    const size_t g = static_cast<size_t>(row) * (P.K / 128) + (blk0 + j) * 2 + (kk >> 1);
+                    psc[0] = __bfloat162float(__ldg(P.pl_scale + g));
+                    pzp[0] = P.pl_zero != nullptr ? __bfloat162float(__ldg(P.pl_zero + g)) : 0.0f;
                 }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ctl.w_empty[sw]);            // every lane's codes are in registers
-            const uint32_t w[8] = {c[0].x, c[0].y, c[0].z, c[0].w, c[1].x, c[1].y, c[1].z, c[1].w};
-            if (kFmt == kFmtNvfp4) {
-                const float2 f0 = decode_e4m3x2(static_cast<uint16_t>(sc)), f1 = decode_e4m3x2(static_cast<uint16_t>(sc >> 16));
-                const float f[4] = {f0.x, f0.y, f1.x, f1.y};
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const __nv_bfloat162 s2 = __float2bfloat162_rn(f[b]);
-                    dequant_e2m1x8(w[2 * b], s2, out + 8 * b);
-                    dequant_e2m1x8(w[2 * b + 1], s2, out + 8 * b + 4);
+                const uint8_t* slot = sW + sw * kWSlot;
+                uint32_t out[32];
+                uint4 c[2];
+                if (kFmt == kFmtKblock) {
+                    c[0] = *reinterpret_cast<const uint4*>(slot + (2 * kk) * 2048 + r * 16);
+                    c[1] = *reinterpret_cast<const uint4*>(slot + (2 * kk + 1) * 2048 + r * 16);
+                } else {
+                    c[0] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk) ^ (r & 7)) << 4));
+                    c[1] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk + 1) ^ (r & 7)) << 4));
                 }
-            } else {
+                uint32_t sc = 0;
+                if (kFmt == kFmtNvfp4) sc = *reinterpret_cast<const uint32_t*>(slot + kCodeBytes + kk * 512 + sf_off);
+                if (kFmt == kFmtKblock) {
+                    if (P.kb_scale == nullptr) {
+                        const __half* sp = reinterpret_cast<const __half*>(slot + kCodeBytes) + (2 * kk) * kRows + r;
+                        psc[0] = __half2float(sp[0]);
+                        psc[1] = __half2float(sp[kRows]);
+                    } else if (row < P.N) {
+                        const __half* sp = P.kb_scale + static_cast<size_t>((blk0 + j) * 8 + 2 * kk) * P.N + row;
+                        psc[0] = __half2float(__ldg(sp));
+                        psc[1] = __half2float(__ldg(sp + P.N));
+                    }
+                }
+                if (u == parts - 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctl.w_empty[sw]);        // every lane's codes are in registers
+                }
+                const uint32_t w[8] = {c[0].x, c[0].y, c[0].z, c[0].w, c[1].x, c[1].y, c[1].z, c[1].w};
+                if (kFmt == kFmtNvfp4) {
+                    const __half2 s01 = decode_e4m3x2_h(static_cast<uint16_t>(sc)), s23 = decode_e4m3x2_h(static_cast<uint16_t>(sc >> 16));
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const float s = kFmt == kFmtKblock ? psc[b] : psc[0];
-                    const __nv_bfloat162 s_hi = __float2bfloat162_rn(s);
-                    const __nv_bfloat162 s_lo = __float2bfloat162_rn(s - __low2float(s_hi));
-                    const __nv_bfloat162 zp = __float2bfloat162_rn(pzp[0]);
+                    for (int b = 0; b < 4; ++b) {
+                        const __half2 s2 = b < 2 ? (b ? __high2half2(s01) : __low2half2(s01)) : b == 3 ? __high2half2(s23) : __low2half2(s23);
+                        dequant_e2m1x8(w[2 * b], s2, out + 8 * b);
+                        dequant_e2m1x8(w[2 * b + 1], s2, out + 8 * b + 4);
+                    }
+                } else {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        __nv_bfloat162 q[4];
-                        nibbles_minus8(w[4 * b + u] ^ (kFmt == kFmtPlugin ? 0x88888888u : 0u), q);
+                    for (int b = 0; b < 2; ++b) {
+                        const float s = kFmt == kFmtKblock ? psc[b] : psc[0];
+                        const __nv_bfloat162 s_hi = __float2bfloat162_rn(s);
+                        const __nv_bfloat162 s_lo = __float2bfloat162_rn(s - __low2float(s_hi));
+                        const __nv_bfloat162 zp = __float2bfloat162_rn(pzp[0]);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            out[16 * b + 4 * u + e] = kFmt == kFmtKblock ? bits(__hfma2(q[e], s_hi, __hmul2(q[e], s_lo)))
-                                                                         : bits(__hfma2(q[e], s_hi, zp));
+                        for (int wd = 0; wd < 4; ++wd) {
+                            __nv_bfloat162 q[4];
+                            nibbles_minus8(w[4 * b + wd] ^ (kFmt == kFmtPlugin ? 0x88888888u : 0u), q);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                out[16 * b + 4 * wd + e] = kFmt == kFmtKblock ? bits(__hfma2(q[e], s_hi, __hmul2(q[e], s_lo)))
+                                                                             : bits(__hfma2(q[e], s_hi, zp));
+                            }
                         }
                     }
                 }
+                if (u == 0) {                                        // the arithmetic above needs no free slot
+                    if (i >= P.n_s && !mbar_wait_bounded(&ctl.empty[sa], sph, kWaitG)) ok = false;
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc::fence_after_thread_sync();
+                }
+                tmem_st_32x32b_x32(lane_addr + P.a_col + (sa * parts + u) * 32, out);
             }
-            if (i >= P.n_s && !mbar_wait_bounded(&ctl.empty[sa], ((i / P.n_s) - 1) & 1, kWaitG)) ok = false;
-            ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 if (lane == 0) record_error(kErrGemmEmptyBarrierTimeout);
                 break;
             }
-            tc::fence_after_thread_sync();
-            tmem_st_32x32b_x32(lane_addr + P.a_col + sa * 32, out);
             tmem_st_wait();
             tc::fence_before_thread_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl.full[sa]);
+            sa += groups;
+            while (sa >= P.n_s) { sa -= P.n_s; sph ^= 1; }
         }
         // ------------------------------------------------------------ accumulator -> shared memory, [token][128 rows]
         if (ok && !mbar_wait_bounded(&ctl.acc_full, 0, kWaitG)) {
@@ -604,13 +628,18 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
             const long long ctas = static_cast<long long>(tiles) * tt * s;
             const bool half = nt <= 128 && ctas > sms;
             const int steps = (k_blocks + s - 1) / s * 4;
-            const float split = l == 0 ? 0.0f : l == 1 ? 0.9f : l == 2 ? 1.5f : 3.2f;
-            // A K step: 0.25 us with 16 dequantising warps, 0.37 with 8; two CTAs on one SM share it.
-            const float step = half ? (ctas > sms ? 0.74f : 0.37f) : 0.25f + 0.0003f * nt;
-            const long long waves = (ctas + (half ? 2 * sms : sms) - 1) / (half ? 2 * sms : sms);
+            const float split = l == 0 ? 0.0f : l == 1 ? 0.5f : l == 2 ? 1.0f : 3.0f;
+            const float step = half ? 0.40f : 0.19f + 0.0005f * nt;     // 64 K values
+            // clusters that fit the machine at once (GPCs of 16 to 20 SMs hold whole clusters only): 148, 74, 33 and 15 of 1, 2,
+            // 4 and 8 CTAs with an SM each, twice that with two CTAs per SM
+            constexpr int kFit[4] = {148, 74, 33, 15};
+            const long long fit = std::max(1, kFit[l] * sms / 148 * (half ? 2 : 1));
+            const long long waves = (static_cast<long long>(tiles) * tt + fit - 1) / fit;
             // a grid of more than half the SMs leaves the next launch no room to start its weight loads
             const float crowd = half || 2 * ctas > sms ? 1.6f : 0.0f;
-            const float cost = waves * (1.9f + steps * step + 0.008f * nt) + split + crowd + 0.004f * std::min(ctas, 150LL);
+            // summing a cluster's tiles through distributed shared memory moves NT x 512 bytes per CTA
+            const float cost = waves * (1.9f + steps * step + 0.008f * nt) + split + (l > 0 ? 0.012f * nt : 0.0f) + crowd +
+                               0.004f * std::min(ctas, 150LL);
             if (cost < best_cost) {
                 best_cost = cost;
                 best = {nt, s, half};
@@ -664,7 +693,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
     const int fmt = nv ? kFmtNvfp4 : a->format == TPB200_W4_INT4_KBLOCK ? kFmtKblock : kFmtPlugin;
     const int tiles = (N + kRows - 1) / kRows;
     P.k_blocks = (K + kBlkK - 1) / kBlkK;
-    P.k_steps = (K + kStepK - 1) / kStepK;
+    P.k_steps = (K + kPartK - 1) / kPartK;
     P.img_kblocks = P.k_blocks;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -720,9 +749,13 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
     const int blocks_per = (P.k_blocks + P.splits - 1) / P.splits, steps_per = std::min(blocks_per * 4, P.k_steps);
     const int budget = (half ? 112 : 225) * 1024 - 1024;
     const int b_bytes = P.nt * 128;
+    // Two 64-K parts per step for narrow token tiles: a step costs the issuing warp ~280 cycles of waiting and issuing
+    // whatever its size, more than the MMAs of one part (2 NT cycles)
+    P.parts = P.nt <= 64 ? 2 : 1;
     P.n_w = std::min(half ? (P.nt <= 64 ? 3 : 2) : 3, blocks_per);
-    P.n_s = std::min(std::min(std::min(kMaxS, (P.tmem_cols - P.a_col) / 32), steps_per), (budget - P.n_w * kWSlot) / b_bytes);
-    int smem = P.n_w * kWSlot + P.n_s * b_bytes;
+    P.n_s = std::min(std::min(kMaxS, (P.tmem_cols - P.a_col) / (32 * P.parts)),
+                     std::min((steps_per + P.parts - 1) / P.parts, (budget - P.n_w * kWSlot) / (b_bytes * P.parts)));
+    int smem = P.n_w * kWSlot + P.n_s * b_bytes * P.parts;
     smem = std::max(smem, P.nt * kRows * 4) + 1024;
 
     static void (*const kernels[3])(const W4gParams) = {w4_gemm_kernel<kFmtNvfp4>, w4_gemm_kernel<kFmtKblock>,
