@@ -201,7 +201,7 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
 }
 
 template <int kFmt>
-__global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__ W4gParams P) {
+__device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sW = smem;                                              // [n_w][16 KB codes | 2 scale slabs]
@@ -610,6 +610,18 @@ __global__ void __launch_bounds__(704, 1) w4_gemm_kernel(const __grid_constant__
     }
 }
 
+// at most 93 registers: two CTAs of 352 threads, or one of 608, fit an SM
+constexpr int kBoundThreads = 704;
+__global__ void __launch_bounds__(kBoundThreads, 1) w4_nvfp4_gemm_kernel(const __grid_constant__ W4gParams P) {
+    w4_gemm_tile<kFmtNvfp4>(P);
+}
+__global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_kblock_gemm_kernel(const __grid_constant__ W4gParams P) {
+    w4_gemm_tile<kFmtKblock>(P);
+}
+__global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_plugin_gemm_kernel(const __grid_constant__ W4gParams P) {
+    w4_gemm_tile<kFmtPlugin>(P);
+}
+
 // ---------------------------------------------------------------- launch plan
 // Tokens per tile, K ranges per tile, and whether two CTAs share an SM (8 dequantising warps each) or one has it
 // to itself (16 warps).  Measured (B200, us per launch; 50 tokens, K = 1024 / 2048 / 1024 / 4096): qkv 5.4, o 5.3, gate_up
@@ -758,8 +770,8 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
     int smem = P.n_w * kWSlot + P.n_s * b_bytes * P.parts;
     smem = std::max(smem, P.nt * kRows * 4) + 1024;
 
-    static void (*const kernels[3])(const W4gParams) = {w4_gemm_kernel<kFmtNvfp4>, w4_gemm_kernel<kFmtKblock>,
-                                                        w4_gemm_kernel<kFmtPlugin>};
+    static void (*const kernels[3])(const W4gParams) = {w4_nvfp4_gemm_kernel, w4_int4_kblock_gemm_kernel,
+                                                        w4_int4_plugin_gemm_kernel};
     auto kernel = kernels[fmt];
     static std::atomic<uint64_t> configured[3] = {};
     const uint64_t bit = 1ull << (dev & 63);

@@ -95,6 +95,16 @@ def _operand_buffer(module, T, K, device):
     return q
 
 
+def _dense_is_faster(T, N, K, gated=False):
+    """Whether [N, K] weights on the tiled image take T tokens faster through the GEMM that dequantises them (bf16
+    activations as they are) than through the e2m1-piece GEMM behind its quantiser: the first dequantises the weights once
+    per 256 tokens, the second pays one launch more, two in a gated MLP.  Measured, us for pieces / dequantising.  Gated MLP
+    of 1024 -> 4096: 17 tokens 26 / 11, 256 33 / 23, 1000 51 / 48; of 1152 -> 8000: 256 40 / 33, 712 67 / 65; of 2048 -> 16384:
+    50 44 / 35, 192 63 / 61, 256 64 / 68.  One linear 8000 -> 1152: 256 21 / 18, 712 26 / 23; 16384 -> 2048: 128 23 / 21,
+    192 26 / 27."""
+    return T * N * K <= (13_000_000_000 if gated else 6_000_000_000)
+
+
 def _split_k_scratch(module, T, N, K, device):
     """Zeroed split-K scratch of `module`'s GEMM, as large as the launch planner wants for T tokens (a scratch
     that is too small makes the planner cut K less and leaves SMs idle: 712 x 2048 x 16384 runs on 48 CTAs
@@ -194,6 +204,9 @@ class NVFP4PackedLinear(nn.Module):
         if T <= 16:
             return ops.tc_gemv(x2, image, self.out_features, out, self.global_scale, bias, act, 3, gemv_ws)
         xb = x2 if x2.dtype == torch.bfloat16 else x2.to(torch.bfloat16)
+        if self.out_features % 8 == 0 and _dense_is_faster(T, self.out_features, self.in_features):
+            return ops.w4_gemm(xb, image, self.out_features, _lib.W4_NVFP4_TILED, alpha=self.global_scale, bias=bias,
+                               activation=act, out=out)
         q = _operand_buffer(self, T, self.in_features, x2.device)
         # the quantiser and the GEMM are chained by programmatic dependent launch: the weights are static, so
         # the GEMM may fetch them while the quantiser still runs
@@ -317,6 +330,13 @@ class NVFP4PackedMLP(nn.Module):
                 ops.nvfp4_gemv_out(h, d.weight_packed, d.weight_scales, out, d_bias, 0, 16, d.global_scale)
             else:
                 ops.tc_gemv(h, d_image, self.hidden_size, out, d.global_scale, d_bias, 0, 3, d_gemv_ws)
+        elif I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True):
+            # two launches: gate_up with act(gate) * up in its epilogue, down on its bf16 result
+            h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
+            with ops.launch_flags(ops.FLAG_PDL):
+                ops.w4_gemm(x2, gu_image, 2 * I, _lib.W4_NVFP4_TILED, alpha=g.global_scale, activation=ACTIVATIONS[g.activation],
+                            gated=True, out=h)
+                ops.w4_gemm(h, d_image, self.hidden_size, _lib.W4_NVFP4_TILED, alpha=d.global_scale, bias=d_bias, out=out)
         else:
             qx = _operand_buffer(g, T, self.hidden_size, x2.device)
             q = _operand_buffer(d, T, I, x2.device)
