@@ -136,7 +136,7 @@ class NVFP4Linear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         batch_shape = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
+        x2 = x if x.dim() == 2 and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
         if x2.dtype not in (torch.float16, torch.bfloat16, torch.float32):
             x2 = x2.float()
         M = x2.shape[0]
@@ -146,7 +146,7 @@ class NVFP4Linear(nn.Module):
                            self.in_features, alpha=1.0 / self.weight_scale_multiplier,
                            bias=None if self.bias is None else self.bias.detach(), activation=self.activation,
                            out_dtype=out_dtype)
-        return y.reshape(*batch_shape, self.out_features).to(x.dtype)
+        return y if x.dim() == 2 and y.dtype == x.dtype else y.reshape(*batch_shape, self.out_features).to(x.dtype)
 
 
 class NVFP4MLP(nn.Module):

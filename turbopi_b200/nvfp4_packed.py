@@ -17,6 +17,7 @@ import torch.nn as nn
 from . import _lib, ops
 from ._lib import ACTIVATIONS
 
+_FLOATS = frozenset((torch.float16, torch.bfloat16, torch.float32))
 BLOCK_SIZE = 32
 NVFP4_MAX = 6.0
 E4M3_MAX = 448.0
@@ -174,14 +175,16 @@ class NVFP4PackedLinear(nn.Module):
     # ------------------------------------------------------------------ tensor-core path ("nvfp4" format)
     def tensor_core_ready(self) -> bool:
         """True if the weights are standard NVFP4 (E4M3 scale per 16 + global scale) on a CUDA device."""
-        return (self.block_size == 16 and self.weight_scales is not None and self.weight_scales.dtype == torch.uint8
+        scales = self.weight_scales
+        return (self.block_size == 16 and scales is not None and scales.dtype == torch.uint8
                 and self.weight_packed.is_cuda and self.in_features % 16 == 0)
 
     def _tc_state(self):
         """(tiled weight image, GEMV scratch), built on first use and whenever the packed
         weights were replaced (load_state_dict, .to(device))."""
-        key = (self.weight_packed.data_ptr(), self.weight_scales.data_ptr(), str(self.weight_packed.device))
-        st = getattr(self, "_tc", None)
+        packed = self.weight_packed
+        key = (packed.data_ptr(), self.weight_scales.data_ptr(), packed.get_device())
+        st = self.__dict__.get("_tc")
         if st is None or st[0] != key:
             N, K = self.out_features, self.in_features
             dev = self.weight_packed.device
@@ -221,15 +224,18 @@ class NVFP4PackedLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         batch_shape = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
-        if x2.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+        x2 = x if x.dim() == 2 and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
+        if x2.dtype not in _FLOATS:
             x2 = x2.float()
         x2 = x2.contiguous()
         T = x2.shape[0]
         act = ACTIVATIONS.get(self.activation, 0)
-        bias = None if self.bias is None else self.bias.detach().float().contiguous()
+        bias = self.bias
+        if bias is not None:
+            bias = bias.detach().float().contiguous()
         if self.tensor_core_ready():
-            return self._forward_tensor_cores(x2, act, bias).reshape(*batch_shape, self.out_features).to(x.dtype)
+            out = self._forward_tensor_cores(x2, act, bias)
+            return out if x.dim() == 2 and out.dtype == x.dtype else out.reshape(*batch_shape, self.out_features).to(x.dtype)
         out = torch.empty((T, self.out_features), dtype=x2.dtype, device=x2.device)
         for t0 in range(0, T, 16):
             t1 = min(T, t0 + 16)
@@ -289,7 +295,7 @@ class NVFP4PackedMLP(nn.Module):
         (each was quantised on its own: the stacked launch needs a common fp32 multiplier)."""
         g, u = self.gate_proj, self.up_proj
         key = (g.weight_packed.data_ptr(), u.weight_packed.data_ptr())
-        st = getattr(self, "_gu", None)
+        st = self.__dict__.get("_gu")
         if st is None or st[0] != key:
             if g.global_scale != u.global_scale:
                 st = (key, None)
@@ -310,26 +316,29 @@ class NVFP4PackedMLP(nn.Module):
         st = self._stacked_gate_up() if fast else None
         if st is None or st[1] is None:
             return self.down_proj(self.gate_proj(x) * self.up_proj(x))
-        from . import _lib
         _, gu_image, gu_gemv_ws = st
         batch_shape = x.shape[:-1]
-        x2 = x.reshape(-1, self.hidden_size).contiguous()
+        x2 = (x if x.dim() == 2 and x.shape[1] == self.hidden_size else x.reshape(-1, self.hidden_size)).contiguous()
         if x2.dtype != torch.bfloat16:
             x2 = x2.to(torch.bfloat16)
         T, I = x2.shape[0], self.intermediate_size
-        gu = torch.empty((T, 2 * I), dtype=torch.bfloat16, device=x2.device)
         mode = _lib.ROW_GELU_MUL if g.activation == "gelu" else _lib.ROW_SILU_MUL
         d_image, d_gemv_ws = d._tc_state()
-        d_bias = None if d.bias is None else d.bias.detach().float().contiguous()
+        d_bias = d.bias
+        if d_bias is not None:
+            d_bias = d_bias.detach().float().contiguous()
         out = torch.empty((T, self.hidden_size), dtype=torch.bfloat16, device=x2.device)
         if T <= 16:
-            ops.tc_gemv(x2, gu_image, 2 * I, gu, g.global_scale, None, 0, 3, gu_gemv_ws)
+            # three launches chained by programmatic dependent launch: each starts on its weights while the one before runs
+            gu = torch.empty((T, 2 * I), dtype=torch.bfloat16, device=x2.device)
             h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
-            ops.rowop(mode, gu, I, None, y_out=h, M=T)
+            ops.tc_gemv(x2, gu_image, 2 * I, gu, g.global_scale, None, 0, 3, gu_gemv_ws, pdl=True)
+            with ops.launch_flags(ops.FLAG_PDL):
+                ops.rowop(mode, gu, I, None, y_out=h, M=T)
             if T <= 4 and d.in_features % 32 == 0 and d.weight_packed.is_contiguous():
-                ops.nvfp4_gemv_out(h, d.weight_packed, d.weight_scales, out, d_bias, 0, 16, d.global_scale)
+                ops.nvfp4_gemv_out(h, d.weight_packed, d.weight_scales, out, d_bias, 0, 16, d.global_scale, pdl=True)
             else:
-                ops.tc_gemv(h, d_image, self.hidden_size, out, d.global_scale, d_bias, 0, 3, d_gemv_ws)
+                ops.tc_gemv(h, d_image, self.hidden_size, out, d.global_scale, d_bias, 0, 3, d_gemv_ws, pdl=True)
         elif I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True):
             # two launches: gate_up with act(gate) * up in its epilogue, down on its bf16 result
             h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
@@ -338,6 +347,7 @@ class NVFP4PackedMLP(nn.Module):
                             gated=True, out=h)
                 ops.w4_gemm(h, d_image, self.hidden_size, _lib.W4_NVFP4_TILED, alpha=d.global_scale, bias=d_bias, out=out)
         else:
+            gu = torch.empty((T, 2 * I), dtype=torch.bfloat16, device=x2.device)
             qx = _operand_buffer(g, T, self.hidden_size, x2.device)
             q = _operand_buffer(d, T, I, x2.device)
             with ops.launch_flags(ops.FLAG_PDL):     # four launches chained by programmatic dependent launch
@@ -353,7 +363,7 @@ class NVFP4PackedMLP(nn.Module):
                                      out=ops._ptr(out), out_dtype=ops._dt(out), ldo=out.stride(0), M=T, N=self.hidden_size,
                                      K=I, layout=ops.OPERANDS_TILED)
                 ops._gemm_ex(args, x2.device, _split_k_scratch(d, T, self.hidden_size, I, x2.device))
-        return out.reshape(*batch_shape, self.hidden_size).to(x.dtype)
+        return out if x.dim() == 2 and x.dtype == out.dtype else out.reshape(*batch_shape, self.hidden_size).to(x.dtype)
 
 
 def replace_mlp_with_nvfp4_packed(model, block_size: int = BLOCK_SIZE, target_layers: Optional[list] = None,

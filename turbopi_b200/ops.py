@@ -11,6 +11,7 @@ and add the B200-native forms (bf16 in/out, E4M3 block-16 scales, grouped launch
 Every tensor must live on a CUDA device; nothing here computes on the CPU.
 """
 import ctypes
+import threading
 
 import torch
 
@@ -38,8 +39,29 @@ def _ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
-def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+# The device check and the stream handle of a call: plain integers (about 0.3 us together) where the context manager and
+# the stream object cost 5 us of a call whose kernel takes ten.
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+
+
+def _run(t, fn, *args):
+    """fn(*args, stream) on the GPU that holds `t` and its current stream; switches the device only when another one
+    is current."""
+    i = t.get_device()
+    if _current_device() == i:
+        return fn(*args, _raw_stream(i))
+    with torch.cuda.device(i):
+        return fn(*args, _raw_stream(i))
+
+
+def _run_on(device, fn, *args):
+    """_run for a torch.device."""
+    i = device.index
+    if i is None or _current_device() != i:
+        with torch.cuda.device(device):
+            return fn(*args, _raw_stream(_current_device()))
+    return fn(*args, _raw_stream(i))
 
 
 def _scale_kind(scales):
@@ -60,11 +82,9 @@ def w4a16_gemv_out(input, weight_packed, scales, out, bias=None, group_size=32, 
     _cuda(input, weight_packed, scales, out, bias)
     M, K = input.shape
     N = out.shape[1]
-    with torch.cuda.device(input.device):
-        st = _lib.load().tpb200_w4a16_gemv(
-            _ptr(input), _dt(input), _ptr(weight_packed), _ptr(scales), _scale_kind(scales), _ptr(bias),
-            _dt(bias) if bias is not None else F32, _ptr(out), _dt(out), M, N, K, group_size, layout,
-            FLAG_PDL if pdl else FLAG_NONE, _stream(input))
+    st = _run(input, _lib.load().tpb200_w4a16_gemv, _ptr(input), _dt(input), _ptr(weight_packed), _ptr(scales),
+              _scale_kind(scales), _ptr(bias), _dt(bias) if bias is not None else F32, _ptr(out), _dt(out), M, N, K,
+              group_size, layout, FLAG_PDL if pdl else FLAG_NONE)
     _lib.check(st, "tpb200_w4a16_gemv")
     return out
 
@@ -92,15 +112,14 @@ def w4a16_gemm(x, weight, scales, zeros=None, bias=None, out=None, layout=INT4_K
     _cuda(x, weight, scales, zeros, bias, out)
     M, K = x.shape
     N = weight.shape[1] if layout == INT4_KBLOCK else weight.shape[0]
-    xb = x.to(torch.bfloat16).contiguous()
+    xb = x if x.dtype == torch.bfloat16 and x.is_contiguous() else x.to(torch.bfloat16).contiguous()
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     if bias is not None:
-        bias = bias.float().contiguous()
-    with torch.cuda.device(x.device):
-        st = _lib.load().tpb200_w4a16_gemm(_ptr(xb), _ptr(weight), _ptr(scales), _ptr(zeros), _ptr(bias), F32, _ptr(out),
-                                           _dt(out), M, N, K, out.stride(0), int(layout), float(alpha), float(beta),
-                                           _launch_flags, _stream(x))
+        bias = (bias if bias.dtype in _DTYPES else bias.float()).contiguous()
+    st = _run(x, _lib.load().tpb200_w4a16_gemm, _ptr(xb), _ptr(weight), _ptr(scales), _ptr(zeros), _ptr(bias),
+              _dt(bias) if bias is not None else F32, _ptr(out), _dt(out), M, N, K, out.stride(0), int(layout),
+              float(alpha), float(beta), _flags.value)
     _lib.check(st, "tpb200_w4a16_gemm")
     return out
 
@@ -112,11 +131,10 @@ def nvfp4_gemv_out(x, weight_packed, weight_scales, out, bias=None, activation=A
     _cuda(x, weight_packed, weight_scales, out, bias, x_scales)
     M, K = x.shape
     N = out.shape[1]
-    with torch.cuda.device(x.device):
-        st = _lib.load().tpb200_nvfp4_gemv(
-            _ptr(x), _dt(x), _ptr(x_scales), _ptr(weight_packed), _ptr(weight_scales), _scale_kind(weight_scales),
-            block_size, float(global_scale), _ptr(bias), _dt(bias) if bias is not None else F32, _ptr(out),
-            _dt(out), M, N, K, int(activation), FLAG_PDL if pdl else FLAG_NONE, _stream(x))
+    st = _run(x, _lib.load().tpb200_nvfp4_gemv, _ptr(x), _dt(x), _ptr(x_scales), _ptr(weight_packed),
+              _ptr(weight_scales), _scale_kind(weight_scales), block_size, float(global_scale), _ptr(bias),
+              _dt(bias) if bias is not None else F32, _ptr(out), _dt(out), M, N, K, int(activation),
+              FLAG_PDL if pdl else FLAG_NONE)
     _lib.check(st, "tpb200_nvfp4_gemv")
     return out
 
@@ -202,8 +220,7 @@ def quantize_weight_to_int4(weight_bf16, group_size=128):
     packed = torch.empty((N, K // 2), dtype=torch.int8, device=w.device)
     scales = torch.empty((N, K // group_size), dtype=torch.bfloat16, device=w.device)
     zeros = torch.empty_like(scales)
-    with torch.cuda.device(w.device):
-        _lib.load().quantizeWeightToINT4(_ptr(w), _ptr(packed), _ptr(scales), _ptr(zeros), N, K, group_size, _stream(w))
+    _run(w, _lib.load().quantizeWeightToINT4, _ptr(w), _ptr(packed), _ptr(scales), _ptr(zeros), N, K, group_size)
     _lib.check_void("quantizeWeightToINT4")
     return packed, scales, zeros
 
@@ -212,9 +229,8 @@ def dequantize_int4_to_bf16(packed, scales, zeros, group_size=128):
     _cuda(packed, scales, zeros)
     N, Kh = packed.shape
     out = torch.empty((N, Kh * 2), dtype=torch.bfloat16, device=packed.device)
-    with torch.cuda.device(packed.device):
-        _lib.load().dequantizeINT4ToBF16(_ptr(packed), _ptr(scales), _ptr(zeros), _ptr(out), N, Kh * 2, group_size,
-                                         _stream(packed))
+    _run(packed, _lib.load().dequantizeINT4ToBF16, _ptr(packed), _ptr(scales), _ptr(zeros), _ptr(out), N, Kh * 2,
+         group_size)
     _lib.check_void("dequantizeINT4ToBF16")
     return out
 
@@ -226,8 +242,7 @@ def quantize_activation_to_fp8(x_bf16):
     M, K = x.shape
     out = torch.empty((M, K), dtype=torch.uint8, device=x.device)
     scales = torch.empty((M, K // 16), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        _lib.load().quantizeActivationToFP8(_ptr(x), _ptr(out), _ptr(scales), M, K, _stream(x))
+    _run(x, _lib.load().quantizeActivationToFP8, _ptr(x), _ptr(out), _ptr(scales), M, K)
     _lib.check_void("quantizeActivationToFP8")
     return out, scales
 
@@ -239,8 +254,7 @@ def quantize_weight_to_nvfp4(weight_bf16):
     N, K = w.shape
     packed = torch.empty((K // 2, N), dtype=torch.uint8, device=w.device)
     scales = torch.empty((K // 16, N), dtype=torch.uint8, device=w.device)
-    with torch.cuda.device(w.device):
-        _lib.load().quantizeWeightToNVFP4(_ptr(w), _ptr(packed), _ptr(scales), N, K, _stream(w))
+    _run(w, _lib.load().quantizeWeightToNVFP4, _ptr(w), _ptr(packed), _ptr(scales), N, K)
     _lib.check_void("quantizeWeightToNVFP4")
     return packed, scales
 
@@ -277,8 +291,7 @@ def nvfp4_quantize_act(x, packed=None, sf=None):
         packed = torch.empty((M, pitch), dtype=torch.uint8, device=x.device)
     if sf is None:
         sf = torch.empty(nvfp4_sf_bytes(M, K), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        st = _lib.load().tpb200_nvfp4_quantize_act(_ptr(x), _dt(x), K, _ptr(packed), pitch, _ptr(sf), M, K, _stream(x))
+    st = _run(x, _lib.load().tpb200_nvfp4_quantize_act, _ptr(x), _dt(x), K, _ptr(packed), pitch, _ptr(sf), M, K)
     _lib.check(st, "tpb200_nvfp4_quantize_act")
     return packed, sf
 
@@ -291,11 +304,9 @@ def nvfp4_gemm(a_packed, a_sf, b_packed, b_sf, M, N, K, alpha=1.0, bias=None, ac
         out = torch.empty((M, N), dtype=out_dtype, device=a_packed.device)
     if bias is not None:
         bias = bias.float().contiguous()
-    with torch.cuda.device(a_packed.device):
-        st = _lib.load().tpb200_nvfp4_gemm(
-            _ptr(a_packed), a_packed.stride(0), _ptr(a_sf), _ptr(b_packed), b_packed.stride(0), _ptr(b_sf),
-            float(alpha), _ptr(bias), int(activation), _ptr(out), _dt(out), out.stride(0), M, N, K, FLAG_NONE,
-            _stream(a_packed))
+    st = _run(a_packed, _lib.load().tpb200_nvfp4_gemm, _ptr(a_packed), a_packed.stride(0), _ptr(a_sf), _ptr(b_packed),
+              b_packed.stride(0), _ptr(b_sf), float(alpha), _ptr(bias), int(activation), _ptr(out), _dt(out),
+              out.stride(0), M, N, K, FLAG_NONE)
     _lib.check(st, "tpb200_nvfp4_gemm")
     return out
 
@@ -312,9 +323,8 @@ def nvfp4_quantize_act_pieces(x, pieces=3):
     packed = torch.empty((pieces * piece_rows, pitch), dtype=torch.uint8, device=x.device)
     sf = torch.empty(nvfp4_sf_bytes(pieces * piece_rows, K), dtype=torch.uint8, device=x.device)
     row_scale = torch.empty((M,), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        st = _lib.load().tpb200_nvfp4_quantize_act_pieces(_ptr(x), _dt(x), K, _ptr(packed), pitch, _ptr(sf),
-                                                          _ptr(row_scale), M, K, pieces, piece_rows, _stream(x))
+    st = _run(x, _lib.load().tpb200_nvfp4_quantize_act_pieces, _ptr(x), _dt(x), K, _ptr(packed), pitch, _ptr(sf),
+              _ptr(row_scale), M, K, pieces, piece_rows)
     _lib.check(st, "tpb200_nvfp4_quantize_act_pieces")
     return packed, sf, row_scale, piece_rows
 
@@ -329,8 +339,12 @@ def nvfp4_gemm_workspace_size(M, N, K, pieces=1, layout=0):
     return int(_lib.load().tpb200_nvfp4_gemm_workspace_size(M, N, K, pieces, layout))
 
 
-# Launch flags applied to the tensor-core GEMM and the row kernel (see `launch_flags`)
-_launch_flags = FLAG_NONE
+# Launch flags applied to the tensor-core GEMM and the row kernel (see `launch_flags`); each host thread has its own
+class _Flags(threading.local):
+    value = FLAG_NONE
+
+
+_flags = _Flags()
 
 
 class launch_flags:
@@ -341,24 +355,21 @@ class launch_flags:
         self.flags = int(flags)
 
     def __enter__(self):
-        global _launch_flags
-        self.prev, _launch_flags = _launch_flags, self.flags
+        self.prev, _flags.value = _flags.value, self.flags
         return self
 
     def __exit__(self, *exc):
-        global _launch_flags
-        _launch_flags = self.prev
+        _flags.value = self.prev
         return False
 
 
 def _gemm_ex(args, device, workspace=None):
-    args.flags = _launch_flags
+    args.flags = _flags.value
     if workspace is not None:
         _cuda(workspace)
         args.workspace = _ptr(workspace)
         args.workspace_bytes = workspace.numel() * workspace.element_size()
-    with torch.cuda.device(device):
-        st = _lib.load().tpb200_nvfp4_gemm_ex(ctypes.byref(args), torch.cuda.current_stream(device).cuda_stream)
+    st = _run_on(device, _lib.load().tpb200_nvfp4_gemm_ex, args)
     _lib.check(st, "tpb200_nvfp4_gemm_ex")
 
 
@@ -403,9 +414,8 @@ def w4_gemm(x, w, N, format, w_scales=None, w_zeros=None, alpha=1.0, beta=0.0, b
 
 
 def _w4_gemm(args, device):
-    args.flags = _launch_flags
-    with torch.cuda.device(device):
-        st = _lib.load().tpb200_w4_gemm(ctypes.byref(args), torch.cuda.current_stream(device).cuda_stream)
+    args.flags = _flags.value
+    st = _run_on(device, _lib.load().tpb200_w4_gemm, args)
     _lib.check(st, "tpb200_w4_gemm")
 
 
@@ -494,9 +504,8 @@ def tile_weights(b_packed, b_sf, N, K):
     blocks [ceil(N/256)][ceil(K/256)] of 36 KB that carry codes and scales of 256 rows for one K stage."""
     _cuda(b_packed, b_sf)
     image = torch.empty(int(_lib.load().tpb200_nvfp4_tiled_b_bytes(N, K)), dtype=torch.uint8, device=b_packed.device)
-    with torch.cuda.device(b_packed.device):
-        st = _lib.load().tpb200_nvfp4_tile_weights(_ptr(b_packed), b_packed.stride(0), _ptr(b_sf), _ptr(image), N, K,
-                                                   _stream(b_packed))
+    st = _run(b_packed, _lib.load().tpb200_nvfp4_tile_weights, _ptr(b_packed), b_packed.stride(0), _ptr(b_sf),
+              _ptr(image), N, K)
     _lib.check(st, "tpb200_nvfp4_tile_weights")
     # weight preparation is a one-off: finish it here, so that a following launch with FLAG_PDL (which reads
     # weights before it waits for its predecessor) can never start on an incomplete image
@@ -538,9 +547,8 @@ def rowop(mode, x, K, q=None, res_in=None, gate=None, h_out=None, w0=None, w1=No
                        packed=p(q.packed) if q is not None else 0, pitch=q.pitch if q is not None else 0,
                        sf=p(q.sf) if q is not None else 0, row_scale=p(q.row_scale) if q is not None else 0,
                        pieces=q.pieces if q is not None else 0, piece_rows=q.piece_rows if q is not None else 0,
-                       layout=q.layout if q is not None else 0, flags=_launch_flags)
-    with torch.cuda.device(x.device):
-        st = _lib.load().tpb200_row_transform_quantize(ctypes.byref(a), torch.cuda.current_stream(x.device).cuda_stream)
+                       layout=q.layout if q is not None else 0, flags=_flags.value)
+    st = _run(x, _lib.load().tpb200_row_transform_quantize, a)
     _lib.check(st, "tpb200_row_transform_quantize")
 
 
@@ -572,6 +580,9 @@ def attention_workspace(n_rows, n_keys, head_dim, groups, device):
     return torch.empty(n, dtype=torch.uint8, device=device)
 
 
+_Two = ctypes.c_longlong * 2
+
+
 def attention(q, k, v, out, scale, key_bias=None, workspace=None, quant=None, rows_per_token=1):
     """out = softmax(scale * q k^T + key_bias) v on the tensor cores; bf16 tensors.
     q / out: [rows, D] or [A, B, rows, D] views (any strides with a unit last stride); k / v: [keys, D] or
@@ -580,19 +591,18 @@ def attention(q, k, v, out, scale, key_bias=None, workspace=None, quant=None, ro
     out=None only, written as the operand of the next tensor-core GEMM -- what rowop(ROW_NONE, out, ...) would
     produce, without that launch (2-D problems only)."""
     _cuda(q, k, v, out, key_bias, workspace)
-    if q.dim() == 2:
-        q, k, v = q[None, None], k[None, None], v[None, None]
-        out = None if out is None else out[None, None]
     if out is None and quant is None:
         raise TurboPiError("attention: neither out nor quant given")
-    if not (q.dim() == k.dim() == v.dim() == 4 and (out is None or out.dim() == 4)):
+    nd = q.dim()
+    if nd not in (2, 4) or k.dim() != nd or v.dim() != nd or (out is not None and out.dim() != nd):
         raise TurboPiError("attention: q, k, v, out must all be 2-D or all 4-D")
     for t in (q, k, v, out):
-        if t is not None and (t.dtype != torch.bfloat16 or t.stride(3) != 1):
+        if t is not None and (t.dtype != torch.bfloat16 or t.stride(-1) != 1):
             raise TurboPiError("attention: bf16 tensors with a contiguous last dimension")
-    A, B, R, D = q.shape
-    S = k.shape[2]
-    if tuple(k.shape) != (A, B, S, D) or tuple(v.shape) != (A, B, S, D) or (out is not None and tuple(out.shape) != (A, B, R, D)):
+    A, B, R, D = q.shape if nd == 4 else (1, 1, *q.shape)
+    S = k.shape[-2]
+    kv_shape, q_shape = ((A, B, S, D), (A, B, R, D)) if nd == 4 else ((S, D), (R, D))
+    if tuple(k.shape) != kv_shape or tuple(v.shape) != kv_shape or (out is not None and tuple(out.shape) != q_shape):
         raise TurboPiError("attention: shapes of q, k, v, out do not agree")
     if key_bias is not None and (key_bias.dtype != torch.bfloat16 or key_bias.numel() < S or not key_bias.is_contiguous()):
         raise TurboPiError("attention: key_bias must be a contiguous bf16 vector with one entry per key")
@@ -601,24 +611,22 @@ def attention(q, k, v, out, scale, key_bias=None, workspace=None, quant=None, ro
             raise TurboPiError("attention: quant must be a QuantBuf of [rows / rows_per_token, rows_per_token * D]")
     if workspace is None:
         workspace = attention_workspace(R, S, D, A * B, q.device)
-    two = ctypes.c_longlong * 2
     o = q if out is None else out          # strides only; the pointer stays NULL without `out`
+    group_strides = [_Two(t.stride(0), t.stride(1)) if nd == 4 else _Two(0, 0) for t in (q, k, v, o)]
     args = _lib.AttentionArgs(q=_ptr(q), k=_ptr(k), v=_ptr(v), out=_ptr(out), key_bias=_ptr(key_bias), n_rows=R, n_keys=S,
-                              head_dim=D, ldq=q.stride(2), ldk=k.stride(2), ldv=v.stride(2), ldo=o.stride(2),
-                              groups_outer=A, groups_inner=B, q_stride=two(q.stride(0), q.stride(1)),
-                              k_stride=two(k.stride(0), k.stride(1)), v_stride=two(v.stride(0), v.stride(1)),
-                              o_stride=two(o.stride(0), o.stride(1)), scale=float(scale), workspace=_ptr(workspace),
-                              workspace_bytes=workspace.numel(), flags=_launch_flags,
+                              head_dim=D, ldq=q.stride(-2), ldk=k.stride(-2), ldv=v.stride(-2), ldo=o.stride(-2),
+                              groups_outer=A, groups_inner=B, q_stride=group_strides[0], k_stride=group_strides[1],
+                              v_stride=group_strides[2], o_stride=group_strides[3], scale=float(scale), workspace=_ptr(workspace),
+                              workspace_bytes=workspace.numel(), flags=_flags.value,
                               quant_image=_ptr(quant.packed) if quant is not None else None,
                               quant_row_scale=_ptr(quant.row_scale) if quant is not None else None,
                               quant_pieces=quant.pieces if quant is not None else 0, quant_rows_per_token=rows_per_token,
                               quant_sf=_ptr(quant.sf) if quant is not None and not quant.tiled else None,
                               quant_pitch=quant.pitch if quant is not None else 0,
                               quant_piece_rows=quant.piece_rows if quant is not None else 0)
-    with torch.cuda.device(q.device):
-        st = _lib.load().tpb200_attention(ctypes.byref(args), torch.cuda.current_stream(q.device).cuda_stream)
+    st = _run(q, _lib.load().tpb200_attention, args)
     _lib.check(st, "tpb200_attention")
-    return out
+    return out if nd == 4 or out is None else out[None, None]      # the [1, 1, rows, D] view of a 2-D call
 
 
 # ------------------------------------------------------------------------------------- tensor-core GEMV
@@ -703,17 +711,13 @@ class TcGemv:
                 _lib.check(st, "tpb200_nvfp4_quantize_acts_tc")
 
     def gemv(self):
-        lib = _lib.load()
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream(self.device).cuda_stream
-            if self.fused:
-                st = lib.tpb200_nvfp4_gemv_tc_fused(self._arr, len(self._arr), self.M, self.pieces, self.x_dtype,
-                                                    self.bias_dtype, self.out_dtype, self.activation,
-                                                    _ptr(self.workspace), self.workspace.numel(), self.flags, stream)
-            else:
-                st = lib.tpb200_nvfp4_gemv_tc(self._arr, len(self._arr), self.M, self.pieces, self.bias_dtype,
-                                              self.out_dtype, self.activation, _ptr(self.workspace),
-                                              self.workspace.numel(), self.flags, stream)
+        lib, ws = _lib.load(), self.workspace
+        if self.fused:
+            st = _run(ws, lib.tpb200_nvfp4_gemv_tc_fused, self._arr, len(self._arr), self.M, self.pieces, self.x_dtype,
+                      self.bias_dtype, self.out_dtype, self.activation, _ptr(ws), ws.numel(), self.flags)
+        else:
+            st = _run(ws, lib.tpb200_nvfp4_gemv_tc, self._arr, len(self._arr), self.M, self.pieces, self.bias_dtype,
+                      self.out_dtype, self.activation, _ptr(ws), ws.numel(), self.flags)
         _lib.check(st, "tpb200_nvfp4_gemv_tc")
 
     def gemv_static(self):
@@ -745,30 +749,26 @@ def tc_gemv(x, w_image, N, out, global_scale=1.0, bias=None, activation=ACT_NONE
     lib = _lib.load()
     flags = FLAG_PDL if pdl else FLAG_NONE
     bias_dtype = _dt(bias) if bias is not None else F32
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        if M <= 4:
-            arr = (_lib.GemvTcFusedProblem * 1)(_lib.GemvTcFusedProblem(_ptr(w_image), _ptr(x), x.stride(0), _ptr(bias), _ptr(out),
-                                                                          N, K, out.stride(0), float(global_scale)))
-            if workspace is None:
-                workspace = torch.zeros(int(lib.tpb200_nvfp4_gemv_tc_fused_workspace_size(arr, 1)), dtype=torch.uint8,
-                                        device=x.device)
-            st = lib.tpb200_nvfp4_gemv_tc_fused(arr, 1, M, pieces, _dt(x), bias_dtype, _dt(out), int(activation),
-                                                _ptr(workspace), workspace.numel(), flags, stream)
-            _lib.check(st, "tpb200_nvfp4_gemv_tc_fused")
-        else:
-            xi = torch.empty(int(lib.tpb200_nvfp4_gemv_tc_x_image_bytes(K, pieces)), dtype=torch.uint8, device=x.device)
-            rs = torch.empty(16, dtype=torch.float32, device=x.device)
-            st = lib.tpb200_nvfp4_quantize_act_tc(_ptr(x), _dt(x), x.stride(0), _ptr(xi), _ptr(rs), M, K, pieces, flags, stream)
-            _lib.check(st, "tpb200_nvfp4_quantize_act_tc")
-            arr = (_lib.GemvTcProblem * 1)(_lib.GemvTcProblem(_ptr(w_image), _ptr(xi), _ptr(rs), _ptr(bias), _ptr(out), N, K,
-                                                              out.stride(0), float(global_scale)))
-            if workspace is None:
-                workspace = torch.zeros(int(lib.tpb200_nvfp4_gemv_tc_workspace_size(arr, 1)), dtype=torch.uint8,
-                                        device=x.device)
-            st = lib.tpb200_nvfp4_gemv_tc(arr, 1, M, pieces, bias_dtype, _dt(out), int(activation), _ptr(workspace),
-                                          workspace.numel(), flags, stream)
-            _lib.check(st, "tpb200_nvfp4_gemv_tc")
+    if M <= 4:
+        arr = (_lib.GemvTcFusedProblem * 1)((_ptr(w_image), _ptr(x), x.stride(0), _ptr(bias), _ptr(out), N, K, out.stride(0),
+                                             float(global_scale)))
+        if workspace is None:
+            workspace = tc_gemv_workspace(N, K, x.device)
+        st = _run(x, lib.tpb200_nvfp4_gemv_tc_fused, arr, 1, M, pieces, _dt(x), bias_dtype, _dt(out), int(activation),
+                  _ptr(workspace), workspace.numel(), flags)
+        _lib.check(st, "tpb200_nvfp4_gemv_tc_fused")
+    else:
+        xi = torch.empty(int(lib.tpb200_nvfp4_gemv_tc_x_image_bytes(K, pieces)), dtype=torch.uint8, device=x.device)
+        rs = torch.empty(16, dtype=torch.float32, device=x.device)
+        st = _run(x, lib.tpb200_nvfp4_quantize_act_tc, _ptr(x), _dt(x), x.stride(0), _ptr(xi), _ptr(rs), M, K, pieces, flags)
+        _lib.check(st, "tpb200_nvfp4_quantize_act_tc")
+        arr = (_lib.GemvTcProblem * 1)((_ptr(w_image), _ptr(xi), _ptr(rs), _ptr(bias), _ptr(out), N, K, out.stride(0),
+                                        float(global_scale)))
+        if workspace is None:
+            workspace = tc_gemv_workspace(N, K, x.device)
+        st = _run(x, lib.tpb200_nvfp4_gemv_tc, arr, 1, M, pieces, bias_dtype, _dt(out), int(activation), _ptr(workspace),
+                  workspace.numel(), flags)
+        _lib.check(st, "tpb200_nvfp4_gemv_tc")
     return out
 
 

@@ -18,6 +18,7 @@ from ._lib import INT4_KBLOCK, INT4_ROWMAJOR
 QUANT_BLOCK = 32
 INT4_OFFSET = 8
 INT4_RANGE = 7
+_FLOATS = frozenset((torch.float16, torch.bfloat16, torch.float32))
 
 
 @dataclass
@@ -152,25 +153,31 @@ class W4A16Linear(nn.Module):
         return dequantize_kblock(self.weight_packed, self.scales)
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
-        *batch_dims, K = input.shape
+        K, N = input.shape[-1], self.out_features
         assert K == self.in_features, f"Input last dim ({K}) doesn't match in_features ({self.in_features})"
-        x = input.reshape(-1, K)
-        if x.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+        x = input if input.dim() == 2 else input.reshape(-1, K)
+        if x.dtype not in _FLOATS:
             x = x.float()
-        x = x.contiguous()
+        if not x.is_contiguous():
+            x = x.contiguous()
         T = x.shape[0]
-        out = torch.empty((T, self.out_features), dtype=input.dtype if input.dtype in (
-            torch.float16, torch.bfloat16, torch.float32) else torch.float32, device=input.device)
-        bias = None if self.bias is None else self.bias.detach().contiguous()
-        if bias is not None and bias.dtype not in (torch.float16, torch.bfloat16, torch.float32):
-            bias = bias.float()
-        if T > 16 and K % 128 == 0 and self.out_features % 8 == 0:
-            ops.w4a16_gemm(x, self.weight_packed, self.scales, None, bias, out, INT4_KBLOCK)
-            return out.reshape(*batch_dims, self.out_features)
-        for t0 in range(0, T, 16):
-            t1 = min(T, t0 + 16)
-            ops.w4a16_gemv_out(x[t0:t1], self.weight_packed, self.scales, out[t0:t1], bias, 32, INT4_KBLOCK)
-        return out.reshape(*batch_dims, self.out_features)
+        packed, scales = self.weight_packed, self.scales
+        out = torch.empty((T, N), dtype=input.dtype if input.dtype in _FLOATS else torch.float32, device=input.device)
+        bias = self.bias
+        if bias is not None:
+            bias = bias.detach().contiguous()
+            if bias.dtype not in _FLOATS:
+                bias = bias.float()
+        if T <= 16:
+            if T > 0:
+                ops.w4a16_gemv_out(x, packed, scales, out, bias, 32, INT4_KBLOCK)
+        elif K % 128 == 0 and N % 8 == 0:
+            ops.w4a16_gemm(x, packed, scales, None, bias, out, INT4_KBLOCK)
+        else:
+            for t0 in range(0, T, 16):
+                t1 = min(T, t0 + 16)
+                ops.w4a16_gemv_out(x[t0:t1], packed, scales, out[t0:t1], bias, 32, INT4_KBLOCK)
+        return out if input.dim() == 2 else out.reshape(*input.shape[:-1], N)
 
     def pack_weights(self, weight: torch.Tensor) -> None:
         packed = self._packer.pack(weight, device=self.weight_packed.device)
