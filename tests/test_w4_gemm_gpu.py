@@ -135,3 +135,30 @@ def test_kblock_gemv_with_k_cut_over_a_cluster(cuda_device, M, N, K):
     mag = x.double().abs() @ w.abs().t() + bias.double().abs()
     assert bool(((out.cpu().double() - ref).abs() <= 2.0 ** -10 * mag).all())
     assert _lib.load().tpb200_device_error(0) == 0
+
+
+@pytest.mark.parametrize("M,N,K,shift", [(1, 16, 16, 0), (50, 272, 1040, 0), (130, 144, 272, 0), (256, 2048, 2048, 0),
+                                         (65, 264, 528, 0), (33, 256, 512, 4)])
+def test_w4a8_forward_on_transposed_weights(cuda_device, M, N, K, shift):
+    """The plugin's transposed codes read as they are (N a multiple of 16, aligned pointers) or re-laid out first."""
+    from oracle import w4a8
+    from turbopi_b200 import _lib, ops
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(M + N + K)
+    w = (torch.randn((N, K), generator=g) * 0.05).to(torch.bfloat16).to(cuda_device)
+    x = torch.randn((M, K), generator=g).to(torch.bfloat16).to(cuda_device)
+    wp_t, ws_t = ops.quantize_weight_to_nvfp4(w)
+    a8, sa = ops.quantize_activation_to_fp8(x)
+    held = torch.empty(wp_t.numel() + 16, dtype=torch.uint8, device=cuda_device)
+    held[shift:shift + wp_t.numel()] = wp_t.reshape(-1)                       # `shift` bytes off a 16-byte boundary
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=cuda_device)
+    nws = lib.getW4A8GemmWorkspaceSize(M, N, K)
+    ws = torch.empty(nws, dtype=torch.uint8, device=cuda_device)
+    torch.cuda.synchronize()
+    lib.w4a8GemmForward(a8.data_ptr(), sa.data_ptr(), held.data_ptr() + shift, ws_t.data_ptr(), out.data_ptr(), M, N, K, 0.5,
+                        ws.data_ptr(), nws, torch.cuda.current_stream().cuda_stream)
+    _lib.check_void("w4a8GemmForward")
+    ref = torch.from_numpy(np.asarray(w4a8.gemm(a8.cpu().numpy(), sa.cpu().numpy(), wp_t.cpu().numpy(), ws_t.cpu().numpy(), 0.5)))
+    # exact products in bf16 x bf16, fp32 sums, one rounding to bf16
+    assert bool(((out.cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all())
+    assert lib.tpb200_device_error(0) == 0

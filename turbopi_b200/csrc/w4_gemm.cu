@@ -51,7 +51,7 @@ constexpr int kXWarp = 0, kMmaWarp = 1, kWWarp = 2, kDqWarp0 = 3;
 constexpr int kDqWarpsPerSm = 16;                // 16 dequantisation warps with an SM of its own, 8 with two CTAs per SM
 constexpr long long kWaitG = 400000000LL;        // ~0.2 s
 
-enum { kFmtNvfp4 = 0, kFmtKblock = 1, kFmtPlugin = 2 };
+enum { kFmtNvfp4 = 0, kFmtKblock = 1, kFmtPlugin = 2, kFmtNvfp4T = 3 };   // 3: the w4a8 plugin's transposed operand
 enum { kEpiPlain = 0, kEpiQkv = 1, kEpiGated = 2 };
 
 struct W4gParams {
@@ -270,7 +270,8 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
         const uint64_t policy = l2_policy_evict_first();
         const bool gated = P.epilogue == kEpiGated;
         const uint32_t bytes = kFmt == kFmtNvfp4 ? (gated ? kCodeBytes + 2 * kSlabBytes : kCodeBytes + kSlabBytes)
-                               : kFmt == kFmtKblock && P.kb_scale == nullptr ? kCodeBytes + kSlabBytes : kCodeBytes;
+                               : kFmt == kFmtNvfp4T || (kFmt == kFmtKblock && P.kb_scale == nullptr) ? kCodeBytes + kSlabBytes
+                                                                                                      : kCodeBytes;
         for (int j = 0; j < nblk; ++j) {
             const int s = j % P.n_w, kb = blk0 + j;
             uint8_t* slot = sW + s * kWSlot;
@@ -298,6 +299,9 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                                              : P.sf + (static_cast<size_t>(row >> 7) * P.img_kblocks + kb) * kSlabBytes;
                     bulk_copy_g2s_hint(slot + kCodeBytes + half * kSlabBytes, src, kSlabBytes, &ctl.w_full[s], policy);
                 }
+            } else if (kFmt == kFmtNvfp4T) {                         // [128 code bytes of K][128 rows], [16 scales][128 rows]
+                if (lane == 0) tc::tma_load_2d(slot, &P.map_w, row_a, kb * 128, &ctl.w_full[s]);
+                if (lane == 1) tc::tma_load_2d(slot + kCodeBytes, &P.map_s, row_a, kb * 16, &ctl.w_full[s]);
             } else if (kFmt == kFmtKblock) {
                 if (lane == 0) tc::tma_load_2d(slot, &P.map_w, row_a * 2, kb * 8, &ctl.w_full[s]);
                 if (lane == 1 && P.kb_scale == nullptr) tc::tma_load_2d(slot + kCodeBytes, &P.map_s, row_a, kb * 8, &ctl.w_full[s]);
@@ -373,7 +377,14 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                 const uint8_t* slot = sW + sw * kWSlot;
                 uint32_t out[32];
                 uint4 c[2];
-                if (kFmt == kFmtKblock) {
+                if (kFmt == kFmtNvfp4T) {                            // a row's codes lie 128 bytes apart
+                    uint32_t* cw = reinterpret_cast<uint32_t*>(c);
+#pragma unroll
+                    for (int wd = 0; wd < 8; ++wd) {
+                        const uint8_t* p4 = slot + (32 * kk + 4 * wd) * kRows + r;
+                        cw[wd] = p4[0] | p4[kRows] << 8 | p4[2 * kRows] << 16 | static_cast<uint32_t>(p4[3 * kRows]) << 24;
+                    }
+                } else if (kFmt == kFmtKblock) {
                     c[0] = *reinterpret_cast<const uint4*>(slot + (2 * kk) * 2048 + r * 16);
                     c[1] = *reinterpret_cast<const uint4*>(slot + (2 * kk + 1) * 2048 + r * 16);
                 } else {
@@ -382,6 +393,10 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                 }
                 uint32_t sc = 0;
                 if (kFmt == kFmtNvfp4) sc = *reinterpret_cast<const uint32_t*>(slot + kCodeBytes + kk * 512 + sf_off);
+                if (kFmt == kFmtNvfp4T) {
+                    const uint8_t* p4 = slot + kCodeBytes + 4 * kk * kRows + r;
+                    sc = p4[0] | p4[kRows] << 8 | p4[2 * kRows] << 16 | static_cast<uint32_t>(p4[3 * kRows]) << 24;
+                }
                 if (kFmt == kFmtKblock) {
                     if (P.kb_scale == nullptr) {
                         const __half* sp = reinterpret_cast<const __half*>(slot + kCodeBytes) + (2 * kk) * kRows + r;
@@ -398,7 +413,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                     if (lane == 0) mbar_arrive(&ctl.w_empty[sw]);        // every lane's codes are in registers
                 }
                 const uint32_t w[8] = {c[0].x, c[0].y, c[0].z, c[0].w, c[1].x, c[1].y, c[1].z, c[1].w};
-                if (kFmt == kFmtNvfp4) {
+                if (kFmt == kFmtNvfp4 || kFmt == kFmtNvfp4T) {
                     const __half2 s01 = decode_e4m3x2_h(static_cast<uint16_t>(sc)), s23 = decode_e4m3x2_h(static_cast<uint16_t>(sc >> 16));
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
@@ -615,6 +630,9 @@ constexpr int kBoundThreads = 704;
 __global__ void __launch_bounds__(kBoundThreads, 1) w4_nvfp4_gemm_kernel(const __grid_constant__ W4gParams P) {
     w4_gemm_tile<kFmtNvfp4>(P);
 }
+__global__ void __launch_bounds__(kBoundThreads, 1) w4_nvfp4_gemm_kernel_transposed(const __grid_constant__ W4gParams P) {
+    w4_gemm_tile<kFmtNvfp4T>(P);
+}
 __global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_kblock_gemm_kernel(const __grid_constant__ W4gParams P) {
     w4_gemm_tile<kFmtKblock>(P);
 }
@@ -665,7 +683,8 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
 
 int device_error_w4_gemm(int clear) { return read_device_error(clear); }
 
-int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
+// `transposed` (internal, TPB200_W4_NVFP4_ROWMAJOR only): w = [K / 2, N] code bytes, w_scales = [K / 16, N] UE4M3 bytes, N % 16 == 0
+int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool transposed) {
     TPB_REQUIRE(a != nullptr && a->x != nullptr && a->w != nullptr && a->out != nullptr, TPB200_ERR_NULL);
     TPB_REQUIRE(a->format >= TPB200_W4_NVFP4_ROWMAJOR && a->format <= TPB200_W4_INT4_PLUGIN, TPB200_ERR_ENUM);
     TPB_REQUIRE((a->flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
@@ -702,7 +721,8 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
         TPB_REQUIRE(static_cast<long long>(a->ldo) * tpb_dtype_size(a->out_dtype) % 16 == 0, TPB200_ERR_ALIGN);
     }
     W4gParams P = {};
-    const int fmt = nv ? kFmtNvfp4 : a->format == TPB200_W4_INT4_KBLOCK ? kFmtKblock : kFmtPlugin;
+    TPB_REQUIRE(!transposed || (a->format == TPB200_W4_NVFP4_ROWMAJOR && !qkv && !gated && N % 16 == 0), TPB200_ERR_ENUM);
+    const int fmt = transposed ? kFmtNvfp4T : nv ? kFmtNvfp4 : a->format == TPB200_W4_INT4_KBLOCK ? kFmtKblock : kFmtPlugin;
     const int tiles = (N + kRows - 1) / kRows;
     P.k_blocks = (K + kBlkK - 1) / kBlkK;
     P.k_steps = (K + kPartK - 1) / kPartK;
@@ -714,7 +734,10 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
     P.splits = plan.splits;
     bool ok = make_tensor_map_2d(&P.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a->x, K, M, static_cast<uint64_t>(a->ldx) * 2, 64,
                                  P.nt, true);
-    if (a->format == TPB200_W4_NVFP4_TILED) {
+    if (transposed) {
+        ok = ok && make_tensor_map_2d(&P.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, a->w, N, K / 2, N, 128, 128, false) &&
+             make_tensor_map_2d(&P.map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, a->w_scales, N, K / 16, N, 128, 16, false);
+    } else if (a->format == TPB200_W4_NVFP4_TILED) {
         P.image = static_cast<const uint8_t*>(a->w);
     } else if (a->format == TPB200_W4_INT4_KBLOCK) {
         ok = ok && make_tensor_map_2d(&P.map_w, CU_TENSOR_MAP_DATA_TYPE_UINT64, a->w, 2ull * N, K / 32, 16ull * N, 256, 8, false);
@@ -770,10 +793,10 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
     int smem = P.n_w * kWSlot + P.n_s * b_bytes * P.parts;
     smem = std::max(smem, P.nt * kRows * 4) + 1024;
 
-    static void (*const kernels[3])(const W4gParams) = {w4_nvfp4_gemm_kernel, w4_int4_kblock_gemm_kernel,
-                                                        w4_int4_plugin_gemm_kernel};
+    static void (*const kernels[4])(const W4gParams) = {w4_nvfp4_gemm_kernel, w4_int4_kblock_gemm_kernel,
+                                                        w4_int4_plugin_gemm_kernel, w4_nvfp4_gemm_kernel_transposed};
     auto kernel = kernels[fmt];
-    static std::atomic<uint64_t> configured[3] = {};
+    static std::atomic<uint64_t> configured[4] = {};
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured[fmt].load(std::memory_order_relaxed) & bit)) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) {
@@ -808,7 +831,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream) {
 }  // namespace tpb
 
 extern "C" int tpb200_w4_gemm(const tpb200_w4_gemm_args* a, tpb200_stream_t stream) {
-    return tpb::w4_gemm_launch(a, reinterpret_cast<cudaStream_t>(stream));
+    return tpb::w4_gemm_launch(a, reinterpret_cast<cudaStream_t>(stream), false);
 }
 
 extern "C" int tpb200_w4a16_gemm(const void* x, const void* weight, const void* scales, const void* zeros,
@@ -835,5 +858,5 @@ extern "C" int tpb200_w4a16_gemm(const void* x, const void* weight, const void* 
     a.N = N;
     a.K = K;
     a.flags = flags;
-    return tpb::w4_gemm_launch(&a, reinterpret_cast<cudaStream_t>(stream));
+    return tpb::w4_gemm_launch(&a, reinterpret_cast<cudaStream_t>(stream), false);
 }
