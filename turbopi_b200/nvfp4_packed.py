@@ -98,11 +98,12 @@ def _operand_buffer(module, T, K, device):
 
 def _dense_is_faster(T, N, K, gated=False):
     """Whether [N, K] weights on the tiled image take T tokens faster through the GEMM that dequantises them (bf16
-    activations as they are) than through the e2m1-piece GEMM behind its quantiser: the first dequantises the weights once
-    per 256 tokens, the second pays one launch more, two in a gated MLP.  Measured, us for pieces / dequantising.  Gated MLP
-    of 1024 -> 4096: 17 tokens 26 / 11, 256 33 / 23, 1000 51 / 48; of 1152 -> 8000: 256 40 / 33, 712 67 / 65; of 2048 -> 16384:
-    50 44 / 35, 192 63 / 61, 256 64 / 68.  One linear 8000 -> 1152: 256 21 / 18, 712 26 / 23; 16384 -> 2048: 128 23 / 21,
-    192 26 / 27."""
+    activations as they are) than through the GEMV behind a quantiser (up to 16 tokens) or the e2m1-piece GEMM behind one:
+    the first dequantises the weights once per 256 tokens, the others pay one launch more, two in a gated MLP.  Measured,
+    us for the others / dequantising.  Gated MLP of 1024 -> 4096: 1 token 16 / 10, 16 37 / 10, 17 26 / 11, 256 33 / 23, 1000 51 /
+    48; of 1152 -> 8000: 1 21 / 14, 256 40 / 33, 712 67 / 65; of 2048 -> 16384: 1 31 / 33 (one launch less to issue), 4 57 / 33,
+    50 44 / 35, 192 63 / 61, 256 64 / 68.  One linear 8000 -> 1152: 256 21 / 18, 712 26 / 23; 16384 -> 2048: 128 23 / 21, 192
+    26 / 27."""
     return T * N * K <= (13_000_000_000 if gated else 6_000_000_000)
 
 
@@ -257,10 +258,10 @@ class NVFP4PackedMLP(nn.Module):
     """Gated MLP down(act(gate(x)) * up(x)).  `gate_activation` defaults to the
     reference module's 'silu'; Gemma's own MLP uses 'gelu' (tanh form).
 
-    With "nvfp4" weights the forward is three or four launches whatever the token count: gate and up run as
-    ONE stacked [2I, K] matrix (one GEMV launch for <= 16 tokens, one tensor-core GEMM otherwise), the row
-    kernel applies act(gate) * up with the module's roundings (and, for the GEMM, writes the down
-    projection's operand), then the down projection."""
+    With "nvfp4" weights gate and up run as ONE stacked [2I, K] matrix.  Up to a size limit (`_dense_is_faster`) the forward
+    is two launches: the GEMM that dequantises its weights, with act(gate) * up (the module's roundings) in its epilogue,
+    and the same kernel on the down projection; with more tokens four: quantiser, block-scaled GEMM, the row kernel that
+    applies act(gate) * up and writes the down projection's operand, block-scaled GEMM."""
 
     def __init__(self, hidden_size: int, intermediate_size: int, block_size: int = BLOCK_SIZE,
                  gate_activation: str = "silu"):
@@ -328,7 +329,14 @@ class NVFP4PackedMLP(nn.Module):
         if d_bias is not None:
             d_bias = d_bias.detach().float().contiguous()
         out = torch.empty((T, self.hidden_size), dtype=torch.bfloat16, device=x2.device)
-        if T <= 16:
+        if I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True):
+            # two launches: gate_up with act(gate) * up in its epilogue, down on its bf16 result
+            h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
+            with ops.launch_flags(ops.FLAG_PDL):
+                ops.w4_gemm(x2, gu_image, 2 * I, _lib.W4_NVFP4_TILED, alpha=g.global_scale, activation=ACTIVATIONS[g.activation],
+                            gated=True, out=h)
+                ops.w4_gemm(h, d_image, self.hidden_size, _lib.W4_NVFP4_TILED, alpha=d.global_scale, bias=d_bias, out=out)
+        elif T <= 16:
             # three launches chained by programmatic dependent launch: each starts on its weights while the one before runs
             gu = torch.empty((T, 2 * I), dtype=torch.bfloat16, device=x2.device)
             h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
@@ -339,13 +347,6 @@ class NVFP4PackedMLP(nn.Module):
                 ops.nvfp4_gemv_out(h, d.weight_packed, d.weight_scales, out, d_bias, 0, 16, d.global_scale, pdl=True)
             else:
                 ops.tc_gemv(h, d_image, self.hidden_size, out, d.global_scale, d_bias, 0, 3, d_gemv_ws, pdl=True)
-        elif I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True):
-            # two launches: gate_up with act(gate) * up in its epilogue, down on its bf16 result
-            h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
-            with ops.launch_flags(ops.FLAG_PDL):
-                ops.w4_gemm(x2, gu_image, 2 * I, _lib.W4_NVFP4_TILED, alpha=g.global_scale, activation=ACTIVATIONS[g.activation],
-                            gated=True, out=h)
-                ops.w4_gemm(h, d_image, self.hidden_size, _lib.W4_NVFP4_TILED, alpha=d.global_scale, bias=d_bias, out=out)
         else:
             gu = torch.empty((T, 2 * I), dtype=torch.bfloat16, device=x2.device)
             qx = _operand_buffer(g, T, self.hidden_size, x2.device)
