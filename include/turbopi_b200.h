@@ -162,6 +162,8 @@ int tpb200_nvfp4_gemv_grouped(const tpb200_gemv_problem* problems, int count, in
 size_t tpb200_nvfp4_sf_bytes(int rows, int K);
 int tpb200_nvfp4_quantize_act(const void* x, int x_dtype, int ldx, void* packed, int packed_pitch,
                               void* sf_swizzled, int M, int K, tpb200_stream_t stream);
+/* the same codes and scales as the one-piece tiled A image of tpb200_nvfp4_gemm_ex (tpb200_nvfp4_tiled_a_bytes(M, K, 1)) */
+int tpb200_nvfp4_quantize_act_tiled(const void* x, int x_dtype, int ldx, void* image, int M, int K, tpb200_stream_t stream);
 int tpb200_nvfp4_gemm(const void* a_packed, int a_pitch, const void* a_sf, const void* b_packed, int b_pitch,
                       const void* b_sf, float alpha, const void* bias_f32, int activation, void* out,
                       int out_dtype, int ldo, int M, int N, int K, int flags, tpb200_stream_t stream);

@@ -162,3 +162,30 @@ def test_w4a8_forward_on_transposed_weights(cuda_device, M, N, K, shift):
     # exact products in bf16 x bf16, fp32 sums, one rounding to bf16
     assert bool(((out.cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all())
     assert lib.tpb200_device_error(0) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (129, 264, 272), (200, 1000, 1040), (712, 4096, 2048)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_w4a4_tiled_operands_equal_the_row_major_form(cuda_device, M, N, K, dtype):
+    from turbopi_b200 import _lib, ops
+    b, sf, _ = _nvfp4(N, K, cuda_device, M + N + K)
+    x = torch.randn((M, K), generator=torch.Generator().manual_seed(M)).to(dtype).to(cuda_device)
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(N)).to(cuda_device)
+    a, a_sf = ops.nvfp4_quantize_act(x)
+    want = ops.nvfp4_gemm(a, a_sf, b, sf, M, N, K, alpha=0.25, bias=bias, activation=_lib.ACT_GELU, out_dtype=torch.float32)
+    got = ops.nvfp4_linear_tiled(x, ops.tile_weights(b, sf, N, K), N, 0.25, bias, _lib.ACT_GELU, torch.float32)
+    # the same products; fp32 sums may associate differently
+    assert float((got - want).abs().max()) <= 2e-6 * float(want.abs().max())
+    assert _lib.load().tpb200_device_error(0) == 0
+
+
+@torch.no_grad()
+def test_nvfp4_linear_notices_weights_written_in_place(cuda_device):
+    from turbopi_b200.nvfp4_linear import NVFP4Linear
+    torch.manual_seed(3)
+    l1, l2 = (torch.nn.Linear(256, 25600, bias=False, device=cuda_device) for _ in range(2))
+    a, b = NVFP4Linear.from_linear(l1, use_mse_search=False), NVFP4Linear.from_linear(l2, use_mse_search=False)
+    x = torch.randn(8, 256, device=cuda_device).to(torch.bfloat16)
+    before, want = a(x), b(x)
+    a.load_state_dict(b.state_dict())
+    assert torch.equal(a(x), want) and not torch.equal(before, want)

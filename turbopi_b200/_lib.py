@@ -115,6 +115,7 @@ SIGNATURES = {
     "tpb200_measure_fp4_mma_rate": (c_int, [c_int, c_void_p]),
     "tpb200_nvfp4_tile_weights": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "tpb200_nvfp4_quantize_act": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]),
+    "tpb200_nvfp4_quantize_act_tiled": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p]),
     "tpb200_nvfp4_gemm": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int,
                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "tpb200_w4_gemm": (c_int, [ctypes.POINTER(W4GemmArgs), c_void_p]),

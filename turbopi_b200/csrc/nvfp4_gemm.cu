@@ -1088,13 +1088,22 @@ __device__ __forceinline__ uint32_t e2m1_index(float a) {
 
 __global__ void nvfp4_quantize_act_kernel(const void* __restrict__ x, int x_dtype, int ldx, uint8_t* __restrict__ packed,
                                           int pitch, uint8_t* __restrict__ sf, int M, int K, int rows_pad,
-                                          int kb_pad) {
+                                          int kb_pad, int tiled) {
+    pdl_launch_dependents();
     const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= static_cast<long long>(rows_pad) * kb_pad) return;
     const int row = static_cast<int>(t / kb_pad);
     const int kb = static_cast<int>(t % kb_pad);
-    const size_t sf_off = (static_cast<size_t>(row >> 7) * (kb_pad >> 2) + (kb >> 2)) * 512 + (row & 31) * 16 +
-                          ((row >> 5) & 3) * 4 + (kb & 3);
+    size_t sf_off = (static_cast<size_t>(row >> 7) * (kb_pad >> 2) + (kb >> 2)) * 512 + (row & 31) * 16 +
+                    ((row >> 5) & 3) * 4 + (kb & 3);
+    size_t code_off = static_cast<size_t>(row) * pitch + kb * 8;
+    if (tiled) {   // one-piece A image: blocks [row / 128][k / 256] of 128 swizzled code rows + 2 KB of scale atoms
+        const int rr = row & 127, jj = kb & 15;
+        const size_t blk = (static_cast<size_t>(row >> 7) * (kb_pad >> 4) + (kb >> 4)) * kBlock;
+        code_off = blk + rr * 128 + (((jj >> 1) ^ (rr & 7)) << 4) + (jj & 1) * 8;
+        sf_off = blk + kTile + (jj >> 2) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 + (jj & 3);
+        sf = packed;
+    }
     if (row >= M || kb * 16 >= K) {
         sf[sf_off] = 0;
         return;
@@ -1143,7 +1152,7 @@ __global__ void nvfp4_quantize_act_kernel(const void* __restrict__ x, int x_dtyp
         if (i < 8) lo |= code << (4 * i);
         else hi |= code << (4 * (i - 8));
     }
-    *reinterpret_cast<uint2*>(packed + static_cast<size_t>(row) * pitch + kb * 8) = make_uint2(lo, hi);
+    *reinterpret_cast<uint2*>(packed + code_off) = make_uint2(lo, hi);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1347,7 +1356,22 @@ extern "C" int tpb200_nvfp4_quantize_act(const void* x, int x_dtype, int ldx, vo
     tpb::nvfp4_quantize_act_kernel<<<static_cast<unsigned>((total + threads - 1) / threads), threads, 0,
                                      reinterpret_cast<cudaStream_t>(stream)>>>(
         x, x_dtype, ldx, static_cast<uint8_t*>(packed), packed_pitch, static_cast<uint8_t*>(sf_swizzled), M, K,
-        rows_pad, kb_pad);
+        rows_pad, kb_pad, 0);
+    return tpb_launch_status();
+}
+
+extern "C" int tpb200_nvfp4_quantize_act_tiled(const void* x, int x_dtype, int ldx, void* image, int M, int K,
+                                               tpb200_stream_t stream) {
+    TPB_REQUIRE(x && image, TPB200_ERR_NULL);
+    TPB_REQUIRE(M >= 1 && K >= 16 && K % 16 == 0 && ldx >= K, TPB200_ERR_SHAPE);
+    TPB_REQUIRE(tpb_valid_dtype(x_dtype), TPB200_ERR_ENUM);
+    TPB_REQUIRE(tpb_aligned16(x) && tpb_aligned16(image), TPB200_ERR_ALIGN);
+    TPB_REQUIRE((static_cast<long long>(ldx) * tpb_dtype_size(x_dtype)) % 16 == 0, TPB200_ERR_ALIGN);
+    const int rows_pad = (M + 127) / 128 * 128;
+    const int kb_pad = (K + 255) / 256 * 16;
+    const long long total = static_cast<long long>(rows_pad) * kb_pad;
+    tpb::nvfp4_quantize_act_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        x, x_dtype, ldx, static_cast<uint8_t*>(image), 0, nullptr, M, K, rows_pad, kb_pad, 1);
     return tpb_launch_status();
 }
 

@@ -18,6 +18,10 @@ from ._lib import ACT_GELU, ACT_NONE
 from .nvfp4_packed import NVFP4_MAX, NVFP4_VALUES, _nearest_index, pack_nvfp4
 
 BLOCK_SIZE = 32
+# 128 x 256 output tiles from which the tiled operand images are the faster form.  Measured with the quantiser, us row-major /
+# tiled: 384 tiles (712 x 16384 x 2048) 34.8 / 23.4, 128 (400 x 8192 x 8192) 44.9 / 29.2, 96 (712 x 4096 x 2048) 17.8 / 13.8,
+# 64 (64 x 16384 x 4096) 15.8 / 15.5, 48 (712 x 2048 x 16384) 56.8 / 56.6
+TILED_MIN_TILES = 80
 
 
 def _quantize_block_with_scale(block, scale, values):
@@ -134,14 +138,30 @@ class NVFP4Linear(nn.Module):
                 layer.bias.copy_(linear.bias)
         return layer.to(linear.weight.device)
 
+    def _tiles(self, M):
+        return (M + 127) // 128 * ((self.out_features + 255) // 256)
+
+    def _image(self):
+        """The weights as the GEMM's tiled image, made on first use and again when a buffer was replaced or written to."""
+        p, s = self.weight_packed, self.weight_scales_swizzled
+        key = (p.data_ptr(), p._version, s.data_ptr(), s._version)
+        st = self.__dict__.get("_tiled")
+        if st is None or st[0] != key:
+            st = self.__dict__["_tiled"] = (key, ops.tile_weights(p, s, self.out_features, self.in_features))
+        return st[1]
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         batch_shape = x.shape[:-1]
         x2 = x if x.dim() == 2 and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
         if x2.dtype not in (torch.float16, torch.bfloat16, torch.float32):
             x2 = x2.float()
         M = x2.shape[0]
-        a, a_sf = ops.nvfp4_quantize_act(x2)
         out_dtype = torch.bfloat16 if x.dtype == torch.bfloat16 else torch.float32
+        if self._tiles(M) >= TILED_MIN_TILES:
+            y = ops.nvfp4_linear_tiled(x2, self._image(), self.out_features, 1.0 / self.weight_scale_multiplier,
+                                       None if self.bias is None else self.bias.detach(), self.activation, out_dtype)
+            return y if x.dim() == 2 and y.dtype == x.dtype else y.reshape(*batch_shape, self.out_features).to(x.dtype)
+        a, a_sf = ops.nvfp4_quantize_act(x2)
         y = ops.nvfp4_gemm(a, a_sf, self.weight_packed, self.weight_scales_swizzled, M, self.out_features,
                            self.in_features, alpha=1.0 / self.weight_scale_multiplier,
                            bias=None if self.bias is None else self.bias.detach(), activation=self.activation,

@@ -311,6 +311,27 @@ def nvfp4_gemm(a_packed, a_sf, b_packed, b_sf, M, N, K, alpha=1.0, bias=None, ac
     return out
 
 
+def nvfp4_linear_tiled(x, b_image, N, alpha=1.0, bias=None, activation=ACT_NONE, out_dtype=torch.bfloat16):
+    """nvfp4_gemm(nvfp4_quantize_act(x), ...) on the tiled operand images: the same codes, scales and products in 128 x 256
+    output tiles (half the operand bytes per product).  b_image: tile_weights() of the weight operand."""
+    _cuda(x, b_image, bias)
+    M, K = x.shape
+    x = x.contiguous()
+    lib = _lib.load()
+    a = torch.empty(int(lib.tpb200_nvfp4_tiled_a_bytes(M, K, 1)), dtype=torch.uint8, device=x.device)
+    st = _run(x, lib.tpb200_nvfp4_quantize_act_tiled, _ptr(x), _dt(x), K, _ptr(a), M, K)
+    _lib.check(st, "tpb200_nvfp4_quantize_act_tiled")
+    out = torch.empty((M, N), dtype=out_dtype, device=x.device)
+    if bias is not None:
+        bias = bias.float().contiguous()
+    args = _lib.GemmArgs(a_packed=_ptr(a), a_pieces=1, b_packed=_ptr(b_image), alpha=float(alpha), bias=_ptr(bias),
+                         activation=int(activation), out=_ptr(out), out_dtype=_dt(out), ldo=N, M=M, N=N, K=K,
+                         layout=OPERANDS_TILED)
+    with launch_flags(FLAG_PDL):        # the weight image is complete: its blocks travel while the quantiser runs
+        _gemm_ex(args, x.device)
+    return out
+
+
 def nvfp4_quantize_act_pieces(x, pieces=3):
     """bf16/fp16/fp32 x [M, K] -> `pieces` residual e2m1 operands stacked along rows (piece p of row m at
     row p * piece_rows + m), their swizzled UE4M3 scales, and the per-row multiplier that undoes the
