@@ -11,8 +11,8 @@
 // Every problem is far too small to fill the machine with one CTA per 128 query rows running over all
 // keys (the action expert has 4 such tiles), so the keys are split too: CTA (row tile, key tile of 256,
 // group) computes S = Q K^T as two 128-key tiles side by side in tensor memory (2 x 16 MMAs of K = 16), the
-// softmax of its 128 x 256 block relative to the block's own row maxima (base-2 exponentials, 256 threads:
-// two per row), and O = P V (16 MMAs), and leaves O, the row maxima and the row sums in scratch; a second
+// softmax of its 128 x 256 block relative to the block's own row maxima (base-2 exponentials, 512 threads:
+// four per row), and O = P V (16 MMAs), and leaves O, the row maxima and the row sums in scratch; a second
 // small kernel combines the key tiles' partial results (the usual log-sum-exp merge).  With a single key
 // tile the first kernel writes the final rows itself.  (The key tiles of a row tile as one thread-block cluster that
 // merges through distributed shared memory, without the second kernel, was slower in a chain of launches: 15.7 against
@@ -42,7 +42,12 @@ constexpr int kRows = 128;              // query rows per CTA
 constexpr int kKeyTile = 128;           // keys per S tile (one MMA's N)
 constexpr int kKeysCta = 256;           // keys per CTA: two S tiles side by side in tensor memory
 constexpr int kChunkBytes = kRows * 128;   // one 64-column block of an operand
-constexpr int kThreadsAttn = 256;           // two warps per 32-lane quarter of tensor memory: each takes half the columns
+// Four warps per 32-lane quarter of tensor memory, each with a quarter of the columns: the softmax and the staging of O are
+// latencies in a row, and halving each thread's share against 256 threads took 5696
+// rows on 712 keys from 17.2 to 16.4 us, SigLIP from 8.7 to 8.2, 400 rows on 762 keys from 11.4 to 11.2.
+constexpr int kParts = 4;
+constexpr int kThreadsAttn = kParts * 128;
+constexpr int kPartCols = kKeyTile / kParts;    // columns of an S tile per thread
 constexpr float kMasked = -2.3819763e38f;   // the reference's additive mask value (pi0_pytorch.py:185-188)
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kFloor2 = -3.0e38f;         // lowest score in the base-2 domain (the mask value times log2 e overflows)
@@ -89,8 +94,8 @@ struct AttnControl {
     uint64_t bar_s, bar_v, bar_o;
     uint32_t tmem_base;
     float bias2[kKeysCta];
-    float half_max[2][kRows];                   // row maxima / row sums of the two column halves
-    float half_sum[2][kRows];
+    float part_max[kParts][kRows];              // row maxima / row sums of the column parts
+    float part_sum[kParts][kRows];
 };
 
 // Instruction descriptor for kind::f16 with bf16 operands and an fp32 accumulator, M = 128:
@@ -256,68 +261,65 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     }
 
     // ---------------------------------------------------------------- softmax of this block, P -> shared memory
-    // Thread (half, row): the row's scores in columns [64 * half, 64 * half + 64) of each S tile.
+    // Thread (part, row): the row's scores in columns [32 * part, 32 * part + 32) of each S tile.
     const int row = threadIdx.x & (kRows - 1);            // tensor-memory lane = query row of the tile
-    const int half = threadIdx.x >> 7;
+    const int part = threadIdx.x >> 7;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
     float m = kFloor2;
     float l = 0.0f;
     if (ok) {
-        // pass 1: the maximum over this thread's up to 128 scores (base-2 domain), all loads in flight at once
+        // pass 1: the maximum over this thread's up to 64 scores (base-2 domain)
         for (int t = 0; t < nt; ++t) {
-            uint32_t r[2][32];
-#pragma unroll
-            for (int c = 0; c < 2; ++c) tc::tmem_ld_32x32b_x32(lane_addr + kColS + t * kKeyTile + half * 64 + c * 32, r[c]);
+            uint32_t r[kPartCols];
+            tc::tmem_ld_32x32b_x32(lane_addr + kColS + t * kKeyTile + part * kPartCols, r);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    m = fmaxf(m, fmaf(__uint_as_float(r[c][j]), P.scale2, ctl->bias2[t * kKeyTile + half * 64 + c * 32 + j]));
-                }
+            for (int j = 0; j < kPartCols; ++j) {
+                m = fmaxf(m, fmaf(__uint_as_float(r[j]), P.scale2, ctl->bias2[t * kKeyTile + part * kPartCols + j]));
             }
         }
-        ctl->half_max[half][row] = m;
+        ctl->part_max[part][row] = m;
     }
     __syncthreads();
     if (ok) {
-        m = fmaxf(m, ctl->half_max[half ^ 1][row]);
+#pragma unroll
+        for (int p = 0; p < kParts; ++p) m = fmaxf(m, ctl->part_max[p][row]);
         // pass 2: p = 2^(t - m) rounded to bf16 (what the PyTorch path feeds its second matmul), row sum of the
         // rounded values, 16-byte stores into the K-major image of P
         uint8_t* sP = sQ;
         for (int t = 0; t < nt; ++t) {
-            uint32_t r[2][32];
-#pragma unroll
-            for (int c = 0; c < 2; ++c) tc::tmem_ld_32x32b_x32(lane_addr + kColS + t * kKeyTile + half * 64 + c * 32, r[c]);
+            uint32_t r[kPartCols];
+            tc::tmem_ld_32x32b_x32(lane_addr + kColS + t * kKeyTile + part * kPartCols, r);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int j8 = 0; j8 < kPartCols / 8; ++j8) {
+                uint32_t w[4];
 #pragma unroll
-                for (int j8 = 0; j8 < 4; ++j8) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int j2 = 0; j2 < 4; ++j2) {
-                        const int j = j8 * 8 + j2 * 2;
-                        const float* b2 = &ctl->bias2[t * kKeyTile + half * 64 + c * 32 + j];
-                        const float x0 = fmaf(__uint_as_float(r[c][j]), P.scale2, b2[0]) - m;
-                        const float x1 = fmaf(__uint_as_float(r[c][j + 1]), P.scale2, b2[1]) - m;
-                        const __nv_bfloat162 pb = __floats2bfloat162_rn(ex2(x0), ex2(x1));
-                        l += __bfloat162float(pb.x) + __bfloat162float(pb.y);
-                        w[j2] = *reinterpret_cast<const uint32_t*>(&pb);
-                    }
-                    const int ch = t * 16 + half * 8 + c * 4 + j8;   // 16-byte chunk of the 256-key row: 0..31
-                    uint8_t* dst = sP + (ch >> 3) * kChunkBytes + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
-                    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+                for (int j2 = 0; j2 < 4; ++j2) {
+                    const int j = j8 * 8 + j2 * 2;
+                    const float* b2 = &ctl->bias2[t * kKeyTile + part * kPartCols + j];
+                    const float x0 = fmaf(__uint_as_float(r[j]), P.scale2, b2[0]) - m;
+                    const float x1 = fmaf(__uint_as_float(r[j + 1]), P.scale2, b2[1]) - m;
+                    const __nv_bfloat162 pb = __floats2bfloat162_rn(ex2(x0), ex2(x1));
+                    l += __bfloat162float(pb.x) + __bfloat162float(pb.y);
+                    w[j2] = *reinterpret_cast<const uint32_t*>(&pb);
                 }
+                const int ch = t * 16 + part * (kPartCols / 8) + j8;   // 16-byte chunk of the 256-key row: 0..31
+                uint8_t* dst = sP + (ch >> 3) * kChunkBytes + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
+                *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
             }
         }
-        ctl->half_sum[half][row] = l;
+        ctl->part_sum[part][row] = l;
     }
     fence_proxy_async_smem();
     tc::fence_before_thread_sync();
     __syncthreads();
     tc::fence_after_thread_sync();
-    if (ok) l += ctl->half_sum[half ^ 1][row];
+    if (ok) {                                             // in part order, the same sum in every thread of the row
+        l = 0.0f;
+#pragma unroll
+        for (int p = 0; p < kParts; ++p) l += ctl->part_sum[p][row];
+    }
 
     // ---------------------------------------------------------------- O = P V
     if (warp == 0 && ok) {
@@ -363,13 +365,13 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     if (ok) {
         __nv_bfloat16* o = P.out + ga * P.o_stride[0] + gb * P.o_stride[1] + static_cast<size_t>(store ? grow : 0) * P.ldo;
         uint8_t* srow = sKV + static_cast<size_t>(row) * P.dvp * 4;
-        if (!final_rows && store && half == 0) {
+        if (!final_rows && store && part == 0) {
             float* pml = P.part_ml + (tile * kRows + row) * 2;
             pml[0] = m;
             pml[1] = l;
         }
         const float inv = 1.0f / l;
-        for (int c64 = half * 64; c64 < P.dv; c64 += 128) {   // the halves take alternate 64-column batches
+        for (int c64 = part * 64; c64 < P.dv; c64 += kParts * 64) {   // the parts take alternate 64-column batches
             // up to four 16-column loads in flight, one wait
             uint32_t r4[4][16];
 #pragma unroll
@@ -417,12 +419,12 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
         }
     }
     if (!final_rows && ok) {
-        // the two warps of a lane quarter (one per column half) have staged its 32 rows: they leave as one bulk copy, rows
+        // the four warps of a lane quarter (one per column part) have staged its 32 rows: they leave as one bulk copy, rows
         // past the end of the matrix left out.  Shared memory only has to outlive the copy's READS; the next kernel's
         // wait covers the writes.
         fence_proxy_async_smem();
         const int q = warp & 3;
-        asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "n"(kParts * 32) : "memory");
         const int rows = min(32, P.n_rows - rt * kRows - 32 * q);
         if (warp < 4 && rows > 0 && tc::elect_one()) {
             const size_t off = static_cast<size_t>(32 * q) * P.dvp;
