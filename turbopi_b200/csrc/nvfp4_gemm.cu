@@ -44,6 +44,8 @@ constexpr int kTile = 128 * kBKBytes;    // 16 KB operand tile
 constexpr int kSfSlab = 4 * 512;         // 4 K-atoms of one 128-row tile
 constexpr int kOutBuf = 128 * 128;       // one staged output box: 128 rows x 128 bytes
 constexpr int kThreads = 320;           // warps: 0 producer, 1 MMA issuer, 2..5 and 6..9 two epilogue groups
+constexpr int kMaxThreads = kThreads + 64;   // tiled form with several pieces: the last two warps produce pieces 1 and 2
+constexpr int kMaxChunks = 3;           // tiled form: B + piece 0, piece 1, piece 2
 constexpr int kTmemCols = 512;
 // tensor memory: columns [0, 256) hold two 128-column accumulators (row-major form) or one of 256
 // columns (tiled form); then the B scales (4 columns per K atom and 128 rows) and 16 columns per A piece
@@ -108,8 +110,8 @@ constexpr int kCounterSlots = 2048;
 enum { kEpiPlain = 0, kEpiQkvRope = 1 };
 
 struct SharedControl {
-    uint64_t full[kMaxStages];
-    uint64_t empty[kMaxStages];
+    uint64_t full[kMaxStages][kMaxChunks];    // row-major form: one chunk per stage
+    uint64_t empty[kMaxStages][kMaxChunks];
     alignas(16) float bias_s[2][128];  // the bias of the columns each epilogue group is working on
     uint64_t acc_full[2];
     uint64_t acc_empty[2];
@@ -252,7 +254,7 @@ __device__ __forceinline__ unsigned long long tl_now() {
 #endif
 
 template <bool kTiled>
-__global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_constant__ GemmParams P) {
+__global__ void __launch_bounds__(kMaxThreads, 1) nvfp4_gemm_kernel(const __grid_constant__ GemmParams P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int kBN = tile_n(kTiled);
@@ -278,12 +280,15 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
     // 128-byte boxes): the MMA thread waits for that drain before every tile, the accumulator being single.
     // The split-K hand-over and the fused QKV epilogue stay on group 0.
     const bool two_groups = P.epilogue == kEpiPlain && splits == 1;
+    const int piece_warp0 = kTiled && pieces > 1 ? static_cast<int>(blockDim.x >> 5) - 2 : 1 << 20;
 
     if (threadIdx.x == 0) {
         TL(0);
         for (int s = 0; s < kMaxStages; ++s) {
-            mbar_init(&ctl->full[s], 1);
-            mbar_init(&ctl->empty[s], 1);
+            for (int c = 0; c < kMaxChunks; ++c) {
+                mbar_init(&ctl->full[s][c], 1);
+                mbar_init(&ctl->empty[s][c], 1);
+            }
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&ctl->acc_full[b], 1);
@@ -337,12 +342,12 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
                 const int ks1 = min(P.k_stages, ks0 + P.stages_per_split);
                 const int n_blk = tile / P.m_blocks;
                 for (int ks = ks0; ks < ks1 && pre < nstages; ++ks, ++pre) {
-                    if (lane == 0) mbar_expect_tx(&ctl->full[pre], stage_sz);
+                    if (lane == 0) mbar_expect_tx(&ctl->full[pre][0], 3 * kBlock);
                     __syncwarp();
                     if (lane < 2) {
                         bulk_copy_g2s_hint(smem + pre * stage_sz + lane * kBlock,
                                            P.b_image + (static_cast<size_t>(n_blk) * P.k_stages + ks) * (2 * kBlock) + lane * kBlock,
-                                           kBlock, &ctl->full[pre], weights_policy);
+                                           kBlock, &ctl->full[pre][0], weights_policy);
                     }
                 }
             }
@@ -363,12 +368,12 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
                         bad = 1;
                     } else if (it < pre) {
                         // barrier already armed, B half already on its way
-                    } else if (wrapped && !mbar_wait_bounded(&ctl->empty[s], empty_phase)) {
+                    } else if (wrapped && !mbar_wait_bounded(&ctl->empty[s][0], empty_phase)) {
                         record_error(kErrGemmEmptyBarrierTimeout);
                         *abort_flag = 1;
                         bad = 1;
                     } else {
-                        mbar_expect_tx(&ctl->full[s], stage_sz);
+                        mbar_expect_tx(&ctl->full[s][0], kTiled ? 3 * kBlock : stage_sz);
                     }
                 }
                 bad = __shfl_sync(0xffffffffu, bad, 0);
@@ -378,30 +383,35 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
                 }
                 uint8_t* st = smem + s * stage_sz;
                 if (kTiled) {
-                    if (lane < 2 + pieces && (lane >= 2 || it >= pre)) {
-                        const uint8_t* src =
-                            lane < 2 ? P.b_image + (static_cast<size_t>(n_blk) * P.k_stages + ks) * (2 * kBlock) + lane * kBlock
-                                     : P.a_image + (static_cast<size_t>(m_blk) * P.k_stages + ks) * (pieces * kBlock) +
-                                           (lane - 2) * kBlock;
-                        if (lane < 2) bulk_copy_g2s_hint(st + lane * kBlock, src, kBlock, &ctl->full[s], weights_policy);
-                        else bulk_copy_g2s(st + lane * kBlock, src, kBlock, &ctl->full[s]);
+                    // chunk 0: the B block and piece 0 (codes, scale slab); the other pieces have producers of their own
+                    const uint8_t* a_blk = P.a_image + (static_cast<size_t>(m_blk) * P.k_stages + ks) * (pieces * kBlock);
+                    if (lane < 2) {
+                        if (it >= pre) {
+                            bulk_copy_g2s_hint(st + lane * kBlock,
+                                               P.b_image + (static_cast<size_t>(n_blk) * P.k_stages + ks) * (2 * kBlock) + lane * kBlock,
+                                               kBlock, &ctl->full[s][0], weights_policy);
+                        }
+                    } else if (lane == 2) {
+                        bulk_copy_g2s(st + off_a, a_blk, kTile, &ctl->full[s][0]);
+                    } else if (lane == 3) {
+                        bulk_copy_g2s(st + off_sfa, a_blk + pieces * kTile, kSfSlab, &ctl->full[s][0]);
                     }
                 } else if (lane == 0) {
-                    tc::tma_load_2d(st, &P.map_b, ks * kBKBytes, n_blk * kBN, &ctl->full[s]);
+                    tc::tma_load_2d(st, &P.map_b, ks * kBKBytes, n_blk * kBN, &ctl->full[s][0]);
                 } else if (lane == 1) {
                     bulk_copy_g2s(st + off_sfb,
                                   P.sfb + static_cast<size_t>(n_blk) * sf_row_stride + static_cast<size_t>(ks) * kSfSlab,
-                                  kSfSlab, &ctl->full[s]);
+                                  kSfSlab, &ctl->full[s][0]);
                 } else if (lane < 2 + 2 * pieces) {
                     const int p = (lane - 2) >> 1;
                     const int a_row_tile = p * (P.a_piece_rows >> 7) + m_blk;
                     if ((lane & 1) == 0) {
-                        tc::tma_load_2d(st + off_a + p * kTile, &P.map_a, ks * kBKBytes, a_row_tile * kBM, &ctl->full[s]);
+                        tc::tma_load_2d(st + off_a + p * kTile, &P.map_a, ks * kBKBytes, a_row_tile * kBM, &ctl->full[s][0]);
                     } else {
                         bulk_copy_g2s(st + off_sfa + p * kSfSlab,
                                       P.sfa + static_cast<size_t>(a_row_tile) * sf_row_stride +
                                           static_cast<size_t>(ks) * kSfSlab,
-                                      kSfSlab, &ctl->full[s]);
+                                      kSfSlab, &ctl->full[s][0]);
                     }
                 }
                 if (++s == nstages) {
@@ -411,6 +421,41 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
                 }
             }
             if (lane == 0 && w == blockIdx.x) TL(3);
+        }
+    } else if (warp >= piece_warp0) {
+        // ------------------------------------------------------------ producer of activation piece p (tiled form).
+        // A piece's room is free again as soon as ITS MMAs are done and its copy only has to land before its own turn a
+        // ring later: with one barrier for the whole 90 KB stage the refill of a two-stage ring began with the last
+        // piece and was waited for by the first (712 x 2048 x 16384 36.3 us, now 35.0; 712 x 32768 x 2048 61.5 and 60.7: what is
+        // left is the rate at which L2 feeds the SMs, 90 KB per stage and SM at 10 TB/s in all).
+        const int p = warp - piece_warp0 + 1;
+        int s = 0;
+        uint32_t phase = 0;
+        bool wrapped = false, stop = p >= pieces;
+        for (int w = blockIdx.x; w < total_items && !stop; w += gridDim.x) {
+            const int tile = w / splits;
+            const int ks0 = (w - tile * splits) * P.stages_per_split;
+            const int ks1 = min(P.k_stages, ks0 + P.stages_per_split);
+            const uint8_t* a_blk = P.a_image + (static_cast<size_t>(tile % P.m_blocks) * P.k_stages + ks0) * (pieces * kBlock);
+            for (int ks = ks0; ks < ks1; ++ks, a_blk += pieces * kBlock) {
+                if (__any_sync(0xffffffffu, *abort_flag != 0) ||
+                    (wrapped && !__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->empty[s][p], phase)))) {
+                    if (lane == 0 && *abort_flag == 0) record_error(kErrGemmEmptyBarrierTimeout);
+                    *abort_flag = 1;
+                    stop = true;
+                    break;
+                }
+                uint8_t* st = smem + s * stage_sz;
+                if (lane == 0) mbar_expect_tx(&ctl->full[s][p], kBlock);
+                __syncwarp();
+                if (lane == 0) bulk_copy_g2s(st + off_a + p * kTile, a_blk + p * kTile, kTile, &ctl->full[s][p]);
+                if (lane == 1) bulk_copy_g2s(st + off_sfa + p * kSfSlab, a_blk + pieces * kTile + p * kSfSlab, kSfSlab, &ctl->full[s][p]);
+                if (++s == nstages) {
+                    s = 0;
+                    phase ^= wrapped ? 1u : 0u;
+                    wrapped = true;
+                }
+            }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -447,32 +492,32 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
                 const uint32_t tmem_acc = tm + buf * 128;
                 uint32_t accumulate = 0;           // the first MMA of the item overwrites the accumulator
                 for (int ks = ks0; ks < ks1; ++ks) {
-                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], full_phase))) {
-                        if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
-                        *abort_flag = 1;
-                        break;
-                    }
-                    tc::fence_after_thread_sync();
-                    if (tile_iter == 0 && ks == ks0 && lane == 0) TL(4);
-                    if (tc::elect_one()) {
-                        // B scales of K atom a sit in kSubTiles * 4 consecutive columns (4 per 128 rows)
+                    uint32_t lo_a = lo0 + off_a16;             // piece p's code tile
+                    uint32_t lo_sfa = lo0 + off_sfa16;         // piece p's scale slab
+                    uint32_t t_sfa_p = t_sfa;
+                    bool landed = true;
+                    for (int p = 0; p < pieces; ++p) {
+                        // tiled form: chunk p (with p = 0: and the B block); row-major form: the whole stage at once
+                        if (kTiled || p == 0) landed = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s][p], full_phase));
+                        if (!landed) break;
+                        tc::fence_after_thread_sync();
+                        if (tile_iter == 0 && ks == ks0 && p == 0 && lane == 0) TL(4);
+                        if (tc::elect_one()) {
+                            if (p == 0) {
+                                // B scales of K atom a sit in kSubTiles * 4 consecutive columns (4 per 128 rows)
 #pragma unroll
-                        for (int a = 0; a < 4; ++a) {
+                                for (int a = 0; a < 4; ++a) {
 #pragma unroll
-                            for (int h = 0; h < kSubTiles; ++h) {
-                                tc::cp_sf_32x128b(t_sfb + 4 * (kSubTiles * a + h),
-                                                  tc::desc_from_words(lo0 + off_sfb16 + ((h * kSfSlab + a * 512) >> 4),
-                                                                      tc::kDescHiSfAtom));
+                                    for (int h = 0; h < kSubTiles; ++h) {
+                                        tc::cp_sf_32x128b(t_sfb + 4 * (kSubTiles * a + h),
+                                                          tc::desc_from_words(lo0 + off_sfb16 + ((h * kSfSlab + a * 512) >> 4),
+                                                                              tc::kDescHiSfAtom));
+                                    }
+                                }
                             }
-                        }
-                        uint32_t lo_a = lo0 + off_a16;         // piece p's code tile
-                        uint32_t lo_sfa = lo0 + off_sfa16;     // piece p's scale slab
-                        uint32_t t_sfa_p = t_sfa;
-                        for (int p = 0; p < pieces; ++p) {
 #pragma unroll
                             for (int a = 0; a < 4; ++a) {
-                                tc::cp_sf_32x128b(t_sfa_p + 4 * a,
-                                                  tc::desc_from_words(lo_sfa + ((a * 512) >> 4), tc::kDescHiSfAtom));
+                                tc::cp_sf_32x128b(t_sfa_p + 4 * a, tc::desc_from_words(lo_sfa + ((a * 512) >> 4), tc::kDescHiSfAtom));
                             }
 #pragma unroll
                             for (int a = 0; a < 4; ++a) {
@@ -480,13 +525,20 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemm_kernel(const __grid_co
                                                  tc::desc_from_words(lo0 + ((a * 32) >> 4), tc::kDescHiKmajorSw128), idesc,
                                                  t_sfa_p + 4 * a, t_sfb + 4 * kSubTiles * a, (accumulate | p | a) ? 1u : 0u);
                             }
-                            lo_a += kTile >> 4;
-                            lo_sfa += kSfSlab >> 4;
-                            t_sfa_p += 16;
+                            // a chunk may be refilled once its MMAs have read it; chunk 0 holds B, which all of them read
+                            if (kTiled && p > 0) tc::commit(&ctl->empty[s][p]);
+                            if (p == pieces - 1) tc::commit(&ctl->empty[s][0]);
                         }
-                        tc::commit(&ctl->empty[s]);   // stage s may be refilled once these MMAs have read it
+                        __syncwarp();
+                        lo_a += kTile >> 4;
+                        lo_sfa += kSfSlab >> 4;
+                        t_sfa_p += 16;
                     }
-                    __syncwarp();
+                    if (!landed) {
+                        if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
+                        *abort_flag = 1;
+                        break;
+                    }
                     accumulate = 1;
                     if (++s == nstages) {
                         s = 0;
@@ -1558,7 +1610,7 @@ extern "C" int tpb200_nvfp4_gemm_ex(const tpb200_nvfp4_gemm_args* a, tpb200_stre
     cfg.gridDim = dim3(grid, 1, 1);
     // the second epilogue group (warps 6..9) only has work in unsplit launches with the plain epilogue
     const bool two_groups = P.epilogue == tpb::kEpiPlain && P.splits == 1;
-    cfg.blockDim = dim3(two_groups ? tpb::kThreads : tpb::kThreads - 128, 1, 1);
+    cfg.blockDim = dim3((two_groups ? tpb::kThreads : tpb::kThreads - 128) + (tiled && pieces > 1 ? 64 : 0), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = reinterpret_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[2];
