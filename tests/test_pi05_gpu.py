@@ -97,6 +97,24 @@ def test_reduced_pi05_matches_oracle(cuda_device, steps):
     assert cosine(graphed.numpy(), ref.numpy()) >= 0.999
 
 
+@torch.no_grad()
+def test_expert_mlp_that_has_no_gated_epilogue(cuda_device):
+    """expert_mlp % 64 != 0: gate and up leave as two halves and the row kernel multiplies them."""
+    from turbopi_b200 import _lib
+    from turbopi_b200.pi05 import Pi05, Pi05Config
+    cfg = Pi05Config(image_size=56, patch=14, vision_layers=1, vision_width=128, vision_mlp=272, vision_heads=2,
+                     prefix_layers=2, width=256, mlp=512, text_len=24, vocab=1000, expert_layers=2, expert_width=128,
+                     expert_mlp=272, action_horizon=50, action_dim=32, max_seq=256)
+    model = Pi05(cfg, cuda_device, seed=1, keep_raw=True)
+    g = torch.Generator().manual_seed(2)
+    images = torch.randint(0, 256, (2, 56, 56, 3), generator=g, dtype=torch.uint8)
+    tokens, noise = torch.randint(0, 1000, (24,), generator=g), torch.randn(50, 32, generator=g)
+    out = model.infer(images, tokens, noise, num_steps=2).cpu()
+    assert _lib.load().tpb200_device_error(0) == 0
+    ref, _ = opi.sample_actions(_extract(model), images, tokens, noise, 2, _ocfg(cfg), model.cos.float().cpu(), model.sin.float().cpu())
+    assert (out - ref).abs().max().item() <= 2e-2            # as test_reduced_pi05_matches_oracle
+
+
 def _ocfg(cfg):
     return dict(image_size=cfg.image_size, patch=cfg.patch, vision_width=cfg.vision_width, vision_heads=cfg.vision_heads,
                 eps=cfg.eps, width=cfg.width, q_dim=cfg.q_dim, head_dim=cfg.head_dim, heads=cfg.heads,

@@ -112,6 +112,10 @@ def test_int4(cuda_device, M, N, K, plugin):
     xd, wd = x.to(cuda_device), w.double().to(cuda_device)
     y = ops.w4_gemm(xd, *args, out_dtype=torch.float32)
     _check(y, xd.double() @ wd.t(), xd.double().abs() @ wd.abs().t(), 2.0 ** -22)
+    if not plugin:                                                                        # scales that TMA cannot fetch
+        odd = torch.empty(args[3].numel() + 1, dtype=torch.float16, device=cuda_device)[1:].view(args[3].shape)
+        assert odd.copy_(args[3]).data_ptr() % 16 == 2
+        assert torch.equal(ops.w4_gemm(xd, *args[:3], odd, out_dtype=torch.float32), y)
     assert _lib.load().tpb200_device_error(0) == 0
 
 
