@@ -193,3 +193,50 @@ def test_nvfp4_linear_notices_weights_written_in_place(cuda_device):
     before, want = a(x), b(x)
     a.load_state_dict(b.state_dict())
     assert torch.equal(a(x), want) and not torch.equal(before, want)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("T", [1, 8, 40])
+def test_packed_mlp_notices_weights_loaded_in_place(cuda_device, T):
+    from types import SimpleNamespace
+    from turbopi_b200.nvfp4_packed import NVFP4PackedMLP
+    torch.manual_seed(5)
+    mods = []
+    for _ in range(2):
+        p = {n: torch.nn.Linear(*s, bias=False, device=cuda_device) for n, s in (("gate_proj", (128, 256)), ("up_proj", (128, 256)), ("down_proj", (256, 128)))}
+        mods.append(NVFP4PackedMLP.from_gemma_mlp(SimpleNamespace(**p), gate_activation="gelu", fmt="nvfp4"))
+    a, b = mods
+    x = torch.randn(T, 128, device=cuda_device).to(torch.bfloat16)
+    before, want = a(x), b(x)
+    for la, lb in ((a.gate_proj, b.gate_proj), (a.up_proj, b.up_proj), (a.down_proj, b.down_proj)):
+        la.weight_packed.copy_(lb.weight_packed)
+        la.weight_scales.copy_(lb.weight_scales)
+        la.global_scale = lb.global_scale
+    assert torch.equal(a(x), want) and not torch.equal(before, want)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("features", [256, 25600])           # either side of the rule on output tiles
+def test_nvfp4_linear_reads_the_weights_it_has_now(cuda_device, features):
+    """A module built in inference mode; a first call that is captured."""
+    from turbopi_b200.nvfp4_linear import TILED_MIN_TILES, NVFP4Linear
+    torch.manual_seed(4)
+    l1, l2 = (torch.nn.Linear(256, features, bias=False, device=cuda_device) for _ in range(2))
+    a, b = NVFP4Linear.from_linear(l1, use_mse_search=False), NVFP4Linear.from_linear(l2, use_mse_search=False)
+    assert (a._tiles(8) >= TILED_MIN_TILES) == (features == 25600)
+    x = torch.randn(8, 256, device=cuda_device).to(torch.bfloat16)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = a(x)
+    want = b(x)
+    # the forms may sum in another order (fp32), then each rounds to bf16
+    tol = 2e-6 * float(want.abs().max())
+    for name, buf in a.named_buffers():
+        buf.copy_(dict(b.named_buffers())[name])
+    assert torch.equal(a(x), want)
+    with torch.inference_mode():
+        c = NVFP4Linear.from_linear(l2, use_mse_search=False)
+        assert torch.allclose(c(x).float(), want.float(), rtol=2.0 ** -7, atol=tol)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.allclose(y.float(), want.float(), rtol=2.0 ** -7, atol=tol)

@@ -142,11 +142,16 @@ class NVFP4Linear(nn.Module):
         return (M + 127) // 128 * ((self.out_features + 255) // 256)
 
     def _image(self):
-        """The weights as the GEMM's tiled image, made on first use and again when a buffer was replaced or written to."""
+        """The weights as the GEMM's tiled image, made on first use and again when a buffer was replaced or written to.  None
+        where writes are not counted (inference tensors) and where making it would be captured."""
         p, s = self.weight_packed, self.weight_scales_swizzled
+        if p.is_inference() or s.is_inference():
+            return None
         key = (p.data_ptr(), p._version, s.data_ptr(), s._version)
         st = self.__dict__.get("_tiled")
         if st is None or st[0] != key:
+            if torch.cuda.is_current_stream_capturing():
+                return None
             st = self.__dict__["_tiled"] = (key, ops.tile_weights(p, s, self.out_features, self.in_features))
         return st[1]
 
@@ -157,8 +162,9 @@ class NVFP4Linear(nn.Module):
             x2 = x2.float()
         M = x2.shape[0]
         out_dtype = torch.bfloat16 if x.dtype == torch.bfloat16 else torch.float32
-        if self._tiles(M) >= TILED_MIN_TILES:
-            y = ops.nvfp4_linear_tiled(x2, self._image(), self.out_features, 1.0 / self.weight_scale_multiplier,
+        image = self._image() if self._tiles(M) >= TILED_MIN_TILES else None
+        if image is not None:
+            y = ops.nvfp4_linear_tiled(x2, image, self.out_features, 1.0 / self.weight_scale_multiplier,
                                        None if self.bias is None else self.bias.detach(), self.activation, out_dtype)
             return y if x.dim() == 2 and y.dtype == x.dtype else y.reshape(*batch_shape, self.out_features).to(x.dtype)
         a, a_sf = ops.nvfp4_quantize_act(x2)

@@ -96,6 +96,11 @@ def _operand_buffer(module, T, K, device):
     return q
 
 
+def _state_of(*tensors):
+    """What changes when a weight buffer is replaced or written to in place (inference tensors count no versions)."""
+    return tuple((t.data_ptr(), t.get_device(), 0 if t.is_inference() else t._version) for t in tensors)
+
+
 def _dense_is_faster(T, N, K, gated=False):
     """Whether [N, K] weights on the tiled image take T tokens faster through the GEMM that dequantises them (bf16
     activations as they are) than through the GEMV behind a quantiser (up to 16 tokens) or the e2m1-piece GEMM behind one:
@@ -127,10 +132,11 @@ class NVFP4PackedLinear(nn.Module):
     "nvfp4").  forward() accepts any leading shape and dispatches on the token count:
 
       "nvfp4" weights   <= 4 tokens: the CUDA-core GEMV on the packed rows as stored; 5..16 tokens: one
-                        tensor-core GEMV launch behind a quantiser launch; more tokens: the tcgen05
-                        block-scaled GEMM on the tiled weight image (bf16 activations as three residual
-                        e2m1 pieces).  The tiled image is built once, on the first forward that needs it,
-                        and serves both tensor-core kernels.
+                        tensor-core GEMV launch behind a quantiser launch; more tokens, up to a size limit
+                        (`_dense_is_faster`): the GEMM that dequantises its weights, activations in bf16;
+                        beyond it the tcgen05 block-scaled GEMM (bf16 activations as three residual e2m1
+                        pieces).  The tiled weight image is built once, on the first forward that needs it,
+                        and serves all three tensor-core kernels.
       "ref" weights     fp32 scales per 32 are not an operand format of the block-scaled tensor cores:
                         rows go through the CUDA-core GEMV 16 at a time, exactly as stored.
 
@@ -182,9 +188,8 @@ class NVFP4PackedLinear(nn.Module):
 
     def _tc_state(self):
         """(tiled weight image, GEMV scratch), built on first use and whenever the packed
-        weights were replaced (load_state_dict, .to(device))."""
-        packed = self.weight_packed
-        key = (packed.data_ptr(), self.weight_scales.data_ptr(), packed.get_device())
+        weights were replaced or written to (load_state_dict, .to(device))."""
+        key = _state_of(self.weight_packed, self.weight_scales)
         st = self.__dict__.get("_tc")
         if st is None or st[0] != key:
             N, K = self.out_features, self.in_features
@@ -295,7 +300,7 @@ class NVFP4PackedMLP(nn.Module):
         """Tiled image of [W_gate; W_up] under ONE global scale, or None if the projections do not share one
         (each was quantised on its own: the stacked launch needs a common fp32 multiplier)."""
         g, u = self.gate_proj, self.up_proj
-        key = (g.weight_packed.data_ptr(), u.weight_packed.data_ptr())
+        key = _state_of(g.weight_packed, u.weight_packed, g.weight_scales, u.weight_scales)
         st = self.__dict__.get("_gu")
         if st is None or st[0] != key:
             if g.global_scale != u.global_scale:
