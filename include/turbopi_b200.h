@@ -102,8 +102,7 @@ int tpb200_w4a16_gemv(const void* x, int x_dtype, const void* weight_packed, con
                       int N, int K, int group_size, int layout, int flags, tpb200_stream_t stream);
 
 /* W4A16 GEMM for more than 16 tokens on the tensor cores: INT4 weights are dequantised to bf16 on their way
- * into shared memory (once per CTA and K stage, shared by up to 384 token rows) and multiplied by tcgen05.mma
- * kind::f16; fp32 accumulation.  out = alpha * x @ dequant(W)^T + bias + beta * out.
+ * into tensor memory (once per 256 tokens) and multiplied by tcgen05.mma kind::f16; fp32 accumulation.  out = alpha * x @ dequant(W)^T + bias + beta * out.
  *   layout TPB200_INT4_PLUGIN: w = q * scale + zero, the operands of w4a16GemmForward
  *          (openpi/w4a16_plugin/src/w4a16_gemm_kernel.cu:54-153,336-406 is the reference's mixed-input GEMM);
  *   layout TPB200_INT4_KBLOCK: W4A16Linear's buffers, w = (q - 8) * scale (fp16, per 32; `zeros` must be NULL),
@@ -420,7 +419,8 @@ size_t getW4A16GemmWorkspaceSize(int M, int N, int K);
 
 /* openpi/w4a8_plugin/src/w4a8_gemm_plugin.h:39-73: out bf16 [M,N] = alpha * (fp8 act * act scale) @ (e2m1 * w scale),
  * weights and their scales stored transposed ([K/2, N], [K/16, N]); N % 8 == 0; the workspace (size from
- * getW4A8GemmWorkspaceSize) holds the re-laid-out operands.  bf16 -> E4M3 values + E4M3 scale per 16 along K;
+ * getW4A8GemmWorkspaceSize) holds the activations in bf16 and, where the weights cannot be read as they are (N % 16 != 0
+ * or an unaligned base), their re-laid-out copy.  bf16 -> E4M3 values + E4M3 scale per 16 along K;
  * bf16 [N, K] weight -> e2m1 packed TRANSPOSED [K/2, N] + E4M3 scales [K/16, N]. */
 void w4a8GemmForward(const void* activation_fp8, const void* activation_scale, const void* weight_packed,
                      const void* weight_scale, void* output_bf16, int M, int N, int K, float alpha, void* workspace,

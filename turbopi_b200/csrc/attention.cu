@@ -28,8 +28,8 @@
 //                                         MN-major B operand (the 128-byte direction is head_dim = N, the rows
 //                                         are keys = K): no transposed copy of V.
 // Loads are TMA tile copies through 4-dimensional tensor maps (head_dim, rows, groups; zero fill past the end
-// of a matrix), issued by one thread; the partial O of a CTA is staged where V was and leaves as one bulk
-// copy.  Nothing here waits on another CTA; every wait is bounded and reports through the device error word.
+// of a matrix), issued by one thread; the partial O of a CTA is staged where V was and leaves as four bulk
+// copies, each as soon as its 32 rows are staged.  Nothing here waits on another CTA; every wait is bounded and reports through the device error word.
 #include <algorithm>
 #include <atomic>
 
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     // The tensor-memory loads are warp-collective: every lane executes them, rows past the end of the matrix
     // only skip the stores.  With a single key tile the rows are final (bf16, normalised); otherwise the
     // unnormalised fp32 rows are staged in shared memory where V was (chunk c of row r at c ^ (r & 7), so the
-    // stores of a quarter warp spread over all banks) and leave as ONE bulk copy, image and all.
+    // stores of a quarter warp spread over all banks) and leave as bulk copies, image and all.
     const int grow = rt * kRows + row;
     const bool store = grow < P.n_rows;
     const bool final_rows = P.key_tiles == 1 && P.qa_image == nullptr;

@@ -474,8 +474,8 @@ __global__ void __launch_bounds__(kThreads, 1) nvfp4_gemv_tc_kernel(const __grid
         }
     } else if (warp == 6) {
         // ------------------------------------------------------------ scale copier.
-        // One thread issues every tcgen05 instruction it is given at ~60 cycles apiece; with the 12 scale
-        // copies of a stage on the MMA thread that thread, not the weight stream, set the pace.  Here they
+        // A thread issued every tcgen05 instruction at ~60 cycles apiece (~25 with warp-uniform control flow); with the 12
+        // scale copies of a stage on the MMA thread that thread, not the weight stream, set the pace.  Here they
         // run one stage ahead into the other set of scale columns.  The copies do not depend on the tile, so
         // this lane only needs the number of stages of each unit.
         {

@@ -9,12 +9,14 @@
 // One persistent CTA per SM, warp-specialised:
 //   warp 0     TMA producer: per 256-wide K stage one 128B-swizzled box of B (128 rows), one per
 //              A piece, and their 2 KB scale slabs (plain bulk copies), ring of 2..5 stages;
-//   warp 1     allocates tensor memory; one lane copies the stage's scale atoms shared->tensor
+//   warp 1     allocates tensor memory; one elected lane copies the stage's scale atoms shared->tensor
 //              memory (tcgen05.cp) and issues 4 tcgen05.mma kind::mxf4nvf4 (K = 64 each) per piece
 //              into one of two 128x128 fp32 accumulators, committing the stage back to the producer;
-//   warps 2-5  epilogue: tcgen05.ld, alpha / row scale / bias / activation (or rotary embedding for
-//              the fused QKV form), conversion, 128B-swizzled staging in shared memory and TMA
-//              tile stores (full-line writes, clipped at the matrix edge by the tensor map).
+//   warps 2-5  (and 6-9, unsplit launches with the plain epilogue) epilogue: tcgen05.ld, alpha / row
+//              scale / bias / activation (or rotary embedding for the fused QKV form), conversion,
+//              128B-swizzled staging in shared memory and TMA tile stores (full-line writes, clipped at
+//              the matrix edge by the tensor map);
+//   last two   tiled form with several pieces: producers of pieces 1 and 2, each with its own barriers.
 // One CTA per SM, no clusters: no operand is shared between CTAs; every wait is bounded and reports
 // through the device error word.
 //
@@ -26,7 +28,7 @@
 // tiles of 128 x 256 outputs.  An SM takes in roughly 0.3 us per copy request whatever its size (the
 // measured rate grows from ~25 GB/s with 8 KB requests to ~100 GB/s with 32 KB+), and this kernel is
 // bound by exactly that intake, so the tiled form both halves the bytes per flop (B shared by twice
-// the columns) and moves them in requests of 36-54 KB instead of 2-16 KB.
+// the columns) and moves them in requests of 16-18 KB a lane.
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
@@ -1364,8 +1366,8 @@ SplitPlan plan_splits(int tiles, int k_stages, int pieces, bool tiled, int sms, 
     SplitPlan best{1, k_stages, 0};
     if (2 * tiles > sms || tiles > kCounterSlots || k_stages < 2) return best;
     const size_t item_bytes = static_cast<size_t>(128) * tile_n(tiled) * 4;   // one partial accumulator
-    // Device timestamps of this kernel (three pieces, tiled): a stage takes 1.4 us (two stages of 90 KB in
-    // flight per SM); a split launch adds parking the sums (1.8 us for 50 valid rows, 3.4 for 128), the wait for
+    // Device timestamps of this kernel (three pieces, tiled): a stage took 1.4 us with one barrier per stage (two stages of
+    // 90 KB in flight per SM; the costs only have to rank the splits); a split launch adds parking the sums (1.8 us for 50 valid rows, 3.4 for 128), the wait for
     // the slowest partner (1-1.5 us) and the slice pass (1.7 / 4.4 us) where an unsplit tile has a 2 us epilogue.
     const float t_stage = stage_bytes(pieces, tiled) / 1024.0f / (tiled ? 64.0f : 70.0f);
     const float t_split = 1.0f + 0.05f * static_cast<float>(std::min(rows, 128));

@@ -17,15 +17,15 @@
 // memory, summed in rank order (deterministic; no workspace, no counters, no waiting on other clusters).
 //
 // What bounds it: four 128 x NT x 16 MMAs with A in tensor memory take exactly 2 NT cycles (measured, NT 32..256), the
-// dequantisation of their 128 x 64 weights ~320 ALU cycles of an SM, and the token tiles are re-read once per 128 weight
-// rows (8-9 TB/s from L2 at 712 x 16384 x 2048).  B200, in a chain of programmatic dependent launches: INT4
-// 712 x 16384 x 2048 49 us (975 TFLOP/s; 85 us with weights dequantised through shared memory), 397 x 2048 x 16384 33 us
-// with four K ranges (265 us without split K).  Pairs of CTAs sharing the token tile (cta_group::2) halve those reads
+// dequantisation of their 128 x 64 weights 470-530 cycles of an SM with 16 warps, and the token tiles are re-read once per
+// 128 weight rows (434 MB through the L2 at 712 x 16384 x 2048).  B200, in a chain of programmatic dependent launches: INT4
+// 712 x 16384 x 2048 49 us (85 us with weights dequantised through shared memory), 397 x 2048 x 16384 33 us
+// with K split (265 us without).  Pairs of CTAs sharing the token tile (cta_group::2) halve those reads
 // but were slower (147 against 103 us at 712 x 32768 x 2048): the barrier round trips between the two SMs sit on the
 // issuing warp's path.
 //
-// Roles (352 threads): warp 0 activation tiles (TMA), warp 1 tensor memory + MMA issue, warps 2..9 dequantisation
-// and epilogue, warp 10 weight blocks (256 K values of 128 rows: 16 KB of codes + scales).  Weight blocks are
+// Roles: warp 0 activation tiles (TMA), warp 1 tensor memory + MMA issue, warp 2 weight blocks (256 K values of 128 rows:
+// 16 KB of codes + scales), then 16 warps (8 where two CTAs share an SM) of dequantisation and epilogue.  Weight blocks are
 // requested and dequantised BEFORE griddepcontrol.wait: under programmatic dependent launch a launch's weights are
 // already in tensor memory when its predecessor's activations arrive.  Every wait is bounded.
 #include <algorithm>
@@ -642,8 +642,8 @@ __global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_plugin_gemm_kernel(c
 
 // ---------------------------------------------------------------- launch plan
 // Tokens per tile, K ranges per tile, and whether two CTAs share an SM (8 dequantising warps each) or one has it
-// to itself (16 warps).  Measured (B200, us per launch; 50 tokens, K = 1024 / 2048 / 1024 / 4096): qkv 5.4, o 5.3, gate_up
-// 6.2, down 6.8, where the e2m1-piece GEMM takes 7.8, 7.9, 8.5 and 8.8 behind a quantiser.
+// to itself (16 warps).  Measured (B200, us per launch; 50 tokens, K = 1024 / 2048 / 1024 / 4096): qkv 4.5, o 4.9, gate_up
+// 5.7, down 6.0, where the e2m1-piece GEMM takes 7.8, 7.9, 8.5 and 8.8 behind a quantiser.
 struct W4gPlan { int nt, splits; bool half; };
 
 W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {

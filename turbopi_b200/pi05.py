@@ -84,8 +84,8 @@ class TcLinear:
     the tiled image (`sf is None`; 128 x 256 output tiles, one contiguous block per K stage: the form for the
     large prefix MLP matrices), or
     row-major codes [N, pitch] + swizzled scale atoms.  A call with a `QuantBuf` (in the weight's form) runs the
-    block-scaled GEMM; `dense` / `dense_qkv` take bf16 activations and dequantise the weights inside the kernel.  `raw` keeps the reference-layout codes / scale bytes for
-    dequantisation in tests."""
+    block-scaled GEMM; `dense` / `dense_qkv` take bf16 activations and dequantise the weights inside the kernel.
+    `raw` keeps the reference-layout codes / scale bytes for dequantisation in tests."""
 
     def __init__(self, image, g, N, K, bias=None, raw=None, sf=None):
         self.b, self.sf, self.g, self.N, self.K = image, sf, float(g), int(N), int(K)
@@ -258,7 +258,7 @@ class Pi05:
         EX = "paligemma_with_expert.gemma_expert.model."
 
         # Operand form per linear: the tiled image for the large prefix MLP matrices (gate_up, down: 712 x 32768 x 2048 in
-        # 71 us + 27 us of row kernel against 114 us on the dequantising GEMM, 712 x 2048 x 16384 in 40 against 49), row-major
+        # 61 us + 28 us of row kernel against 107 us on the dequantising GEMM, 712 x 2048 x 16384 in 35 against 47), row-major
         # for everything else (the vision tower, the attention projections, the action expert, the small projections).
         def lin(wname, bias=True, perm=None, rm=True):
             return TcLinear.from_weight(get(wname + ".weight"), get(wname + ".bias") if bias else None, perm, kr, rm)
