@@ -253,6 +253,13 @@ typedef struct {
     int flags;
 } tpb200_w4_gemm_args;
 int tpb200_w4_gemm(const tpb200_w4_gemm_args* args, tpb200_stream_t stream);
+/* What a launch of that shape looks like on a GPU of `sms` SMs (host only, no device needed): tokens per tile, K ranges
+ * per tile, CTAs per SM, groups of four dequantising warps, 64-K parts per step, slots of the weight and of the step ring,
+ * 256-K blocks and 64-K parts of the whole K. */
+typedef struct {
+    int tokens_per_tile, splits, ctas_per_sm, groups, parts, weight_slots, step_slots, k_blocks, k_steps;
+} tpb200_w4_gemm_plan_info;
+int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_plan_info* info);
 
 /* ---------------------------------------------------------------------------------------------
  * NVFP4 weight-only GEMV for decode shapes (M <= 16) on the tensor cores: same result as

@@ -234,7 +234,8 @@ def test_ctypes_structures_follow_the_header_field_by_field():
     mirrors = {"tpb200_gemv_problem": _lib.GemvProblem, "tpb200_nvfp4_gemm_args": _lib.GemmArgs,
                "tpb200_gemv_tc_problem": _lib.GemvTcProblem, "tpb200_gemv_tc_fused_problem": _lib.GemvTcFusedProblem,
                "tpb200_gemv_tc_plan_info": _lib.GemvTcPlanInfo, "tpb200_attention_args": _lib.AttentionArgs,
-               "tpb200_rowop_args": _lib.RowOpArgs, "tpb200_w4_gemm_args": _lib.W4GemmArgs}
+               "tpb200_rowop_args": _lib.RowOpArgs, "tpb200_w4_gemm_args": _lib.W4GemmArgs,
+               "tpb200_w4_gemm_plan_info": _lib.W4GemmPlanInfo}
     for name, mirror in mirrors.items():
         m = re.search(r"typedef struct(?:\s+\w+)?\s*\{([^}]*)\}\s*" + name + r"\s*;", header, re.S)
         assert m, name

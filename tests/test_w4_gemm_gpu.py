@@ -119,6 +119,100 @@ def test_int4(cuda_device, M, N, K, plugin):
     assert _lib.load().tpb200_device_error(0) == 0
 
 
+def _ring_wraps(M, N, K):
+    """Whether the launch has narrow token tiles, an SM per CTA and more weight blocks than ring slots."""
+    import ctypes
+    from turbopi_b200 import _lib
+    p = _lib.W4GemmPlanInfo()
+    assert _lib.load().tpb200_w4_gemm_plan(M, N, K, 148, ctypes.byref(p)) == 0
+    return p.parts == 2 and p.groups == 4 and -(-p.k_blocks // p.splits) > p.weight_slots
+
+
+def _repeat_cold(call, y, device):
+    """The same bits again under programmatic dependent launch, with the operands out of L2 and in it."""
+    from turbopi_b200 import _lib, ops
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device=device)
+    for _ in range(4):
+        flush.zero_()
+        with ops.launch_flags(ops.FLAG_PDL):
+            ys = [call() for _ in range(3)]
+        assert all(torch.equal(v, y) for v in ys)
+    assert _lib.load().tpb200_device_error(0) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 2048, 16384), (17, 2048, 16384), (50, 2048, 16384), (64, 2048, 16384), (17, 16384, 2048),
+                                   (64, 16384, 2048), (50, 8192, 1280), (512, 1152, 4304)])
+def test_few_tokens_and_a_long_k(cuda_device, M, N, K):
+    """K ranges of more 256-K blocks than the weight ring holds, with each group of warps on every second block."""
+    from turbopi_b200 import _lib, ops
+    assert _ring_wraps(M, N, K)
+    b, sf, w = _nvfp4(N, K, cuda_device, M + N + K)
+    x = torch.randn((M, K), generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(cuda_device)
+    ref, mag = x.double() @ w.t(), x.double().abs() @ w.abs().t()
+    for weight in ((ops.tile_weights(b, sf, N, K), N, _lib.W4_NVFP4_TILED), (b, N, _lib.W4_NVFP4_ROWMAJOR, sf)):
+        call = lambda: ops.w4_gemm(x, *weight, alpha=0.25, out_dtype=torch.float32)      # noqa: E731
+        y = call()
+        _check(y, 0.25 * ref, mag, 2.0 ** -22)
+        _repeat_cold(call, y, cuda_device)
+
+
+@pytest.mark.parametrize("M,I,K", [(1, 8192, 2048), (50, 8192, 2048), (64, 1024, 8192)])
+def test_gated_few_tokens_and_a_long_k(cuda_device, M, I, K):
+    from turbopi_b200 import _lib, ops
+    assert _ring_wraps(M, 2 * I, K)
+    b, sf, w = _nvfp4(2 * I, K, cuda_device, M + I + K)
+    x = torch.randn((M, K), generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(cuda_device)
+    gu = x.double() @ w.t()
+    a = 1.0 / float(gu.std())
+    image = ops.tile_weights(b, sf, 2 * I, K)
+    call = lambda: ops.w4_gemm(x, image, 2 * I, _lib.W4_NVFP4_TILED, alpha=a, activation=_lib.ACT_GELU, gated=True)   # noqa: E731
+    y = call()
+    r16 = lambda v: v.to(torch.bfloat16).double()      # noqa: E731
+    gate, up = r16(a * gu[:, :I]), r16(a * gu[:, I:])
+    ref = r16(torch.nn.functional.gelu(gate, approximate="tanh")) * up
+    # gate may round to its neighbour, 2^-8 of it, which GELU passes on with a slope of at most 1.13; up, the activation and
+    # the product round likewise; the fp32 sums of K terms are off by 2e-6 * mag before all that
+    mag = a * (x.double().abs() @ w.abs().t())
+    tol = 2.0 ** -8 * (1.13 * (gate * up).abs() + 3 * ref.abs()) + 2e-6 * 1.13 * (mag[:, :I] * up.abs() + mag[:, I:] * gate.abs())
+    assert bool(((y.double() - ref).abs() <= tol + 1e-6).all())
+    _repeat_cold(call, y, cuda_device)
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 2048, 16384), (64, 2048, 16384), (17, 16384, 2048), (64, 16384, 2048)])
+@pytest.mark.parametrize("plugin", [False, True])
+def test_int4_few_tokens_and_a_long_k(cuda_device, M, N, K, plugin):
+    from turbopi_b200 import ops
+    assert _ring_wraps(M, N, K)
+    xd, args, wd = _int4(M, N, K, plugin, cuda_device)
+    call = lambda: ops.w4_gemm(xd, *args, out_dtype=torch.float32)      # noqa: E731
+    y = call()
+    _check(y, xd.double() @ wd.t(), xd.double().abs() @ wd.abs().t(), 2.0 ** -22)
+    _repeat_cold(call, y, cuda_device)
+
+
+def _int4(M, N, K, plugin, device):
+    """(bf16 activations, operands of w4_gemm, dequantised float64 weights)"""
+    from turbopi_b200 import _lib
+    from turbopi_b200.w4a16 import _codes_to_words
+    g = torch.Generator().manual_seed(M + N + K)
+    codes = torch.randint(0, 16, (N, K), generator=g, dtype=torch.uint8)
+    x = torch.randn((M, K), generator=g).to(torch.bfloat16)
+    q = codes.double() - 8
+    words = _codes_to_words(codes)
+    if plugin:
+        sc = (torch.rand((N, K // 128), generator=g) * 0.1).to(torch.bfloat16)
+        zp = (torch.randn((N, K // 128), generator=g) * 0.1).to(torch.bfloat16)
+        w = (q * sc.double().repeat_interleave(128, 1) + zp.double().repeat_interleave(128, 1)).float().to(torch.bfloat16)
+        packed = (words.view(torch.uint8).reshape(N, K // 2) ^ 0x88).to(device)               # two's-complement nibbles
+        args = (packed, N, _lib.W4_INT4_PLUGIN, sc.to(device), zp.to(device))
+    else:
+        sc = (torch.rand((N, K // 32), generator=g) * 0.1).half()
+        w = (q * sc.double().repeat_interleave(32, 1)).float().to(torch.bfloat16)             # exact in fp32, one rounding
+        packed = words.reshape(N, K // 32, 4).permute(1, 0, 2).contiguous().to(device)
+        args = (packed, N, _lib.W4_INT4_KBLOCK, sc.t().contiguous().to(device))
+    return x.to(device), args, w.double().to(device)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 512), (1, 72, 1024), (2, 136, 8192), (5, 1000, 4096), (1, 2048, 16384), (16, 8, 2080),
                                    (3, 61, 1056)])
 def test_kblock_gemv_with_k_cut_over_a_cluster(cuda_device, M, N, K):

@@ -53,6 +53,11 @@ class W4GemmArgs(ctypes.Structure):
                 ("qkv_positions", c_void_p), ("qkv_rope_cos", c_void_p), ("qkv_rope_sin", c_void_p), ("flags", c_int)]
 
 
+class W4GemmPlanInfo(ctypes.Structure):
+    _fields_ = [(n, c_int) for n in ("tokens_per_tile", "splits", "ctas_per_sm", "groups", "parts", "weight_slots", "step_slots",
+                                     "k_blocks", "k_steps")]
+
+
 class GemvTcProblem(ctypes.Structure):
     _fields_ = [("w_image", c_void_p), ("x_image", c_void_p),
                 ("x_row_scale", c_void_p), ("bias", c_void_p), ("out", c_void_p),
@@ -118,6 +123,7 @@ SIGNATURES = {
     "tpb200_nvfp4_quantize_act_tiled": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p]),
     "tpb200_nvfp4_gemm": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int,
                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "tpb200_w4_gemm_plan": (c_int, [c_int, c_int, c_int, c_int, ctypes.POINTER(W4GemmPlanInfo)]),
     "tpb200_w4_gemm": (c_int, [ctypes.POINTER(W4GemmArgs), c_void_p]),
     "tpb200_nvfp4_gemm_ex": (c_int, [ctypes.POINTER(GemmArgs), c_void_p]),
     "tpb200_nvfp4_quantize_act_pieces": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,

@@ -679,6 +679,35 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
     return best;
 }
 
+// Ring depths.  Up to 128 tokens: half an SM's shared and tensor memory, so that two CTAs (of this launch or of the
+// next one in the stream) share an SM; more tokens: one CTA per SM.
+struct W4gRing { int groups, parts, n_w, n_s, tmem_cols, a_col; };
+
+W4gRing ring_of(const W4gPlan& plan, int k_blocks, int k_steps) {
+    W4gRing r;
+    r.groups = kDqWarpsPerSm / 4 / (plan.half ? 2 : 1);
+    r.tmem_cols = plan.half ? 256 : 512;
+    r.a_col = (plan.nt + 31) / 32 * 32;
+    // Two 64-K parts per step for narrow token tiles: a step costs the issuing warp ~280 cycles of waiting and issuing
+    // whatever its size, more than the MMAs of one part (2 NT cycles)
+    r.parts = plan.nt <= 64 ? 2 : 1;
+    const int blocks_per = (k_blocks + plan.splits - 1) / plan.splits, steps_per = std::min(blocks_per * 4, k_steps);
+    const int budget = (plan.half ? 112 : 225) * 1024 - 1024;
+    // A group takes every `stride`-th weight block.  A parity wait tells a phase from the one before it only, so a group
+    // must have waited for EVERY earlier block of a slot it comes to: with more blocks than slots, the number of slots is
+    // a multiple of the stride.  (Three slots under a stride of two: a group could take a block's codes out of a slot that
+    // was still receiving the block before, and hand the slot back in another group's place.)
+    const int stride = std::max(1, r.groups * r.parts / 4);
+    const int slots = stride == 2 ? 4 : plan.half && plan.nt > 64 ? 2 : 3;
+    static_assert(kMaxW >= 4, "two blocks ahead for each half of the groups");
+    r.n_w = std::min(slots, blocks_per);
+    // Operand steps: a group's wait for the MMAs of its previous step covers every slot's last but one use as long as there
+    // are at least as many slots as groups (5 for 256 tokens, the fewest), or no slot is used twice.
+    r.n_s = std::min(std::min(kMaxS, (r.tmem_cols - r.a_col) / (32 * r.parts)),
+                     std::min((steps_per + r.parts - 1) / r.parts, (budget - r.n_w * kWSlot) / (plan.nt * 128 * r.parts)));
+    return r;
+}
+
 }  // namespace
 
 int device_error_w4_gemm(int clear) { return read_device_error(clear); }
@@ -776,21 +805,13 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     P.rope_cos = static_cast<const __nv_bfloat16*>(a->qkv_rope_cos);
     P.rope_sin = static_cast<const __nv_bfloat16*>(a->qkv_rope_sin);
 
-    // Ring depths.  Up to 128 tokens: half an SM's shared and tensor memory, so that two CTAs (of this launch or of the
-    // next one in the stream) share an SM; more tokens: one CTA per SM.
-    const bool half = plan.half;
-    P.tmem_cols = half ? 256 : 512;
-    P.a_col = (P.nt + 31) / 32 * 32;
-    const int blocks_per = (P.k_blocks + P.splits - 1) / P.splits, steps_per = std::min(blocks_per * 4, P.k_steps);
-    const int budget = (half ? 112 : 225) * 1024 - 1024;
-    const int b_bytes = P.nt * 128;
-    // Two 64-K parts per step for narrow token tiles: a step costs the issuing warp ~280 cycles of waiting and issuing
-    // whatever its size, more than the MMAs of one part (2 NT cycles)
-    P.parts = P.nt <= 64 ? 2 : 1;
-    P.n_w = std::min(half ? (P.nt <= 64 ? 3 : 2) : 3, blocks_per);
-    P.n_s = std::min(std::min(kMaxS, (P.tmem_cols - P.a_col) / (32 * P.parts)),
-                     std::min((steps_per + P.parts - 1) / P.parts, (budget - P.n_w * kWSlot) / (b_bytes * P.parts)));
-    int smem = P.n_w * kWSlot + P.n_s * b_bytes * P.parts;
+    const W4gRing ring = ring_of(plan, P.k_blocks, P.k_steps);
+    P.tmem_cols = ring.tmem_cols;
+    P.a_col = ring.a_col;
+    P.parts = ring.parts;
+    P.n_w = ring.n_w;
+    P.n_s = ring.n_s;
+    int smem = P.n_w * kWSlot + P.n_s * P.nt * 128 * P.parts;
     smem = std::max(smem, P.nt * kRows * 4) + 1024;
 
     static void (*const kernels[4])(const W4gParams) = {w4_nvfp4_gemm_kernel, w4_int4_kblock_gemm_kernel,
@@ -806,7 +827,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles * P.splits, (M + P.nt - 1) / P.nt, 1);
-    cfg.blockDim = dim3((kDqWarp0 + kDqWarpsPerSm / (half ? 2 : 1)) * 32, 1, 1);
+    cfg.blockDim = dim3((kDqWarp0 + 4 * ring.groups) * 32, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -832,6 +853,16 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
 
 extern "C" int tpb200_w4_gemm(const tpb200_w4_gemm_args* a, tpb200_stream_t stream) {
     return tpb::w4_gemm_launch(a, reinterpret_cast<cudaStream_t>(stream), false);
+}
+
+extern "C" int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_plan_info* info) {
+    TPB_REQUIRE(info != nullptr, TPB200_ERR_NULL);
+    TPB_REQUIRE(M >= 1 && M <= 65535 * 256 && N >= 8 && K >= 16 && sms >= 1, TPB200_ERR_SHAPE);
+    const int k_blocks = (K + tpb::kBlkK - 1) / tpb::kBlkK, k_steps = (K + tpb::kPartK - 1) / tpb::kPartK;
+    const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms);
+    const tpb::W4gRing r = tpb::ring_of(plan, k_blocks, k_steps);
+    *info = {plan.nt, plan.splits, plan.half ? 2 : 1, r.groups, r.parts, r.n_w, r.n_s, k_blocks, k_steps};
+    return TPB200_OK;
 }
 
 extern "C" int tpb200_w4a16_gemm(const void* x, const void* weight, const void* scales, const void* zeros,
