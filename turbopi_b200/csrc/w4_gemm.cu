@@ -446,6 +446,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                     if (!ok) break;
                     tc::fence_after_thread_sync();
                 }
+                __syncwarp();                                        // lane 0 may be behind: it has arrived on w_empty
                 tmem_st_32x32b_x32(lane_addr + P.a_col + (sa * parts + u) * 32, out);
             }
             if (!ok) {
