@@ -203,14 +203,15 @@ typedef struct {
      * at chunk c ^ (r & 7), then the 2048-byte scale slabs (4 atoms) of rows 0..127 and 128..255.  A image
      * (tpb200_row_transform_quantize with TPB200_OPERANDS_TILED writes it): blocks [ceil(M/128)][ceil(K/256)]
      * of a_pieces * 18432 bytes = one 128-row code tile per piece in the same chunk pattern, then one scale
-     * slab per piece; a_pieces <= 3.  Padding rows / K must hold zero scales. */
+     * slab per piece; a_pieces <= 3.  Padding rows / K must hold zero scales.  TPB200_OPERANDS_TILED_A: a_packed is the A
+     * image, b_packed / b_pitch / b_sf the row-major operand, read as it is at the launch; the same 128 x 256 tiles. */
     int layout;
     /* TPB200_FLAG_PDL: launch with programmatic stream serialisation.  The kernel sets itself up (barriers,
      * tensor memory) while the previous kernel of the stream is still running and waits for it before it
      * reads an operand or writes a result. */
     int flags;
 } tpb200_nvfp4_gemm_args;
-enum { TPB200_OPERANDS_ROWMAJOR = 0, TPB200_OPERANDS_TILED = 1 };
+enum { TPB200_OPERANDS_ROWMAJOR = 0, TPB200_OPERANDS_TILED = 1, TPB200_OPERANDS_TILED_A = 2 };
 size_t tpb200_nvfp4_gemm_workspace_size(int M, int N, int K, int a_pieces, int layout);
 size_t tpb200_nvfp4_tiled_a_bytes(int M, int K, int pieces);
 size_t tpb200_nvfp4_tiled_b_bytes(int N, int K);

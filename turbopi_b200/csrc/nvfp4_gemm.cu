@@ -73,7 +73,7 @@ struct alignas(64) GemmParams {
     const uint8_t* sfa;
     const uint8_t* sfb;
     const uint8_t* a_image;    // tiled form: blocks [m_blk][ks] of pieces * 18 KB
-    const uint8_t* b_image;    // tiled form: blocks [n_blk][ks] of 36 KB
+    const uint8_t* b_image;    // tiled B: blocks [n_blk][ks] of 36 KB
     const float* bias;
     int M, N, K;
     int out_dtype;
@@ -128,6 +128,29 @@ __device__ __forceinline__ float gelu_tanh_fast(float x) {
     return __fdividef(x, 1.0f + __expf(-z2));
 }
 __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+
+// Tiled form: the 256 rows of B that K stage `ks` of column tile `n_blk` needs, [codes of 256 rows][their two scale slabs],
+// from the tiled image or from row-major codes and scale atoms (one 256-row box in the same swizzle; rows past N arrive as
+// zeros, their scales are the last row tile's).  `full` counts 2 * kBlock bytes either way.  With the quantiser in a chain of
+// launches, image / row-major, us (B200): 712 x 16384 x 2048 23.3 / 23.8 (24.2 with two 128-row boxes), 400 x 8192 x 8192 29.0 /
+// 29.7, 712 x 4096 x 2048 13.6 / 13.9; rows that do not start on 128 bytes 1000 x 12000 x 3008 32.1 / 33.5.
+template <bool kBRows>
+__device__ __forceinline__ void request_b_block(const GemmParams& P, uint8_t* st, int n_blk, int ks, uint64_t* full, uint64_t policy,
+                                                int lane) {
+    if (!kBRows) {
+        if (lane < 2) {
+            bulk_copy_g2s_hint(st + lane * kBlock,
+                               P.b_image + (static_cast<size_t>(n_blk) * P.k_stages + ks) * (2 * kBlock) + lane * kBlock, kBlock,
+                               full, policy);
+        }
+    } else if (lane == 0) {
+        tc::tma_load_2d(st, &P.map_b, ks * kBKBytes, n_blk * 256, full);
+    } else if (lane < 3) {
+        const int row_tile = min(2 * n_blk + lane - 1, (P.N + 127) / 128 - 1);
+        bulk_copy_g2s(st + 2 * kTile + (lane - 1) * kSfSlab,
+                      P.sfb + (static_cast<size_t>(row_tile) * P.k_stages + ks) * kSfSlab, kSfSlab, full);
+    }
+}
 
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
@@ -255,7 +278,9 @@ __device__ __forceinline__ unsigned long long tl_now() {
 #define TL(point) ((void)0)
 #endif
 
-template <bool kTiled>
+// kBRows: B in its row-major form (always without kTiled).  A form of its own: asking at run time whose requests to make took
+// 0.7 us of the 145 of a 712-token MLP on images.
+template <bool kTiled, bool kBRows>
 __global__ void __launch_bounds__(kMaxThreads, 1) nvfp4_gemm_kernel(const __grid_constant__ GemmParams P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -322,10 +347,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1) nvfp4_gemm_kernel(const __grid
         // Lane 0 owns the barrier hand-shakes; the stage's copy requests are issued by DIFFERENT lanes.  A
         // thread that issues a bulk copy is held for ~0.3 us whatever the size, so one lane issuing a stage's
         // requests back to back tops out near 60-90 GB/s per SM; the same requests issued side by side from
-        // several lanes reach ~130 GB/s.  Tiled form: the stage is (2 + pieces) chunks of 18 KB, one per lane
-        // (two from the B block, the rest from the contiguous A block).  Row-major form: one lane per box.
-        if (!kTiled && lane == 0) {
-            tc::prefetch_tensormap(&P.map_a);
+        // several lanes reach ~130 GB/s.  Tiled form: the B block (two chunks of 18 KB, or a box and two slabs) and
+        // piece 0 of A (codes and slab); pieces 1 and 2 have producers of their own.  Row-major form: one lane per box.
+        if (kBRows && lane == 0) {
+            if (!kTiled) tc::prefetch_tensormap(&P.map_a);
             tc::prefetch_tensormap(&P.map_b);
         }
         const int sf_row_stride = P.k_stages * kSfSlab;   // bytes per 128-row tile of scales
@@ -346,11 +371,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) nvfp4_gemm_kernel(const __grid
                 for (int ks = ks0; ks < ks1 && pre < nstages; ++ks, ++pre) {
                     if (lane == 0) mbar_expect_tx(&ctl->full[pre][0], 3 * kBlock);
                     __syncwarp();
-                    if (lane < 2) {
-                        bulk_copy_g2s_hint(smem + pre * stage_sz + lane * kBlock,
-                                           P.b_image + (static_cast<size_t>(n_blk) * P.k_stages + ks) * (2 * kBlock) + lane * kBlock,
-                                           kBlock, &ctl->full[pre][0], weights_policy);
-                    }
+                    request_b_block<kBRows>(P, smem + pre * stage_sz, n_blk, ks, &ctl->full[pre][0], weights_policy, lane);
                 }
             }
         }
@@ -387,15 +408,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1) nvfp4_gemm_kernel(const __grid
                 if (kTiled) {
                     // chunk 0: the B block and piece 0 (codes, scale slab); the other pieces have producers of their own
                     const uint8_t* a_blk = P.a_image + (static_cast<size_t>(m_blk) * P.k_stages + ks) * (pieces * kBlock);
-                    if (lane < 2) {
-                        if (it >= pre) {
-                            bulk_copy_g2s_hint(st + lane * kBlock,
-                                               P.b_image + (static_cast<size_t>(n_blk) * P.k_stages + ks) * (2 * kBlock) + lane * kBlock,
-                                               kBlock, &ctl->full[s][0], weights_policy);
-                        }
-                    } else if (lane == 2) {
+                    constexpr int kBLanes = kBRows ? 3 : 2;
+                    if (lane < kBLanes) {
+                        if (it >= pre) request_b_block<kBRows>(P, st, n_blk, ks, &ctl->full[s][0], weights_policy, lane);
+                    } else if (lane == kBLanes) {
                         bulk_copy_g2s(st + off_a, a_blk, kTile, &ctl->full[s][0]);
-                    } else if (lane == 3) {
+                    } else if (lane == kBLanes + 1) {
                         bulk_copy_g2s(st + off_sfa, a_blk + pieces * kTile, kSfSlab, &ctl->full[s][0]);
                     }
                 } else if (lane == 0) {
@@ -1476,7 +1494,7 @@ extern "C" int tpb200_nvfp4_tile_weights(const void* packed, int pitch, const vo
 
 extern "C" size_t tpb200_nvfp4_gemm_workspace_size(int M, int N, int K, int a_pieces, int layout) {
     if (M < 1 || N < 1 || K < 16) return 0;
-    const bool tiled = layout == TPB200_OPERANDS_TILED;
+    const bool tiled = layout != TPB200_OPERANDS_ROWMAJOR;
     const int bn = tpb::tile_n(tiled);
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1490,8 +1508,9 @@ extern "C" size_t tpb200_nvfp4_gemm_workspace_size(int M, int N, int K, int a_pi
 extern "C" int tpb200_nvfp4_gemm_ex(const tpb200_nvfp4_gemm_args* a, tpb200_stream_t stream) {
     TPB_REQUIRE(a != nullptr, TPB200_ERR_NULL);
     const int M = a->M, N = a->N, K = a->K;
-    TPB_REQUIRE(a->layout == TPB200_OPERANDS_ROWMAJOR || a->layout == TPB200_OPERANDS_TILED, TPB200_ERR_ENUM);
-    const bool tiled = a->layout == TPB200_OPERANDS_TILED;
+    TPB_REQUIRE(a->layout >= TPB200_OPERANDS_ROWMAJOR && a->layout <= TPB200_OPERANDS_TILED_A, TPB200_ERR_ENUM);
+    const bool tiled = a->layout != TPB200_OPERANDS_ROWMAJOR;           // tiles of 128 x 256, A as its tiled image
+    const bool b_rows = a->layout != TPB200_OPERANDS_TILED;             // B as row-major codes + scale atoms
     TPB_REQUIRE(a->a_packed && a->b_packed, TPB200_ERR_NULL);
     TPB_REQUIRE(M >= 1 && N >= 8 && N % 8 == 0 && K >= 16 && K % 16 == 0, TPB200_ERR_SHAPE);
     TPB_REQUIRE(a->activation >= TPB200_ACT_NONE && a->activation <= TPB200_ACT_GEGLU, TPB200_ERR_ENUM);
@@ -1503,13 +1522,15 @@ extern "C" int tpb200_nvfp4_gemm_ex(const tpb200_nvfp4_gemm_args* a, tpb200_stre
     const int n_out = geglu ? N / 2 : N;
     const int pieces = a->a_pieces <= 0 ? 1 : a->a_pieces;
     TPB_REQUIRE(tpb_aligned16(a->a_packed) && tpb_aligned16(a->b_packed), TPB200_ERR_ALIGN);
+    if (b_rows) {
+        TPB_REQUIRE(a->b_sf, TPB200_ERR_NULL);
+        TPB_REQUIRE(a->b_pitch >= K / 2 && a->b_pitch % 16 == 0 && tpb_aligned16(a->b_sf), TPB200_ERR_ALIGN);
+    }
     if (tiled) {
         TPB_REQUIRE(pieces <= 3, TPB200_ERR_SHAPE);
     } else {
-        TPB_REQUIRE(a->a_sf && a->b_sf, TPB200_ERR_NULL);
-        TPB_REQUIRE(a->a_pitch >= K / 2 && a->b_pitch >= K / 2 && a->a_pitch % 16 == 0 && a->b_pitch % 16 == 0,
-                    TPB200_ERR_ALIGN);
-        TPB_REQUIRE(tpb_aligned16(a->a_sf) && tpb_aligned16(a->b_sf), TPB200_ERR_ALIGN);
+        TPB_REQUIRE(a->a_sf, TPB200_ERR_NULL);
+        TPB_REQUIRE(a->a_pitch >= K / 2 && a->a_pitch % 16 == 0 && tpb_aligned16(a->a_sf), TPB200_ERR_ALIGN);
         TPB_REQUIRE(pieces <= 4, TPB200_ERR_SHAPE);
         TPB_REQUIRE(pieces == 1 || (a->a_piece_rows >= M && a->a_piece_rows % 128 == 0), TPB200_ERR_SHAPE);
     }
@@ -1532,10 +1553,9 @@ extern "C" int tpb200_nvfp4_gemm_ex(const tpb200_nvfp4_gemm_args* a, tpb200_stre
 
     tpb::GemmParams P;
     const uint64_t a_rows = pieces == 1 ? static_cast<uint64_t>(M) : static_cast<uint64_t>(pieces) * a->a_piece_rows;
-    if (!tiled &&
-        (!tpb::make_tensor_map_bytes_sw128(&P.map_a, a->a_packed, static_cast<uint64_t>(K) / 2, a_rows, a->a_pitch,
-                                           tpb::kBM) ||
-         !tpb::make_tensor_map_bytes_sw128(&P.map_b, a->b_packed, static_cast<uint64_t>(K) / 2, N, a->b_pitch, 128))) {
+    if ((!tiled && !tpb::make_tensor_map_bytes_sw128(&P.map_a, a->a_packed, static_cast<uint64_t>(K) / 2, a_rows, a->a_pitch,
+                                                     tpb::kBM)) ||
+        (b_rows && !tpb::make_tensor_map_bytes_sw128(&P.map_b, a->b_packed, static_cast<uint64_t>(K) / 2, N, a->b_pitch, tiled ? 256 : 128))) {
         return TPB200_ERR_CUDA;
     }
     P.a_image = static_cast<const uint8_t*>(a->a_packed);
@@ -1584,11 +1604,10 @@ extern "C" int tpb200_nvfp4_gemm_ex(const tpb200_nvfp4_gemm_args* a, tpb200_stre
     static std::atomic<uint64_t> configured{0};
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {
-        if (cudaFuncSetAttribute(tpb::nvfp4_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 227 * 1024) != cudaSuccess ||
-            cudaFuncSetAttribute(tpb::nvfp4_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 227 * 1024) != cudaSuccess) {
-            return TPB200_ERR_CUDA;
+        for (auto k : {tpb::nvfp4_gemm_kernel<false, true>, tpb::nvfp4_gemm_kernel<true, true>, tpb::nvfp4_gemm_kernel<true, false>}) {
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
+                return TPB200_ERR_CUDA;
+            }
         }
         configured.fetch_or(bit, std::memory_order_relaxed);
     }
@@ -1638,8 +1657,9 @@ extern "C" int tpb200_nvfp4_gemm_ex(const tpb200_nvfp4_gemm_args* a, tpb200_stre
     static std::atomic<int> launch_no{0};
     P.debug_slot = launch_no.fetch_add(1);
 #endif
-    const cudaError_t err = tiled ? cudaLaunchKernelEx(&cfg, tpb::nvfp4_gemm_kernel<true>, P)
-                                  : cudaLaunchKernelEx(&cfg, tpb::nvfp4_gemm_kernel<false>, P);
+    auto kernel = !tiled ? tpb::nvfp4_gemm_kernel<false, true> : b_rows ? tpb::nvfp4_gemm_kernel<true, true>
+                                                                       : tpb::nvfp4_gemm_kernel<true, false>;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, P);
     if (err != cudaSuccess) return TPB200_ERR_CUDA;
     return tpb_launch_status();
 }

@@ -18,9 +18,10 @@ from ._lib import ACT_GELU, ACT_NONE
 from .nvfp4_packed import NVFP4_MAX, NVFP4_VALUES, _nearest_index, pack_nvfp4
 
 BLOCK_SIZE = 32
-# 128 x 256 output tiles from which the tiled operand images are the faster form.  Measured with the quantiser, us row-major /
-# tiled: 384 tiles (712 x 16384 x 2048) 34.8 / 23.4, 128 (400 x 8192 x 8192) 44.9 / 29.2, 96 (712 x 4096 x 2048) 17.8 / 13.8,
-# 64 (64 x 16384 x 4096) 15.8 / 15.5, 48 (712 x 2048 x 16384) 56.8 / 56.6
+# 128 x 256 output tiles from which activations in the tiled form are the faster ones; the weights are read as stored either
+# way.  Measured with the quantiser, us row-major / tiled: 384 tiles (712 x 16384 x 2048) 32.8 / 24.1, 128 (400 x 8192 x 8192) 41.2
+# / 30.0, 96 (712 x 4096 x 2048) 16.7 / 13.9, 80 (640 x 4096 x 4096) 25.4 / 19.6, 64 (512 x 4096 x 2048) 11.9 / 13.2, 48 (712 x
+# 2048 x 16384) 53.6 / 59.0
 TILED_MIN_TILES = 80
 
 
@@ -141,20 +142,6 @@ class NVFP4Linear(nn.Module):
     def _tiles(self, M):
         return (M + 127) // 128 * ((self.out_features + 255) // 256)
 
-    def _image(self):
-        """The weights as the GEMM's tiled image, made on first use and again when a buffer was replaced or written to.  None
-        where writes are not counted (inference tensors) and where making it would be captured."""
-        p, s = self.weight_packed, self.weight_scales_swizzled
-        if p.is_inference() or s.is_inference():
-            return None
-        key = (p.data_ptr(), p._version, s.data_ptr(), s._version)
-        st = self.__dict__.get("_tiled")
-        if st is None or st[0] != key:
-            if torch.cuda.is_current_stream_capturing():
-                return None
-            st = self.__dict__["_tiled"] = (key, ops.tile_weights(p, s, self.out_features, self.in_features))
-        return st[1]
-
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         batch_shape = x.shape[:-1]
         x2 = x if x.dim() == 2 and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
@@ -162,10 +149,10 @@ class NVFP4Linear(nn.Module):
             x2 = x2.float()
         M = x2.shape[0]
         out_dtype = torch.bfloat16 if x.dtype == torch.bfloat16 else torch.float32
-        image = self._image() if self._tiles(M) >= TILED_MIN_TILES else None
-        if image is not None:
-            y = ops.nvfp4_linear_tiled(x2, image, self.out_features, 1.0 / self.weight_scale_multiplier,
-                                       None if self.bias is None else self.bias.detach(), self.activation, out_dtype)
+        if self._tiles(M) >= TILED_MIN_TILES:
+            y = ops.nvfp4_linear_tiled(x2, self.weight_packed, self.out_features, 1.0 / self.weight_scale_multiplier,
+                                       None if self.bias is None else self.bias.detach(), self.activation, out_dtype,
+                                       self.weight_scales_swizzled)
             return y if x.dim() == 2 and y.dtype == x.dtype else y.reshape(*batch_shape, self.out_features).to(x.dtype)
         a, a_sf = ops.nvfp4_quantize_act(x2)
         y = ops.nvfp4_gemm(a, a_sf, self.weight_packed, self.weight_scales_swizzled, M, self.out_features,

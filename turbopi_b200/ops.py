@@ -311,10 +311,11 @@ def nvfp4_gemm(a_packed, a_sf, b_packed, b_sf, M, N, K, alpha=1.0, bias=None, ac
     return out
 
 
-def nvfp4_linear_tiled(x, b_image, N, alpha=1.0, bias=None, activation=ACT_NONE, out_dtype=torch.bfloat16):
-    """nvfp4_gemm(nvfp4_quantize_act(x), ...) on the tiled operand images: the same codes, scales and products in 128 x 256
-    output tiles (half the operand bytes per product).  b_image: tile_weights() of the weight operand."""
-    _cuda(x, b_image, bias)
+def nvfp4_linear_tiled(x, b_image, N, alpha=1.0, bias=None, activation=ACT_NONE, out_dtype=torch.bfloat16, b_sf=None):
+    """nvfp4_gemm(nvfp4_quantize_act(x), ...) with the activations as a tiled operand image: the same codes, scales and
+    products in 128 x 256 output tiles (half the operand bytes per product).  b_image: tile_weights() of the weight operand,
+    or with `b_sf` its row-major codes, read where they are."""
+    _cuda(x, b_image, bias, b_sf)
     M, K = x.shape
     x = x.contiguous()
     lib = _lib.load()
@@ -324,10 +325,11 @@ def nvfp4_linear_tiled(x, b_image, N, alpha=1.0, bias=None, activation=ACT_NONE,
     out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     if bias is not None:
         bias = bias.float().contiguous()
-    args = _lib.GemmArgs(a_packed=_ptr(a), a_pieces=1, b_packed=_ptr(b_image), alpha=float(alpha), bias=_ptr(bias),
-                         activation=int(activation), out=_ptr(out), out_dtype=_dt(out), ldo=N, M=M, N=N, K=K,
-                         layout=OPERANDS_TILED)
-    with launch_flags(FLAG_PDL):        # the weight image is complete: its blocks travel while the quantiser runs
+    args = _lib.GemmArgs(a_packed=_ptr(a), a_pieces=1, b_packed=_ptr(b_image), b_pitch=0 if b_sf is None else b_image.stride(0),
+                         b_sf=_ptr(b_sf), alpha=float(alpha), bias=_ptr(bias), activation=int(activation), out=_ptr(out),
+                         out_dtype=_dt(out), ldo=N, M=M, N=N, K=K, layout=OPERANDS_TILED if b_sf is None else OPERANDS_TILED_A)
+    # the quantiser is a plain launch, so what wrote the weights is complete when it starts: their blocks travel while it runs
+    with launch_flags(FLAG_PDL):
         _gemm_ex(args, x.device)
     return out
 
@@ -517,7 +519,7 @@ def fused_qkv_rope_append(x, w_packed, w_sf, q_dim, k_rows, v_rows, positions, r
 
 
 # ------------------------------------------------------------------------- tiled operands for the GEMM
-OPERANDS_ROWMAJOR, OPERANDS_TILED = 0, 1
+OPERANDS_ROWMAJOR, OPERANDS_TILED, OPERANDS_TILED_A = 0, 1, 2
 
 
 def tile_weights(b_packed, b_sf, N, K):
