@@ -9,6 +9,8 @@ Two weight formats are carried:
   "nvfp4" block 16, E4M3 scale per block + fp32 global (standard NVFP4; what the
           prefix tensor-core GEMM consumes as well)
 """
+import threading
+import weakref
 from typing import Optional, Tuple
 
 import torch
@@ -96,9 +98,63 @@ def _operand_buffer(module, T, K, device):
     return q
 
 
-def _state_of(*tensors):
-    """What changes when a weight buffer is replaced or written to in place (inference tensors count no versions)."""
-    return tuple((t.data_ptr(), t.get_device(), 0 if t.is_inference() else t._version) for t in tensors)
+class _TiledWeights:
+    """A module's tiled weight image, the scratch of the GEMV on it, and what it was made from: the buffers themselves, their
+    addresses and version counters (inference tensors count no versions)."""
+
+    lock = threading.Lock()                # one thread remakes an image, the others find it made
+
+    def __init__(self, image, scratch):
+        self.image, self.scratch, self.marks = image, scratch, ()
+
+    @staticmethod
+    def marks_of(tensors):
+        return tuple((weakref.ref(t), t.data_ptr(), None if t.is_inference() else t._version) for t in tensors)
+
+    def is_of(self, tensors):
+        for t, (ref, address, version) in zip(tensors, self.marks):
+            if ref() is not t or t.data_ptr() != address or (version is not None and t._version != version):
+                return False
+        return len(self.marks) == len(tensors)
+
+
+class _TiledWeightsOwner(nn.Module):
+    """Keeps `_TiledWeights` under an attribute that is neither copied nor saved with the module."""
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_tiled_weights"}
+
+    def _tiled(self, codes, scales, N, K):
+        """(image, GEMV scratch, finished) of the packed matrices stacked along N.  The image is made on first use and made
+        again, in the same memory, when a buffer was replaced or written to: a captured graph that reads it stays valid and
+        sees the new weights after the next eager call.  Inside a capture nothing is kept: without a current image the tiling
+        becomes part of the capture, and `finished` is False (the next launch must not overlap it)."""
+        held = self.__dict__.get("_tiled_weights")
+        sources = codes + scales
+        if held is not None and held.is_of(sources):
+            return held.image, held.scratch, True
+        dev = codes[0].device
+        with torch.cuda.device(dev), _TiledWeights.lock:
+            held = self.__dict__.get("_tiled_weights")
+            if held is not None and held.is_of(sources):
+                return held.image, held.scratch, True
+            capturing = torch.cuda.is_current_stream_capturing()
+            marks = _TiledWeights.marks_of(sources)         # before the reads: a write in between shows at the next call
+            b = torch.zeros((N, ops.packed_pitch(K)), dtype=torch.uint8, device=dev)
+            b[:, :K // 2] = codes[0] if len(codes) == 1 else torch.cat(codes, 0)
+            sf = ops.swizzle_scales(scales[0] if len(scales) == 1 else torch.cat(scales, 0))
+            if capturing:
+                return ops.tile_weights(b, sf, N, K, finish=False), ops.tc_gemv_workspace(N, K, dev), False
+            fits = (held is not None and held.image.device == dev
+                    and held.image.numel() == int(_lib.load().tpb200_nvfp4_tiled_b_bytes(N, K)))
+            if fits:
+                held.marks = ()                             # a failure below leaves no half-written image behind
+                ops.tile_weights(b, sf, N, K, held.image)
+            else:
+                held = _TiledWeights(ops.tile_weights(b, sf, N, K), ops.tc_gemv_workspace(N, K, dev))
+            held.marks = marks
+            self.__dict__["_tiled_weights"] = held
+            return held.image, held.scratch, True
 
 
 def _dense_is_faster(T, N, K, gated=False):
@@ -124,7 +180,7 @@ def _split_k_scratch(module, T, N, K, device):
     return ws
 
 
-class NVFP4PackedLinear(nn.Module):
+class NVFP4PackedLinear(_TiledWeightsOwner):
     """Linear layer over packed e2m1 weights with fused bias + GELU-tanh / SiLU.
 
     Buffers follow the reference: weight_packed [N, K/2] uint8 and weight_scales
@@ -182,24 +238,19 @@ class NVFP4PackedLinear(nn.Module):
     # ------------------------------------------------------------------ tensor-core path ("nvfp4" format)
     def tensor_core_ready(self) -> bool:
         """True if the weights are standard NVFP4 (E4M3 scale per 16 + global scale) on a CUDA device."""
-        scales = self.weight_scales
+        codes, scales = self._stored()
         return (self.block_size == 16 and scales is not None and scales.dtype == torch.uint8
-                and self.weight_packed.is_cuda and self.in_features % 16 == 0)
+                and codes.is_cuda and self.in_features % 16 == 0)
+
+    def _stored(self):
+        """(weight_packed, weight_scales), without the module's attribute search (a third of a microsecond each)"""
+        b = self._buffers
+        return b["weight_packed"], b["weight_scales"]
 
     def _tc_state(self):
-        """(tiled weight image, GEMV scratch), built on first use and whenever the packed
-        weights were replaced or written to (load_state_dict, .to(device))."""
-        key = _state_of(self.weight_packed, self.weight_scales)
-        st = self.__dict__.get("_tc")
-        if st is None or st[0] != key:
-            N, K = self.out_features, self.in_features
-            dev = self.weight_packed.device
-            b = torch.zeros((N, ops.packed_pitch(K)), dtype=torch.uint8, device=dev)
-            b[:, :K // 2] = self.weight_packed
-            image = ops.tile_weights(b, ops.swizzle_scales(self.weight_scales.contiguous()), N, K)
-            st = (key, image, ops.tc_gemv_workspace(N, K, dev))
-            self._tc = st
-        return st[1], st[2]
+        """(tiled weight image, GEMV scratch, whether the image is finished)"""
+        codes, scales = self._stored()
+        return self._tiled((codes,), (scales,), self.out_features, self.in_features)
 
     def _forward_tensor_cores(self, x2, act, bias):
         T = x2.shape[0]
@@ -209,18 +260,20 @@ class NVFP4PackedLinear(nn.Module):
             # split-K hand-over at the end (4.5-12 us against 9-27 us for the tensor-core kernel, whose
             # ground is many matrices per launch)
             return ops.nvfp4_gemv_out(x2, self.weight_packed, self.weight_scales, out, bias, act, 16, self.global_scale)
-        image, gemv_ws = self._tc_state()
+        image, gemv_ws, finished = self._tc_state()
         if T <= 16:
             return ops.tc_gemv(x2, image, self.out_features, out, self.global_scale, bias, act, 3, gemv_ws)
         xb = x2 if x2.dtype == torch.bfloat16 else x2.to(torch.bfloat16)
         if self.out_features % 8 == 0 and _dense_is_faster(T, self.out_features, self.in_features):
-            return ops.w4_gemm(xb, image, self.out_features, _lib.W4_NVFP4_TILED, alpha=self.global_scale, bias=bias,
-                               activation=act, out=out)
+            with ops.launch_flags(ops.launch_flags.current() if finished else ops.FLAG_NONE):
+                return ops.w4_gemm(xb, image, self.out_features, _lib.W4_NVFP4_TILED, alpha=self.global_scale, bias=bias,
+                                   activation=act, out=out)
         q = _operand_buffer(self, T, self.in_features, x2.device)
         # the quantiser and the GEMM are chained by programmatic dependent launch: the weights are static, so
         # the GEMM may fetch them while the quantiser still runs
-        with ops.launch_flags(ops.FLAG_PDL):
+        with ops.launch_flags(ops.FLAG_PDL if finished else ops.FLAG_NONE) as flags:
             ops.rowop(_lib.ROW_NONE, xb, self.in_features, q)
+            flags.set(ops.FLAG_PDL)
             args = _lib.GemmArgs(a_packed=ops._ptr(q.packed), a_pieces=3, a_row_scale=ops._ptr(q.row_scale),
                                  b_packed=ops._ptr(image), alpha=float(self.global_scale), bias=ops._ptr(bias),
                                  activation=int(act), out=ops._ptr(out), out_dtype=ops._dt(out), ldo=out.stride(0), M=T,
@@ -259,7 +312,7 @@ class NVFP4PackedLinear(nn.Module):
                 f"bias={self.bias is not None}, activation={self.activation}")
 
 
-class NVFP4PackedMLP(nn.Module):
+class NVFP4PackedMLP(_TiledWeightsOwner):
     """Gated MLP down(act(gate(x)) * up(x)).  `gate_activation` defaults to the
     reference module's 'silu'; Gemma's own MLP uses 'gelu' (tanh form).
 
@@ -297,39 +350,30 @@ class NVFP4PackedMLP(nn.Module):
         return layer
 
     def _stacked_gate_up(self):
-        """Tiled image of [W_gate; W_up] under ONE global scale, or None if the projections do not share one
-        (each was quantised on its own: the stacked launch needs a common fp32 multiplier)."""
+        """(tiled image of [W_gate; W_up], GEMV scratch, whether the image is finished), or None if the projections do not
+        share a global scale (each was quantised on its own: the stacked launch needs a common fp32 multiplier)."""
         g, u = self.gate_proj, self.up_proj
-        key = _state_of(g.weight_packed, u.weight_packed, g.weight_scales, u.weight_scales)
-        st = self.__dict__.get("_gu")
-        if st is None or st[0] != key:
-            if g.global_scale != u.global_scale:
-                st = (key, None)
-            else:
-                dev = g.weight_packed.device
-                N, K = 2 * self.intermediate_size, self.hidden_size
-                b = torch.zeros((N, ops.packed_pitch(K)), dtype=torch.uint8, device=dev)
-                b[:, :K // 2] = torch.cat([g.weight_packed, u.weight_packed], 0)
-                sc = torch.cat([g.weight_scales, u.weight_scales], 0).contiguous()
-                st = (key, ops.tile_weights(b, ops.swizzle_scales(sc), N, K), ops.tc_gemv_workspace(N, K, dev))
-            self._gu = st
-        return st
+        if g.global_scale != u.global_scale:
+            return None
+        (gc, gs), (uc, us) = g._stored(), u._stored()
+        return self._tiled((gc, uc), (gs, us), 2 * self.intermediate_size, self.hidden_size)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         g, u, d = self.gate_proj, self.up_proj, self.down_proj
         fast = (g.tensor_core_ready() and u.tensor_core_ready() and d.tensor_core_ready() and g.bias is None
                 and u.bias is None and g.activation in ("gelu", "silu") and self.intermediate_size % 16 == 0)
         st = self._stacked_gate_up() if fast else None
-        if st is None or st[1] is None:
+        if st is None:
             return self.down_proj(self.gate_proj(x) * self.up_proj(x))
-        _, gu_image, gu_gemv_ws = st
+        gu_image, gu_gemv_ws, finished = st
         batch_shape = x.shape[:-1]
         x2 = (x if x.dim() == 2 and x.shape[1] == self.hidden_size else x.reshape(-1, self.hidden_size)).contiguous()
         if x2.dtype != torch.bfloat16:
             x2 = x2.to(torch.bfloat16)
         T, I = x2.shape[0], self.intermediate_size
         mode = _lib.ROW_GELU_MUL if g.activation == "gelu" else _lib.ROW_SILU_MUL
-        d_image, d_gemv_ws = d._tc_state()
+        d_image, d_gemv_ws, d_finished = d._tc_state()
+        first = ops.FLAG_PDL if finished and d_finished else ops.FLAG_NONE     # the flags of the first launch on an image
         d_bias = d.bias
         if d_bias is not None:
             d_bias = d_bias.detach().float().contiguous()
@@ -337,15 +381,16 @@ class NVFP4PackedMLP(nn.Module):
         if I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True):
             # two launches: gate_up with act(gate) * up in its epilogue, down on its bf16 result
             h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
-            with ops.launch_flags(ops.FLAG_PDL):
+            with ops.launch_flags(first) as flags:
                 ops.w4_gemm(x2, gu_image, 2 * I, _lib.W4_NVFP4_TILED, alpha=g.global_scale, activation=ACTIVATIONS[g.activation],
                             gated=True, out=h)
+                flags.set(ops.FLAG_PDL)
                 ops.w4_gemm(h, d_image, self.hidden_size, _lib.W4_NVFP4_TILED, alpha=d.global_scale, bias=d_bias, out=out)
         elif T <= 16:
             # three launches chained by programmatic dependent launch: each starts on its weights while the one before runs
             gu = torch.empty((T, 2 * I), dtype=torch.bfloat16, device=x2.device)
             h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
-            ops.tc_gemv(x2, gu_image, 2 * I, gu, g.global_scale, None, 0, 3, gu_gemv_ws, pdl=True)
+            ops.tc_gemv(x2, gu_image, 2 * I, gu, g.global_scale, None, 0, 3, gu_gemv_ws, pdl=first == ops.FLAG_PDL)
             with ops.launch_flags(ops.FLAG_PDL):
                 ops.rowop(mode, gu, I, None, y_out=h, M=T)
             if T <= 4 and d.in_features % 32 == 0 and d.weight_packed.is_contiguous():
@@ -356,8 +401,10 @@ class NVFP4PackedMLP(nn.Module):
             gu = torch.empty((T, 2 * I), dtype=torch.bfloat16, device=x2.device)
             qx = _operand_buffer(g, T, self.hidden_size, x2.device)
             q = _operand_buffer(d, T, I, x2.device)
-            with ops.launch_flags(ops.FLAG_PDL):     # four launches chained by programmatic dependent launch
+            # four launches chained by programmatic dependent launch
+            with ops.launch_flags(first) as flags:
                 ops.rowop(_lib.ROW_NONE, x2, self.hidden_size, qx)
+                flags.set(ops.FLAG_PDL)
                 args = _lib.GemmArgs(a_packed=ops._ptr(qx.packed), a_pieces=3, a_row_scale=ops._ptr(qx.row_scale),
                                      b_packed=ops._ptr(gu_image), alpha=float(g.global_scale), out=ops._ptr(gu),
                                      out_dtype=ops._dt(gu), ldo=gu.stride(0), M=T, N=2 * I, K=self.hidden_size,

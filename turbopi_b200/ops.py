@@ -377,6 +377,15 @@ class launch_flags:
     def __init__(self, flags):
         self.flags = int(flags)
 
+    @staticmethod
+    def current():
+        return _flags.value
+
+    @staticmethod
+    def set(flags):
+        """Other flags for the rest of the block."""
+        _flags.value = flags
+
     def __enter__(self):
         self.prev, _flags.value = _flags.value, self.flags
         return self
@@ -522,17 +531,24 @@ def fused_qkv_rope_append(x, w_packed, w_sf, q_dim, k_rows, v_rows, positions, r
 OPERANDS_ROWMAJOR, OPERANDS_TILED, OPERANDS_TILED_A = 0, 1, 2
 
 
-def tile_weights(b_packed, b_sf, N, K):
+def tile_weights(b_packed, b_sf, N, K, image=None, finish=True):
     """Row-major GEMM B operand (codes [N, pitch] + swizzled scales) -> the tiled image of the fast path:
-    blocks [ceil(N/256)][ceil(K/256)] of 36 KB that carry codes and scales of 256 rows for one K stage."""
-    _cuda(b_packed, b_sf)
-    image = torch.empty(int(_lib.load().tpb200_nvfp4_tiled_b_bytes(N, K)), dtype=torch.uint8, device=b_packed.device)
+    blocks [ceil(N/256)][ceil(K/256)] of 36 KB that carry codes and scales of 256 rows for one K stage.
+    `image`: an image of the same [N, K] to write into.  `finish=False` (inside a capture): do not wait for it; the next
+    launch of the stream must then be one without FLAG_PDL."""
+    _cuda(b_packed, b_sf, image)
+    size = int(_lib.load().tpb200_nvfp4_tiled_b_bytes(N, K))
+    if image is None:
+        image = torch.empty(size, dtype=torch.uint8, device=b_packed.device)
+    elif image.numel() != size or image.device != b_packed.device:
+        raise TurboPiError("tile_weights: image of another shape or device")
     st = _run(b_packed, _lib.load().tpb200_nvfp4_tile_weights, _ptr(b_packed), b_packed.stride(0), _ptr(b_sf),
               _ptr(image), N, K)
     _lib.check(st, "tpb200_nvfp4_tile_weights")
     # weight preparation is a one-off: finish it here, so that a following launch with FLAG_PDL (which reads
     # weights before it waits for its predecessor) can never start on an incomplete image
-    torch.cuda.current_stream(b_packed.device).synchronize()
+    if finish:
+        torch.cuda.current_stream(b_packed.device).synchronize()
     return image
 
 
