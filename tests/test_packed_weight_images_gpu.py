@@ -141,3 +141,38 @@ def test_moved_replaced_copied(cuda_device, monkeypatch, kind, T):
     for m in _linears(d):
         m.weight_packed.data = m.weight_packed.data.clone()     # the same object on other memory
     assert torch.equal(d(x), before)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("H,I", [(2048, 14144), (2048, 14208), (2048, 16384)])
+def test_one_token_inside_a_capture(cuda_device, H, I):
+    """Either side of the size from which a captured single token takes the GEMVs: both against float64."""
+    from turbopi_b200.nvfp4_packed import NVFP4PackedMLP, unpack_nvfp4
+    g = torch.Generator(device=cuda_device).manual_seed(I)
+    w = {n: torch.randn(s, generator=g, device=cuda_device) * 0.02
+         for n, s in (("gate_proj", (I, H)), ("up_proj", (I, H)), ("down_proj", (H, I)))}
+    lin = {n: torch.nn.Linear(v.shape[1], v.shape[0], bias=False, device="meta") for n, v in w.items()}
+    for n, l in lin.items():
+        l.weight = torch.nn.Parameter(w[n], requires_grad=False)
+    mlp = NVFP4PackedMLP.from_gemma_mlp(SimpleNamespace(**lin), gate_activation="gelu", fmt="nvfp4")
+    x = torch.randn((1, H), generator=g, device=cuda_device).to(torch.bfloat16)
+    eager = mlp(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = mlp(x)
+    graph.replay()
+
+    def dense(m):
+        s = m.weight_scales.view(torch.float8_e4m3fn).double().repeat_interleave(16, 1)
+        return unpack_nvfp4(m.weight_packed, m.out_features, m.in_features).double() * s * m.global_scale
+
+    gate, up = x.double() @ dense(mlp.gate_proj).t(), x.double() @ dense(mlp.up_proj).t()
+    h = torch.nn.functional.gelu(gate, approximate="tanh") * up
+    wd = dense(mlp.down_proj)
+    ref = h @ wd.t()
+    # gate, up, the activation and the product are rounded to bf16 (2^-9 each) at random: 4 * 2^-9 of the 2-norm of the terms,
+    # five standard deviations, and the last rounding
+    tol = 5 * 4 * 2.0 ** -9 * ((h * h) @ (wd * wd).t()).sqrt() + 2.0 ** -8 * ref.abs()
+    for out in (eager, y):
+        assert bool(((out.double() - ref).abs() <= tol).all())
+    assert torch.equal(eager, y) == (2 * I * H < 58_000_000)

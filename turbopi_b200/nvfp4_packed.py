@@ -161,11 +161,19 @@ def _dense_is_faster(T, N, K, gated=False):
     """Whether [N, K] weights on the tiled image take T tokens faster through the GEMM that dequantises them (bf16
     activations as they are) than through the GEMV behind a quantiser (up to 16 tokens) or the e2m1-piece GEMM behind one:
     the first dequantises the weights once per 256 tokens, the others pay one launch more, two in a gated MLP.  Measured,
-    us for the others / dequantising.  Gated MLP of 1024 -> 4096: 1 token 16 / 10, 16 37 / 10, 17 26 / 11, 256 33 / 23, 1000 51 /
-    48; of 1152 -> 8000: 1 21 / 14, 256 40 / 33, 712 67 / 65; of 2048 -> 16384: 1 31 / 33 (one launch less to issue), 4 57 / 33,
-    50 44 / 35, 192 63 / 61, 256 64 / 68.  One linear 8000 -> 1152: 256 21 / 18, 712 26 / 23; 16384 -> 2048: 128 23 / 21, 192
-    26 / 27."""
+    us for the others / dequantising.  Gated MLP of 1024 -> 4096: 1 token 17 / 9, 16 37 / 10, 17 26 / 11, 256 33 / 23, 1000 51 /
+    48; of 1152 -> 8000: 1 21 / 14, 256 40 / 33, 712 67 / 65; of 2048 -> 16384: 2 38 / 34, 4 57 / 34, 50 44 / 35, 192 63 / 61,
+    256 64 / 68.  One linear 8000 -> 1152: 256 21 / 18, 712 26 / 23 (on the far side of the line); 16384 -> 2048: 128 23 / 21,
+    192 26 / 27."""
     return T * N * K <= (13_000_000_000 if gated else 6_000_000_000)
+
+
+def _captured_single_token(T, N, K):
+    """One token of a large gated MLP inside a capture.  The GEMVs stream the weights faster than the other form dequantises
+    them, but a call issues three launches instead of two.  Us for the GEMVs / dequantising, replayed: 2048 -> 16384 31.3 / 33.6, 2048
+    -> 12288 28.5 / 26.6; as a call 45 / 33 and 46 / 30.  So the GEMVs are taken where issuing costs nothing, above the sizes'
+    middle.  (The two forms round their sums differently.)"""
+    return T == 1 and N * K >= 58_000_000 and torch.cuda.is_current_stream_capturing()
 
 
 def _split_k_scratch(module, T, N, K, device):
@@ -378,7 +386,8 @@ class NVFP4PackedMLP(_TiledWeightsOwner):
         if d_bias is not None:
             d_bias = d_bias.detach().float().contiguous()
         out = torch.empty((T, self.hidden_size), dtype=torch.bfloat16, device=x2.device)
-        if I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True):
+        if (I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True)
+                and not _captured_single_token(T, 2 * I, self.hidden_size)):
             # two launches: gate_up with act(gate) * up in its epilogue, down on its bf16 result
             h = torch.empty((T, I), dtype=torch.bfloat16, device=x2.device)
             with ops.launch_flags(first) as flags:
