@@ -3,9 +3,9 @@
 //
 // A tile is 128 weight rows x NT tokens (NT a multiple of 16, up to 256).  The weight rows are the M side of
 // tcgen05.mma kind::f16 and come from tensor memory, the tokens are the N side and come from shared memory, so a
-// few tokens cost a few columns instead of a padded 128-row tile.  Two groups of four warps turn codes into bf16
-// in registers (thread = weight row) and store them with tcgen05.st; nothing dequantised passes through shared
-// memory, whose port the activation tiles and the MMAs need.  What a weight becomes:
+// few tokens cost a few columns instead of a padded 128-row tile.  Groups of four warps (four groups, or two where two CTAs
+// share an SM) turn codes into bf16 in registers (thread = weight row) and store them with tcgen05.st; nothing dequantised
+// passes through shared memory, whose port the activation tiles and the MMAs need.  What a weight becomes:
 //   NVFP4        e2m1 x UE4M3 has six significant bits: the product is EXACT in bf16, and so is the result up to the
 //                fp32 accumulation -- activations need no residual pieces and no quantiser launch in front
 //   INT4 k-block (q - 8) * scale with an 11-bit fp16 scale, rounded once to bf16: the scale is split into two bf16
@@ -50,6 +50,7 @@ constexpr int kMaxW = 4, kMaxS = 14;
 constexpr int kXWarp = 0, kMmaWarp = 1, kWWarp = 2, kDqWarp0 = 3;
 constexpr int kDqWarpsPerSm = 16;                // 16 dequantisation warps with an SM of its own, 8 with two CTAs per SM
 constexpr long long kWaitG = 400000000LL;        // ~0.2 s
+constexpr long long kLandCycles = 2000000LL;     // ~1 ms
 
 enum { kFmtNvfp4 = 0, kFmtKblock = 1, kFmtPlugin = 2, kFmtNvfp4T = 3 };   // 3: the w4a8 plugin's transposed operand
 enum { kEpiPlain = 0, kEpiQkv = 1, kEpiGated = 2 };
@@ -90,7 +91,13 @@ struct W4gControl {
     uint64_t full[kMaxS], empty[kMaxS];          // operand steps: weights in tensor memory + activations in shared memory
     uint64_t acc_full;
     uint32_t tmem_base;
+    int failed;                                  // a wait ran out
 };
+
+__device__ __forceinline__ void give_up(W4gControl& ctl, int error) {
+    record_error(error);
+    ctl.failed = 1;
+}
 
 __device__ __forceinline__ uint32_t idesc_bf16(int n) {
     // D = f32, A = B = bf16, both K-major, N >> 3 at [17,23), M = 128
@@ -233,6 +240,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
             mbar_init(&ctl.empty[s], 1);
         }
         mbar_init(&ctl.acc_full, 1);
+        ctl.failed = 0;
         fence_mbar_init();
     }
     if (warp == kMmaWarp) {
@@ -255,7 +263,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
             int s = 0, ph = 1;
             for (int i = 0; i < steps; ++i) {
                 if (i >= P.n_s && !mbar_wait_bounded(&ctl.empty[s], ph, kWaitG)) {
-                    record_error(kErrGemmEmptyBarrierTimeout);
+                    give_up(ctl, kErrGemmEmptyBarrierTimeout);
                     break;
                 }
                 mbar_expect_tx(&ctl.full[s], b_bytes);
@@ -275,13 +283,16 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
         for (int j = 0; j < nblk; ++j) {
             const int s = j % P.n_w, kb = blk0 + j;
             uint8_t* slot = sW + s * kWSlot;
+            int stop = 0;
             if (lane == 0) {
                 if (j >= P.n_w && !mbar_wait_bounded(&ctl.w_empty[s], ((j / P.n_w) - 1) & 1, kWaitG)) {
-                    record_error(kErrGemmEmptyBarrierTimeout);
+                    give_up(ctl, kErrGemmEmptyBarrierTimeout);
+                    stop = 1;
+                } else {
+                    mbar_expect_tx(&ctl.w_full[s], bytes);
                 }
-                mbar_expect_tx(&ctl.w_full[s], bytes);
             }
-            __syncwarp();
+            if (__shfl_sync(0xffffffffu, stop, 0)) break;            // the slot may still be read
             // the requests of a block leave from different lanes: one lane needs ~0.3 us per request
             if (kFmt == kFmtNvfp4) {
                 const int half = lane & 1, row = half ? row_b : row_a;
@@ -322,7 +333,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
             int s = 0, ph = 0;
             for (int i = 0; i < steps; ++i) {
                 if (!__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[s], ph, kWaitG))) {
-                    if (lane == 0) record_error(kErrGemmTmaBarrierTimeout);
+                    if (lane == 0) give_up(ctl, kErrGemmTmaBarrierTimeout);
                     break;
                 }
                 tc::fence_after_thread_sync();
@@ -450,7 +461,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                 tmem_st_32x32b_x32(lane_addr + P.a_col + (sa * parts + u) * 32, out);
             }
             if (!ok) {
-                if (lane == 0) record_error(kErrGemmEmptyBarrierTimeout);
+                if (lane == 0) give_up(ctl, kErrGemmEmptyBarrierTimeout);
                 break;
             }
             tmem_st_wait();
@@ -462,7 +473,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
         }
         // ------------------------------------------------------------ accumulator -> shared memory, [token][128 rows]
         if (ok && !mbar_wait_bounded(&ctl.acc_full, 0, kWaitG)) {
-            record_error(kErrGemmMmaBarrierTimeout);
+            give_up(ctl, kErrGemmMmaBarrierTimeout);
             ok = false;
         }
         ok = __all_sync(0xffffffffu, ok);
@@ -497,8 +508,13 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
     }
 
     // ---------------------------------------------------------------- this CTA's share of the tokens, all 128 rows
-    {
-        pdl_wait_prior_grids();                                      // a no-op by now; orders reads of `out` (beta)
+    pdl_wait_prior_grids();                                          // a no-op by now; orders reads of `out` (beta)
+    if (ctl.failed) {
+        // Nothing is stored, and the CTA stays until the copies it has requested (microseconds of work) have landed: its
+        // shared memory goes to another CTA afterwards.
+        const long long start = clock64();
+        while (clock64() - start < kLandCycles) __nanosleep(1000);
+    } else {
         const int valid = min(P.nt, P.M - t0);
         const int tb = rank * valid / splits, te = (rank + 1) * valid / splits;
         const uint32_t base = smem_u32(smem);
