@@ -170,8 +170,8 @@ def test_one_token_inside_a_capture(cuda_device, H, I):
     h = torch.nn.functional.gelu(gate, approximate="tanh") * up
     wd = dense(mlp.down_proj)
     ref = h @ wd.t()
-    # gate, up, the activation and the product are rounded to bf16 (2^-9 each) at random: 4 * 2^-9 of the 2-norm of the terms,
-    # five standard deviations, and the last rounding
+    # gate, up, the activation and the product round to bf16, each by 2^-8 / sqrt(3) of its value in the mean square: together
+    # less than 4 * 2^-9 of the 2-norm of the terms; five times that, and the last rounding
     tol = 5 * 4 * 2.0 ** -9 * ((h * h) @ (wd * wd).t()).sqrt() + 2.0 ** -8 * ref.abs()
     for out in (eager, y):
         assert bool(((out.double() - ref).abs() <= tol).all())

@@ -88,6 +88,42 @@ def test_qkv_epilogue_equals_the_piecewise_gemm(cuda_device, M):
     assert float((kv[2:, M:]).abs().max()) == 0
 
 
+@pytest.mark.parametrize("M", [1, 50, 177])
+@pytest.mark.parametrize("tiled", [False, True])
+def test_qkv_epilogue_against_float64(cuda_device, M, tiled):
+    from turbopi_b200 import _lib, ops
+    K, q_dim, N = 1024, 2048, 2560
+    b, sf, w = _nvfp4(N, K, cuda_device, M)
+    x = torch.randn((M, K), generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(cuda_device)
+    cos, sin = ops.rope_tables(1024, device=cuda_device)
+    pos = torch.randperm(1024, generator=torch.Generator().manual_seed(1))[:M].to(torch.int32).to(cuda_device)
+    kv = torch.zeros((2, M + 2, 256), dtype=torch.bfloat16, device=cuda_device)
+    q = torch.empty((M, q_dim), dtype=torch.bfloat16, device=cuda_device)
+    p, alpha = ops._ptr, 2.0 ** -9
+    image = ops.tile_weights(b, sf, N, K)
+    weight = (dict(format=_lib.W4_NVFP4_TILED, w=p(image)) if tiled
+              else dict(format=_lib.W4_NVFP4_ROWMAJOR, w=p(b), w_pitch=b.stride(0), w_scales=p(sf)))
+    ops._w4_gemm(_lib.W4GemmArgs(x=p(x), ldx=K, alpha=alpha, out=p(q), out_dtype=_lib.BF16, ldo=q_dim, M=M, N=N, K=K,
+                                 qkv_q_dim=q_dim, qkv_k_rows=p(kv[0]), qkv_v_rows=p(kv[1]), qkv_positions=p(pos),
+                                 qkv_rope_cos=p(cos), qkv_rope_sin=p(sin), **weight), cuda_device)
+    rows = torch.empty_like(w)
+    rows[ops.qkv_tile_permutation(q_dim).to(cuda_device)] = w              # the kernel's rows are permuted by tile
+    ref, mag = alpha * (x.double() @ rows.t()), alpha * (x.double().abs() @ rows.abs().t())
+    c, s = cos[pos.long()].double()[:, None], sin[pos.long()].double()[:, None]
+    heads, hm = ref[:, :q_dim + 256].view(M, -1, 2, 128), mag[:, :q_dim + 256].view(M, -1, 2, 128)
+    lo, hi, ml, mh = heads[:, :, 0], heads[:, :, 1], hm[:, :, 0], hm[:, :, 1]
+    got = torch.cat([q, kv[0, :M]], 1).double().view(M, -1, 2, 128)
+    u = 2.0 ** -8                                                          # unit roundoff of bf16 (eight significant bits)
+    for y, r, m, ms in ((got[:, :, 0], lo * c - hi * s, (lo * c).abs() + (hi * s).abs(), (ml * c.abs()) + (mh * s.abs())),
+                        (got[:, :, 1], hi * c + lo * s, (hi * c).abs() + (lo * s).abs(), (mh * c.abs()) + (ml * s.abs()))):
+        # both projections, both products and the sum round once each; fp32 sums of K terms
+        assert bool(((y - r).abs() <= 1.02 * u * (2 * m + r.abs()) + 2e-6 * ms + 1e-30).all())
+    v, mv = ref[:, q_dim + 256:], mag[:, q_dim + 256:]
+    assert bool(((kv[1, :M].double() - v).abs() <= 1.02 * u * v.abs() + 2e-6 * mv + 1e-30).all())
+    assert float(kv[:, M:].abs().max()) == 0
+    assert _lib.load().tpb200_device_error(0) == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(17, 8, 128), (50, 1032, 1024), (200, 136, 384), (257, 512, 2048), (712, 2048, 1024)])
 @pytest.mark.parametrize("plugin", [False, True])
 def test_int4(cuda_device, M, N, K, plugin):
