@@ -492,11 +492,12 @@ def run_extras(device, sets, x):
         pk, sf = ops.nvfp4_quantize_act(xq)
         t = time_launches(lambda i: ops.nvfp4_quantize_act(xq, pk, sf), 16)
         ex[f"nvfp4_quantize_act_{M}x{K}"] = {"us": t * 1e6, "gbps": (M * K * 2 + M * K // 2 + M * K // 16) / t / 1e9}
-    # (g) the model's linears as they run in the pipeline: bf16 activations -> 3 residual e2m1 pieces (row
-    # kernel), NVFP4 weights; the two large prefix MLP matrices on the tiled images (128 x 256 output tiles), the
-    # other shapes in the row-major operand form (128 x 128 tiles), chained by programmatic dependent launch as
-    # in the pipeline (benchmark config 4 with weight-only semantics; `tflops` counts the useful 2 M N K once,
-    # not the 3 pieces; `tiled_gemm_us`: the same shape on the tiled images)
+    # (g) the model's linears as they run in the pipeline, launches chained by programmatic dependent launch as there: the
+    # two large prefix MLP matrices on the tiled images behind the quantising row kernel (three residual e2m1 pieces,
+    # 128 x 256 output tiles), every other linear on its bf16 activations through the GEMM that dequantises its weights
+    # (the expert's gate_up with GELU(gate) * up in the epilogue); benchmark config 4 with weight-only semantics.
+    # `tflops` counts the useful 2 M N K once; `e2m1_pieces_us`: the same linear through the row-major piece GEMM,
+    # without the quantiser in front of it
     from turbopi_b200 import _lib as tlib
     from turbopi_b200.pi05 import TcLinear
     gemm_ws = ops.gemm_workspace(device)
@@ -504,33 +505,34 @@ def run_extras(device, sets, x):
                             (712, 2560, 2048, "gemma2b_qkv_M712"), (512, 4304, 1152, "siglip_fc1_M512"),
                             (512, 1152, 4304, "siglip_fc2_M512"), (50, 8192, 1024, "expert_gate_up_M50"),
                             (50, 1024, 4096, "expert_down_M50")):
-        rowmajor = N * K < (1 << 25)            # the pipeline's rule: everything but the prefix gate_up / down
+        dense = N * K < (1 << 25)               # the pipeline's rule: everything but the prefix gate_up / down
+        gated = name.startswith("expert_gate_up")
         xq = torch.randn(M, K, device=device).to(torch.bfloat16)
         o = torch.empty((M, N), dtype=torch.bfloat16, device=device)
-        weights_ = [torch.randn(N, K, device=device) * 0.02 for _ in range(2)]
-        times = {}
-        for form in ((False, True) if rowmajor else (False,)):
-            q = ops.QuantBuf(M, K, 3, device, tiled=not form)
-            lins = [TcLinear.from_weight(w_, rowmajor=form) for w_ in weights_]
-            for l_ in lins:
-                l_.ws = gemm_ws
-            ops.rowop(tlib.ROW_NONE, xq, K, q)
-            with ops.launch_flags(ops.FLAG_PDL):
-                times[form] = (time_launches(lambda i: lins[i % 2](q, o), 16),
-                               time_launches(lambda i: ops.rowop(tlib.ROW_NONE, xq, K, q), 16))
-            del lins
-        del weights_
-        t, tq = times[rowmajor]
+        og = torch.empty((M, N // 2), dtype=torch.bfloat16, device=device) if gated else o
+        copies = max(2, min(32, (256 << 20) // (N * K * 9 // 16)))        # rotating weights larger than L2
+        lins = [TcLinear.from_weight(torch.randn(N, K, device=device) * 0.02, rowmajor=dense) for _ in range(copies)]
+        for l_ in lins:
+            l_.ws = gemm_ws
+        q = ops.QuantBuf(M, K, 3, device, tiled=not dense)
+        ops.rowop(tlib.ROW_NONE, xq, K, q)
+        with ops.launch_flags(ops.FLAG_PDL):
+            pieces = time_launches(lambda i: lins[i % copies](q, o), 32)
+            tq = time_launches(lambda i: ops.rowop(tlib.ROW_NONE, xq, K, q), 16)
+            t = pieces
+            if dense:
+                t = time_launches(lambda i: lins[i % copies].dense(xq, og, tlib.ACT_GELU if gated else tlib.ACT_NONE, gated), 32)
+        del lins
         # the library comparator on the same shape: torch F.linear in bf16 (cuBLAS), weights rotating too
-        wb = [(torch.randn(N, K, device=device) * 0.02).to(torch.bfloat16) for _ in range(2)]
-        tb = time_launches(lambda i: torch.nn.functional.linear(xq, wb[i % 2]), 16)
-        ex[f"w4a16_tc_linear_{name}"] = {"gemm_us": t * 1e6, "quantise_us": tq * 1e6,
-                                         "form": "row-major operands, 128x128 tiles" if rowmajor else "tiled images, 128x256 tiles",
-                                         "tflops": 2.0 * M * N * K / t / 1e12,
-                                         "tensor_tflops": 3 * 2.0 * M * N * K / t / 1e12,
-                                         "cublas_bf16_us": tb * 1e6, "cublas_bf16_tflops": 2.0 * M * N * K / tb / 1e12}
-        if rowmajor:
-            ex[f"w4a16_tc_linear_{name}"]["tiled_gemm_us"] = times[False][0] * 1e6
+        wb = [(torch.randn(N, K, device=device) * 0.02).to(torch.bfloat16) for _ in range(copies)]
+        tb = time_launches(lambda i: torch.nn.functional.linear(xq, wb[i % copies]), 32)
+        row = {"gemm_us": t * 1e6, "tflops": 2.0 * M * N * K / t / 1e12,
+               "cublas_bf16_us": tb * 1e6, "cublas_bf16_tflops": 2.0 * M * N * K / tb / 1e12}
+        if dense:
+            row.update(form="bf16 activations, weights dequantised into tensor memory", e2m1_pieces_us=pieces * 1e6)
+        else:
+            row.update(form="tiled images, 128x256 tiles", quantise_us=tq * 1e6, tensor_tflops=3 * 2.0 * M * N * K / t / 1e12)
+        ex[f"w4a16_tc_linear_{name}"] = row
         del wb
     # (e2) the same NVFP4 x NVFP4 products on the tiled operand images (one e2m1 activation piece, 128 x 256 tiles):
     # the form the prefix would run with e2m1 activations

@@ -59,7 +59,7 @@ class Pi05Config:
     action_horizon: int = 50
     action_dim: int = 32
     max_seq: int = 1024
-    pieces: int = 3
+    pieces: int = 3          # residual e2m1 pieces of the prefix MLP's activations (every other linear takes them in bf16)
     eps: float = 1e-6
 
     @property
@@ -129,18 +129,6 @@ class TcLinear:
         args.out, args.out_dtype, args.ldo = ops._ptr(out), ops._dt(out), out.stride(0)
         ops._gemm_ex(args, out.device, self.ws)
         return out
-
-    def qkv(self, q, q_out, k_rows, v_rows, positions, cos, sin, q_dim, M=None):
-        M = q.M if M is None else M
-        if k_rows.shape[0] < M or v_rows.shape[0] < M or positions.numel() < M:
-            raise TurboPiError("fused QKV: cache rows / positions shorter than the token count")
-        p = ops._ptr
-        args = self._args(q, M)
-        args.qkv_q_out, args.qkv_ldq, args.qkv_q_dim = p(q_out), q_out.stride(0), q_dim
-        args.qkv_k_rows, args.qkv_v_rows, args.qkv_positions = p(k_rows), p(v_rows), p(positions)
-        args.qkv_rope_cos, args.qkv_rope_sin = p(cos), p(sin)
-        ops._gemm_ex(args, q_out.device, self.ws)
-        return q_out
 
     def _w4_args(self, x, M, out, ldo):
         p = ops._ptr
