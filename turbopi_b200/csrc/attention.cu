@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     const uint32_t tmem = ctl->tmem_base;
     pdl_wait_prior_grids();                               // q, k, v (and the bias) may come from the previous kernel
 
-    // warps 1..7: the keys' additive bias in the base-2 domain (visible to all after the barrier behind the S wait)
+    // warps 1..8: the keys' additive bias in the base-2 domain (visible to all after the barrier behind the S wait)
     for (int i = threadIdx.x - 32; i >= 0 && i < kKeysCta; i += kThreadsAttn - 32) {
         const int key = key0 + i;
         float b = kFloor2;                                // keys past the end never count
