@@ -176,3 +176,34 @@ def test_one_token_inside_a_capture(cuda_device, H, I):
     for out in (eager, y):
         assert bool(((out.double() - ref).abs() <= tol).all())
     assert torch.equal(eager, y) == (2 * I * H < 58_000_000)
+
+
+@torch.no_grad()
+def test_scratch_of_a_capture(cuda_device, monkeypatch):
+    """Operand buffers and split-K scratch: those a captured graph uses outlive calls with other token counts; those made
+    inside a capture, whose zeros only a replay writes, serve no other call."""
+    a, b = _pair("mlp_pieces", cuda_device, monkeypatch)
+    xs = {T: torch.randn(T, 128, device=cuda_device).to(torch.bfloat16) for T in (1, 200, 300, 17, 33, 65, 130, 260, 390)}
+    for m, n in zip(_linears(a), _linears(b)):
+        n.global_scale = m.global_scale
+    _load(b, a)
+    want = {T: b(x) for T, x in xs.items()}
+    a(xs[1])
+    a(xs[200])
+    graphs, ys = {}, {}
+    for T in (200, 300):                                    # warmed up, and not
+        graphs[T] = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graphs[T]):
+            ys[T] = a(xs[T])
+    for m in _linears(a):
+        assert all(key[0] != 300 for key in m.__dict__.get("_operands", {}))
+    assert torch.equal(a(xs[300]), want[300])
+    for T in (17, 33, 65, 130, 260, 390):
+        assert torch.equal(a(xs[T]), want[T])
+    _scribble(cuda_device)
+    for _ in range(2):
+        for T, graph in graphs.items():
+            graph.replay()
+            assert torch.equal(ys[T], want[T])
+    from turbopi_b200 import _lib
+    assert _lib.load().tpb200_device_error(0) == 0

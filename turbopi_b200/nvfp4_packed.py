@@ -83,18 +83,28 @@ def quantize_nvfp4_two_level(weight: torch.Tensor, block_size: int = 16):
     return packed, s8.view(torch.uint8), g
 
 
+def _pin_if_captured(module, buffer):
+    """A captured graph reads and writes `buffer` by address: it then lives as long as the module."""
+    if torch.cuda.is_current_stream_capturing():
+        module.__dict__.setdefault("_captured", {})[id(buffer)] = buffer
+    return buffer
+
+
 def _operand_buffer(module, T, K, device):
     """The tiled A operand of `module`'s GEMM for T tokens, kept on the module: allocating (and zero-filling) 3 x T x K / 2
     bytes per call costs more than the quantiser that fills them.  Padding rows and columns are never written, so
     they stay zero from one call to the next.  (Calls on one module are expected in stream order, as with any
-    module that owns scratch.)"""
+    module that owns scratch.)  One made inside a capture is the graph's own: its zeros are written by the replays."""
     cache = module.__dict__.setdefault("_operands", {})
     key = (int(T), int(K), str(device))
     q = cache.get(key)
-    if q is None:
+    if q is not None:
+        return _pin_if_captured(module, q)
+    q = ops.QuantBuf(T, K, 3, device)
+    if not torch.cuda.is_current_stream_capturing():
         if len(cache) >= 4:
             cache.clear()
-        q = cache[key] = ops.QuantBuf(T, K, 3, device)
+        cache[key] = q
     return q
 
 
@@ -119,10 +129,12 @@ class _TiledWeights:
 
 
 class _TiledWeightsOwner(nn.Module):
-    """Keeps `_TiledWeights` under an attribute that is neither copied nor saved with the module."""
+    """Keeps `_TiledWeights` and the scratch above under attributes that are neither copied nor saved with the module."""
+
+    _OWN = frozenset(("_tiled_weights", "_operands", "_gemm_ws", "_captured"))
 
     def __getstate__(self):
-        return {k: v for k, v in self.__dict__.items() if k != "_tiled_weights"}
+        return {k: v for k, v in self.__dict__.items() if k not in self._OWN}
 
     def _tiled(self, codes, scales, N, K):
         """(image, GEMV scratch, finished) of the packed matrices stacked along N.  The image is made on first use and made
@@ -180,11 +192,14 @@ def _split_k_scratch(module, T, N, K, device):
     """Zeroed split-K scratch of `module`'s GEMM, as large as the launch planner wants for T tokens (a scratch
     that is too small makes the planner cut K less and leaves SMs idle: 712 x 2048 x 16384 runs on 48 CTAs
     without it).  Grown when a larger token count arrives; owned by the module, so calls on different modules
-    never share counters."""
+    never share counters.  Scratch made inside a capture is the graph's own, like an operand buffer."""
     need = ops.nvfp4_gemm_workspace_size(T, N, K, 3, ops.OPERANDS_TILED)
     ws = module.__dict__.get("_gemm_ws")
-    if ws is None or ws.numel() < need or ws.device != torch.device(device):
-        ws = module.__dict__["_gemm_ws"] = ops.gemm_workspace(device, max(int(need), 1 << 20))
+    if ws is not None and ws.numel() >= need and ws.device == torch.device(device):
+        return _pin_if_captured(module, ws)
+    ws = ops.gemm_workspace(device, max(int(need), 1 << 20))
+    if not torch.cuda.is_current_stream_capturing():
+        module.__dict__["_gemm_ws"] = ws
     return ws
 
 
