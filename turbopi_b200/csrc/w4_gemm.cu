@@ -283,16 +283,12 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
         for (int j = 0; j < nblk; ++j) {
             const int s = j % P.n_w, kb = blk0 + j;
             uint8_t* slot = sW + s * kWSlot;
-            int stop = 0;
-            if (lane == 0) {
-                if (j >= P.n_w && !mbar_wait_bounded(&ctl.w_empty[s], ((j / P.n_w) - 1) & 1, kWaitG)) {
-                    give_up(ctl, kErrGemmEmptyBarrierTimeout);
-                    stop = 1;
-                } else {
-                    mbar_expect_tx(&ctl.w_full[s], bytes);
-                }
+            if (j >= P.n_w && !__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.w_empty[s], ((j / P.n_w) - 1) & 1, kWaitG))) {
+                if (lane == 0) give_up(ctl, kErrGemmEmptyBarrierTimeout);
+                break;                                               // the slot may still be read
             }
-            if (__shfl_sync(0xffffffffu, stop, 0)) break;            // the slot may still be read
+            if (lane == 0) mbar_expect_tx(&ctl.w_full[s], bytes);
+            __syncwarp();
             // the requests of a block leave from different lanes: one lane needs ~0.3 us per request
             if (kFmt == kFmtNvfp4) {
                 const int half = lane & 1, row = half ? row_b : row_a;
@@ -509,12 +505,8 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
 
     // ---------------------------------------------------------------- this CTA's share of the tokens, all 128 rows
     pdl_wait_prior_grids();                                          // a no-op by now; orders reads of `out` (beta)
-    if (ctl.failed) {
-        // Nothing is stored, and the CTA stays until the copies it has requested (microseconds of work) have landed: its
-        // shared memory goes to another CTA afterwards.
-        const long long start = clock64();
-        while (clock64() - start < kLandCycles) __nanosleep(1000);
-    } else {
+    const bool failed = ctl.failed != 0;                             // then nothing is stored
+    {
         const int valid = min(P.nt, P.M - t0);
         const int tb = rank * valid / splits, te = (rank + 1) * valid / splits;
         const uint32_t base = smem_u32(smem);
@@ -563,6 +555,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
 #pragma unroll
                     for (int e = 0; e < 8; ++e) v[e] = act_fast(v[e], P.activation);
                 }
+                if (failed) continue;                                // asked here: the flag arrives beside the sums
                 const size_t o = static_cast<size_t>(t0 + t) * P.ldo + n;
                 if (P.beta != 0.0f) {
 #pragma unroll
@@ -594,6 +587,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                 sum8(t, c + 64, up);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) g[e] = bf16r(act_fast(bf16r(g[e]), P.activation)) * bf16r(up[e]);
+                if (failed) continue;
                 *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.out) + static_cast<size_t>(t0 + t) * P.ldo + row_a + c) =
                     pack8(g);
             }
@@ -628,12 +622,19 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                     olo[e] = bits(a);
                     ohi[e] = bits(b);
                 }
+                if (failed) continue;
                 __nv_bfloat16* dst = head < heads ? static_cast<__nv_bfloat16*>(P.out) + static_cast<size_t>(m) * P.ldq + head * 256
                                      : (head == heads ? P.k_rows : P.v_rows) + static_cast<size_t>(m) * 256;
                 *reinterpret_cast<uint4*>(dst + i0 + c) = make_uint4(olo[0], olo[1], olo[2], olo[3]);
                 *reinterpret_cast<uint4*>(dst + i0 + c + 128) = make_uint4(ohi[0], ohi[1], ohi[2], ohi[3]);
             }
         }
+    }
+    if (failed) {
+        // The CTA stays until the copies it has requested (microseconds of work) have landed: its shared memory goes to
+        // another CTA afterwards.
+        const long long start = clock64();
+        while (clock64() - start < kLandCycles) __nanosleep(1000);
     }
     if (splits > 1) {                                                // nobody leaves while a peer still reads its sums
         __syncwarp();
