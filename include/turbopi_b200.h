@@ -254,6 +254,21 @@ typedef struct {
     int flags;
 } tpb200_w4_gemm_args;
 int tpb200_w4_gemm(const tpb200_w4_gemm_args* args, tpb200_stream_t stream);
+/* The same launch (NVFP4 weights) with the RMS norms around it folded in (GemmaRMSNorm and _gated_residual,
+ * openpi/src/openpi/models_pytorch/transformers_replace/models/gemma/modeling_gemma.py:49-129):
+ *   in_sumsq != NULL: the rows of x are h * (1 + scale) without their RMS factor.  Every sum is multiplied by
+ *          rsqrt(sum of the row's in_parts partial sums / K + in_eps), then in_shift[n] (fp32: W * shift, alpha included, or
+ *          NULL) is added, then bias and activation.  in_sumsq [M, in_parts] fp32, in_parts % 4 == 0.
+ *   h_out != NULL: h = bf16(res_in + bf16(y * gate)) with y the linear's bf16 result (res_in, gate may be NULL) goes to h_out
+ *          [M, N] (may be res_in), bf16(h * (1 + scale)) to `out`, the sums of h^2 over 128 columns to out_sumsq
+ *          [M, N / 128].  N % 128 == 0, bf16 out, no activation, no beta, neither gated nor QKV.
+ * in_shift, gate and scale are parameters like the weights: under TPB200_FLAG_PDL they may be read while the kernel before
+ * this one still runs. */
+typedef struct {
+    const float* in_sumsq; const float* in_shift; int in_parts; float in_eps;
+    const void* res_in; const void* gate; const void* scale; void* h_out; float* out_sumsq;
+} tpb200_w4_norm_args;
+int tpb200_w4_gemm_norm(const tpb200_w4_gemm_args* args, const tpb200_w4_norm_args* norm, tpb200_stream_t stream);
 /* What a launch of that shape looks like on a GPU of `sms` SMs (host only, no device needed): tokens per tile, K ranges
  * per tile, CTAs per SM, groups of four dequantising warps, 64-K parts per step, slots of the weight and of the step ring,
  * 256-K blocks and 64-K parts of the whole K. */

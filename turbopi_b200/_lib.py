@@ -53,6 +53,11 @@ class W4GemmArgs(ctypes.Structure):
                 ("qkv_positions", c_void_p), ("qkv_rope_cos", c_void_p), ("qkv_rope_sin", c_void_p), ("flags", c_int)]
 
 
+class W4NormArgs(ctypes.Structure):
+    _fields_ = [("in_sumsq", c_void_p), ("in_shift", c_void_p), ("in_parts", c_int), ("in_eps", c_float),
+                ("res_in", c_void_p), ("gate", c_void_p), ("scale", c_void_p), ("h_out", c_void_p), ("out_sumsq", c_void_p)]
+
+
 class W4GemmPlanInfo(ctypes.Structure):
     _fields_ = [(n, c_int) for n in ("tokens_per_tile", "splits", "ctas_per_sm", "groups", "parts", "weight_slots", "step_slots",
                                      "k_blocks", "k_steps")]
@@ -125,6 +130,7 @@ SIGNATURES = {
                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "tpb200_w4_gemm_plan": (c_int, [c_int, c_int, c_int, c_int, ctypes.POINTER(W4GemmPlanInfo)]),
     "tpb200_w4_gemm": (c_int, [ctypes.POINTER(W4GemmArgs), c_void_p]),
+    "tpb200_w4_gemm_norm": (c_int, [ctypes.POINTER(W4GemmArgs), ctypes.POINTER(W4NormArgs), c_void_p]),
     "tpb200_nvfp4_gemm_ex": (c_int, [ctypes.POINTER(GemmArgs), c_void_p]),
     "tpb200_nvfp4_quantize_act_pieces": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                                  c_int, c_int, c_int, c_void_p]),

@@ -8,7 +8,8 @@
 #include "common.cuh"
 
 namespace tpb {
-int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool transposed);
+int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool transposed,
+                   const tpb200_w4_norm_args* norm = nullptr);
 }
 
 namespace tpb {

@@ -53,7 +53,7 @@ constexpr long long kWaitG = 400000000LL;        // ~0.2 s
 constexpr long long kLandCycles = 2000000LL;     // ~1 ms
 
 enum { kFmtNvfp4 = 0, kFmtKblock = 1, kFmtPlugin = 2, kFmtNvfp4T = 3 };   // 3: the w4a8 plugin's transposed operand
-enum { kEpiPlain = 0, kEpiQkv = 1, kEpiGated = 2 };
+enum { kEpiPlain = 0, kEpiQkv = 1, kEpiGated = 2, kEpiResidual = 3 };
 
 struct W4gParams {
     CUtensorMap map_x;                           // bf16 [M, K], box 64 x NT, 128-byte swizzle
@@ -84,6 +84,17 @@ struct W4gParams {
     const int* positions;
     const __nv_bfloat16* rope_cos;
     const __nv_bfloat16* rope_sin;
+    // The norm in front of this linear, folded: x holds h * (1 + scale), the row's RMS factor and W * shift come here
+    const float* in_sumsq;                       // [M, in_parts] partial sums of h^2, or null
+    const float* in_shift;                       // fp32 [N] or null
+    int in_parts;
+    float in_eps, in_inv_k;
+    // kEpiResidual: the residual stream and the next norm's input
+    const __nv_bfloat16* res;
+    const __nv_bfloat16* gate;
+    const __nv_bfloat16* scale;
+    __nv_bfloat16* h_out;
+    float* out_sumsq;                            // [M, N / 128]
 };
 
 struct W4gControl {
@@ -140,6 +151,7 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
 }
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
     uint32_t a;
@@ -202,9 +214,142 @@ __device__ __forceinline__ float act_fast(float x, int act) {
 }
 __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
-    return make_uint4(bits(__floats2bfloat162_rn(v[0], v[1])), bits(__floats2bfloat162_rn(v[2], v[3])),
-                      bits(__floats2bfloat162_rn(v[4], v[5])), bits(__floats2bfloat162_rn(v[6], v[7])));
+__device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
+    return make_uint2(bits(__floats2bfloat162_rn(v[0], v[1])), bits(__floats2bfloat162_rn(v[2], v[3])));
+}
+__device__ __forceinline__ void unpack4(uint2 u, float (&v)[4]) {
+    const float2 a = __bfloat1622float2(as_bf162(u.x)), b = __bfloat1622float2(as_bf162(u.y));
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void act4(float (&v)[4], int act) {
+    if (act == TPB200_ACT_GELU) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = act_fast(v[e], TPB200_ACT_GELU);
+    } else if (act == TPB200_ACT_SILU) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = act_fast(v[e], TPB200_ACT_SILU);
+    }
+}
+
+// Sums of up to S CTAs' partial results at one offset, in rank order.  All loads leave before the first sum needs one (a
+// loop that added while it loaded paid a distributed-shared-memory round trip per CTA: 1.4 us of a 5 us launch at 8).
+template <int S>
+__device__ __forceinline__ float4 sum_ranks(uint32_t base, uint32_t off, int splits) {
+    float4 x[S];
+#pragma unroll
+    for (int p = 0; p < S; ++p) x[p] = ld_cluster_f4(map_to_rank(base, p < splits ? p : 0) + off);
+    float4 a = x[0];
+#pragma unroll
+    for (int p = 1; p < S; ++p) {
+        if (p < splits) { a.x += x[p].x; a.y += x[p].y; a.z += x[p].z; a.w += x[p].w; }
+    }
+    return a;
+}
+
+// A load for the line's sake: into this SM's L1, the value unused
+__device__ __forceinline__ void touch(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+}
+
+// What one unit of the epilogue (a token, 4 weight rows or 4 + 4) reads for the norms folded into a launch.
+//   in:   RMSNorm(h) (1 + scale) + shift in front of a linear is  rstd * W (h (1 + scale)) + W shift.  The elementwise
+//         product is what the launch before wrote as x; rstd needs its sums of squares and W * shift is a constant vector.
+//   out:  (kEpiResidual) the launch that ends a residual branch writes h, h (1 + scale) and the sums of squares itself.
+// Between them no launch has to see a whole row before it can start, and the row kernel that stood there is gone.
+struct NormUnit {
+    float rstd;
+    float4 shift_a, shift_b;
+    uint2 res, gate, scale, h, cos, sin;
+
+    template <bool kPairs>
+    __device__ __forceinline__ void load(const W4gParams& P, int m, int n, int n2) {
+        if (P.in_sumsq != nullptr) {
+            const float4* sp = reinterpret_cast<const float4*>(P.in_sumsq + static_cast<size_t>(m) * P.in_parts);
+            float4 a = sp[0];
+            for (int i = 1; i < P.in_parts / 4; ++i) {
+                const float4 f = sp[i];
+                a.x += f.x; a.y += f.y; a.z += f.z; a.w += f.w;
+            }
+            rstd = rsqrtf(((a.x + a.y) + (a.z + a.w)) * P.in_inv_k + P.in_eps);
+            shift_a = shift_b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (P.in_shift != nullptr) {
+                shift_a = *reinterpret_cast<const float4*>(P.in_shift + n);
+                if (kPairs) shift_b = *reinterpret_cast<const float4*>(P.in_shift + n2);
+            }
+        }
+        if (kPairs && P.epilogue == kEpiQkv && n < P.q_dim + 256) {  // a Q or K head: 128-row tiles, two per head
+            const size_t p = static_cast<size_t>(P.positions[m]) * 128 + (n >> 7 & 1) * 64 + (n & 63);
+            cos = *reinterpret_cast<const uint2*>(P.rope_cos + p);
+            sin = *reinterpret_cast<const uint2*>(P.rope_sin + p);
+        }
+        if (!kPairs && P.epilogue == kEpiResidual) {
+            if (P.res != nullptr) res = *reinterpret_cast<const uint2*>(P.res + static_cast<size_t>(m) * P.N + n);
+            if (P.gate != nullptr) gate = *reinterpret_cast<const uint2*>(P.gate + n);
+            scale = *reinterpret_cast<const uint2*>(P.scale + n);
+        }
+    }
+    __device__ __forceinline__ void apply(const W4gParams& P, const float4& s, float (&v)[4]) const {
+        if (P.in_sumsq == nullptr) return;
+        v[0] = fmaf(v[0], rstd, s.x);
+        v[1] = fmaf(v[1], rstd, s.y);
+        v[2] = fmaf(v[2], rstd, s.z);
+        v[3] = fmaf(v[3], rstd, s.w);
+    }
+    // y (this linear's output) -> h, and in `v` the next norm's input; returns the token's sum of h^2 over the tile's 128
+    // rows, which are the 32 lanes of a warp
+    __device__ __forceinline__ float residual(const W4gParams& P, float (&v)[4]) {
+        float r[4], s[4], ss = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = bf16r(v[e]);
+        if (P.gate != nullptr) {
+            float g[4];
+            unpack4(gate, g);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = bf16r(v[e] * g[e]);
+        }
+        if (P.res != nullptr) {
+            unpack4(res, r);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = bf16r(r[e] + v[e]);
+        }
+        h = pack4(v);
+        unpack4(scale, s);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            ss = fmaf(v[e], v[e], ss);
+            v[e] *= 1.0f + s[e];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        return ss;
+    }
+};
+
+// What the epilogue will read besides the sums, brought into the SM's L1 by one warp that has nothing else left to do: read
+// first behind the last barrier, these lines (some from HBM) were 1.2 us of a 6 us launch.  Vectors that are parameters of
+// the launch like the weights come before griddepcontrol.wait, rows of the launches before it behind it.
+__device__ __forceinline__ void touch_parameters(const W4gParams& P, int row_a, int row_b, int lane) {
+    const int row = (lane < 16 ? row_a : row_b) + (lane & 15) * 4;   // 64 rows from row_a, 64 from row_b
+    if (P.in_shift != nullptr && row < P.N && (lane & 7) == 0) touch(P.in_shift + row);
+    if (P.epilogue == kEpiResidual && (lane & 15) == 0) {
+        touch(P.scale + row);
+        if (P.gate != nullptr) touch(P.gate + row);
+    }
+}
+__device__ __forceinline__ void touch_rows(const W4gParams& P, int row_a, int m0, int m1, int lane) {
+    for (int m = m0 + lane; m < m1; m += 32) {
+        if (P.in_sumsq != nullptr) touch(P.in_sumsq + static_cast<size_t>(m) * P.in_parts);
+        if (P.epilogue == kEpiResidual && P.res != nullptr) {
+            touch(P.res + static_cast<size_t>(m) * P.N + row_a);
+            touch(P.res + static_cast<size_t>(m) * P.N + row_a + 64);
+        }
+        if (P.epilogue == kEpiQkv && row_a < P.q_dim + 256) {
+            const size_t p = static_cast<size_t>(P.positions[m]) * 128 + (row_a >> 7 & 1) * 64;
+            touch(P.rope_cos + p);
+            touch(P.rope_sin + p);
+        }
+    }
 }
 
 template <int kFmt>
@@ -316,6 +461,12 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                 if (lane < 2) tc::tma_load_2d(slot + lane * 8192, &P.map_w, kb * 128, lane ? row_b : row_a, &ctl.w_full[s]);
             }
             __syncwarp();
+        }
+        if (kFmt == kFmtNvfp4) {
+            touch_parameters(P, row_a, row_b, lane);
+            pdl_wait_prior_grids();
+            const int valid = min(P.nt, P.M - t0);
+            touch_rows(P, row_a, t0 + rank * valid / splits, t0 + (rank + 1) * valid / splits, lane);
         }
     } else if (warp == kMmaWarp) {
         // ------------------------------------------------------------ MMA issue
@@ -490,6 +641,15 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
         tc::fence_before_thread_sync();
     }
 
+    pdl_wait_prior_grids();                                          // a no-op by now; orders reads of `out` (beta) and of the norms' inputs
+    const int valid = min(P.nt, P.M - t0);
+    const int tb = rank * valid / splits, te = (rank + 1) * valid / splits;
+    // A unit of the epilogue is a token x 4 weight rows (4 + 4 where rows come in pairs): neighbouring lanes read and write
+    // neighbouring 16 and 8 bytes.
+    const bool pairs = P.epilogue == kEpiGated || P.epilogue == kEpiQkv;
+    const int per_token = pairs ? 16 : 32;
+    const int u_first = tb * per_token + threadIdx.x, u_end = te * per_token;
+
     if (splits > 1) {
         __syncwarp();
         cluster_arrive();
@@ -504,112 +664,103 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
     }
 
     // ---------------------------------------------------------------- this CTA's share of the tokens, all 128 rows
-    pdl_wait_prior_grids();                                          // a no-op by now; orders reads of `out` (beta)
     const bool failed = ctl.failed != 0;                             // then nothing is stored
     {
-        const int valid = min(P.nt, P.M - t0);
-        const int tb = rank * valid / splits, te = (rank + 1) * valid / splits;
         const uint32_t base = smem_u32(smem);
-        uint32_t peer[8];
-#pragma unroll
-        for (int p = 0; p < 8; ++p) peer[p] = p < splits && splits > 1 ? map_to_rank(base, p) : base;
-        auto sum8 = [&](int t, int c, float (&v)[8]) {
+        auto sum4 = [&](int t, int c, float (&v)[4]) {
             const uint32_t off = static_cast<uint32_t>((t * kRows + c) * 4);
-            float4 a, b;
-            if (splits == 1) {
-                a = *reinterpret_cast<const float4*>(smem + off);
-                b = *reinterpret_cast<const float4*>(smem + off + 16);
-            } else {
-                a = ld_cluster_f4(peer[0] + off);
-                b = ld_cluster_f4(peer[0] + off + 16);
-#pragma unroll
-                for (int p = 1; p < 8; ++p) {
-                    if (p < splits) {
-                        const float4 x = ld_cluster_f4(peer[p] + off), y = ld_cluster_f4(peer[p] + off + 16);
-                        a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
-                        b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
-                    }
-                }
-            }
+            float4 a;
+            if (splits == 1) a = *reinterpret_cast<const float4*>(smem + off);
+            else if (splits == 2) a = sum_ranks<2>(base, off, 2);
+            else if (splits <= 4) a = sum_ranks<4>(base, off, splits);
+            else a = sum_ranks<8>(base, off, splits);
             v[0] = a.x * P.alpha; v[1] = a.y * P.alpha; v[2] = a.z * P.alpha; v[3] = a.w * P.alpha;
-            v[4] = b.x * P.alpha; v[5] = b.y * P.alpha; v[6] = b.z * P.alpha; v[7] = b.w * P.alpha;
         };
-        if (P.epilogue == kEpiPlain) {
-            for (int u = tb * 16 + threadIdx.x; u < te * 16; u += static_cast<int>(blockDim.x)) {
-                const int t = u >> 4, c = (u & 15) * 8, n = row_a + c;
+        if (!pairs) {
+            for (int u = u_first; u < u_end; u += static_cast<int>(blockDim.x)) {
+                const int t = u >> 5, c = (u & 31) * 4, n = row_a + c;
                 if (n >= P.N) continue;                              // N is a multiple of 8
-                float v[8];
-                sum8(t, c, v);
+                float v[4];
+                NormUnit nu;
+                if (kFmt == kFmtNvfp4) nu.load<false>(P, t0 + t, n, 0);
+                sum4(t, c, v);
+                if (kFmt == kFmtNvfp4) nu.apply(P, nu.shift_a, v);
                 if (P.bias != nullptr) {
                     if (P.bias_dtype == TPB200_F32 && (reinterpret_cast<uintptr_t>(P.bias) & 15) == 0) {
-                        const float4* bp = reinterpret_cast<const float4*>(static_cast<const float*>(P.bias) + n);
-                        const float4 b0 = __ldg(bp), b1 = __ldg(bp + 1);
+                        const float4 b0 = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(P.bias) + n));
                         v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
-                        v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
                     } else {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] += load_as_float(P.bias, P.bias_dtype, n + e);
+                        for (int e = 0; e < 4; ++e) v[e] += load_as_float(P.bias, P.bias_dtype, n + e);
                     }
                 }
-                if (P.activation != TPB200_ACT_NONE) {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = act_fast(v[e], P.activation);
+                act4(v, P.activation);
+                if (kFmt == kFmtNvfp4 && P.epilogue == kEpiResidual) {
+                    // h = res + y * gate and the next norm's input h * (1 + scale), each rounded to bf16 (N % 128 == 0: all
+                    // 32 lanes are here)
+                    const float ss = nu.residual(P, v);
+                    if (failed) continue;
+                    *reinterpret_cast<uint2*>(P.h_out + static_cast<size_t>(t0 + t) * P.N + n) = nu.h;
+                    if ((threadIdx.x & 31) == 0) P.out_sumsq[static_cast<size_t>(t0 + t) * (P.N / kRows) + tile] = ss;
                 }
                 if (failed) continue;                                // asked here: the flag arrives beside the sums
                 const size_t o = static_cast<size_t>(t0 + t) * P.ldo + n;
                 if (P.beta != 0.0f) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = fmaf(P.beta, load_as_float(P.out, P.out_dtype, o + e), v[e]);
+                    for (int e = 0; e < 4; ++e) v[e] = fmaf(P.beta, load_as_float(P.out, P.out_dtype, o + e), v[e]);
                 }
                 if (P.out_dtype == TPB200_BF16) {
-                    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.out) + o) = pack8(v);
+                    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(P.out) + o) = pack4(v);
                 } else if (P.out_dtype == TPB200_F32) {
-                    float4* op = reinterpret_cast<float4*>(static_cast<float*>(P.out) + o);
-                    op[0] = make_float4(v[0], v[1], v[2], v[3]);
-                    op[1] = make_float4(v[4], v[5], v[6], v[7]);
+                    *reinterpret_cast<float4*>(static_cast<float*>(P.out) + o) = make_float4(v[0], v[1], v[2], v[3]);
                 } else {
-                    uint32_t h[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const __half2 h2 = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-                        h[e] = *reinterpret_cast<const uint32_t*>(&h2);
-                    }
-                    *reinterpret_cast<uint4*>(static_cast<__half*>(P.out) + o) = make_uint4(h[0], h[1], h[2], h[3]);
+                    const __half2 h0 = __floats2half2_rn(v[0], v[1]), h1 = __floats2half2_rn(v[2], v[3]);
+                    *reinterpret_cast<uint2*>(static_cast<__half*>(P.out) + o) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
                 }
             }
         } else if (P.epilogue == kEpiGated) {
             // gate rows 0..63, up rows 64..127 of the tile; the roundings of the module: both projections, the
             // activation and the product go to bf16
-            for (int u = tb * 8 + threadIdx.x; u < te * 8; u += static_cast<int>(blockDim.x)) {
-                const int t = u >> 3, c = (u & 7) * 8;
-                float g[8], up[8];
-                sum8(t, c, g);
-                sum8(t, c + 64, up);
+            for (int u = u_first; u < u_end; u += static_cast<int>(blockDim.x)) {
+                const int t = u >> 4, c = (u & 15) * 4;
+                float g[4], up[4];
+                NormUnit nu;
+                if (kFmt == kFmtNvfp4) nu.load<true>(P, t0 + t, row_a + c, row_b + c);
+                sum4(t, c, g);
+                sum4(t, c + 64, up);
+                if (kFmt == kFmtNvfp4) {
+                    nu.apply(P, nu.shift_a, g);
+                    nu.apply(P, nu.shift_b, up);
+                }
 #pragma unroll
-                for (int e = 0; e < 8; ++e) g[e] = bf16r(act_fast(bf16r(g[e]), P.activation)) * bf16r(up[e]);
+                for (int e = 0; e < 4; ++e) g[e] = bf16r(g[e]);
+                act4(g, P.activation);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) g[e] = bf16r(g[e]) * bf16r(up[e]);
                 if (failed) continue;
-                *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.out) + static_cast<size_t>(t0 + t) * P.ldo + row_a + c) =
-                    pack8(g);
+                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(P.out) + static_cast<size_t>(t0 + t) * P.ldo + row_a + c) =
+                    pack4(g);
             }
         } else {
             // rows 0..63 of the tile are head offsets i, rows 64..127 their rotate-half partners i + 128; the rotation
             // in bf16, each product and the sum rounded, as torch does it.  V heads pass through.
             const int head = tile >> 1, i0 = (tile & 1) * 64, heads = P.q_dim >> 8;
-            for (int u = tb * 8 + threadIdx.x; u < te * 8; u += static_cast<int>(blockDim.x)) {
-                const int t = u >> 3, c = (u & 7) * 8, m = t0 + t;
-                float lo[8], hi[8];
-                sum8(t, c, lo);
-                sum8(t, c + 64, hi);
-                uint32_t olo[4], ohi[4];
-                uint4 cv = make_uint4(0, 0, 0, 0), sv = cv;
-                if (head <= heads) {
-                    const size_t p = static_cast<size_t>(__ldg(P.positions + m)) * 128 + i0 + c;
-                    cv = __ldg(reinterpret_cast<const uint4*>(P.rope_cos + p));
-                    sv = __ldg(reinterpret_cast<const uint4*>(P.rope_sin + p));
+            for (int u = u_first; u < u_end; u += static_cast<int>(blockDim.x)) {
+                const int t = u >> 4, c = (u & 15) * 4, m = t0 + t;
+                float lo[4], hi[4];
+                NormUnit nu;
+                if (kFmt == kFmtNvfp4) nu.load<true>(P, m, row_a + c, row_b + c);
+                sum4(t, c, lo);
+                sum4(t, c + 64, hi);
+                if (kFmt == kFmtNvfp4) {
+                    nu.apply(P, nu.shift_a, lo);
+                    nu.apply(P, nu.shift_b, hi);
                 }
-                const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w}, sw[4] = {sv.x, sv.y, sv.z, sv.w};
+                uint32_t olo[2], ohi[2];
+                const uint32_t cw[2] = {nu.cos.x, nu.cos.y}, sw[2] = {nu.sin.x, nu.sin.y};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
+                for (int e = 0; e < 2; ++e) {
                     __nv_bfloat162 a = __floats2bfloat162_rn(lo[2 * e], lo[2 * e + 1]);
                     __nv_bfloat162 b = __floats2bfloat162_rn(hi[2 * e], hi[2 * e + 1]);
                     if (head <= heads) {
@@ -625,8 +776,8 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                 if (failed) continue;
                 __nv_bfloat16* dst = head < heads ? static_cast<__nv_bfloat16*>(P.out) + static_cast<size_t>(m) * P.ldq + head * 256
                                      : (head == heads ? P.k_rows : P.v_rows) + static_cast<size_t>(m) * 256;
-                *reinterpret_cast<uint4*>(dst + i0 + c) = make_uint4(olo[0], olo[1], olo[2], olo[3]);
-                *reinterpret_cast<uint4*>(dst + i0 + c + 128) = make_uint4(ohi[0], ohi[1], ohi[2], ohi[3]);
+                *reinterpret_cast<uint2*>(dst + i0 + c) = make_uint2(olo[0], olo[1]);
+                *reinterpret_cast<uint2*>(dst + i0 + c + 128) = make_uint2(ohi[0], ohi[1]);
             }
         }
     }
@@ -638,7 +789,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
     }
     if (splits > 1) {                                                // nobody leaves while a peer still reads its sums
         __syncwarp();
-        cluster_arrive();
+        cluster_arrive_relaxed();                                    // its loads have returned; the stores need not land first
         cluster_wait();
     }
 }
@@ -731,7 +882,7 @@ W4gRing ring_of(const W4gPlan& plan, int k_blocks, int k_steps) {
 int device_error_w4_gemm(int clear) { return read_device_error(clear); }
 
 // `transposed` (internal, TPB200_W4_NVFP4_ROWMAJOR only): w = [K / 2, N] code bytes, w_scales = [K / 16, N] UE4M3 bytes, N % 16 == 0
-int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool transposed) {
+int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool transposed, const tpb200_w4_norm_args* norm) {
     TPB_REQUIRE(a != nullptr && a->x != nullptr && a->w != nullptr && a->out != nullptr, TPB200_ERR_NULL);
     TPB_REQUIRE(a->format >= TPB200_W4_NVFP4_ROWMAJOR && a->format <= TPB200_W4_INT4_PLUGIN, TPB200_ERR_ENUM);
     TPB_REQUIRE((a->flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
@@ -767,7 +918,36 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
         TPB_REQUIRE(a->ldo >= N, TPB200_ERR_SHAPE);
         TPB_REQUIRE(static_cast<long long>(a->ldo) * tpb_dtype_size(a->out_dtype) % 16 == 0, TPB200_ERR_ALIGN);
     }
+    const bool norm_in = norm != nullptr && norm->in_sumsq != nullptr, norm_out = norm != nullptr && norm->h_out != nullptr;
+    if (norm_in) {
+        TPB_REQUIRE(nv, TPB200_ERR_ENUM);
+        TPB_REQUIRE(norm->in_parts >= 4 && norm->in_parts % 4 == 0, TPB200_ERR_SHAPE);
+        TPB_REQUIRE(tpb_aligned16(norm->in_sumsq) && tpb_aligned16(norm->in_shift), TPB200_ERR_ALIGN);
+    }
+    if (norm_out) {
+        TPB_REQUIRE(nv && !qkv && !gated && a->out_dtype == TPB200_BF16 && a->activation == TPB200_ACT_NONE && a->beta == 0.0f,
+                    TPB200_ERR_ENUM);
+        TPB_REQUIRE(norm->scale != nullptr && norm->out_sumsq != nullptr, TPB200_ERR_NULL);
+        TPB_REQUIRE(N % kRows == 0, TPB200_ERR_SHAPE);
+        TPB_REQUIRE(tpb_aligned16(norm->h_out) && tpb_aligned16(norm->res_in) && tpb_aligned16(norm->gate) &&
+                        tpb_aligned16(norm->scale),
+                    TPB200_ERR_ALIGN);
+    }
     W4gParams P = {};
+    if (norm_in) {
+        P.in_sumsq = norm->in_sumsq;
+        P.in_shift = norm->in_shift;
+        P.in_parts = norm->in_parts;
+        P.in_eps = norm->in_eps;
+        P.in_inv_k = 1.0f / static_cast<float>(K);
+    }
+    if (norm_out) {
+        P.res = static_cast<const __nv_bfloat16*>(norm->res_in);
+        P.gate = static_cast<const __nv_bfloat16*>(norm->gate);
+        P.scale = static_cast<const __nv_bfloat16*>(norm->scale);
+        P.h_out = static_cast<__nv_bfloat16*>(norm->h_out);
+        P.out_sumsq = norm->out_sumsq;
+    }
     TPB_REQUIRE(!transposed || (a->format == TPB200_W4_NVFP4_ROWMAJOR && !qkv && !gated && N % 16 == 0), TPB200_ERR_ENUM);
     const int fmt = transposed ? kFmtNvfp4T : nv ? kFmtNvfp4 : a->format == TPB200_W4_INT4_KBLOCK ? kFmtKblock : kFmtPlugin;
     const int tiles = (N + kRows - 1) / kRows;
@@ -813,7 +993,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     P.M = M;
     P.N = N;
     P.K = K;
-    P.epilogue = qkv ? kEpiQkv : gated ? kEpiGated : kEpiPlain;
+    P.epilogue = qkv ? kEpiQkv : gated ? kEpiGated : norm_out ? kEpiResidual : kEpiPlain;
     P.gated_rows = N / 2;
     P.q_dim = a->qkv_q_dim;
     P.ldq = a->ldo;
@@ -870,7 +1050,12 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
 }  // namespace tpb
 
 extern "C" int tpb200_w4_gemm(const tpb200_w4_gemm_args* a, tpb200_stream_t stream) {
-    return tpb::w4_gemm_launch(a, reinterpret_cast<cudaStream_t>(stream), false);
+    return tpb::w4_gemm_launch(a, reinterpret_cast<cudaStream_t>(stream), false, nullptr);
+}
+
+extern "C" int tpb200_w4_gemm_norm(const tpb200_w4_gemm_args* a, const tpb200_w4_norm_args* norm, tpb200_stream_t stream) {
+    TPB_REQUIRE(norm != nullptr, TPB200_ERR_NULL);
+    return tpb::w4_gemm_launch(a, reinterpret_cast<cudaStream_t>(stream), false, norm);
 }
 
 extern "C" int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_plan_info* info) {
@@ -907,5 +1092,5 @@ extern "C" int tpb200_w4a16_gemm(const void* x, const void* weight, const void* 
     a.N = N;
     a.K = K;
     a.flags = flags;
-    return tpb::w4_gemm_launch(&a, reinterpret_cast<cudaStream_t>(stream), false);
+    return tpb::w4_gemm_launch(&a, reinterpret_cast<cudaStream_t>(stream), false, nullptr);
 }

@@ -445,9 +445,12 @@ def w4_gemm(x, w, N, format, w_scales=None, w_zeros=None, alpha=1.0, beta=0.0, b
     return out
 
 
-def _w4_gemm(args, device):
+def _w4_gemm(args, device, norm=None):
     args.flags = _flags.value
-    st = _run_on(device, _lib.load().tpb200_w4_gemm, args)
+    if norm is None:
+        st = _run_on(device, _lib.load().tpb200_w4_gemm, args)
+    else:
+        st = _run_on(device, _lib.load().tpb200_w4_gemm_norm, args, norm)
     _lib.check(st, "tpb200_w4_gemm")
 
 

@@ -136,14 +136,15 @@ class TcLinear:
                                w=p(self.b), w_pitch=self.b.stride(0) if self.rowmajor else 0, w_scales=p(self.sf),
                                alpha=float(self.g), out=p(out), out_dtype=ops._dt(out), ldo=ldo, M=M, N=self.N, K=self.K)
 
-    def dense(self, x, out, activation=ACT_NONE, gated=False):
-        """out = act(x W^T + bias) for bf16 x [M, >= K]; `gated`: W = [gate; up], out = act(gate) * up."""
+    def dense(self, x, out, activation=ACT_NONE, gated=False, norm=None, bias=True):
+        """out = act(x W^T + bias) for bf16 x [M, >= K]; `gated`: W = [gate; up], out = act(gate) * up.  `norm`
+        (_lib.W4NormArgs): the RMS norms around the linear, see tpb200_w4_gemm_norm."""
         args = self._w4_args(x, x.shape[0], out, out.stride(0))
-        args.bias, args.activation, args.gated = ops._ptr(self.bias), int(activation), int(gated)
-        ops._w4_gemm(args, out.device)
+        args.bias, args.activation, args.gated = ops._ptr(self.bias if bias else None), int(activation), int(gated)
+        ops._w4_gemm(args, out.device, norm)
         return out
 
-    def dense_qkv(self, x, q_out, k_rows, v_rows, positions, cos, sin, q_dim):
+    def dense_qkv(self, x, q_out, k_rows, v_rows, positions, cos, sin, q_dim, norm=None):
         M = x.shape[0]
         if k_rows.shape[0] < M or v_rows.shape[0] < M or positions.numel() < M:
             raise TurboPiError("fused QKV: cache rows / positions shorter than the token count")
@@ -151,7 +152,7 @@ class TcLinear:
         args = self._w4_args(x, M, q_out, q_out.stride(0))
         args.qkv_q_dim, args.qkv_k_rows, args.qkv_v_rows, args.qkv_positions = q_dim, p(k_rows), p(v_rows), p(positions)
         args.qkv_rope_cos, args.qkv_rope_sin = p(cos), p(sin)
-        ops._w4_gemm(args, q_out.device)
+        ops._w4_gemm(args, q_out.device, norm)
         return q_out
 
 
@@ -195,7 +196,10 @@ class Pi05:
         self._graph = None
         self._graph_steps = None
         self._time_emb = {}
-        self._mod = {}            # per step count: the adaptive norms' modulation table
+        self._mod = {}            # per step count: the adaptive norms' modulation tables
+        # The expert's norms ride in the epilogues of the linears around them where a row's sums of squares come in
+        # whole 16-byte groups of 128-column parts; other widths take the row kernel between two linears.
+        self.fold_norms = cfg.expert_width % 512 == 0 and cfg.expert_mlp % 64 == 0
         self.set_valid()
 
     @classmethod
@@ -403,6 +407,7 @@ class Pi05:
             ex=torch.empty((A, ew), dtype=bf, device=d), e_q=torch.empty((A, c.q_dim), dtype=bf, device=d),
             e_attn=torch.empty((A, c.q_dim), dtype=bf, device=d), e_mlp=torch.empty((A, c.expert_mlp), dtype=bf, device=d),
             e_gu=torch.empty((A if c.expert_mlp % 64 else 0, 2 * c.expert_mlp), dtype=bf, device=d),
+            e_ss=torch.empty((A, max(1, ew // 128)), dtype=torch.float32, device=d),
             v_out=torch.empty((A, c.action_dim), dtype=torch.float32, device=d),
             pos_suffix=torch.arange(S, S + A, dtype=torch.int32, device=d),
         )
@@ -532,11 +537,50 @@ class Pi05:
         self.ada_dense.dense(t1[1], mod)
         return mod.view(num_steps, self.n_norms, 3, ew)
 
-    def denoise_step(self, mod, dt):
-        """One Euler step: v = expert(x_t | cache); x_t += dt * v."""
+    def _shifts(self, mod):
+        """W * shift of every linear behind an adaptive norm, per step: what is left of the norm's shift when its RMS
+        factor is applied behind the linear.  fp32, alpha included; rows in the order of the weights."""
+        c, n = self.cfg, mod.shape[0]
+
+        def through(lin, norm, bias=False):
+            return lin.dense(mod[:, norm, 1], torch.empty((n, lin.N), dtype=torch.float32, device=self.device), bias=bias)
+        return dict(qkv=[through(L["qkv"], 2 * l) for l, L in enumerate(self.expert)],
+                    gate_up=[through(L["gate_up"], 2 * l + 1) for l, L in enumerate(self.expert)],
+                    out=through(self.action_out, 2 * c.expert_layers, bias=True))
+
+    def _norm_in(self, shift):
+        b, c = self.b, self.cfg
+        return _lib.W4NormArgs(in_sumsq=ops._ptr(b["e_ss"]), in_shift=ops._ptr(shift), in_parts=c.expert_width // 128, in_eps=c.eps)
+
+    def _norm_out(self, scale, gate=None, first=False):
+        b, p = self.b, ops._ptr
+        return _lib.W4NormArgs(res_in=0 if first else p(b["eh"]), gate=p(gate), scale=p(scale), h_out=p(b["eh"]),
+                               out_sumsq=p(b["e_ss"]))
+
+    def denoise_step(self, mod, dt, shift=None):
+        """One Euler step: v = expert(x_t | cache); x_t += dt * v.  `shift` (one row per linear, `_shifts`): the norms run in
+        the epilogues of the linears around them; None: in row kernels between the linears."""
         c, b = self.cfg, self.b
         S, A, ew = c.prefix_len, c.action_horizon, c.expert_width
         b["x_bf"].copy_(b["x_t"])
+        if shift is None:
+            self._expert_with_row_kernels(mod)
+        else:
+            self.action_in.dense(b["x_bf"], b["ex"], norm=self._norm_out(mod[0, 0], first=True))
+            for l, L in enumerate(self.expert):
+                m_in, m_post = mod[2 * l], mod[2 * l + 1]
+                L["qkv"].dense_qkv(b["ex"], b["e_q"], self.cache[l, 0, S:], self.cache[l, 1, S:], b["pos_suffix"], self.cos,
+                                   self.sin, c.q_dim, norm=self._norm_in(shift["qkv"][l]))
+                self._attention(b["e_q"], self.cache[l, 0, :S + A], self.cache[l, 1, :S + A], b["e_attn"])
+                L["o"].dense(b["e_attn"], b["ex"], norm=self._norm_out(m_post[0], m_in[2]))
+                L["gate_up"].dense(b["ex"], b["e_mlp"], ACT_GELU, gated=True, norm=self._norm_in(shift["gate_up"][l]))
+                L["down"].dense(b["e_mlp"], b["ex"], norm=self._norm_out(mod[2 * l + 2, 0], m_post[2]))
+            self.action_out.dense(b["ex"], b["v_out"], norm=self._norm_in(shift["out"]), bias=False)
+        b["x_t"].add_(b["v_out"], alpha=dt)
+
+    def _expert_with_row_kernels(self, mod):
+        c, b = self.cfg, self.b
+        S, A, ew = c.prefix_len, c.action_horizon, c.expert_width
         self.action_in.dense(b["x_bf"], b["eh"])
         prev_gate = None
         for l, L in enumerate(self.expert):
@@ -563,7 +607,6 @@ class Pi05:
         rowop(_lib.ROW_ADARMS, b["ey"], ew, y_out=b["ex"], res_in=b["eh"], gate=prev_gate, h_out=b["eh"], w0=m_f[0], w1=m_f[1],
               eps=c.eps)
         self.action_out.dense(b["ex"], b["v_out"])
-        b["x_t"].add_(b["v_out"], alpha=dt)
 
     def _modulation(self, num_steps):
         """The adaptive norms' (scale, shift, gate) for every step of an `num_steps` schedule.  They depend on
@@ -574,15 +617,18 @@ class Pi05:
         if mod is None:
             if torch.cuda.is_current_stream_capturing():
                 raise TurboPiError("the modulation table of a new schedule must be built before the capture")
-            mod = self._mod[num_steps] = self._ada_modulation(num_steps)
+            mod = self._ada_modulation(num_steps)
+            mod = self._mod[num_steps] = (mod, self._shifts(mod) if self.fold_norms else None)
         return mod
 
     def denoise_loop(self, num_steps):
-        mod = self._modulation(num_steps)
+        mod, shift = self._modulation(num_steps)
         self.b["x_t"].copy_(self.noise)
         dt = -1.0 / num_steps
         for i in range(num_steps):
-            self.denoise_step(mod[i], dt)
+            at = None if shift is None else dict(qkv=[s[i] for s in shift["qkv"]], gate_up=[s[i] for s in shift["gate_up"]],
+                                                 out=shift["out"][i])
+            self.denoise_step(mod[i], dt, at)
         self.actions.copy_(self.b["x_t"])
 
     def forward(self, num_steps):
