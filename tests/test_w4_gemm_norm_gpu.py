@@ -89,3 +89,24 @@ def test_residual_behind(cuda_device, M, N, K, with_res, with_gate):
     ref = want.double().square().view(M, -1, 128).sum(2)
     assert bool(((ss.double() - ref).abs() <= 128 * 2.0 ** -24 * ref).all())
     assert _lib.load().tpb200_device_error(0) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(33, 8, 16), (65, 136, 2064), (100, 4304, 1152), (241, 264, 528), (712, 2560, 2176)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_tiles_stored_from_tensor_memory(cuda_device, M, N, K, dtype):
+    """Unsplit plain tiles: ragged token and row tiles, a K whose last operand step has parts past its end, strided rows."""
+    from turbopi_b200 import _lib, ops
+    b, sf, w = _nvfp4(N, K, cuda_device, M + N + K)
+    g = torch.Generator().manual_seed(N)
+    x = torch.randn((M, K), generator=g).to(torch.bfloat16).to(cuda_device)
+    bias = torch.randn(N, generator=g).to(cuda_device)
+    out = torch.full((M + 1, N + 8), 7.0, dtype=dtype, device=cuda_device)
+    ops.w4_gemm(x, b, N, _lib.W4_NVFP4_ROWMAJOR, sf, alpha=2.0 ** -8, bias=bias, activation=_lib.ACT_SILU, out=out[:M, :N])
+    z = 2.0 ** -8 * (x.double() @ w.t()) + bias.double()
+    mag = 2.0 ** -8 * (x.double().abs() @ w.abs().t()) + bias.double().abs()
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -21}[dtype]
+    # SiLU's slope is at most 1.1; the hardware exponential and division are good to 2^-20 of the result
+    _check(out[:M, :N], torch.nn.functional.silu(z), 1.1 * mag + 1e-2, eps + 2.0 ** -20)
+    assert bool((out[M] == 7).all()) and bool((out[:, N:] == 7).all())
+    assert _lib.load().tpb200_device_error(0) == 0

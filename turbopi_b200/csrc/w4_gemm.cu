@@ -48,12 +48,14 @@ constexpr int kCodeBytes = kRows * kBlkK / 2;    // 16 KB
 constexpr int kWSlot = kCodeBytes + 2 * kSlabBytes;
 constexpr int kMaxW = 4, kMaxS = 14;
 constexpr int kXWarp = 0, kMmaWarp = 1, kWWarp = 2, kDqWarp0 = 3;
-constexpr int kDqWarpsPerSm = 16;                // 16 dequantisation warps with an SM of its own, 8 with two CTAs per SM
 constexpr long long kWaitG = 400000000LL;        // ~0.2 s
 constexpr long long kLandCycles = 2000000LL;     // ~1 ms
 
 enum { kFmtNvfp4 = 0, kFmtKblock = 1, kFmtPlugin = 2, kFmtNvfp4T = 3 };   // 3: the w4a8 plugin's transposed operand
-enum { kEpiPlain = 0, kEpiQkv = 1, kEpiGated = 2, kEpiResidual = 3 };
+// Epilogues.  Direct (K not split, no partner rows) has a kernel of its own, the others share one: a chain of short launches
+// fetches its instructions anew unless the launches before ran the same ones.  All five in one kernel cost the 50-token
+// launches 0.6 us each, a kernel for each of the five 0.4.
+enum { kEpiDirect = 0, kEpiSplit = 1, kEpiResidual = 2, kEpiGated = 3, kEpiQkv = 4 };
 
 struct W4gParams {
     CUtensorMap map_x;                           // bf16 [M, K], box 64 x NT, 128-byte swizzle
@@ -72,7 +74,8 @@ struct W4gParams {
     int nt;                                      // tokens per tile
     int splits;                                  // CTAs (cluster size) per tile, each with a K range
     int k_blocks, k_steps;
-    int parts;                                   // 64-K parts per operand step: 1, or 2 for narrow token tiles
+    int parts;                                   // consecutive 64-K parts a group of warps dequantises: 1, or 2 for narrow token tiles
+    int merge;                                   // such units per operand step (what one barrier hands to the tensor cores)
     int n_w, n_s;                                // ring depths: weight blocks, operand steps
     int tmem_cols, a_col;
     int epilogue;
@@ -125,6 +128,14 @@ __device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
         "}\n" ::"r"(tmem_d),
         "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc)
         : "memory");
+}
+
+// the four K = 16 products of one 64-K part; `acc` = 0: the first of them starts the sum
+__device__ __forceinline__ void mma_part(uint32_t tmem_d, uint32_t a_col, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        mma_bf16_ts(tmem_d, a_col + kk * 8, tc::desc_from_words(b_lo + kk * 2, tc::kDescHiKmajorSw128), idesc, kk > 0 ? 1u : acc);
+    }
 }
 
 __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -352,28 +363,117 @@ __device__ __forceinline__ void touch_rows(const W4gParams& P, int row_a, int m0
     }
 }
 
-template <int kFmt>
+// Tiles that no other CTA adds to go from tensor memory to the result by the warps that hold them, without a barrier.  A
+// warp has 32 rows of W (its lanes) for 32 tokens; 16-bit results are turned through 2 KB of its own shared memory so that
+// a lane stores 8 neighbouring rows of a token: a 128 x 240 tile is 128 stores of 512 bytes a warp.  (The tile staged as
+// fp32, a barrier and a second pass over it: 4.0 us of the tile's 18; 16 stores of 64 bytes straight from the
+// registers: 3.2; this: 2.3.)
+// kDtype -1: any type, with beta.
+template <int kDtype>
+__device__ __forceinline__ void store_columns(const W4gParams& P, uint32_t lane_addr, int c_first, int c_step, int t0, int valid,
+                                              int row0, float bias, uint8_t* buf, int lane) {
+    auto result = [&](int col, float (&v)[16]) {                             // 16 columns at a time: 64 registers a thread in all
+        uint32_t raw[16];
+        tmem_ld_32x32b_x16(lane_addr + col, raw);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = fmaf(__uint_as_float(raw[e]), P.alpha, bias);
+        if (P.activation == TPB200_ACT_GELU) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] = act_fast(v[e], TPB200_ACT_GELU);
+        } else if (P.activation == TPB200_ACT_SILU) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] = act_fast(v[e], TPB200_ACT_SILU);
+        }
+    };
+    // 16-byte chunk c (8 tokens) of row n lies at c ^ key(n): the lanes' stores and the transposing loads hit all banks
+    auto key = [](int n) { return ((n >> 3) ^ (n >> 1)) & 3; };
+    const int tn = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);     // the row whose address this lane gives to ldmatrix
+    for (int c0 = c_first; c0 < valid; c0 += c_step) {
+        if constexpr (kDtype == TPB200_BF16 || kDtype == TPB200_F16) {
+            __syncwarp();
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float v[16];
+                result(c0 + 16 * half, v);
+                uint32_t w[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    if (kDtype == TPB200_BF16) {
+                        w[e] = bits(__floats2bfloat162_rn(v[2 * e], v[2 * e + 1]));
+                    } else {
+                        const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+                        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    *reinterpret_cast<uint4*>(buf + lane * 64 + (((2 * half + c) ^ key(lane)) << 4)) =
+                        make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+                }
+            }
+            __syncwarp();
+            const int n = row0 + 8 * (lane & 3);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                uint32_t q[4];
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3])
+                             : "r"(smem_u32(buf + tn * 64 + ((c ^ key(tn)) << 4)))
+                             : "memory");
+                const int t = c0 + 8 * c + (lane >> 2);
+                if (t < valid && n < P.N) {                          // N is a multiple of 8
+                    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(P.out) + static_cast<size_t>(t0 + t) * P.ldo + n) =
+                        make_uint4(q[0], q[1], q[2], q[3]);
+                }
+            }
+        } else {
+            for (int half = 0; half < 2; ++half) {
+                float v[16];
+                result(c0 + 16 * half, v);
+                size_t o = static_cast<size_t>(t0 + c0 + 16 * half) * P.ldo + row0 + lane;
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    if (row0 + lane < P.N && c0 + 16 * half + e < valid) {
+                        if (kDtype == TPB200_F32) {
+                            static_cast<float*>(P.out)[o] = v[e];
+                        } else {
+                            const float y = fmaf(P.beta, load_as_float(P.out, P.out_dtype, o), v[e]);
+                            if (P.out_dtype == TPB200_BF16) static_cast<__nv_bfloat16*>(P.out)[o] = __float2bfloat16_rn(y);
+                            else if (P.out_dtype == TPB200_F16) static_cast<__half*>(P.out)[o] = __float2half_rn(y);
+                            else static_cast<float*>(P.out)[o] = y;
+                        }
+                    }
+                    o += P.ldo;
+                }
+            }
+        }
+    }
+}
+
+template <int kFmt, bool kDirect>
 __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sW = smem;                                              // [n_w][16 KB codes | 2 scale slabs]
     uint8_t* sB = sW + P.n_w * kWSlot;                               // [n_b][nt rows of 128 bytes]
-    const int part_bytes = P.nt * 128, b_bytes = part_bytes * P.parts;
+    const int part_bytes = P.nt * 128, step_parts = P.parts * P.merge, b_bytes = part_bytes * step_parts;
     __shared__ W4gControl ctl;
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform, and known to be
-    const int splits = P.splits;
+    const int splits = kDirect ? 1 : P.splits;
     const int tile = blockIdx.x / splits;
     const int rank = blockIdx.x - tile * splits;                     // K range
     const int groups = ((blockDim.x >> 5) - kDqWarp0) >> 2;          // of four dequantisation warps
     const int t0 = blockIdx.y * P.nt;                                // first token
     const int blk0 = rank * P.k_blocks / splits, blk1 = (rank + 1) * P.k_blocks / splits;
     const int nblk = blk1 - blk0;
-    const int parts = P.parts;                                       // a step past the end of K multiplies zeros
-    const int steps = (min(blk1 * 4, P.k_steps) - blk0 * 4 + parts - 1) / parts;
+    const int parts = P.parts, merge = P.merge;                      // a part past the end of K multiplies zeros
+    const int steps = (min(blk1 * 4, P.k_steps) - blk0 * 4 + step_parts - 1) / step_parts;
     // weight rows of the tile: rows 0..63 start at row_a, 64..127 at row_b (apart only in the gated form)
-    const int row_a = P.epilogue == kEpiGated ? tile * 64 : tile * kRows;
-    const int row_b = P.epilogue == kEpiGated ? P.gated_rows + row_a : row_a + 64;
+    const bool gated = !kDirect && kFmt == kFmtNvfp4 && P.epilogue == kEpiGated;
+    const int row_a = gated ? tile * 64 : tile * kRows;
+    const int row_b = gated ? P.gated_rows + row_a : row_a + 64;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.n_w; ++s) {
@@ -381,7 +481,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
             mbar_init(&ctl.w_empty[s], 16 / P.parts);                // 4 or 2 steps x 4 warps
         }
         for (int s = 0; s < P.n_s; ++s) {
-            mbar_init(&ctl.full[s], 5);                              // the activation tile and four dequantising warps
+            mbar_init(&ctl.full[s], 1 + 4 * merge);                  // the activation tiles and four dequantising warps a unit
             mbar_init(&ctl.empty[s], 1);
         }
         mbar_init(&ctl.acc_full, 1);
@@ -412,8 +512,9 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                     break;
                 }
                 mbar_expect_tx(&ctl.full[s], b_bytes);
-                for (int u = 0; u < parts; ++u) {
-                    tc::tma_load_2d(sB + s * b_bytes + u * part_bytes, &P.map_x, (blk0 * 4 + i * parts + u) * kPartK, t0, &ctl.full[s]);
+                for (int u = 0; u < step_parts; ++u) {
+                    tc::tma_load_2d(sB + s * b_bytes + u * part_bytes, &P.map_x, (blk0 * 4 + i * step_parts + u) * kPartK, t0,
+                                    &ctl.full[s]);
                 }
                 if (++s == P.n_s) { s = 0; ph ^= 1; }
             }
@@ -421,7 +522,6 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
     } else if (warp == kWWarp) {
         // ------------------------------------------------------------ weight blocks
         const uint64_t policy = l2_policy_evict_first();
-        const bool gated = P.epilogue == kEpiGated;
         const uint32_t bytes = kFmt == kFmtNvfp4 ? (gated ? kCodeBytes + 2 * kSlabBytes : kCodeBytes + kSlabBytes)
                                : kFmt == kFmtNvfp4T || (kFmt == kFmtKblock && P.kb_scale == nullptr) ? kCodeBytes + kSlabBytes
                                                                                                       : kCodeBytes;
@@ -462,7 +562,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
             }
             __syncwarp();
         }
-        if (kFmt == kFmtNvfp4) {
+        if (kFmt == kFmtNvfp4 && !kDirect) {
             touch_parameters(P, row_a, row_b, lane);
             pdl_wait_prior_grids();
             const int valid = min(P.nt, P.M - t0);
@@ -484,19 +584,13 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                     break;
                 }
                 tc::fence_after_thread_sync();
-                const uint32_t a_col = tm + P.a_col + s * 32 * parts, b_lo = b16 + ((s * b_bytes) >> 4);
+                const uint32_t a_col = tm + P.a_col + s * 32 * step_parts, b_lo = b16 + ((s * b_bytes) >> 4), pb = part_bytes >> 4;
                 if (tc::elect_one()) {
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        mma_bf16_ts(tm, a_col + kk * 8, tc::desc_from_words(b_lo + kk * 2, tc::kDescHiKmajorSw128), idesc,
-                                    (i > 0 || kk > 0) ? 1u : 0u);
-                    }
-                    if (parts == 2) {
-                        const uint32_t b_lo2 = b_lo + (part_bytes >> 4);
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            mma_bf16_ts(tm, a_col + 32 + kk * 8, tc::desc_from_words(b_lo2 + kk * 2, tc::kDescHiKmajorSw128), idesc, 1u);
-                        }
+                    mma_part(tm, a_col, b_lo, idesc, i > 0 ? 1u : 0u);
+                    if (step_parts >= 2) mma_part(tm, a_col + 32, b_lo + pb, idesc, 1u);
+                    if (step_parts == 4) {
+                        mma_part(tm, a_col + 64, b_lo + 2 * pb, idesc, 1u);
+                        mma_part(tm, a_col + 96, b_lo + 3 * pb, idesc, 1u);
                     }
                     tc::commit(&ctl.empty[s]);
                 }
@@ -511,28 +605,41 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
         const int r = (warp & 3) * 32 + lane;                        // the lanes of tensor memory this warp can reach
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         const int row = r < 64 ? row_a + r : row_b + r - 64;
-        const int sf_off = (r >= 64 && P.epilogue == kEpiGated ? kSlabBytes : 0) + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+        const int sf_off = (r >= 64 && gated ? kSlabBytes : 0) + (row & 31) * 16 + ((row >> 5) & 3) * 4;
         bool ok = true;
         float psc[2] = {0.0f, 0.0f}, pzp[2] = {0.0f, 0.0f};
-        // ring positions and phases of this group's steps (kept by counting: four integer divisions a step would cost a
-        // third of the dequantisation's instructions)
-        int sw = 0, wph = 0, last_j = 0, sa = grp, sph = 1;
-        while (sa >= P.n_s) { sa -= P.n_s; sph ^= 1; }
-        for (int i = grp; i < steps; i += groups) {
-            const int j = i * parts >> 2;
-            while (last_j < j) {
-                ++last_j;
-                if (++sw == P.n_w) { sw = 0; wph ^= 1; }
+        // Ring positions and phases of this group's units, kept by counting: the loop is bound by instruction issue (of ~420
+        // instructions per part and warp once, 220 were the arithmetic).
+        int sw = 0, wph = 0, next_j = 1, sa = 0, sub = grp, sph = 1;   // weight slot and phase; operand slot, unit in it, empty phase
+        bool fresh = true;                                           // no operand slot has been used twice yet
+        auto settle = [&] {
+            while (sub >= merge) {
+                sub -= merge;
+                if (++sa == P.n_s) { sa = 0; sph ^= 1; fresh = false; }
             }
+        };
+        settle();
+        const uint32_t code_off = kFmt == kFmtKblock ? r * 16 : r * 128 + ((r & 7) << 4);
+        const int live = P.k_steps - blk0 * 4;                       // parts before the end of K
+        uint8_t* slot = sW;
+        for (int i = grp; i < steps * merge; i += groups) {
+            const int p0 = i * parts;
+            while (next_j <= p0 >> 2) {
+                ++next_j;
+                slot += kWSlot;
+                if (++sw == P.n_w) { sw = 0; wph ^= 1; slot = sW; }
+            }
+            // asked before the arithmetic, used behind it: by then the slot is mostly free and the answer there
+            const bool slot_free = fresh || mbar_test_wait(&ctl.empty[sa], sph);
             if (!mbar_wait_bounded(&ctl.w_full[sw], wph, kWaitG)) ok = false;
             for (int u = 0; u < parts; ++u) {
-                const int kk = (i * parts + u) & 3;
-                if (kFmt == kFmtPlugin && row < P.N) {                   // two scales per 256 K, straight from global memory
-                    const size_t g = static_cast<size_t>(row) * (P.K / 128) + (blk0 + j) * 2 + (kk >> 1);
+                const int kk = (p0 + u) & 3;
+                const bool past = p0 + u >= live;                    // of an operand step's last parts only: zeros
+                if (kFmt == kFmtPlugin && row < P.N && !past) {          // two scales per 256 K, straight from global memory
+                    const size_t g = static_cast<size_t>(row) * (P.K / 128) + (blk0 + (p0 >> 2)) * 2 + (kk >> 1);
                     psc[0] = __bfloat162float(__ldg(P.pl_scale + g));
                     pzp[0] = P.pl_zero != nullptr ? __bfloat162float(__ldg(P.pl_zero + g)) : 0.0f;
                 }
-                const uint8_t* slot = sW + sw * kWSlot;
                 uint32_t out[32];
                 uint4 c[2];
                 if (kFmt == kFmtNvfp4T) {                            // a row's codes lie 128 bytes apart
@@ -543,11 +650,13 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                         cw[wd] = p4[0] | p4[kRows] << 8 | p4[2 * kRows] << 16 | static_cast<uint32_t>(p4[3 * kRows]) << 24;
                     }
                 } else if (kFmt == kFmtKblock) {
-                    c[0] = *reinterpret_cast<const uint4*>(slot + (2 * kk) * 2048 + r * 16);
-                    c[1] = *reinterpret_cast<const uint4*>(slot + (2 * kk + 1) * 2048 + r * 16);
-                } else {
-                    c[0] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk) ^ (r & 7)) << 4));
-                    c[1] = *reinterpret_cast<const uint4*>(slot + r * 128 + (((2 * kk + 1) ^ (r & 7)) << 4));
+                    const uint8_t* p16 = slot + code_off + kk * 4096;
+                    c[0] = *reinterpret_cast<const uint4*>(p16);
+                    c[1] = *reinterpret_cast<const uint4*>(p16 + 2048);
+                } else {                                             // 16-byte chunks 2 kk, 2 kk + 1 of the row, each XOR r & 7
+                    const uint32_t o16 = code_off ^ (kk << 5);
+                    c[0] = *reinterpret_cast<const uint4*>(slot + o16);
+                    c[1] = *reinterpret_cast<const uint4*>(slot + (o16 ^ 16));
                 }
                 uint32_t sc = 0;
                 if (kFmt == kFmtNvfp4) sc = *reinterpret_cast<const uint32_t*>(slot + kCodeBytes + kk * 512 + sf_off);
@@ -560,11 +669,16 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                         const __half* sp = reinterpret_cast<const __half*>(slot + kCodeBytes) + (2 * kk) * kRows + r;
                         psc[0] = __half2float(sp[0]);
                         psc[1] = __half2float(sp[kRows]);
-                    } else if (row < P.N) {
-                        const __half* sp = P.kb_scale + static_cast<size_t>((blk0 + j) * 8 + 2 * kk) * P.N + row;
+                    } else if (row < P.N && !past) {
+                        const __half* sp = P.kb_scale + static_cast<size_t>((blk0 + (p0 >> 2)) * 8 + 2 * kk) * P.N + row;
                         psc[0] = __half2float(__ldg(sp));
                         psc[1] = __half2float(__ldg(sp + P.N));
                     }
+                }
+                if (past) {                                          // codes and scales of zero: zeros, whatever the slot holds
+                    c[0] = c[1] = make_uint4(0, 0, 0, 0);
+                    sc = 0;
+                    psc[0] = psc[1] = pzp[0] = 0.0f;
                 }
                 if (u == parts - 1) {
                     __syncwarp();
@@ -599,13 +713,13 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
                     }
                 }
                 if (u == 0) {                                        // the arithmetic above needs no free slot
-                    if (i >= P.n_s && !mbar_wait_bounded(&ctl.empty[sa], sph, kWaitG)) ok = false;
+                    if (!slot_free && !mbar_wait_bounded(&ctl.empty[sa], sph, kWaitG)) ok = false;
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc::fence_after_thread_sync();
                 }
                 __syncwarp();                                        // lane 0 may be behind: it has arrived on w_empty
-                tmem_st_32x32b_x32(lane_addr + P.a_col + (sa * parts + u) * 32, out);
+                tmem_st_32x32b_x32(lane_addr + P.a_col + (sa * step_parts + sub * parts + u) * 32, out);
             }
             if (!ok) {
                 if (lane == 0) give_up(ctl, kErrGemmEmptyBarrierTimeout);
@@ -615,10 +729,15 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
             tc::fence_before_thread_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl.full[sa]);
-            sa += groups;
-            while (sa >= P.n_s) { sa -= P.n_s; sph ^= 1; }
+            sub += groups;
+            settle();
         }
-        // ------------------------------------------------------------ accumulator -> shared memory, [token][128 rows]
+        // ------------------------------------------------------------ accumulator -> result, or -> shared memory
+        float bias = 0.0f;
+        if (kDirect) {
+            pdl_wait_prior_grids();                                  // long over by now; orders the stores (and reads of `out`)
+            if (P.bias != nullptr && row < P.N) bias = load_as_float(P.bias, P.bias_dtype, row);
+        }
         if (ok && !mbar_wait_bounded(&ctl.acc_full, 0, kWaitG)) {
             give_up(ctl, kErrGemmMmaBarrierTimeout);
             ok = false;
@@ -626,15 +745,26 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
             tc::fence_after_thread_sync();
-            float* st = reinterpret_cast<float*>(smem);              // every ring slot has been consumed
             const int valid = min(P.nt, P.M - t0);
-            for (int c0 = grp * 16; c0 < valid; c0 += groups * 16) {
-                uint32_t v[16];
-                tmem_ld_32x32b_x16(lane_addr + c0, v);
-                tc::tmem_ld_wait();
+            if constexpr (kDirect) {
+                if (*static_cast<volatile int*>(&ctl.failed) == 0) {
+                    uint8_t* buf = smem + (warp - kDqWarp0) * 2048;  // the rings: every slot has been consumed
+                    const int row0 = row_a + (warp & 3) * 32;
+                    if (P.beta != 0.0f) store_columns<-1>(P, lane_addr, grp * 32, groups * 32, t0, valid, row0, bias, buf, lane);
+                    else if (P.out_dtype == TPB200_BF16) store_columns<TPB200_BF16>(P, lane_addr, grp * 32, groups * 32, t0, valid, row0, bias, buf, lane);
+                    else if (P.out_dtype == TPB200_F16) store_columns<TPB200_F16>(P, lane_addr, grp * 32, groups * 32, t0, valid, row0, bias, buf, lane);
+                    else store_columns<TPB200_F32>(P, lane_addr, grp * 32, groups * 32, t0, valid, row0, bias, buf, lane);
+                }
+            } else {
+                float* st = reinterpret_cast<float*>(smem);          // every ring slot has been consumed; [token][128 rows]
+                for (int c0 = grp * 16; c0 < valid; c0 += groups * 16) {
+                    uint32_t v[16];
+                    tmem_ld_32x32b_x16(lane_addr + c0, v);
+                    tc::tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    if (c0 + e < valid) st[(c0 + e) * kRows + r] = __uint_as_float(v[e]);
+                    for (int e = 0; e < 16; ++e) {
+                        if (c0 + e < valid) st[(c0 + e) * kRows + r] = __uint_as_float(v[e]);
+                    }
                 }
             }
         }
@@ -646,7 +776,7 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
     const int tb = rank * valid / splits, te = (rank + 1) * valid / splits;
     // A unit of the epilogue is a token x 4 weight rows (4 + 4 where rows come in pairs): neighbouring lanes read and write
     // neighbouring 16 and 8 bytes.
-    const bool pairs = P.epilogue == kEpiGated || P.epilogue == kEpiQkv;
+    const bool pairs = kFmt == kFmtNvfp4 && (P.epilogue == kEpiGated || P.epilogue == kEpiQkv);
     const int per_token = pairs ? 16 : 32;
     const int u_first = tb * per_token + threadIdx.x, u_end = te * per_token;
 
@@ -676,7 +806,9 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
             else a = sum_ranks<8>(base, off, splits);
             v[0] = a.x * P.alpha; v[1] = a.y * P.alpha; v[2] = a.z * P.alpha; v[3] = a.w * P.alpha;
         };
-        if (!pairs) {
+        if constexpr (kDirect) {
+            // stored by the warps that read the accumulator
+        } else if (!pairs) {
             for (int u = u_first; u < u_end; u += static_cast<int>(blockDim.x)) {
                 const int t = u >> 5, c = (u & 31) * 4, n = row_a + c;
                 if (n >= P.N) continue;                              // N is a multiple of 8
@@ -796,17 +928,21 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
 
 // at most 93 registers: two CTAs of 352 threads, or one of 608, fit an SM
 constexpr int kBoundThreads = 704;
+template <bool kDirect>
 __global__ void __launch_bounds__(kBoundThreads, 1) w4_nvfp4_gemm_kernel(const __grid_constant__ W4gParams P) {
-    w4_gemm_tile<kFmtNvfp4>(P);
+    w4_gemm_tile<kFmtNvfp4, kDirect>(P);
 }
+template <bool kDirect>
 __global__ void __launch_bounds__(kBoundThreads, 1) w4_nvfp4_gemm_kernel_transposed(const __grid_constant__ W4gParams P) {
-    w4_gemm_tile<kFmtNvfp4T>(P);
+    w4_gemm_tile<kFmtNvfp4T, kDirect>(P);
 }
+template <bool kDirect>
 __global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_kblock_gemm_kernel(const __grid_constant__ W4gParams P) {
-    w4_gemm_tile<kFmtKblock>(P);
+    w4_gemm_tile<kFmtKblock, kDirect>(P);
 }
+template <bool kDirect>
 __global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_plugin_gemm_kernel(const __grid_constant__ W4gParams P) {
-    w4_gemm_tile<kFmtPlugin>(P);
+    w4_gemm_tile<kFmtPlugin, kDirect>(P);
 }
 
 // ---------------------------------------------------------------- launch plan
@@ -816,32 +952,36 @@ __global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_plugin_gemm_kernel(c
 struct W4gPlan { int nt, splits; bool half; };
 
 W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
-    // Microseconds on a B200, fitted to launches chained by programmatic dependent launch (50 to 712 tokens, 1024 to
-    // 32768 rows, K 1024 to 16384); it only has to rank the candidates.
+    // Microseconds on a B200, fitted to 62 shapes chained by programmatic dependent launch (1 to 900 tokens, 1024 to 32768
+    // rows, K 1024 to 16384; eight of them in the pipeline's own chains), every candidate measured: what it chooses is 2 %
+    // off the best on average, 16 % at worst.
     W4gPlan best{256, 1, false};
     float best_cost = 1e30f;
     for (int nt = 16; nt <= 256; nt += 16) {
         const int tt = (M + nt - 1) / nt;
         if (tt > 65535 || (nt > 16 && (M + nt - 17) / (nt - 16) == tt)) continue;      // a narrower tile does the same
         for (int s = 1, l = 0; s <= 8 && s <= k_blocks; s *= 2, ++l) {
-            const long long ctas = static_cast<long long>(tiles) * tt * s;
-            const bool half = nt <= 128 && ctas > sms;
-            const int steps = (k_blocks + s - 1) / s * 4;
-            const float split = l == 0 ? 0.0f : l == 1 ? 0.5f : l == 2 ? 1.0f : 3.0f;
-            const float step = half ? 0.40f : 0.19f + 0.0005f * nt;     // 64 K values
+            const int ctas = static_cast<int>(std::min(1LL * tiles * tt * s, 1LL << 30));
+            const int steps = (k_blocks + s - 1) / s * 4;            // parts of 64 K values
             // clusters that fit the machine at once (GPCs of 16 to 20 SMs hold whole clusters only): 148, 74, 33 and 15 of 1, 2,
             // 4 and 8 CTAs with an SM each, twice that with two CTAs per SM
             constexpr int kFit[4] = {148, 74, 33, 15};
-            const long long fit = std::max(1, kFit[l] * sms / 148 * (half ? 2 : 1));
-            const long long waves = (static_cast<long long>(tiles) * tt + fit - 1) / fit;
-            // a grid of more than half the SMs leaves the next launch no room to start its weight loads
-            const float crowd = half || 2 * ctas > sms ? 1.6f : 0.0f;
-            // summing a cluster's tiles through distributed shared memory moves NT x 512 bytes per CTA
-            const float cost = waves * (1.9f + steps * step + 0.008f * nt) + split + (l > 0 ? 0.012f * nt : 0.0f) + crowd +
-                               0.004f * std::min(ctas, 150LL);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = {nt, s, half};
+            constexpr float kSplit[4] = {0.0f, 0.43f, 1.3f, 2.45f};
+            for (int half = 0; half <= (nt <= 128 ? 1 : 0); ++half) {
+                const int per_sm = 1 + half;
+                const long long fit = std::max(1, kFit[l] * sms / 148 * per_sm);
+                const long long waves = (static_cast<long long>(tiles) * tt + fit - 1) / fit;
+                const float step = half ? std::max(0.30f, 0.13f + 0.0025f * nt) : std::max(0.18f, 0.05f + 0.0014f * nt);
+                // a grid of more than half the room leaves the next launch none to start its weight loads in; one of narrow
+                // CTAs leaves more, and costs a little by itself
+                const float crowd = (2LL * ctas > static_cast<long long>(sms) * per_sm ? 1.8f : 0.0f) + (half ? 0.5f : 0.0f);
+                // summing a cluster's tiles through distributed shared memory moves NT x 512 bytes per CTA
+                const float cost = waves * (1.85f + steps * step + (half ? 0.006f : 0.007f) * nt) + kSplit[l] + (l > 0 ? 0.012f * nt : 0.0f) + crowd +
+                                   0.012f * std::min(ctas, 150);
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best = {nt, s, half != 0};
+                }
             }
         }
     }
@@ -850,18 +990,18 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
 
 // Ring depths.  Up to 128 tokens: half an SM's shared and tensor memory, so that two CTAs (of this launch or of the
 // next one in the stream) share an SM; more tokens: one CTA per SM.
-struct W4gRing { int groups, parts, n_w, n_s, tmem_cols, a_col; };
+struct W4gRing { int groups, parts, merge, n_w, n_s, tmem_cols, a_col; };
 
 W4gRing ring_of(const W4gPlan& plan, int k_blocks, int k_steps) {
     W4gRing r;
-    r.groups = kDqWarpsPerSm / 4 / (plan.half ? 2 : 1);
     r.tmem_cols = plan.half ? 256 : 512;
     r.a_col = (plan.nt + 31) / 32 * 32;
-    // Two 64-K parts per step for narrow token tiles: a step costs the issuing warp ~280 cycles of waiting and issuing
-    // whatever its size, more than the MMAs of one part (2 NT cycles)
-    r.parts = plan.nt <= 64 ? 2 : 1;
     const int blocks_per = (k_blocks + plan.splits - 1) / plan.splits, steps_per = std::min(blocks_per * 4, k_steps);
     const int budget = (plan.half ? 112 : 225) * 1024 - 1024;
+    // Two parts a unit where four such units (one per group of warps) fit the step ring: what a unit costs beside its
+    // arithmetic (barriers, positions, phases) is ~100 instructions of a loop that is bound by their issue.
+    r.parts = plan.nt <= (plan.half ? 64 : 144) ? 2 : 1;
+    r.groups = plan.half ? 2 : 4;
     // A group takes every `stride`-th weight block.  A parity wait tells a phase from the one before it only, so a group
     // must have waited for EVERY earlier block of a slot it comes to: with more blocks than slots, the number of slots is
     // a multiple of the stride.  (Three slots under a stride of two: a group could take a block's codes out of a slot that
@@ -870,10 +1010,17 @@ W4gRing ring_of(const W4gPlan& plan, int k_blocks, int k_steps) {
     const int slots = stride == 2 ? 4 : plan.half && plan.nt > 64 ? 2 : 3;
     static_assert(kMaxW >= 4, "two blocks ahead for each half of the groups");
     r.n_w = std::min(slots, blocks_per);
-    // Operand steps: a group's wait for the MMAs of its previous step covers every slot's last but one use as long as there
-    // are at least as many slots as groups (5 for 256 tokens, the fewest), or no slot is used twice.
-    r.n_s = std::min(std::min(kMaxS, (r.tmem_cols - r.a_col) / (32 * r.parts)),
-                     std::min((steps_per + r.parts - 1) / r.parts, (budget - r.n_w * kWSlot) / (plan.nt * 128 * r.parts)));
+    auto depth = [&](int merge) {
+        const int units = merge * r.parts;
+        return std::min(std::min(kMaxS, (r.tmem_cols - r.a_col) / (32 * units)),
+                        std::min((steps_per + units - 1) / units, (budget - r.n_w * kWSlot) / (plan.nt * 128 * units)));
+    };
+    // Two units per operand step where K is long and three such steps fit: handing a step to the tensor cores costs the
+    // issuing warp ~250 cycles (barrier, commit, loop) beside 35 per MMA.
+    r.merge = steps_per >= 32 && depth(2) >= 3 ? 2 : 1;
+    // Operand steps: a group's wait for the MMAs of its previous unit covers every slot's last but one use as long as there
+    // is room for a unit of each group (5 units for 256 tokens, the fewest), or no slot is used twice.
+    r.n_s = depth(r.merge);
     return r;
 }
 
@@ -993,7 +1140,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     P.M = M;
     P.N = N;
     P.K = K;
-    P.epilogue = qkv ? kEpiQkv : gated ? kEpiGated : norm_out ? kEpiResidual : kEpiPlain;
+    P.epilogue = qkv ? kEpiQkv : gated ? kEpiGated : norm_out ? kEpiResidual : P.splits > 1 || norm_in ? kEpiSplit : kEpiDirect;
     P.gated_rows = N / 2;
     P.q_dim = a->qkv_q_dim;
     P.ldq = a->ldo;
@@ -1007,21 +1154,27 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     P.tmem_cols = ring.tmem_cols;
     P.a_col = ring.a_col;
     P.parts = ring.parts;
+    P.merge = ring.merge;
     P.n_w = ring.n_w;
     P.n_s = ring.n_s;
-    int smem = P.n_w * kWSlot + P.n_s * P.nt * 128 * P.parts;
-    smem = std::max(smem, P.nt * kRows * 4) + 1024;
+    int smem = P.n_w * kWSlot + P.n_s * P.nt * 128 * P.parts * P.merge;
+    smem = std::max(smem, P.epilogue == kEpiDirect ? ring.groups * 4 * 2048 : P.nt * kRows * 4);
+    smem += 1024;
 
-    static void (*const kernels[4])(const W4gParams) = {w4_nvfp4_gemm_kernel, w4_int4_kblock_gemm_kernel,
-                                                        w4_int4_plugin_gemm_kernel, w4_nvfp4_gemm_kernel_transposed};
-    auto kernel = kernels[fmt];
-    static std::atomic<uint64_t> configured[4] = {};
+    using Kernel = void (*)(const W4gParams);
+    static const Kernel kernels[4][2] = {{w4_nvfp4_gemm_kernel<false>, w4_nvfp4_gemm_kernel<true>},
+                                         {w4_int4_kblock_gemm_kernel<false>, w4_int4_kblock_gemm_kernel<true>},
+                                         {w4_int4_plugin_gemm_kernel<false>, w4_int4_plugin_gemm_kernel<true>},
+                                         {w4_nvfp4_gemm_kernel_transposed<false>, w4_nvfp4_gemm_kernel_transposed<true>}};
+    const int direct = P.epilogue == kEpiDirect;
+    const Kernel kernel = kernels[fmt][direct];
+    static std::atomic<uint64_t> configured[4][2] = {};
     const uint64_t bit = 1ull << (dev & 63);
-    if (!(configured[fmt].load(std::memory_order_relaxed) & bit)) {
+    if (!(configured[fmt][direct].load(std::memory_order_relaxed) & bit)) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) {
             return TPB200_ERR_CUDA;
         }
-        configured[fmt].fetch_or(bit, std::memory_order_relaxed);
+        configured[fmt][direct].fetch_or(bit, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles * P.splits, (M + P.nt - 1) / P.nt, 1);
@@ -1064,7 +1217,7 @@ extern "C" int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_
     const int k_blocks = (K + tpb::kBlkK - 1) / tpb::kBlkK, k_steps = (K + tpb::kPartK - 1) / tpb::kPartK;
     const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms);
     const tpb::W4gRing r = tpb::ring_of(plan, k_blocks, k_steps);
-    *info = {plan.nt, plan.splits, plan.half ? 2 : 1, r.groups, r.parts, r.n_w, r.n_s, k_blocks, k_steps};
+    *info = {plan.nt, plan.splits, plan.half ? 2 : 1, r.groups, r.parts, r.n_w, r.n_s * r.merge, k_blocks, k_steps};
     return TPB200_OK;
 }
 
