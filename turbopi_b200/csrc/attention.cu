@@ -14,10 +14,9 @@
 // softmax of its 128 x 256 block relative to the block's own row maxima (base-2 exponentials, 512 threads:
 // four per row), and O = P V (16 MMAs), and leaves O, the row maxima and the row sums in scratch; a second
 // small kernel combines the key tiles' partial results (the usual log-sum-exp merge).  With a single key
-// tile the first kernel writes the final rows itself.  (The key tiles of a row tile as one thread-block cluster that
-// merges through distributed shared memory, without the second kernel, was slower in a chain of launches: 15.7 against
-// 12.6 us for 400 rows on 762 keys, 19.5 against 17.6 for 5696 on 712 -- each CTA reads 128 KB from its peers, where
-// the second kernel reads L2 from every SM.)
+// tile the first kernel writes the final rows itself.  Problems of few row tiles (the
+// action expert) take the cluster form further down, which needs neither scratch nor a second kernel; 5696 rows on 712
+// keys leave no SMs for it.
 //
 // Operands in shared memory, all in the 128-byte-swizzle image (rows of 128 B = 64 bf16, 16-byte chunk c of
 // row r at c ^ (r & 7), 8-row groups 1024 B apart, one 16 KB block per 64 columns of head_dim):
@@ -85,6 +84,7 @@ struct AttnParams {
     float* qa_row_scale;
     int qa_pieces;
     int qa_rows_per_token;
+    int dv_parts, dv_part;   // cluster form: head_dim cut into dv_parts pieces of dv_part columns (the N of the second MMA)
     uint8_t* qa_sf;          // not null: the row-major operand form (codes [pieces * piece_rows, pitch] + scale atoms)
     int qa_pitch, qa_piece_rows;
 };
@@ -441,6 +441,317 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     }
 }
 
+// ---------------------------------------------------------------- the cluster form
+// The key tiles of a row tile as one thread-block cluster, merged through distributed shared memory: no scratch, no second
+// launch.  What made that slow with whole rows (each CTA read 128 KB from its peers: 15.7 us for 400 rows on 762 keys
+// against 12.6 with a merge kernel) is the size of the exchange: loads from a peer bring ~15 bytes a nanosecond.  So head_dim is
+// cut as well: CTA (key tile, row tile, piece of head_dim) repeats S = Q K^T and the softmax -- there are SMs to spare -- and
+// computes dv_part columns of O; with 64 columns it stages 32 KB and reads 28 KB.  Chains of dependent launches (B200): 400 rows
+// on 762 keys 11.3 -> 7.7 us, 2744 rows on 343 keys 12.0 -> 9.5.  Of the 7.7: loads of Q and K 1.7, softmax 1.3, O 0.5,
+// staging and cluster barrier 0.9, merge 1.9.  (The rows sent as bulk copies into the peers' K: 8.0.)
+struct ClusterControl {
+    uint64_t bar_qk[4];                         // per 64-column block of head_dim: Q and K have landed
+    uint64_t bar_s, bar_v, bar_o;
+    uint32_t tmem_base;
+    float2 ml[kRows];                           // row maximum (base 2) and row sum over this CTA's keys; read by the peers
+    float bias2[kKeyTile];
+    float part_max[kParts][kRows];
+    float part_sum[kParts][kRows];
+    float weight[kRows / 2][9];                 // of the rows this CTA finishes: 2^(m_p - max) per key tile, 1 / sum
+};
+
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+
+// kTiles: the most key tiles (4 or 8)
+template <int kTiles>
+__global__ void __launch_bounds__(kThreadsAttn, 1) attention_cluster_kernel(const __grid_constant__ AttnParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int nchunk = P.dpad >> 6, vchunks = (P.dv_part + 63) >> 6;
+    uint8_t* sQ = smem;                                   // later P: 128 rows x 128 keys = two 64-key blocks
+    uint8_t* sK = sQ + max(nchunk, 2) * kChunkBytes;
+    uint8_t* sV = sK + nchunk * kChunkBytes;
+    uint8_t* sO = smem;                                   // the partial O, fp32, pitch dvp, once the MMAs have read the operands
+    ClusterControl* ctl = reinterpret_cast<ClusterControl*>(smem + max((max(nchunk, 2) + nchunk + vchunks) * kChunkBytes, kRows * P.dvp * 4));
+
+    const int kt = blockIdx.x, g = blockIdx.z;            // kt: also the rank in the cluster
+    const int rt = blockIdx.y / P.dv_parts, dvp0 = (blockIdx.y - rt * P.dv_parts) * P.dv_part;
+    const int ga = g / P.groups_inner, gb = g - ga * P.groups_inner;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform, and known to be
+    const int key0 = kt * kKeyTile;
+    const uint32_t tmem_cols = P.dv_part <= 128 ? 256 : 512;   // half of it leaves room for the next launch's CTA
+    constexpr uint32_t kColOc = kKeyTile;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 4; ++i) mbar_init(&ctl->bar_qk[i], 2);
+        mbar_init(&ctl->bar_s, 1);
+        mbar_init(&ctl->bar_v, 1);
+        mbar_init(&ctl->bar_o, 1);
+        fence_mbar_init();
+        tc::prefetch_tensormap(&P.q.map);
+        tc::prefetch_tensormap(&P.k.map);
+        tc::prefetch_tensormap(&P.v.map);
+    }
+    if (warp == 1) {
+        __syncwarp();
+        tc::tmem_alloc(&ctl->tmem_base, tmem_cols);
+        tc::tmem_relinquish();
+    }
+    pdl_launch_dependents();
+    tc::fence_before_thread_sync();
+    __syncthreads();
+    tc::fence_after_thread_sync();
+    const uint32_t tmem = ctl->tmem_base;
+    pdl_wait_prior_grids();                               // q, k, v (and the bias) may come from the previous kernel
+
+    if (warp >= 4 && warp < 8) {                          // one key per thread (visible to all behind the S wait)
+        const int key = key0 + threadIdx.x - 128;
+        float b = -INFINITY;                              // keys past the end: weight zero whatever the others are
+        if (key < P.n_keys) b = P.key_bias != nullptr ? fmaxf(__bfloat162float(P.key_bias[key]) * kLog2e, kFloor2) : 0.0f;
+        ctl->bias2[threadIdx.x - 128] = b;
+    }
+    // Q, K and V leave from three warps side by side: one thread is held for 0.1 us by each request
+    if ((warp == 0 || warp == 2) && tc::elect_one()) {
+        for (int c = 0; c < nchunk; ++c) {
+            mbar_expect_tx(&ctl->bar_qk[c], kChunkBytes);
+            if (warp == 0) load_rows(sQ, P.q, rt * kRows, ga, gb, c, c + 1, &ctl->bar_qk[c]);
+            else load_rows(sK, P.k, key0, ga, gb, c, c + 1, &ctl->bar_qk[c]);
+        }
+    }
+    if (warp == 3 && tc::elect_one()) {
+        mbar_expect_tx(&ctl->bar_v, vchunks * kChunkBytes);
+        const int c0 = dvp0 >> 6;
+        load_rows(sV - c0 * kChunkBytes, P.v, key0, ga, gb, c0, c0 + vchunks, &ctl->bar_v);
+    }
+    __syncwarp();
+    if (warp == 0) {
+        // The whole warp walks the loop and one elected lane issues (operands in uniform registers).
+        const uint32_t idesc = make_idesc_bf16(kKeyTile, 0);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint32_t q16 = (smem_u32(sQ) & 0x3FFFFu) >> 4, k16 = (smem_u32(sK) & 0x3FFFFu) >> 4;
+        const int ksteps = (P.head_dim + 15) >> 4;        // 16 columns of head_dim per MMA
+        bool loaded = true;
+        for (int c = 0; c < nchunk && loaded; ++c) {
+            loaded = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->bar_qk[c], 0, kWaitCycles));
+            if (!loaded) {
+                if (threadIdx.x == 0) record_error(kErrAttnBarrierTimeout);
+                break;
+            }
+            tc::fence_after_thread_sync();
+            if (tc::elect_one()) {
+                const int kk1 = min(ksteps, 4 * c + 4);
+                for (int kk = 4 * c; kk < kk1; ++kk) {
+                    const uint32_t off = static_cast<uint32_t>((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4;
+                    mma_bf16(tm + kColS, tc::desc_from_words(q16 + off, tc::kDescHiKmajorSw128),
+                             tc::desc_from_words(k16 + off, tc::kDescHiKmajorSw128), idesc, kk > 0 ? 1u : 0u);
+                }
+            }
+            __syncwarp();
+        }
+        if (loaded && tc::elect_one()) tc::commit(&ctl->bar_s);   // otherwise the wait below runs out for the whole CTA
+        __syncwarp();
+    }
+    bool ok = mbar_wait_bounded(&ctl->bar_s, 0, 2 * kWaitCycles);
+    if (!ok) record_error(kErrAttnBarrierTimeout);
+    ok = __syncthreads_and(ok);
+    tc::fence_after_thread_sync();
+    if (!ok && threadIdx.x == 0) {                        // the copies that are in flight land before the CTA leaves
+        for (int c = 0; c < nchunk; ++c) mbar_wait_bounded(&ctl->bar_qk[c], 0, kWaitCycles);
+        mbar_wait_bounded(&ctl->bar_v, 0, kWaitCycles);
+    }
+
+    // ---------------------------------------------------------------- softmax: thread (part, row), 32 columns each
+    const int row = threadIdx.x & (kRows - 1);            // tensor-memory lane = query row of the tile
+    const int part = threadIdx.x >> 7;
+    const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    float m = kFloor2, l = 0.0f;
+    float t[kPartCols];                                   // the scores in the base-2 domain
+    if (ok) {
+        uint32_t r[kPartCols];
+        tc::tmem_ld_32x32b_x32(lane_addr + kColS + part * kPartCols, r);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < kPartCols; ++j) {
+            t[j] = fmaf(__uint_as_float(r[j]), P.scale2, ctl->bias2[part * kPartCols + j]);
+            m = fmaxf(m, t[j]);
+        }
+        ctl->part_max[part][row] = m;
+    }
+    __syncthreads();
+    if (ok) {
+#pragma unroll
+        for (int p = 0; p < kParts; ++p) m = fmaxf(m, ctl->part_max[p][row]);
+        // p = 2^(t - m) rounded to bf16 (what the PyTorch path feeds its second matmul), row sum of the rounded values
+#pragma unroll
+        for (int j8 = 0; j8 < kPartCols / 8; ++j8) {
+            uint32_t w[4];
+#pragma unroll
+            for (int j2 = 0; j2 < 4; ++j2) {
+                const int j = j8 * 8 + j2 * 2;
+                const __nv_bfloat162 pb = __floats2bfloat162_rn(ex2(t[j] - m), ex2(t[j + 1] - m));
+                l += __bfloat162float(pb.x) + __bfloat162float(pb.y);
+                w[j2] = *reinterpret_cast<const uint32_t*>(&pb);
+            }
+            const int ch = part * (kPartCols / 8) + j8;   // 16-byte chunk of the 128-key row: 0..15
+            uint8_t* dst = sQ + (ch >> 3) * kChunkBytes + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
+            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        ctl->part_sum[part][row] = l;
+    }
+    fence_proxy_async_smem();
+    tc::fence_before_thread_sync();
+    __syncthreads();
+    tc::fence_after_thread_sync();
+
+    // ---------------------------------------------------------------- O = P V, dv_part columns
+    if (warp == 0 && ok) {
+        if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl->bar_v, 0, kWaitCycles))) {
+            tc::fence_after_thread_sync();
+            const uint32_t idesc = make_idesc_bf16(P.dv_part, 1);    // B = V read MN-major, as in attention_partial_kernel
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint32_t p16 = (smem_u32(sQ) & 0x3FFFFu) >> 4, v16 = (smem_u32(sV) & 0x3FFFFu) >> 4;
+            constexpr uint32_t kDescHiMnSw128 = (1024u >> 4) | (1u << 14) | (static_cast<uint32_t>(tc::kSwizzle128B) << 29);
+            constexpr uint32_t kLboField = (static_cast<uint32_t>(kChunkBytes) >> 4) << 16;
+            if (tc::elect_one()) {
+                for (int kk = 0; kk < kKeyTile / 16; ++kk) {
+                    const uint32_t a_off = static_cast<uint32_t>((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4;
+                    mma_bf16(tm + kColOc, tc::desc_from_words(p16 + a_off, tc::kDescHiKmajorSw128),
+                             tc::desc_from_words((v16 + (kk * 2048 >> 4)) | kLboField, kDescHiMnSw128), idesc, kk > 0 ? 1u : 0u);
+                }
+                tc::commit(&ctl->bar_o);
+            }
+            __syncwarp();
+        } else if (threadIdx.x == 0) {
+            record_error(kErrAttnBarrierTimeout);         // the wait below runs out for the whole CTA
+        }
+    }
+    if (ok && part == 0) {                                // in part order
+        for (int p = 0; p < kParts; ++p) l = p == 0 ? ctl->part_sum[0][row] : l + ctl->part_sum[p][row];
+        ctl->ml[row] = make_float2(m, l);
+    }
+    if (ok) {
+        ok = mbar_wait_bounded(&ctl->bar_o, 0, 2 * kWaitCycles);
+        if (!ok) record_error(kErrAttnBarrierTimeout);
+    }
+    ok = __syncthreads_and(ok);
+    tc::fence_after_thread_sync();
+
+    // ---------------------------------------------------------------- O -> shared memory (chunk c of row r at c ^ (r & 7))
+    if (ok) {
+        uint8_t* srow = sO + static_cast<size_t>(row) * P.dvp * 4;
+        for (int c0 = part * 16; c0 < P.dv_part; c0 += kParts * 16) {
+            uint32_t r[16];
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                  "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(lane_addr + kColOc + c0)
+                : "memory");
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+                const int ch = (c0 + j) >> 2;
+                *reinterpret_cast<uint4*>(srow + ((ch ^ (row & 7)) << 4)) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+            }
+        }
+    }
+    tc::fence_before_thread_sync();
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp == 1) {
+        tc::fence_after_thread_sync();
+        tc::tmem_dealloc(tmem, tmem_cols);
+    }
+
+    // ---------------------------------------------------------------- this CTA's share of the rows, from all key tiles
+    {
+        const int rows = min(kRows, P.n_rows - rt * kRows);
+        const int r0 = kt * rows / P.key_tiles, r1 = (kt + 1) * rows / P.key_tiles;
+        const int units = P.dv_part >> 2;                 // of four columns
+        const uint32_t o_base = smem_u32(sO);
+        constexpr int kBatch = 8 / kTiles;                // units whose loads are in flight together
+        float4 o[kBatch][kTiles];
+        auto load = [&](int u0) {
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                const int u = u0 + b * kThreadsAttn;
+                if (u >= (r1 - r0) * units) break;
+                const int rr = r0 + u / units, c = u % units;
+                const uint32_t off = static_cast<uint32_t>(rr * P.dvp * 4 + ((c ^ (rr & 7)) << 4));
+#pragma unroll
+                for (int p = 0; p < kTiles; ++p) {
+                    if (p < P.key_tiles) o[b][p] = ld_cluster_f4(map_to_rank(o_base, p) + off);
+                }
+            }
+        };
+        load(threadIdx.x);
+        // the rows' weights, eight lanes a row, while the first values are on their way
+        const int wr = threadIdx.x >> 3, wp = threadIdx.x & 7;
+        float2 ml = make_float2(kFloor2, 0.0f);
+        if (wr < r1 - r0 && wp < P.key_tiles) ml = ld_cluster_f2(map_to_rank(smem_u32(&ctl->ml[r0 + wr]), wp));
+        float mmax = ml.x;
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) mmax = fmaxf(mmax, __shfl_xor_sync(0xffffffffu, mmax, d));
+        const float w = ex2(ml.x - mmax);
+        float lsum = 0.0f;                                // in tile order, as merge_key_tiles adds
+#pragma unroll
+        for (int p = 0; p < kTiles; ++p) {
+            const float wt = __shfl_sync(0xffffffffu, w, p, 8), lt = __shfl_sync(0xffffffffu, ml.y, p, 8);
+            if (p < P.key_tiles) lsum = fmaf(wt, lt, lsum);
+        }
+        if (wr < r1 - r0) {
+            ctl->weight[wr][wp] = w;
+            if (wp == 0) ctl->weight[wr][8] = 1.0f / lsum;
+        }
+        __syncthreads();
+        for (int u0 = threadIdx.x; u0 < (r1 - r0) * units; u0 += kBatch * kThreadsAttn) {
+            if (u0 != static_cast<int>(threadIdx.x)) load(u0);
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                const int u = u0 + b * kThreadsAttn;
+                if (u >= (r1 - r0) * units) break;
+                const int rr = r0 + u / units, c = u % units;
+                float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (int p = 0; p < kTiles; ++p) {
+                    if (p < P.key_tiles) {
+                        const float wt = ctl->weight[rr - r0][p];
+                        acc.x = fmaf(wt, o[b][p].x, acc.x); acc.y = fmaf(wt, o[b][p].y, acc.y);
+                        acc.z = fmaf(wt, o[b][p].z, acc.z); acc.w = fmaf(wt, o[b][p].w, acc.w);
+                    }
+                }
+                const int col = dvp0 + 4 * c;
+                if (ok && col < P.head_dim) {             // head_dim is a multiple of 8
+                    const float inv = ctl->weight[rr - r0][8];
+                    const __nv_bfloat162 x = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
+                    const __nv_bfloat162 y = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
+                    __nv_bfloat16* dst = P.out + ga * P.o_stride[0] + gb * P.o_stride[1] + static_cast<size_t>(rt * kRows + rr) * P.ldo + col;
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
+                }
+            }
+        }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");    // nobody leaves while a peer still reads its rows
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Columns [8 c, 8 c + 8) of a row merged over its key tiles: acc = sum_j w_j O_j, returns sum_j w_j l_j, w_j = 2^(m_j - max_j
 // m_j).  The loads of kBatch tiles are in flight together: one tile after the other this was a chain of six L2
 // round trips, 2.9 us of the 12.6 of 400 rows on 762 keys.
@@ -617,6 +928,21 @@ int attn_dims(int n_rows, int n_keys, int head_dim, int groups, AttnDims& d) {
     return TPB200_OK;
 }
 
+// The cluster form: 128 keys per CTA, 2 to 8 key tiles, and the finest cut of head_dim (whole 64-column blocks) whose clusters
+// all run at once.  cudaOccupancyMaxActiveClusters with an SM per CTA (GPCs hold whole clusters): kFit.  0: not for it.
+int cluster_dv_parts(int n_rows, int n_keys, int head_dim, int groups) {
+    constexpr int kFit[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+    const int tiles = (n_keys + 127) / 128, row_tiles = (n_rows + 127) / 128;
+    if (tiles < 2 || tiles > 8) return 0;
+    const int blocks = head_dim / 64;
+    for (int parts = head_dim % 64 == 0 ? std::min(blocks, 4) : 1; parts >= 1; parts /= 2) {
+        if (blocks % parts == 0 || parts == 1) {
+            if (static_cast<long long>(row_tiles) * groups * parts <= kFit[tiles]) return parts;
+        }
+    }
+    return 0;
+}
+
 // Tensor map of one operand: [outer groups][inner groups][rows][head_dim] with element strides (stride[0],
 // stride[1], ld, 1).  The three outer dimensions go into the map by ascending stride; a group dimension
 // with stride 0 (every group reads the same rows) becomes a dimension of size 1 whose coordinate stays 0.
@@ -743,6 +1069,39 @@ extern "C" int tpb200_attention(const tpb200_attention_args* a, tpb200_stream_t 
     P.qa_piece_rows = a->quant_piece_rows;
 
     const int nchunk = d.dpad / 64;
+    const int dv_parts = quant || d.key_tiles == 1 || d.keys_per_cta != 128 ? 0 : cluster_dv_parts(a->n_rows, a->n_keys, a->head_dim, d.groups);
+    if (dv_parts > 0) {
+        P.dv_parts = dv_parts;
+        P.dv_part = dv_parts > 1 ? a->head_dim / dv_parts : d.dv;
+        P.dvp = (P.dv_part + 31) / 32 * 32;
+        P.key_tiles = (a->n_keys + 127) / 128;
+        const size_t bytes = std::max((std::max(nchunk, 2) + nchunk + (P.dv_part + 63) / 64) * tpb::kChunkBytes, tpb::kRows * P.dvp * 4) +
+                             sizeof(tpb::ClusterControl) + 1024;
+        static std::atomic<uint64_t> ready[2] = {};
+        const int many = P.key_tiles > 4;
+        auto kernel = many ? tpb::attention_cluster_kernel<8> : tpb::attention_cluster_kernel<4>;
+        int at = 0;
+        cudaGetDevice(&at);
+        const uint64_t one = 1ull << (at & 63);
+        if (!(ready[many].load(std::memory_order_relaxed) & one)) {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return TPB200_ERR_CUDA;
+            ready[many].fetch_or(one, std::memory_order_relaxed);
+        }
+        cudaLaunchAttribute ca[2];
+        ca[0].id = cudaLaunchAttributeClusterDimension;
+        ca[0].val.clusterDim.x = P.key_tiles;
+        ca[0].val.clusterDim.y = ca[0].val.clusterDim.z = 1;
+        ca[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        ca[1].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cc = {};
+        cc.gridDim = dim3(P.key_tiles, d.row_tiles * dv_parts, d.groups);
+        cc.blockDim = dim3(tpb::kThreadsAttn, 1, 1);
+        cc.dynamicSmemBytes = bytes;
+        cc.stream = reinterpret_cast<cudaStream_t>(stream);
+        cc.attrs = ca;
+        cc.numAttrs = (a->flags & TPB200_FLAG_PDL) ? 2 : 1;
+        return cudaLaunchKernelEx(&cc, kernel, P) == cudaSuccess ? TPB200_OK : TPB200_ERR_CUDA;
+    }
     const size_t smem = static_cast<size_t>(std::max(nchunk, 4) + 2 * nchunk) * tpb::kChunkBytes + sizeof(tpb::AttnControl) + 1024;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
