@@ -9,6 +9,7 @@ from ctypes import c_char_p, c_float, c_int, c_size_t, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libturbopi_b200.so"
+CALLS_PATH = LIB_PATH.parent / "_calls.so"
 
 F32, F16, BF16 = 0, 1, 2
 ACT_NONE, ACT_GELU, ACT_SILU, ACT_GEGLU = 0, 1, 2, 3
@@ -170,6 +171,29 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
+
+# the entry points csrc/calls.cpp calls, in the order of its Entries
+_NATIVE_ENTRIES = ("tpb200_w4_gemm", "tpb200_w4a16_gemv", "tpb200_w4a16_gemm", "tpb200_attention", "quantizeActivationToFP8",
+                   "tpb200_last_error", "tpb200_nvfp4_tiled_a_bytes", "tpb200_nvfp4_quantize_act_tiled", "tpb200_nvfp4_gemm_ex")
+
+
+def native():
+    """The tensor-level calls of csrc/calls.cpp, bound to the library that load() has loaded."""
+    global _native
+    if _native is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (the module links against its libraries)
+        if not CALLS_PATH.exists():
+            raise TurboPiError(f"{CALLS_PATH} is missing: build it with `python -m turbopi_b200.build`")
+        spec = importlib.util.spec_from_file_location("_calls", CALLS_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        lib = load()
+        module.bind([ctypes.cast(getattr(lib, name), c_void_p).value for name in _NATIVE_ENTRIES])
+        _native = module
+    return _native
 
 
 def load():

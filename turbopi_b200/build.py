@@ -3,7 +3,7 @@
     python -m turbopi_b200.build [--force]
 
 Every .cu under csrc/ is one translation unit; objects are compiled in parallel
-into csrc/_obj/ and linked into lib/libturbopi_b200.so.  A unit is recompiled only
+into csrc/_obj/ and linked into lib/libturbopi_b200.so; csrc/calls.cpp becomes lib/_calls.so.  A unit is recompiled only
 when it or a header it can see is newer than its object.
 """
 import concurrent.futures
@@ -17,6 +17,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = CSRC / "_obj"
 LIB = PKG / "lib" / "libturbopi_b200.so"
+CALLS_SRC = CSRC / "calls.cpp"
+CALLS = LIB.parent / "_calls.so"
 INCLUDE = PKG.parent / "include"
 
 NVCC_FLAGS = [
@@ -52,14 +54,39 @@ def _compile(src, force):
     return src.name, "compiled", r.stderr
 
 
+def _build_calls(force):
+    """csrc/calls.cpp, the calls that take and return tensors: a Python extension module against torch's headers."""
+    if (not force and CALLS.exists() and CALLS.stat().st_mtime > CALLS_SRC.stat().st_mtime
+            and CALLS.stat().st_mtime > (INCLUDE / "turbopi_b200.h").stat().st_mtime):
+        return "up to date"
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cuda = Path(_nvcc()).resolve().parent.parent
+    includes = [*cpp_extension.include_paths(), str(cuda / "include"), sysconfig.get_paths()["include"], str(INCLUDE)]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_calls",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in includes), str(CALLS_SRC),
+           "-o", str(CALLS), *(f"-L{p}" for p in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+           "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {CALLS_SRC.name}:\n{r.stderr[-4000:]}")
+    return "compiled"
+
+
 def build(force=False, verbose=False):
     OBJ.mkdir(parents=True, exist_ok=True)
     LIB.parent.mkdir(parents=True, exist_ok=True)
     sources = sorted(CSRC.glob("*.cu"))
     if not sources:
         raise RuntimeError("no CUDA sources found")
-    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(sources))) as ex:
+    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(sources) + 1)) as ex:
+        calls = ex.submit(_build_calls, force)
         results = list(ex.map(lambda s: _compile(s, force), sources))
+        state = calls.result()
+    if verbose:
+        print(f"[turbopi_b200.build] {CALLS_SRC.name}: {state}")
     changed = any(state == "compiled" for _, state, _ in results)
     if verbose:
         for name, state, _ in results:

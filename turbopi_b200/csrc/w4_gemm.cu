@@ -988,6 +988,17 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
     return best;
 }
 
+// The last plans of this thread: a call's host side is a few microseconds, ranking the candidates is one of them.
+W4gPlan plan_cached(int tiles, int M, int k_blocks, int sms) {
+    struct Entry { int tiles, M, k_blocks, sms; W4gPlan plan; };
+    static thread_local Entry cache[32] = {};
+    Entry& e = cache[(static_cast<unsigned>(tiles) * 31u + static_cast<unsigned>(M) * 7u + static_cast<unsigned>(k_blocks)) % 32u];
+    if (e.tiles != tiles || e.M != M || e.k_blocks != k_blocks || e.sms != sms) {
+        e = {tiles, M, k_blocks, sms, plan_w4_gemm(tiles, M, k_blocks, sms)};
+    }
+    return e.plan;
+}
+
 // Ring depths.  Up to 128 tokens: half an SM's shared and tensor memory, so that two CTAs (of this launch or of the
 // next one in the stream) share an SM; more tokens: one CTA per SM.
 struct W4gRing { int groups, parts, merge, n_w, n_s, tmem_cols, a_col; };
@@ -1103,7 +1114,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     P.img_kblocks = P.k_blocks;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const W4gPlan plan = plan_w4_gemm(tiles, M, P.k_blocks, sms);
+    const W4gPlan plan = plan_cached(tiles, M, P.k_blocks, sms);
     P.nt = plan.nt;
     P.splits = plan.splits;
     bool ok = make_tensor_map_2d(&P.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a->x, K, M, static_cast<uint64_t>(a->ldx) * 2, 64,

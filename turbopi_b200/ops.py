@@ -64,6 +64,13 @@ def _run_on(device, fn, *args):
     return fn(*args, _raw_stream(i))
 
 
+def _result(done, what):
+    """What a call of csrc/calls.cpp returned: its result, or an int, the status it failed with."""
+    if type(done) is int:
+        _lib.check(done, what)
+    return done
+
+
 def _scale_kind(scales):
     if scales.dtype == torch.float32:
         return SCALE_F32
@@ -237,6 +244,9 @@ def dequantize_int4_to_bf16(packed, scales, zeros, group_size=128):
 
 def quantize_activation_to_fp8(x_bf16):
     """quantizeActivationToFP8: bf16 [M, K] -> (E4M3 bytes [M, K], E4M3 scale bytes [M, K/16])."""
+    done = (_lib._native or _lib.native()).quantize_fp8(x_bf16)
+    if done is not None:
+        return _result(done, "quantizeActivationToFP8")
     _cuda(x_bf16)
     x = x_bf16.to(torch.bfloat16).contiguous()
     M, K = x.shape
@@ -315,6 +325,10 @@ def nvfp4_linear_tiled(x, b_image, N, alpha=1.0, bias=None, activation=ACT_NONE,
     """nvfp4_gemm(nvfp4_quantize_act(x), ...) with the activations as a tiled operand image: the same codes, scales and
     products in 128 x 256 output tiles (half the operand bytes per product).  b_image: tile_weights() of the weight operand,
     or with `b_sf` its row-major codes, read where they are."""
+    if b_sf is not None:
+        done = (_lib._native or _lib.native()).nvfp4_linear(x, b_image, N, alpha, bias, int(activation), _DTYPES.get(out_dtype, -1), b_sf)
+        if done is not None:
+            return _result(done, "tpb200_nvfp4_gemm_ex")
     _cuda(x, b_image, bias, b_sf)
     M, K = x.shape
     x = x.contiguous()
@@ -430,6 +444,10 @@ def w4_gemm(x, w, N, format, w_scales=None, w_zeros=None, alpha=1.0, beta=0.0, b
     inside the kernel (tpb200_w4_gemm).  `format`: _lib.W4_NVFP4_ROWMAJOR (w = codes [N, pitch], w_scales = swizzled
     atoms), W4_NVFP4_TILED (w = the tiled image), W4_INT4_KBLOCK, W4_INT4_PLUGIN.  `gated`: W = [gate; up], the result
     is act(gate) * up with N / 2 columns.  x [M, K] bf16, unit last stride, row stride a multiple of 8."""
+    done = (_lib._native or _lib.native()).w4_gemm(x, w, N, int(format), w_scales, w_zeros, alpha, beta, bias, int(activation),
+                                                   bool(gated), out, _DTYPES.get(out_dtype, -1), _flags.value)
+    if done is not None:
+        return _result(done, "tpb200_w4_gemm")
     _cuda(x, w, w_scales, w_zeros, bias, out)
     M, K = x.shape
     if x.dtype != torch.bfloat16 or x.stride(1) != 1:
@@ -632,6 +650,10 @@ def attention(q, k, v, out, scale, key_bias=None, workspace=None, quant=None, ro
     `quant` (a tiled QuantBuf of [rows / rows_per_token, rows_per_token * D]): the result is also, or with
     out=None only, written as the operand of the next tensor-core GEMM -- what rowop(ROW_NONE, out, ...) would
     produce, without that launch (2-D problems only)."""
+    if quant is None and out is not None and workspace is not None:
+        done = (_lib._native or _lib.native()).attention(q, k, v, out, scale, key_bias, workspace, _flags.value)
+        if done is not None:
+            return _result(done, "tpb200_attention")
     _cuda(q, k, v, out, key_bias, workspace)
     if out is None and quant is None:
         raise TurboPiError("attention: neither out nor quant given")

@@ -12,7 +12,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _lib, ops
 from ._lib import INT4_KBLOCK, INT4_ROWMAJOR
 
 QUANT_BLOCK = 32
@@ -153,6 +153,11 @@ class W4A16Linear(nn.Module):
         return dequantize_kblock(self.weight_packed, self.scales)
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
+        buffers = self._buffers                       # (the module's attribute search costs a third of a microsecond each)
+        done = (_lib._native or _lib.native()).w4a16_linear(input, buffers["weight_packed"], buffers["scales"],
+                                                            self._parameters["bias"], self.out_features, ops._flags.value)
+        if done is not None:
+            return ops._result(done, "W4A16Linear")
         K, N = input.shape[-1], self.out_features
         assert K == self.in_features, f"Input last dim ({K}) doesn't match in_features ({self.in_features})"
         x = input if input.dim() == 2 else input.reshape(-1, K)
