@@ -262,13 +262,23 @@ int tpb200_w4_gemm(const tpb200_w4_gemm_args* args, tpb200_stream_t stream);
  *   h_out != NULL: h = bf16(res_in + bf16(y * gate)) with y the linear's bf16 result (res_in, gate may be NULL) goes to h_out
  *          [M, N] (may be res_in), bf16(h * (1 + scale)) to `out`, the sums of h^2 over 128 columns to out_sumsq
  *          [M, N / 128].  N % 128 == 0, bf16 out, no activation, no beta, neither gated nor QKV.
+ *   copy_out != NULL (with in_sumsq, a plain linear): the result also goes to copy_out [M, N] as bf16.
  * in_shift, gate and scale are parameters like the weights: under TPB200_FLAG_PDL they may be read while the kernel before
  * this one still runs. */
 typedef struct {
     const float* in_sumsq; const float* in_shift; int in_parts; float in_eps;
     const void* res_in; const void* gate; const void* scale; void* h_out; float* out_sumsq;
+    void* copy_out;
 } tpb200_w4_norm_args;
 int tpb200_w4_gemm_norm(const tpb200_w4_gemm_args* args, const tpb200_w4_norm_args* norm, tpb200_stream_t stream);
+
+/* The pipeline's inputs (openpi/src/openpi/models_pytorch/pi0_pytorch.py:215-345): uint8 images [num_images, size, size, 3] to
+ * bf16 rows of one patch each, values x / 127.5 - 1 in (channel, row, column) order, `pitch` elements apart; int64 tokens to
+ * rows of a bf16 table [vocab, width] times `scale` (negative indices count from the end, others outside give zeros). */
+int tpb200_pi05_patches(const void* images_u8, void* patches, int num_images, int size, int patch, int pitch, int flags,
+                        tpb200_stream_t stream);
+int tpb200_pi05_embed(const long long* tokens, const void* table, void* out, int num_tokens, long long vocab, int width, float scale,
+                      int flags, tpb200_stream_t stream);
 /* What a launch of that shape looks like on a GPU of `sms` SMs (host only, no device needed): tokens per tile, K ranges
  * per tile, CTAs per SM, groups of four dequantising warps, 64-K parts per step, slots of the weight and of the step ring,
  * 256-K blocks and 64-K parts of the whole K. */

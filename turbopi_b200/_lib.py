@@ -5,7 +5,7 @@ status, an exception is raised.
 """
 import ctypes
 import os
-from ctypes import c_char_p, c_float, c_int, c_size_t, c_void_p
+from ctypes import c_char_p, c_float, c_int, c_longlong, c_size_t, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libturbopi_b200.so"
@@ -56,7 +56,8 @@ class W4GemmArgs(ctypes.Structure):
 
 class W4NormArgs(ctypes.Structure):
     _fields_ = [("in_sumsq", c_void_p), ("in_shift", c_void_p), ("in_parts", c_int), ("in_eps", c_float),
-                ("res_in", c_void_p), ("gate", c_void_p), ("scale", c_void_p), ("h_out", c_void_p), ("out_sumsq", c_void_p)]
+                ("res_in", c_void_p), ("gate", c_void_p), ("scale", c_void_p), ("h_out", c_void_p), ("out_sumsq", c_void_p),
+                ("copy_out", c_void_p)]
 
 
 class W4GemmPlanInfo(ctypes.Structure):
@@ -132,6 +133,8 @@ SIGNATURES = {
     "tpb200_w4_gemm_plan": (c_int, [c_int, c_int, c_int, c_int, ctypes.POINTER(W4GemmPlanInfo)]),
     "tpb200_w4_gemm": (c_int, [ctypes.POINTER(W4GemmArgs), c_void_p]),
     "tpb200_w4_gemm_norm": (c_int, [ctypes.POINTER(W4GemmArgs), ctypes.POINTER(W4NormArgs), c_void_p]),
+    "tpb200_pi05_patches": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "tpb200_pi05_embed": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_int, c_float, c_int, c_void_p]),
     "tpb200_nvfp4_gemm_ex": (c_int, [ctypes.POINTER(GemmArgs), c_void_p]),
     "tpb200_nvfp4_quantize_act_pieces": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                                  c_int, c_int, c_int, c_void_p]),

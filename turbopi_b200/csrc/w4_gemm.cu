@@ -98,6 +98,7 @@ struct W4gParams {
     const __nv_bfloat16* scale;
     __nv_bfloat16* h_out;
     float* out_sumsq;                            // [M, N / 128]
+    __nv_bfloat16* copy_out;                     // kEpiSplit: the result once more, bf16 [M, N], or null
 };
 
 struct W4gControl {
@@ -841,6 +842,9 @@ __device__ __forceinline__ void w4_gemm_tile(const W4gParams& P) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) v[e] = fmaf(P.beta, load_as_float(P.out, P.out_dtype, o + e), v[e]);
                 }
+                if (kFmt == kFmtNvfp4 && P.copy_out != nullptr) {
+                    *reinterpret_cast<uint2*>(P.copy_out + static_cast<size_t>(t0 + t) * P.N + n) = pack4(v);
+                }
                 if (P.out_dtype == TPB200_BF16) {
                     *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(P.out) + o) = pack4(v);
                 } else if (P.out_dtype == TPB200_F32) {
@@ -1081,6 +1085,8 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
         TPB_REQUIRE(nv, TPB200_ERR_ENUM);
         TPB_REQUIRE(norm->in_parts >= 4 && norm->in_parts % 4 == 0, TPB200_ERR_SHAPE);
         TPB_REQUIRE(tpb_aligned16(norm->in_sumsq) && tpb_aligned16(norm->in_shift), TPB200_ERR_ALIGN);
+        TPB_REQUIRE(norm->copy_out == nullptr || (!qkv && !gated && !norm_out), TPB200_ERR_ENUM);
+        TPB_REQUIRE(tpb_aligned16(norm->copy_out), TPB200_ERR_ALIGN);
     }
     if (norm_out) {
         TPB_REQUIRE(nv && !qkv && !gated && a->out_dtype == TPB200_BF16 && a->activation == TPB200_ACT_NONE && a->beta == 0.0f,
@@ -1097,6 +1103,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
         P.in_shift = norm->in_shift;
         P.in_parts = norm->in_parts;
         P.in_eps = norm->in_eps;
+        P.copy_out = static_cast<__nv_bfloat16*>(norm->copy_out);
         P.in_inv_k = 1.0f / static_cast<float>(K);
     }
     if (norm_out) {

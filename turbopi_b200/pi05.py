@@ -136,10 +136,11 @@ class TcLinear:
                                w=p(self.b), w_pitch=self.b.stride(0) if self.rowmajor else 0, w_scales=p(self.sf),
                                alpha=float(self.g), out=p(out), out_dtype=ops._dt(out), ldo=ldo, M=M, N=self.N, K=self.K)
 
-    def dense(self, x, out, activation=ACT_NONE, gated=False, norm=None, bias=True):
-        """out = act(x W^T + bias) for bf16 x [M, >= K]; `gated`: W = [gate; up], out = act(gate) * up.  `norm`
-        (_lib.W4NormArgs): the RMS norms around the linear, see tpb200_w4_gemm_norm."""
+    def dense(self, x, out, activation=ACT_NONE, gated=False, norm=None, bias=True, scale=1.0, beta=0.0):
+        """out = act(scale * x W^T + bias) + beta * out for bf16 x [M, >= K]; `gated`: W = [gate; up], out = act(gate) * up.
+        `norm` (_lib.W4NormArgs): the RMS norms around the linear, see tpb200_w4_gemm_norm."""
         args = self._w4_args(x, x.shape[0], out, out.stride(0))
+        args.alpha, args.beta = float(self.g) * scale, beta
         args.bias, args.activation, args.gated = ops._ptr(self.bias if bias else None), int(activation), int(gated)
         ops._w4_gemm(args, out.device, norm)
         return out
@@ -390,7 +391,7 @@ class Pi05:
         self.cache = torch.zeros((c.prefix_layers, 2, c.max_seq, c.head_dim), dtype=bf, device=d)
         self.b = dict(
             # vision
-            patches=torch.zeros((T, self.patch_k), dtype=bf, device=d),
+            patches=torch.zeros((T, self.patch_k), dtype=bf, device=d), pos=self.pos_emb.repeat(c.num_images, 1),
             vh=torch.empty((T, vw), dtype=bf, device=d), vy=torch.empty((T, vw), dtype=bf, device=d),
             vx=torch.empty((T, vw), dtype=bf, device=d), v_qkv=torch.empty((T, 3 * vw), dtype=bf, device=d),
             v_attn=torch.empty((T, vw), dtype=bf, device=d),
@@ -467,17 +468,16 @@ class Pi05:
     def vision_tower(self):
         c, b = self.cfg, self.b
         T, vw = c.num_images * c.image_tokens, c.vision_width
-        n = c.image_size // c.patch
-        img = self.images.float().div_(127.5).sub_(1.0)                               # [-1, 1]
-        pt = img.view(c.num_images, n, c.patch, n, c.patch, 3).permute(0, 1, 3, 5, 2, 4).reshape(T, -1)   # (c, i, j)
-        b["patches"][:, :pt.shape[1]].copy_(pt)
+        st = ops._run_on(self.images.device, _lib.load().tpb200_pi05_patches, ops._ptr(self.images), ops._ptr(b["patches"]),
+                         c.num_images, c.image_size, c.patch, self.patch_k, ops._flags.value)
+        _lib.check(st, "tpb200_pi05_patches")
         self.patch_embed.dense(b["patches"], b["vh"])
-        b["vh"].view(c.num_images, c.image_tokens, vw).add_(self.pos_emb)
         hd = vw // c.vision_heads
         first = True
         for L in self.vision:
             if first:
-                rowop(_lib.ROW_LAYERNORM, b["vh"], vw, y_out=b["vx"], w0=L["ln1_w"], w1=L["ln1_b"], eps=c.eps)
+                rowop(_lib.ROW_LAYERNORM, b["vh"], vw, y_out=b["vx"], res_in=b["pos"], h_out=b["vh"], w0=L["ln1_w"], w1=L["ln1_b"],
+                      eps=c.eps)
                 first = False
             else:
                 rowop(_lib.ROW_LAYERNORM, b["vy"], vw, y_out=b["vx"], res_in=b["vh"], h_out=b["vh"], w0=L["ln1_w"],
@@ -499,7 +499,11 @@ class Pi05:
     def prefix_pass(self):
         c, b = self.cfg, self.b
         T, S = c.num_images * c.image_tokens, c.prefix_len
-        b["ph"][T:].copy_(self.embed_tokens[self.tokens] * math.sqrt(c.width))
+        if c.text_len:
+            st = ops._run_on(self.tokens.device, _lib.load().tpb200_pi05_embed, ops._ptr(self.tokens), ops._ptr(self.embed_tokens),
+                             ops._ptr(b["ph"][T:]), c.text_len, self.embed_tokens.shape[0], c.width, math.sqrt(c.width),
+                             ops._flags.value)
+            _lib.check(st, "tpb200_pi05_embed")
         first = True
         for l, L in enumerate(self.prefix):
             if first:
@@ -546,7 +550,7 @@ class Pi05:
             return lin.dense(mod[:, norm, 1], torch.empty((n, lin.N), dtype=torch.float32, device=self.device), bias=bias)
         return dict(qkv=[through(L["qkv"], 2 * l) for l, L in enumerate(self.expert)],
                     gate_up=[through(L["gate_up"], 2 * l + 1) for l, L in enumerate(self.expert)],
-                    out=through(self.action_out, 2 * c.expert_layers, bias=True))
+                    out=through(self.action_out, 2 * c.expert_layers, bias=True).mul_(-1.0 / n))    # times the Euler step
 
     def _norm_in(self, shift):
         b, c = self.b, self.cfg
@@ -558,13 +562,15 @@ class Pi05:
                                out_sumsq=p(b["e_ss"]))
 
     def denoise_step(self, mod, dt, shift=None):
-        """One Euler step: v = expert(x_t | cache); x_t += dt * v.  `shift` (one row per linear, `_shifts`): the norms run in
-        the epilogues of the linears around them; None: in row kernels between the linears."""
+        """One Euler step: v = expert(x_t | cache); x_t += dt * v.  `shift` (one row per linear, `_shifts`): the norms and the
+        Euler update run in the epilogues of the linears around them, x_bf holds bf16(x_t) before and after; None: in row
+        kernels between the linears."""
         c, b = self.cfg, self.b
         S, A, ew = c.prefix_len, c.action_horizon, c.expert_width
-        b["x_bf"].copy_(b["x_t"])
         if shift is None:
+            b["x_bf"].copy_(b["x_t"])
             self._expert_with_row_kernels(mod)
+            b["x_t"].add_(b["v_out"], alpha=dt)
         else:
             self.action_in.dense(b["x_bf"], b["ex"], norm=self._norm_out(mod[0, 0], first=True))
             for l, L in enumerate(self.expert):
@@ -575,8 +581,9 @@ class Pi05:
                 L["o"].dense(b["e_attn"], b["ex"], norm=self._norm_out(m_post[0], m_in[2]))
                 L["gate_up"].dense(b["ex"], b["e_mlp"], ACT_GELU, gated=True, norm=self._norm_in(shift["gate_up"][l]))
                 L["down"].dense(b["e_mlp"], b["ex"], norm=self._norm_out(mod[2 * l + 2, 0], m_post[2]))
-            self.action_out.dense(b["ex"], b["v_out"], norm=self._norm_in(shift["out"]), bias=False)
-        b["x_t"].add_(b["v_out"], alpha=dt)
+            norm = self._norm_in(shift["out"])
+            norm.copy_out = ops._ptr(b["x_bf"])
+            self.action_out.dense(b["ex"], b["x_t"], norm=norm, bias=False, scale=dt, beta=1.0)
 
     def _expert_with_row_kernels(self, mod):
         c, b = self.cfg, self.b
@@ -624,6 +631,7 @@ class Pi05:
     def denoise_loop(self, num_steps):
         mod, shift = self._modulation(num_steps)
         self.b["x_t"].copy_(self.noise)
+        self.b["x_bf"].copy_(self.noise)
         dt = -1.0 / num_steps
         for i in range(num_steps):
             at = None if shift is None else dict(qkv=[s[i] for s in shift["qkv"]], gate_up=[s[i] for s in shift["gate_up"]],
