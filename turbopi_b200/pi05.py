@@ -10,8 +10,8 @@ Every linear layer runs as NVFP4 weights x bf16 activations on the tensor cores.
 matrices take the block-scaled e2m1 GEMM (activations as residual e2m1 pieces, written by the row kernels);
 every other linear takes the GEMM that dequantises its weights into tensor memory and reads the bf16
 activations as they are (csrc/w4_gemm.cu): no quantiser in front of it, GELU(gate) * up and Q/K/V + RoPE +
-KV-cache append in its epilogue.  Norms and residuals are the fused row kernels; attention is the
-tensor-core kernel of csrc/attention.cu (`ops.attention`).  All buffers are
+KV-cache append in its epilogue.  Norms and residuals are the fused row kernels, in the action expert the
+epilogues of the linears around them; attention is the tensor-core kernel of csrc/attention.cu (`ops.attention`).  All buffers are
 allocated once, so the whole inference (or just the denoise loop) replays as ONE CUDA graph.
 
 Weights come from a reference-named state dict (`Pi05.from_state_dict`, tensor names of
