@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
     // warps 1..8: the keys' additive bias in the base-2 domain (visible to all after the barrier behind the S wait)
     for (int i = threadIdx.x - 32; i >= 0 && i < kKeysCta; i += kThreadsAttn - 32) {
         const int key = key0 + i;
-        float b = kFloor2;                                // keys past the end never count
+        float b = -INFINITY;                              // keys past the end: weight zero whatever the others are
         if (key < P.n_keys) {
             b = P.key_bias != nullptr ? fmaxf(__bfloat162float(P.key_bias[key]) * kLog2e, kFloor2) : 0.0f;
         }
