@@ -67,6 +67,7 @@ enum {
 /* launch flags */
 enum {
     TPB200_FLAG_NONE = 0,
+    TPB200_FLAG_STRICT_TOKENS = 2, /* tpb200_pi05_embed only: see there */
     TPB200_FLAG_PDL = 1 /* launch with programmatic stream serialisation: the kernel prefetches its
                            weights while the previous kernel in the stream is still running, and
                            waits for that kernel before it reads activations or writes outputs.
@@ -81,8 +82,8 @@ int tpb200_version(void);
 const char* tpb200_status_string(int status);
 /* last non-OK status produced on this host thread by a void-returning entry point (and clears it) */
 int tpb200_last_error(void);
-/* code recorded by a kernel whose bounded wait ran out on the current device, 0 if none; synchronises
- * the device.  `clear` != 0 resets the word.
+/* code recorded by a kernel whose bounded wait ran out on the current device (or 401: a prompt token outside the embedding
+ * table, see TPB200_FLAG_STRICT_TOKENS), 0 if none; synchronises the device.  `clear` != 0 resets the word.
  * Recovery: a kernel that gave up may have left its split-K counters non-zero.  After a non-zero code
  * every workspace that was passed to a GEMM / GEMV / attention launch since the last check must be set
  * to zero again (cudaMemsetAsync) before it is reused; results of the failed launch are undefined. */
@@ -274,7 +275,8 @@ int tpb200_w4_gemm_norm(const tpb200_w4_gemm_args* args, const tpb200_w4_norm_ar
 
 /* The pipeline's inputs (openpi/src/openpi/models_pytorch/pi0_pytorch.py:215-345): uint8 images [num_images, size, size, 3] to
  * bf16 rows of one patch each, values x / 127.5 - 1 in (channel, row, column) order, `pitch` elements apart; int64 tokens to
- * rows of a bf16 table [vocab, width] times `scale` (negative indices count from the end, others outside give zeros). */
+ * rows of a bf16 table [vocab, width] times `scale` (negative indices count from the end, others outside give zeros; under
+ * TPB200_FLAG_STRICT_TOKENS they give rows of NaN and tpb200_device_error() returns 401). */
 int tpb200_pi05_patches(const void* images_u8, void* patches, int num_images, int size, int patch, int pitch, int flags,
                         tpb200_stream_t stream);
 int tpb200_pi05_embed(const long long* tokens, const void* table, void* out, int num_tokens, long long vocab, int width, float scale,

@@ -16,7 +16,7 @@ ACT_NONE, ACT_GELU, ACT_SILU, ACT_GEGLU = 0, 1, 2, 3
 SCALE_F32, SCALE_E4M3, SCALE_F16, SCALE_BF16 = 0, 1, 2, 3
 INT4_KBLOCK, INT4_ROWMAJOR, INT4_PLUGIN = 0, 1, 2
 W4_NVFP4_ROWMAJOR, W4_NVFP4_TILED, W4_INT4_KBLOCK, W4_INT4_PLUGIN = 0, 1, 2, 3
-FLAG_NONE, FLAG_PDL = 0, 1
+FLAG_NONE, FLAG_PDL, FLAG_STRICT_TOKENS = 0, 1, 2
 MAX_GROUP = 64
 
 ACTIVATIONS = {"none": ACT_NONE, "gelu": ACT_GELU, "silu": ACT_SILU}

@@ -31,6 +31,7 @@ enum DeviceErrorCode : int {
     kErrGemmEmptyBarrierTimeout = 204,
     kErrGemmSplitTimeout = 205,
     kErrAttnBarrierTimeout = 301,
+    kErrTokenOutOfRange = 401,
 };
 
 __device__ __forceinline__ void record_error(int code) { atomicCAS(&g_device_error, 0, code); }

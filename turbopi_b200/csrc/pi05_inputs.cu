@@ -20,16 +20,19 @@ __global__ void __launch_bounds__(256) pi05_patches_kernel(const uint8_t* images
     }
 }
 
-// one CTA per token; a negative index counts from the end, one outside the table gives zeros
+// one CTA per token; a negative index counts from the end.  One outside the table gives zeros, or with `strict` NaN and an
+// error: masked or not, a prompt row of NaN reaches every action through the attention
 __global__ void __launch_bounds__(256) pi05_embed_kernel(const long long* tokens, const __nv_bfloat16* table, __nv_bfloat16* out,
-                                                         long long vocab, int width, float scale) {
+                                                         long long vocab, int width, float scale, bool strict) {
     pdl_launch_dependents();
     pdl_wait_prior_grids();
     long long t = tokens[blockIdx.x];
     if (t < 0) t += vocab;
     const bool in = t >= 0 && t < vocab;
+    const float outside = strict ? __int_as_float(0x7fffffff) : 0.0f;
+    if (!in && strict && threadIdx.x == 0) record_error(kErrTokenOutOfRange);
     for (int e = threadIdx.x * 2; e < width; e += 2 * blockDim.x) {
-        __nv_bfloat162 v = __floats2bfloat162_rn(0.0f, 0.0f);
+        __nv_bfloat162 v = __floats2bfloat162_rn(outside, outside);
         if (in) {
             const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(table + t * width + e));
             v = __floats2bfloat162_rn(f.x * scale, f.y * scale);
@@ -51,6 +54,9 @@ cudaLaunchConfig_t config(int blocks, int flags, cudaLaunchAttribute* attr, cuda
 }
 
 }  // namespace
+
+int device_error_pi05_inputs(int clear) { return read_device_error(clear); }
+
 }  // namespace tpb
 
 extern "C" int tpb200_pi05_patches(const void* images_u8, void* patches, int num_images, int size, int patch, int pitch, int flags,
@@ -68,11 +74,11 @@ extern "C" int tpb200_pi05_patches(const void* images_u8, void* patches, int num
 extern "C" int tpb200_pi05_embed(const long long* tokens, const void* table, void* out, int num_tokens, long long vocab, int width,
                                  float scale, int flags, tpb200_stream_t stream) {
     TPB_REQUIRE(tokens != nullptr && table != nullptr && out != nullptr, TPB200_ERR_NULL);
-    TPB_REQUIRE((flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
+    TPB_REQUIRE((flags & ~(TPB200_FLAG_PDL | TPB200_FLAG_STRICT_TOKENS)) == 0, TPB200_ERR_ENUM);
     TPB_REQUIRE(num_tokens >= 1 && vocab >= 1 && width >= 2 && width % 2 == 0, TPB200_ERR_SHAPE);
     TPB_REQUIRE(((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 3) == 0, TPB200_ERR_ALIGN);
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = tpb::config(num_tokens, flags, &attr, reinterpret_cast<cudaStream_t>(stream));
     return cudaLaunchKernelEx(&cfg, tpb::pi05_embed_kernel, tokens, static_cast<const __nv_bfloat16*>(table),
-                              static_cast<__nv_bfloat16*>(out), vocab, width, scale) == cudaSuccess ? TPB200_OK : TPB200_ERR_CUDA;
+                              static_cast<__nv_bfloat16*>(out), vocab, width, scale, (flags & TPB200_FLAG_STRICT_TOKENS) != 0) == cudaSuccess ? TPB200_OK : TPB200_ERR_CUDA;
 }

@@ -502,7 +502,7 @@ class Pi05:
         if c.text_len:
             st = ops._run_on(self.tokens.device, _lib.load().tpb200_pi05_embed, ops._ptr(self.tokens), ops._ptr(self.embed_tokens),
                              ops._ptr(b["ph"][T:]), c.text_len, self.embed_tokens.shape[0], c.width, math.sqrt(c.width),
-                             ops._flags.value)
+                             ops._flags.value | _lib.FLAG_STRICT_TOKENS)
             _lib.check(st, "tpb200_pi05_embed")
         first = True
         for l, L in enumerate(self.prefix):
@@ -661,7 +661,13 @@ class Pi05:
     def infer(self, images_u8, tokens, noise, num_steps=10, use_graph=True, image_valid=None, prompt_len=None):
         """images_u8 [num_images, H, W, 3] uint8, tokens [text_len] int64, noise [horizon, action_dim] fp32
         (host or device tensors); `image_valid` / `prompt_len` as in `set_valid` (default: everything valid).
-        Returns the device tensor of actions [horizon, action_dim] fp32."""
+        A token outside the embedding table is refused where it lies on the host; on the device it makes every action NaN
+        and is recorded (tpb200_device_error: 401).  Returns the device tensor of actions [horizon, action_dim] fp32."""
+        if not tokens.is_cuda and tokens.numel():
+            low, high = torch.aminmax(tokens)
+            vocab = self.embed_tokens.shape[0]
+            if low < -vocab or high >= vocab:
+                raise TurboPiError(f"token ids {int(low)}..{int(high)} are outside the embedding table of {vocab} rows")
         if image_valid is not None or prompt_len is not None or not bool(self.valid.all()):
             self.set_valid(image_valid, prompt_len)
         self.images.copy_(images_u8, non_blocking=True)
