@@ -25,6 +25,7 @@ buffers (positions, additive key bias), so one captured graph serves every mask.
 """
 import ctypes
 import math
+import operator
 from dataclasses import dataclass
 
 import torch
@@ -165,6 +166,30 @@ def sinusoidal_time_embedding(t, dim, min_period=4e-3, max_period=4.0):
     return torch.cat([torch.sin(ang), torch.cos(ang)], dim=1)
 
 
+_version = operator.attrgetter("_version")
+
+
+class _Marks:
+    """The tensors a kept table was made from, with their version counters (inference tensors count no versions) and the
+    plain numbers beside them."""
+
+    def __init__(self, tensors, numbers=()):
+        self.tensors, self.numbers = tensors, numbers
+        self.counting = [t for t in tensors if not t.is_inference()]
+        self.versions = list(map(_version, self.counting))
+
+    @classmethod
+    def of(cls, linears):
+        return cls([t for l in linears for t in (l.b, l.sf, l.bias) if t is not None], [l.g for l in linears])
+
+    def written(self):
+        return list(map(_version, self.counting)) != self.versions
+
+    def same(self, other):
+        return (self.versions == other.versions and self.numbers == other.numbers
+                and all(map(operator.is_, self.tensors, other.tensors)))
+
+
 class Pi05:
     """Pi0.5-shaped model; `infer(images_u8, tokens, noise, num_steps)` -> actions [50, 32].
 
@@ -197,7 +222,8 @@ class Pi05:
         self._graph = None
         self._graph_steps = None
         self._time_emb = {}
-        self._mod = {}            # per step count: the adaptive norms' modulation tables
+        self._mod = {}            # per step count: the adaptive norms' modulation tables, and the weights they follow
+        self._pos_marks = _Marks([self.pos_emb])
         # The expert's norms ride in the epilogues of the linears around them where a row's sums of squares come in
         # whole 16-byte groups of 128-column parts; other widths take the row kernel between two linears.
         self.fold_norms = cfg.expert_width % 512 == 0 and cfg.expert_mlp % 64 == 0
@@ -465,8 +491,27 @@ class Pi05:
         ops.attention(q.view(L * c.heads, c.head_dim), k, v, out.view(L * c.heads, c.head_dim), c.head_dim ** -0.5,
                       self.key_bias, self.attn_ws)
 
+    def weights_changed(self):
+        """Weights may be written in place at any time; what is kept of products of them (the positions once per image, the
+        adaptive norms' modulation and the linears' share of their shifts) is made again, in its own memory, when PyTorch's
+        version counters have moved.  After a write that they do not see (through `.data`, from another library, to
+        tensors made in inference mode) call this: the next inference makes the tables again, also for a captured graph."""
+        self._pos_marks = None
+        self._mod = {n: (mod, shift, None) for n, (mod, shift, _) in self._mod.items()}
+
+    def _positions(self):
+        """The position embeddings, once per image: the first LayerNorm's row kernel adds them."""
+        marks = _Marks([self.pos_emb])
+        if self._pos_marks is None or not marks.same(self._pos_marks):
+            c = self.cfg
+            self.b["pos"].view(c.num_images, c.image_tokens, c.vision_width).copy_(self.pos_emb)
+            if not torch.cuda.is_current_stream_capturing():
+                self._pos_marks = marks
+        return self.b["pos"]
+
     def vision_tower(self):
         c, b = self.cfg, self.b
+        pos = self._positions()
         T, vw = c.num_images * c.image_tokens, c.vision_width
         st = ops._run_on(self.images.device, _lib.load().tpb200_pi05_patches, ops._ptr(self.images), ops._ptr(b["patches"]),
                          c.num_images, c.image_size, c.patch, self.patch_k, ops._flags.value)
@@ -476,7 +521,7 @@ class Pi05:
         first = True
         for L in self.vision:
             if first:
-                rowop(_lib.ROW_LAYERNORM, b["vh"], vw, y_out=b["vx"], res_in=b["pos"], h_out=b["vh"], w0=L["ln1_w"], w1=L["ln1_b"],
+                rowop(_lib.ROW_LAYERNORM, b["vh"], vw, y_out=b["vx"], res_in=pos, h_out=b["vh"], w0=L["ln1_w"], w1=L["ln1_b"],
                       eps=c.eps)
                 first = False
             else:
@@ -524,7 +569,7 @@ class Pi05:
             rowop(_lib.ROW_GELU_MUL, b["p_gu"], c.mlp, b["q_pmlp"])
             L["down"](b["q_pmlp"], b["py"])
 
-    def _ada_modulation(self, num_steps):
+    def _ada_modulation(self, num_steps, out=None):
         """adarms_cond per step and every adaptive norm's (scale, shift, gate): [steps, n_norms, 3, width]
         (pi0_pytorch.py:817-839; GemmaRMSNorm.dense, modeling_gemma.py:96-103)."""
         c, d = self.cfg, self.device
@@ -537,20 +582,23 @@ class Pi05:
         t1 = torch.empty((2, num_steps, ew), dtype=torch.bfloat16, device=d)
         self.time_mlp_in.dense(emb, t1[0], ACT_SILU)
         self.time_mlp_out.dense(t1[0], t1[1], ACT_SILU)
-        mod = torch.empty((num_steps, self.n_norms * 3 * ew), dtype=torch.bfloat16, device=d)
+        mod = torch.empty((num_steps, self.n_norms * 3 * ew), dtype=torch.bfloat16, device=d) if out is None else out.view(num_steps, -1)
         self.ada_dense.dense(t1[1], mod)
         return mod.view(num_steps, self.n_norms, 3, ew)
 
-    def _shifts(self, mod):
+    def _shifts(self, mod, out=None):
         """W * shift of every linear behind an adaptive norm, per step: what is left of the norm's shift when its RMS
         factor is applied behind the linear.  fp32, alpha included; rows in the order of the weights."""
         c, n = self.cfg, mod.shape[0]
-
-        def through(lin, norm, bias=False):
-            return lin.dense(mod[:, norm, 1], torch.empty((n, lin.N), dtype=torch.float32, device=self.device), bias=bias)
-        return dict(qkv=[through(L["qkv"], 2 * l) for l, L in enumerate(self.expert)],
-                    gate_up=[through(L["gate_up"], 2 * l + 1) for l, L in enumerate(self.expert)],
-                    out=through(self.action_out, 2 * c.expert_layers, bias=True).mul_(-1.0 / n))    # times the Euler step
+        if out is None:
+            empty = lambda lin: torch.empty((n, lin.N), dtype=torch.float32, device=self.device)    # noqa: E731
+            out = dict(qkv=[empty(L["qkv"]) for L in self.expert], gate_up=[empty(L["gate_up"]) for L in self.expert],
+                       out=empty(self.action_out))
+        for l, L in enumerate(self.expert):
+            L["qkv"].dense(mod[:, 2 * l, 1], out["qkv"][l], bias=False)
+            L["gate_up"].dense(mod[:, 2 * l + 1, 1], out["gate_up"][l], bias=False)
+        self.action_out.dense(mod[:, 2 * c.expert_layers, 1], out["out"]).mul_(-1.0 / n)             # times the Euler step
+        return out
 
     def _norm_in(self, shift):
         b, c = self.b, self.cfg
@@ -619,14 +667,24 @@ class Pi05:
         """The adaptive norms' (scale, shift, gate) for every step of an `num_steps` schedule.  They depend on
         the schedule and the weights only, not on the observation (the reference precomputes the per-step
         conditioning vectors for its graphs too: pi0_pytorch.py:770-839), so they are computed once per schedule -- by
-        the warm-up pass that precedes a capture -- and stay out of the per-inference graph."""
-        mod = self._mod.get(num_steps)
-        if mod is None:
-            if torch.cuda.is_current_stream_capturing():
+        the warm-up pass that precedes a capture -- and stay out of the per-inference graph.  Made again in the same memory
+        when a weight has been written since (a capture that finds them out of date contains the making)."""
+        mod, shift, held = self._mod.get(num_steps, (None, None, None))
+        linears = [self.time_mlp_in, self.time_mlp_out, self.ada_dense]
+        if self.fold_norms:
+            linears.append(self.action_out)
+            for L in self.expert:
+                linears += L["qkv"], L["gate_up"]
+        marks = _Marks.of(linears)
+        if held is None or not marks.same(held):
+            capturing = torch.cuda.is_current_stream_capturing()
+            if capturing and mod is None:
                 raise TurboPiError("the modulation table of a new schedule must be built before the capture")
-            mod = self._ada_modulation(num_steps)
-            mod = self._mod[num_steps] = (mod, self._shifts(mod) if self.fold_norms else None)
-        return mod
+            mod = self._ada_modulation(num_steps, mod)
+            shift = self._shifts(mod, shift) if self.fold_norms else None
+            if not capturing:
+                self._mod[num_steps] = (mod, shift, marks)
+        return mod, shift
 
     def denoise_loop(self, num_steps):
         mod, shift = self._modulation(num_steps)
@@ -649,6 +707,7 @@ class Pi05:
     def capture(self, num_steps):
         """Capture vision + prefix + the whole denoise loop as one CUDA graph."""
         side = torch.cuda.Stream(device=self.device)
+        side.wait_stream(torch.cuda.current_stream(self.device))     # the warm-up makes tables of weights written there
         with torch.cuda.stream(side):
             self.forward(num_steps)            # warm-up: attribute setup, allocator pools
         torch.cuda.synchronize(self.device)
@@ -676,6 +735,12 @@ class Pi05:
         if use_graph:
             if self._graph is None or self._graph_steps != num_steps:
                 self.capture(num_steps)
+            else:                              # tables that a write has made stale: in the memory the graph reads them from
+                if self._pos_marks is None or self._pos_marks.written():
+                    self._positions()
+                marks = self._mod[num_steps][2]
+                if marks is None or marks.written():
+                    self._modulation(num_steps)
             self._graph.replay()
         else:
             self.forward(num_steps)
