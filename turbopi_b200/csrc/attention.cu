@@ -176,11 +176,13 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
         tc::tmem_alloc(&ctl->tmem_base, kTmemColsAttn);
         tc::tmem_relinquish();
     }
-    pdl_launch_dependents();
     tc::fence_before_thread_sync();
     __syncthreads();
     tc::fence_after_thread_sync();
     const uint32_t tmem = ctl->tmem_base;
+    // Behind the barrier: this CTA has its columns.  A CTA of the next launch that took them first would hold them until this
+    // grid ends, and this CTA would wait for them.
+    pdl_launch_dependents();
     pdl_wait_prior_grids();                               // q, k, v (and the bias) may come from the previous kernel
 
     // warps 1..8: the keys' additive bias in the base-2 domain (visible to all after the barrier behind the S wait)
@@ -511,11 +513,13 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_cluster_kernel(cons
         tc::tmem_alloc(&ctl->tmem_base, tmem_cols);
         tc::tmem_relinquish();
     }
-    pdl_launch_dependents();
     tc::fence_before_thread_sync();
     __syncthreads();
     tc::fence_after_thread_sync();
     const uint32_t tmem = ctl->tmem_base;
+    // Behind the barrier: this CTA has its columns.  A CTA of the next launch that took them first would hold them until this
+    // grid ends, and this CTA would wait for them.
+    pdl_launch_dependents();
     pdl_wait_prior_grids();                               // q, k, v (and the bias) may come from the previous kernel
 
     if (warp >= 4 && warp < 8) {                          // one key per thread (visible to all behind the S wait)
