@@ -288,6 +288,13 @@ typedef struct {
     int tokens_per_tile, splits, ctas_per_sm, groups, parts, weight_slots, step_slots, k_blocks, k_steps;
 } tpb200_w4_gemm_plan_info;
 int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_plan_info* info);
+/* The same for a plain linear of one weight format, launched with `flags`, and what a CTA takes of an SM.  `parts` 64-K parts
+ * are dequantised at a time by a group, `units_per_step` such units go to the tensor cores together; step_slots counts steps. */
+typedef struct {
+    int tokens_per_tile, splits, ctas_per_sm, groups, parts, units_per_step, weight_slots, step_slots, k_blocks, k_steps;
+    int tmem_columns, smem_bytes;
+} tpb200_w4_gemm_launch_info;
+int tpb200_w4_gemm_describe(int M, int N, int K, int format, int flags, int sms, tpb200_w4_gemm_launch_info* info);
 
 /* ---------------------------------------------------------------------------------------------
  * NVFP4 weight-only GEMV for decode shapes (M <= 16) on the tensor cores: same result as
@@ -400,6 +407,12 @@ typedef struct {
 } tpb200_attention_args;
 size_t tpb200_attention_workspace_size(int n_rows, int n_keys, int head_dim, int groups);
 int tpb200_attention(const tpb200_attention_args* args, tpb200_stream_t stream);
+/* What a launch of that shape looks like (host only, no device needed): CTAs of a cluster (0: no clusters) and the pieces
+ * head_dim is cut into, tensor memory columns and dynamic shared memory of a CTA. */
+typedef struct {
+    int cluster_ctas, head_dim_parts, tmem_columns, smem_bytes;
+} tpb200_attention_launch_info;
+int tpb200_attention_describe(int n_rows, int n_keys, int head_dim, int groups, int fused_quant, tpb200_attention_launch_info* info);
 
 /* ---------------------------------------------------------------------------------------------
  * Row-wise glue between two linears, fused with the activation quantiser of the tensor-core GEMM:

@@ -60,6 +60,15 @@ class W4NormArgs(ctypes.Structure):
                 ("copy_out", c_void_p)]
 
 
+class W4GemmLaunchInfo(ctypes.Structure):
+    _fields_ = [(n, c_int) for n in ("tokens_per_tile", "splits", "ctas_per_sm", "groups", "parts", "units_per_step", "weight_slots",
+                                     "step_slots", "k_blocks", "k_steps", "tmem_columns", "smem_bytes")]
+
+
+class AttentionLaunchInfo(ctypes.Structure):
+    _fields_ = [(n, c_int) for n in ("cluster_ctas", "head_dim_parts", "tmem_columns", "smem_bytes")]
+
+
 class W4GemmPlanInfo(ctypes.Structure):
     _fields_ = [(n, c_int) for n in ("tokens_per_tile", "splits", "ctas_per_sm", "groups", "parts", "weight_slots", "step_slots",
                                      "k_blocks", "k_steps")]
@@ -131,6 +140,7 @@ SIGNATURES = {
     "tpb200_nvfp4_gemm": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int,
                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "tpb200_w4_gemm_plan": (c_int, [c_int, c_int, c_int, c_int, ctypes.POINTER(W4GemmPlanInfo)]),
+    "tpb200_w4_gemm_describe": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(W4GemmLaunchInfo)]),
     "tpb200_w4_gemm": (c_int, [ctypes.POINTER(W4GemmArgs), c_void_p]),
     "tpb200_w4_gemm_norm": (c_int, [ctypes.POINTER(W4GemmArgs), ctypes.POINTER(W4NormArgs), c_void_p]),
     "tpb200_pi05_patches": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
@@ -151,6 +161,7 @@ SIGNATURES = {
     "tpb200_nvfp4_gemv_tc_plan": (c_int, [ctypes.POINTER(c_int), ctypes.POINTER(c_int), c_int, c_int,
                                           ctypes.POINTER(GemvTcPlanInfo)]),
     "tpb200_attention_workspace_size": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "tpb200_attention_describe": (c_int, [c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(AttentionLaunchInfo)]),
     "tpb200_attention": (c_int, [ctypes.POINTER(AttentionArgs), c_void_p]),
     "tpb200_w4a16_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                                   c_int, c_int, c_int, c_float, c_float, c_int, c_void_p]),

@@ -85,6 +85,7 @@ struct AttnParams {
     int qa_pieces;
     int qa_rows_per_token;
     int dv_parts, dv_part;   // cluster form: head_dim cut into dv_parts pieces of dv_part columns (the N of the second MMA)
+    int tmem_cols;
     uint8_t* qa_sf;          // not null: the row-major operand form (codes [pieces * piece_rows, pitch] + scale atoms)
     int qa_pitch, qa_piece_rows;
 };
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_cluster_kernel(cons
     const int ga = g / P.groups_inner, gb = g - ga * P.groups_inner;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform, and known to be
     const int key0 = kt * kKeyTile;
-    const uint32_t tmem_cols = P.dv_part <= 128 ? 256 : 512;   // half of it leaves room for the next launch's CTA
+    const uint32_t tmem_cols = P.tmem_cols;
     constexpr uint32_t kColOc = kKeyTile;
 
     if (threadIdx.x == 0) {
@@ -932,19 +933,40 @@ int attn_dims(int n_rows, int n_keys, int head_dim, int groups, AttnDims& d) {
     return TPB200_OK;
 }
 
+size_t partial_smem(const AttnDims& d) {
+    const int nchunk = d.dpad / 64;
+    return static_cast<size_t>(std::max(nchunk, 4) + 2 * nchunk) * tpb::kChunkBytes + sizeof(tpb::AttnControl) + 1024;
+}
+
 // The cluster form: 128 keys per CTA, 2 to 8 key tiles, and the finest cut of head_dim (whole 64-column blocks) whose clusters
 // all run at once.  cudaOccupancyMaxActiveClusters with an SM per CTA (GPCs hold whole clusters): kFit.  0: not for it.
-int cluster_dv_parts(int n_rows, int n_keys, int head_dim, int groups) {
+int cluster_dv_parts(const AttnDims& d, int n_rows, int n_keys, int head_dim) {
+    if (d.key_tiles == 1 || d.keys_per_cta != 128) return 0;
     constexpr int kFit[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
     const int tiles = (n_keys + 127) / 128, row_tiles = (n_rows + 127) / 128;
     if (tiles < 2 || tiles > 8) return 0;
     const int blocks = head_dim / 64;
     for (int parts = head_dim % 64 == 0 ? std::min(blocks, 4) : 1; parts >= 1; parts /= 2) {
         if (blocks % parts == 0 || parts == 1) {
-            if (static_cast<long long>(row_tiles) * groups * parts <= kFit[tiles]) return parts;
+            if (static_cast<long long>(row_tiles) * d.groups * parts <= kFit[tiles]) return parts;
         }
     }
     return 0;
+}
+
+// Tensor memory and shared memory of a CTA of the cluster form; half of the tensor memory where it is enough
+struct ClusterDims { int dv_part, dvp, tmem_cols, smem; };
+
+ClusterDims cluster_dims(const AttnDims& d, int head_dim, int dv_parts) {
+    ClusterDims c;
+    const int nchunk = d.dpad / 64;
+    c.dv_part = dv_parts > 1 ? head_dim / dv_parts : d.dv;
+    c.dvp = (c.dv_part + 31) / 32 * 32;
+    c.tmem_cols = c.dv_part <= 128 ? 256 : 512;
+    c.smem = std::max((std::max(nchunk, 2) + nchunk + (c.dv_part + 63) / 64) * tpb::kChunkBytes, tpb::kRows * c.dvp * 4) +
+             static_cast<int>(sizeof(tpb::ClusterControl)) + 1024;
+    c.smem = std::max(c.smem, tpb::min_smem_of_columns(c.tmem_cols));
+    return c;
 }
 
 // Tensor map of one operand: [outer groups][inner groups][rows][head_dim] with element strides (stride[0],
@@ -995,6 +1017,21 @@ extern "C" size_t tpb200_attention_workspace_size(int n_rows, int n_keys, int he
     AttnDims d;
     if (attn_dims(n_rows, n_keys, head_dim, groups, d) != TPB200_OK) return 0;
     return (d.part_o_floats + d.part_ml_floats) * sizeof(float) + 256;
+}
+
+extern "C" int tpb200_attention_describe(int n_rows, int n_keys, int head_dim, int groups, int fused_quant, tpb200_attention_launch_info* info) {
+    TPB_REQUIRE(info != nullptr, TPB200_ERR_NULL);
+    AttnDims d;
+    const int st = attn_dims(n_rows, n_keys, head_dim, groups, d);
+    if (st != TPB200_OK) return st;
+    const int parts = fused_quant ? 0 : cluster_dv_parts(d, n_rows, n_keys, head_dim);
+    if (parts == 0) {
+        *info = {0, 0, static_cast<int>(tpb::kTmemColsAttn), static_cast<int>(partial_smem(d))};
+    } else {
+        const ClusterDims c = cluster_dims(d, head_dim, parts);
+        *info = {(n_keys + 127) / 128, parts, c.tmem_cols, c.smem};
+    }
+    return TPB200_OK;
 }
 
 extern "C" int tpb200_attention(const tpb200_attention_args* a, tpb200_stream_t stream) {
@@ -1072,15 +1109,14 @@ extern "C" int tpb200_attention(const tpb200_attention_args* a, tpb200_stream_t 
     P.qa_pitch = a->quant_pitch;
     P.qa_piece_rows = a->quant_piece_rows;
 
-    const int nchunk = d.dpad / 64;
-    const int dv_parts = quant || d.key_tiles == 1 || d.keys_per_cta != 128 ? 0 : cluster_dv_parts(a->n_rows, a->n_keys, a->head_dim, d.groups);
+    const int dv_parts = quant ? 0 : cluster_dv_parts(d, a->n_rows, a->n_keys, a->head_dim);
     if (dv_parts > 0) {
         P.dv_parts = dv_parts;
-        P.dv_part = dv_parts > 1 ? a->head_dim / dv_parts : d.dv;
-        P.dvp = (P.dv_part + 31) / 32 * 32;
+        const ClusterDims c = cluster_dims(d, a->head_dim, dv_parts);
+        P.dv_part = c.dv_part;
+        P.dvp = c.dvp;
+        P.tmem_cols = c.tmem_cols;
         P.key_tiles = (a->n_keys + 127) / 128;
-        const size_t bytes = std::max((std::max(nchunk, 2) + nchunk + (P.dv_part + 63) / 64) * tpb::kChunkBytes, tpb::kRows * P.dvp * 4) +
-                             sizeof(tpb::ClusterControl) + 1024;
         static std::atomic<uint64_t> ready[2] = {};
         const int many = P.key_tiles > 4;
         auto kernel = many ? tpb::attention_cluster_kernel<8> : tpb::attention_cluster_kernel<4>;
@@ -1100,13 +1136,13 @@ extern "C" int tpb200_attention(const tpb200_attention_args* a, tpb200_stream_t 
         cudaLaunchConfig_t cc = {};
         cc.gridDim = dim3(P.key_tiles, d.row_tiles * dv_parts, d.groups);
         cc.blockDim = dim3(tpb::kThreadsAttn, 1, 1);
-        cc.dynamicSmemBytes = bytes;
+        cc.dynamicSmemBytes = c.smem;
         cc.stream = reinterpret_cast<cudaStream_t>(stream);
         cc.attrs = ca;
         cc.numAttrs = (a->flags & TPB200_FLAG_PDL) ? 2 : 1;
         return cudaLaunchKernelEx(&cc, kernel, P) == cudaSuccess ? TPB200_OK : TPB200_ERR_CUDA;
     }
-    const size_t smem = static_cast<size_t>(std::max(nchunk, 4) + 2 * nchunk) * tpb::kChunkBytes + sizeof(tpb::AttnControl) + 1024;
+    const size_t smem = partial_smem(d);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);

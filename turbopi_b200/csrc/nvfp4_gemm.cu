@@ -1599,8 +1599,9 @@ extern "C" int tpb200_nvfp4_gemm_ex(const tpb200_nvfp4_gemm_args* a, tpb200_stre
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         return TPB200_ERR_CUDA;
     }
-    const size_t smem = tpb::num_stages(pieces, tiled) * tpb::stage_bytes(pieces, tiled) + 2 * tpb::kOutBuf +
-                        sizeof(tpb::SharedControl) + 1024;
+    const size_t smem = std::max<size_t>(tpb::num_stages(pieces, tiled) * tpb::stage_bytes(pieces, tiled) + 2 * tpb::kOutBuf +
+                                             sizeof(tpb::SharedControl) + 1024,
+                                         tpb::min_smem_of_columns(tpb::kTmemCols));
     static std::atomic<uint64_t> configured{0};
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {

@@ -154,6 +154,13 @@ __device__ __forceinline__ bool elect_one() {
 
 }  // namespace tc
 
+// ------------------------------------------------------------------ host: launches that wait while they hold tensor memory
+// The least dynamic shared memory of a launch whose CTAs wait for one another (a cluster, the partners of a split K) with `cols`
+// columns of tensor memory each.  Two such launches in two streams must not share an SM unless their columns fit side by side:
+// CTAs of each could hold one SM and want the other's.  An SM has 228 KB, 1 KB of them goes to every CTA: three CTAs of 256
+// columns never meet (3 x 78 KB), nor does one of 512 with another of either kind (154 + 78).
+constexpr int min_smem_of_columns(int cols) { return (cols <= 256 ? 77 : 153) * 1024; }
+
 // ------------------------------------------------------------------ host: tensor maps
 // 2-D byte tensor [rows, row_bytes] with pitch `pitch_bytes`, box 128 bytes x box_rows, 128-byte swizzle.
 // Returns false if the driver entry point is unavailable or refuses the shape.

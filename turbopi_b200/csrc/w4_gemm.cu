@@ -1039,6 +1039,14 @@ W4gRing ring_of(const W4gPlan& plan, int k_blocks, int k_steps) {
     return r;
 }
 
+// Dynamic shared memory: the rings, then the accumulators of the epilogue in their place; K ranges summed inside a cluster
+// keep other clusters off the SM if their tensor memory would not fit beside this one's.
+int smem_of(const W4gPlan& plan, const W4gRing& r, bool direct) {
+    const int rings = r.n_w * kWSlot + r.n_s * plan.nt * 128 * r.parts * r.merge;
+    const int smem = std::max(rings, direct ? r.groups * 4 * 2048 : plan.nt * kRows * 4) + 1024;
+    return plan.splits > 1 ? std::max(smem, min_smem_of_columns(r.tmem_cols)) : smem;
+}
+
 }  // namespace
 
 int device_error_w4_gemm(int clear) { return read_device_error(clear); }
@@ -1175,9 +1183,6 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     P.merge = ring.merge;
     P.n_w = ring.n_w;
     P.n_s = ring.n_s;
-    int smem = P.n_w * kWSlot + P.n_s * P.nt * 128 * P.parts * P.merge;
-    smem = std::max(smem, P.epilogue == kEpiDirect ? ring.groups * 4 * 2048 : P.nt * kRows * 4);
-    smem += 1024;
 
     using Kernel = void (*)(const W4gParams);
     static const Kernel kernels[4][2] = {{w4_nvfp4_gemm_kernel<false>, w4_nvfp4_gemm_kernel<true>},
@@ -1197,7 +1202,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles * P.splits, (M + P.nt - 1) / P.nt, 1);
     cfg.blockDim = dim3((kDqWarp0 + 4 * ring.groups) * 32, 1, 1);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = smem_of(plan, ring, direct != 0);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
@@ -1236,6 +1241,18 @@ extern "C" int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_
     const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms);
     const tpb::W4gRing r = tpb::ring_of(plan, k_blocks, k_steps);
     *info = {plan.nt, plan.splits, plan.half ? 2 : 1, r.groups, r.parts, r.n_w, r.n_s * r.merge, k_blocks, k_steps};
+    return TPB200_OK;
+}
+
+extern "C" int tpb200_w4_gemm_describe(int M, int N, int K, int format, int flags, int sms, tpb200_w4_gemm_launch_info* info) {
+    TPB_REQUIRE(info != nullptr, TPB200_ERR_NULL);
+    TPB_REQUIRE(M >= 1 && M <= 65535 * 256 && N >= 8 && K >= 16 && sms >= 1, TPB200_ERR_SHAPE);
+    TPB_REQUIRE(format >= TPB200_W4_NVFP4_ROWMAJOR && format <= TPB200_W4_INT4_PLUGIN && (flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
+    const int k_blocks = (K + tpb::kBlkK - 1) / tpb::kBlkK, k_steps = (K + tpb::kPartK - 1) / tpb::kPartK;
+    const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms);
+    const tpb::W4gRing r = tpb::ring_of(plan, k_blocks, k_steps);
+    *info = {plan.nt, plan.splits, plan.half ? 2 : 1, r.groups, r.parts, r.merge, r.n_w, r.n_s, k_blocks, k_steps, r.tmem_cols,
+             tpb::smem_of(plan, r, plan.splits == 1)};
     return TPB200_OK;
 }
 
