@@ -266,9 +266,8 @@ class NVFP4PackedLinear(_TiledWeightsOwner):
                 and codes.is_cuda and self.in_features % 16 == 0)
 
     def _stored(self):
-        """(weight_packed, weight_scales), without the module's attribute search (a third of a microsecond each)"""
-        b = self._buffers
-        return b["weight_packed"], b["weight_scales"]
+        """(weight_packed, weight_scales)"""
+        return ops.registered(self, "_buffers", "weight_packed"), ops.registered(self, "_buffers", "weight_scales")
 
     def _tc_state(self):
         """(tiled weight image, GEMV scratch, whether the image is finished)"""
@@ -375,17 +374,16 @@ class NVFP4PackedMLP(_TiledWeightsOwner):
     def _stacked_gate_up(self):
         """(tiled image of [W_gate; W_up], GEMV scratch, whether the image is finished), or None if the projections do not
         share a global scale (each was quantised on its own: the stacked launch needs a common fp32 multiplier)."""
-        g, u = self._modules["gate_proj"], self._modules["up_proj"]
+        g, u = ops.registered(self, "_modules", "gate_proj"), ops.registered(self, "_modules", "up_proj")
         if g.global_scale != u.global_scale:
             return None
         (gc, gs), (uc, us) = g._stored(), u._stored()
         return self._tiled((gc, uc), (gs, us), 2 * self.intermediate_size, self.hidden_size)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        m = self._modules                             # (the module's attribute search costs a third of a microsecond each)
-        g, u, d = m["gate_proj"], m["up_proj"], m["down_proj"]
-        fast = (g.tensor_core_ready() and u.tensor_core_ready() and d.tensor_core_ready() and g._parameters["bias"] is None
-                and u._parameters["bias"] is None and g.activation in ("gelu", "silu") and self.intermediate_size % 16 == 0)
+        g, u, d = (ops.registered(self, "_modules", name) for name in ("gate_proj", "up_proj", "down_proj"))
+        fast = (g.tensor_core_ready() and u.tensor_core_ready() and d.tensor_core_ready() and ops.registered(g, "_parameters", "bias") is None
+                and ops.registered(u, "_parameters", "bias") is None and g.activation in ("gelu", "silu") and self.intermediate_size % 16 == 0)
         st = self._stacked_gate_up() if fast else None
         if st is None:
             return self.down_proj(self.gate_proj(x) * self.up_proj(x))
@@ -398,7 +396,7 @@ class NVFP4PackedMLP(_TiledWeightsOwner):
         mode = _lib.ROW_GELU_MUL if g.activation == "gelu" else _lib.ROW_SILU_MUL
         d_image, d_gemv_ws, d_finished = d._tc_state()
         first = ops.FLAG_PDL if finished and d_finished else ops.FLAG_NONE     # the flags of the first launch on an image
-        d_bias = d._parameters["bias"]
+        d_bias = ops.registered(d, "_parameters", "bias")
         if d_bias is not None:
             d_bias = d_bias.detach().float().contiguous()
         dense = (I % 64 == 0 and self.hidden_size % 16 == 0 and _dense_is_faster(T, 2 * I, self.hidden_size, True)

@@ -153,9 +153,9 @@ class W4A16Linear(nn.Module):
         return dequantize_kblock(self.weight_packed, self.scales)
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
-        buffers = self._buffers                       # (the module's attribute search costs a third of a microsecond each)
-        done = (_lib._native or _lib.native()).w4a16_linear(input, buffers["weight_packed"], buffers["scales"],
-                                                            self._parameters["bias"], self.out_features, ops._flags.value)
+        packed, scales = ops.registered(self, "_buffers", "weight_packed"), ops.registered(self, "_buffers", "scales")
+        bias = ops.registered(self, "_parameters", "bias")
+        done = (_lib._native or _lib.native()).w4a16_linear(input, packed, scales, bias, self.out_features, ops._flags.value)
         if done is not None:
             return ops._result(done, "W4A16Linear")
         K, N = input.shape[-1], self.out_features
@@ -166,9 +166,7 @@ class W4A16Linear(nn.Module):
         if not x.is_contiguous():
             x = x.contiguous()
         T = x.shape[0]
-        packed, scales = self.weight_packed, self.scales
         out = torch.empty((T, N), dtype=input.dtype if input.dtype in _FLOATS else torch.float32, device=input.device)
-        bias = self.bias
         if bias is not None:
             bias = bias.detach().contiguous()
             if bias.dtype not in _FLOATS:
