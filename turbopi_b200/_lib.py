@@ -9,7 +9,6 @@ from ctypes import c_char_p, c_float, c_int, c_longlong, c_size_t, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libturbopi_b200.so"
-CALLS_PATH = LIB_PATH.parent / "_calls.so"
 
 F32, F16, BF16 = 0, 1, 2
 ACT_NONE, ACT_GELU, ACT_SILU, ACT_GEGLU = 0, 1, 2, 3
@@ -192,19 +191,36 @@ _NATIVE_ENTRIES = ("tpb200_w4_gemm", "tpb200_w4a16_gemv", "tpb200_w4a16_gemm", "
                    "tpb200_last_error", "tpb200_nvfp4_tiled_a_bytes", "tpb200_nvfp4_quantize_act_tiled", "tpb200_nvfp4_gemm_ex")
 
 
+def calls_path():
+    """csrc/calls.cpp's module for this torch and this Python: with another of either there is no file, not another ABI."""
+    import sysconfig
+
+    import torch
+    return LIB_PATH.parent / f"_calls.torch{torch.__version__}.{sysconfig.get_config_var('SOABI')}.so"
+
+
+class _PythonForms:
+    """Stands in for the module where it has not been built (a library from a host without torch): recognises nothing, so
+    that every call takes its Python form, which launches the same kernels."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def native():
     """The tensor-level calls of csrc/calls.cpp, bound to the library that load() has loaded."""
     global _native
     if _native is None:
         import importlib.util
-
-        import torch  # noqa: F401  (the module links against its libraries)
-        if not CALLS_PATH.exists():
-            raise TurboPiError(f"{CALLS_PATH} is missing: build it with `python -m turbopi_b200.build`")
-        spec = importlib.util.spec_from_file_location("_calls", CALLS_PATH)
+        path, lib = calls_path(), load()
+        if not path.exists():
+            import warnings
+            warnings.warn(f"{path.name} is missing (`python -m turbopi_b200.build` makes it): short calls are issued from Python")
+            _native = _PythonForms()
+            return _native
+        spec = importlib.util.spec_from_file_location("_calls", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
-        lib = load()
         module.bind([ctypes.cast(getattr(lib, name), c_void_p).value for name in _NATIVE_ENTRIES])
         _native = module
     return _native

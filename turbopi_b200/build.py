@@ -3,7 +3,8 @@
     python -m turbopi_b200.build [--force]
 
 Every .cu under csrc/ is one translation unit; objects are compiled in parallel
-into csrc/_obj/ and linked into lib/libturbopi_b200.so; csrc/calls.cpp becomes lib/_calls.so.  A unit is recompiled only
+into csrc/_obj/ and linked into lib/libturbopi_b200.so, which needs nvcc only.  Where torch is installed,
+csrc/calls.cpp becomes lib/_calls.<torch>.<python>.so besides.  A unit is recompiled only
 when it or a header it can see is newer than its object.
 """
 import concurrent.futures
@@ -18,7 +19,6 @@ CSRC = PKG / "csrc"
 OBJ = CSRC / "_obj"
 LIB = PKG / "lib" / "libturbopi_b200.so"
 CALLS_SRC = CSRC / "calls.cpp"
-CALLS = LIB.parent / "_calls.so"
 INCLUDE = PKG.parent / "include"
 
 NVCC_FLAGS = [
@@ -55,23 +55,35 @@ def _compile(src, force):
 
 
 def _build_calls(force):
-    """csrc/calls.cpp, the calls that take and return tensors: a Python extension module against torch's headers."""
-    if (not force and CALLS.exists() and CALLS.stat().st_mtime > CALLS_SRC.stat().st_mtime
-            and CALLS.stat().st_mtime > (INCLUDE / "turbopi_b200.h").stat().st_mtime):
-        return "up to date"
+    """csrc/calls.cpp, the calls that take and return tensors: a Python extension module against torch's headers.  Its name
+    carries the torch and the Python it was built for; after an upgrade of either it is built anew."""
+    import importlib.util
+    if importlib.util.find_spec("torch") is None:
+        return "skipped (no torch)"
     import sysconfig
 
     import torch
     from torch.utils import cpp_extension
+
+    from ._lib import calls_path
+    if torch.version.cuda is None:
+        return "skipped (torch without CUDA)"
+    out = calls_path()
+    if (not force and out.exists() and out.stat().st_mtime > CALLS_SRC.stat().st_mtime
+            and out.stat().st_mtime > (INCLUDE / "turbopi_b200.h").stat().st_mtime):
+        return "up to date"
     cuda = Path(_nvcc()).resolve().parent.parent
     includes = [*cpp_extension.include_paths(), str(cuda / "include"), sysconfig.get_paths()["include"], str(INCLUDE)]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_calls",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in includes), str(CALLS_SRC),
-           "-o", str(CALLS), *(f"-L{p}" for p in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+           "-o", str(out), *(f"-L{p}" for p in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
            "-ltorch_python"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {CALLS_SRC.name}:\n{r.stderr[-4000:]}")
+    for other in out.parent.glob("_calls*.so"):
+        if other != out:
+            other.unlink()
     return "compiled"
 
 
@@ -84,9 +96,6 @@ def build(force=False, verbose=False):
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(sources) + 1)) as ex:
         calls = ex.submit(_build_calls, force)
         results = list(ex.map(lambda s: _compile(s, force), sources))
-        state = calls.result()
-    if verbose:
-        print(f"[turbopi_b200.build] {CALLS_SRC.name}: {state}")
     changed = any(state == "compiled" for _, state, _ in results)
     if verbose:
         for name, state, _ in results:
@@ -100,6 +109,9 @@ def build(force=False, verbose=False):
             raise RuntimeError(f"link failed:\n{r.stderr[-4000:]}")
         if verbose:
             print(f"[turbopi_b200.build] linked {LIB}")
+    state = calls.result()                     # a failure there leaves the library built
+    if verbose:
+        print(f"[turbopi_b200.build] {CALLS_SRC.name}: {state}")
     return LIB
 
 
