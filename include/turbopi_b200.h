@@ -264,6 +264,7 @@ int tpb200_w4_gemm(const tpb200_w4_gemm_args* args, tpb200_stream_t stream);
  *          [M, N] (may be res_in), bf16(h * (1 + scale)) to `out`, the sums of h^2 over 128 columns to out_sumsq
  *          [M, N / 128].  N % 128 == 0, bf16 out, no activation, no beta, neither gated nor QKV.
  *   copy_out != NULL (with in_sumsq, a plain linear): the result also goes to copy_out [M, N] as bf16.
+ * in_shift and copy_out without in_sumsq are refused (TPB200_ERR_NULL).
  * in_shift, gate and scale are parameters like the weights: under TPB200_FLAG_PDL they may be read while the kernel before
  * this one still runs. */
 typedef struct {

@@ -1089,6 +1089,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
         TPB_REQUIRE(static_cast<long long>(a->ldo) * tpb_dtype_size(a->out_dtype) % 16 == 0, TPB200_ERR_ALIGN);
     }
     const bool norm_in = norm != nullptr && norm->in_sumsq != nullptr, norm_out = norm != nullptr && norm->h_out != nullptr;
+    TPB_REQUIRE(norm == nullptr || norm_in || (norm->in_shift == nullptr && norm->copy_out == nullptr), TPB200_ERR_NULL);
     if (norm_in) {
         TPB_REQUIRE(nv, TPB200_ERR_ENUM);
         TPB_REQUIRE(norm->in_parts >= 4 && norm->in_parts % 4 == 0, TPB200_ERR_SHAPE);
