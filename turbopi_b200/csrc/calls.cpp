@@ -123,7 +123,7 @@ py::object w4a16_linear(const at::Tensor& input, const at::Tensor& packed, const
     const int dev = here(input);
     const int code = code_of(input.scalar_type());
     if (dev < 0 || code < 0 || input.dim() < 1 || !input.is_contiguous() || !on(packed, dev) || !on(scales, dev) || !on(bias, dev) ||
-        packed.dim() != 3 || input.size(-1) != packed.size(0) * 32 ||
+        packed.dim() != 3 || packed.size(0) == 0 || input.size(-1) != packed.size(0) * 32 ||
         (bias.has_value() && (code_of(bias->scalar_type()) < 0 || !bias->is_contiguous())) || scales.scalar_type() != at::kHalf) {
         return py::none();
     }
