@@ -21,6 +21,11 @@ WRITES = {
 }
 
 
+def _moved(w):
+    """Other values of the same kind: rows reversed, images of bytes turned by 512, vectors by one."""
+    return w.flip(0) if w.dim() > 1 else w.roll(512 if w.dtype == torch.uint8 else 1)
+
+
 @torch.no_grad()
 @pytest.mark.parametrize("expert_width", [128, 512])           # row kernels / the norms in the linears' epilogues
 @pytest.mark.parametrize("use_graph", [False, True])
@@ -34,11 +39,11 @@ def test_written_weights_are_followed(cuda_device, expert_width, use_graph, what
     run = lambda m: m.infer(images, tokens, noise, num_steps=2, use_graph=use_graph).clone()     # noqa: E731
     before = run(model)
     w = WRITES[what](model)
-    w.copy_(w.flip(0) if w.dim() > 1 else w.roll(512))
+    w.copy_(_moved(w))
     after = run(model)
     fresh = run(Pi05.sharing_weights(model))                   # the same weights, tables of its own
     assert torch.equal(after, fresh) and not torch.equal(after, before)
-    w.data.copy_(w.data.flip(0) if w.dim() > 1 else w.data.roll(512))      # a write that no version counter sees
+    w.data.copy_(_moved(w.data))      # a write that no version counter sees
     model.weights_changed()
     assert torch.equal(run(model), run(Pi05.sharing_weights(model)))
 
