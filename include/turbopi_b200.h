@@ -282,14 +282,15 @@ int tpb200_pi05_patches(const void* images_u8, void* patches, int num_images, in
                         tpb200_stream_t stream);
 int tpb200_pi05_embed(const long long* tokens, const void* table, void* out, int num_tokens, long long vocab, int width, float scale,
                       int flags, tpb200_stream_t stream);
-/* What a launch of that shape looks like on a GPU of `sms` SMs (host only, no device needed): tokens per tile, K ranges
- * per tile, CTAs per SM, groups of four dequantising warps, 64-K parts per step, slots of the weight and of the step ring,
- * 256-K blocks and 64-K parts of the whole K. */
+/* What a launch of that shape looks like with NVFP4 weights on a GPU of `sms` SMs (host only, no device
+ * needed): tokens per tile, K ranges per tile, CTAs per SM, groups of four dequantising warps, 64-K parts that a group
+ * dequantises at a time, slots of the weight ring and of the ring of operand steps (tpb200_w4_gemm_describe: how many such
+ * units a step is), 256-K blocks and 64-K parts of the whole K. */
 typedef struct {
     int tokens_per_tile, splits, ctas_per_sm, groups, parts, weight_slots, step_slots, k_blocks, k_steps;
 } tpb200_w4_gemm_plan_info;
 int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_plan_info* info);
-/* The same for a plain linear of one weight format, launched with `flags`, and what a CTA takes of an SM.  `parts` 64-K parts
+/* The same for a plain linear of one weight format (the flags do not change the plan), and what a CTA takes of an SM.  `parts` 64-K parts
  * are dequantised at a time by a group, `units_per_step` such units go to the tensor cores together; step_slots counts steps. */
 typedef struct {
     int tokens_per_tile, splits, ctas_per_sm, groups, parts, units_per_step, weight_slots, step_slots, k_blocks, k_steps;

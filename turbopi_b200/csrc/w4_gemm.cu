@@ -950,38 +950,74 @@ __global__ void __launch_bounds__(kBoundThreads, 1) w4_int4_plugin_gemm_kernel(c
 }
 
 // ---------------------------------------------------------------- launch plan
+// 64-K parts per unit, the share of a weight block that a group of warps dequantises at a time: two where four such units
+// (one per group) fit the step ring.  What a unit costs beside its arithmetic (barriers, positions, phases) is ~100
+// instructions of a loop that is bound by their issue.
+constexpr int unit_parts(int nt, bool half) { return nt <= (half ? 64 : 144) ? 2 : 1; }
+
 // Tokens per tile, K ranges per tile, and whether two CTAs share an SM (8 dequantising warps each) or one has it
-// to itself (16 warps).  Measured (B200, us per launch; 50 tokens, K = 1024 / 2048 / 1024 / 4096): qkv 4.5, o 4.9, gate_up
-// 5.7, down 6.0, where the e2m1-piece GEMM takes 7.8, 7.9, 8.5 and 8.8 behind a quantiser.
+// to itself (16 warps).
 struct W4gPlan { int nt, splits; bool half; };
 
-W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
-    // Microseconds on a B200, fitted to 62 shapes chained by programmatic dependent launch (1 to 900 tokens, 1024 to 32768
-    // rows, K 1024 to 16384; eight of them in the pipeline's own chains), every candidate measured: what it chooses is 2 %
-    // off the best on average, 16 % at worst.
+// What a launch takes, about in microseconds on a B200; it only has to rank the candidates.  One per weight form, fitted to 485 shapes
+// (1 to 1000 tokens, 512 to 32768 rows, K 512 to 16384) with every candidate measured as a plain launch and in a chain of
+// programmatic dependent ones.  A shape has one plan for both (a launch flag does not change a result's bits): NVFP4 weighs the chains
+// of the modules and the pipeline more, INT4 plain calls; the transposed form is fitted to plain launches alone.  Off the best
+// candidate on average, plain / in a chain: INT4 2.4 / 1.2 %, NVFP4 3.3 / 1.2, transposed 0.7.  One model for all forms was 10 / 6, 7 /
+// 4 and 9 % off, 86 % at worst: it had 0.33 us per 64 K for two CTAs that share an SM, which take 0.62 with INT4 codes, as
+// long as one after the other (712 x 2048 x 16384: 89 us, 49 as planned now).
+struct W4gCost {
+    // 64 K values: max(a, b + c NT), for a CTA with an SM of its own, two that share one, and the narrow form of a CTA
+    // where it has the SM to itself
+    float own[3], shared[3], alone[3];
+    float unpaired;                                  // more where a unit is one part only (ring_of)
+    float round[2], round_nt[2];                     // per round of CTAs, whole and narrow, and its NT x ...
+    float narrow;                                    // a launch of narrow CTAs
+    float split[4], split_nt;                        // 1, 2, 4, 8 K ranges: barrier and sums; NT x 512 bytes per CTA move
+    float cta;                                       // each of up to 150
+    float crowd;                                     // a grid of more than half the room: the next launch of a chain cannot start
+};
+constexpr W4gCost kCostNvfp4 = {{0.0751f, 0.0396f, 0.000391f}, {0.278f, 0.0011f, 0.00152f}, {0.0263f, 0.107f, 0.00137f},
+    -0.00485f, {4.0f, 2.97f}, {0.0109f, 0.0123f}, 0.373f,
+    {0.0f, 0.0402f, 0.00588f, 0.119f}, 0.00461f, 0.0111f, 0.573f};
+constexpr W4gCost kCostInt4 = {{0.0152f, 0.0929f, 0.000222f}, {0.694f, 0.0332f, 0.00325f}, {0.787f, 0.0718f, 0.0357f},
+    0.0143f, {4.05f, 1.1f}, {0.0112f, 0.0149f}, -0.0602f,
+    {0.0f, -0.0167f, 0.0528f, 0.794f}, 0.00374f, 0.0116f, 0.686f};
+constexpr W4gCost kCostTransposed = {{0.308f, 0.0662f, 0.00107f}, {0.744f, 0.332f, 0.00168f}, {0.347f, 0.0999f, 0.00141f},
+    0.0599f, {5.9f, 6.86f}, {0.0382f, 0.0202f}, 0.574f,
+    {0.0f, 0.361f, 0.131f, -0.147f}, 0.00485f, 0.0121f, 0.0f};
+
+// Clusters of 1, 2, 4 and 8 CTAs that run at once with an SM each (GPCs of 16 to 20 SMs hold whole clusters only), as
+// cudaOccupancyMaxActiveClusters has it for every one of these kernels.  Two narrow CTAs do share an SM: times step where
+// twice as many clusters are exceeded (296 CTAs, 148 pairs, 66 fours).  The occupancy calls cannot be asked for that: they allow
+// a kernel that allocates tensor memory one CTA per SM.
+constexpr int kFit[4] = {148, 74, 33, 15};
+
+W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms, int fmt) {
+    const W4gCost& C = fmt == kFmtNvfp4 ? kCostNvfp4 : fmt == kFmtNvfp4T ? kCostTransposed : kCostInt4;
     W4gPlan best{256, 1, false};
     float best_cost = 1e30f;
     for (int nt = 16; nt <= 256; nt += 16) {
         const int tt = (M + nt - 1) / nt;
         if (tt > 65535 || (nt > 16 && (M + nt - 17) / (nt - 16) == tt)) continue;      // a narrower tile does the same
+        const long long clusters = static_cast<long long>(tiles) * tt;
         for (int s = 1, l = 0; s <= 8 && s <= k_blocks; s *= 2, ++l) {
-            const int ctas = static_cast<int>(std::min(1LL * tiles * tt * s, 1LL << 30));
+            const long long ctas = clusters * s, fit = std::max(1, kFit[l] * sms / 148);
             const int steps = (k_blocks + s - 1) / s * 4;            // parts of 64 K values
-            // clusters that fit the machine at once (GPCs of 16 to 20 SMs hold whole clusters only): 148, 74, 33 and 15 of 1, 2,
-            // 4 and 8 CTAs with an SM each, twice that with two CTAs per SM
-            constexpr int kFit[4] = {148, 74, 33, 15};
-            constexpr float kSplit[4] = {0.0f, 0.43f, 1.3f, 2.45f};
             for (int half = 0; half <= (nt <= 128 ? 1 : 0); ++half) {
-                const int per_sm = 1 + half;
-                const long long fit = std::max(1, kFit[l] * sms / 148 * per_sm);
-                const long long waves = (static_cast<long long>(tiles) * tt + fit - 1) / fit;
-                const float step = half ? std::max(0.30f, 0.13f + 0.0025f * nt) : std::max(0.18f, 0.05f + 0.0014f * nt);
-                // a grid of more than half the room leaves the next launch none to start its weight loads in; one of narrow
-                // CTAs leaves more, and costs a little by itself
-                const float crowd = (2LL * ctas > static_cast<long long>(sms) * per_sm ? 1.8f : 0.0f) + (half ? 0.5f : 0.0f);
-                // summing a cluster's tiles through distributed shared memory moves NT x 512 bytes per CTA
-                const float cost = waves * (1.85f + steps * step + (half ? 0.006f : 0.007f) * nt) + kSplit[l] + (l > 0 ? 0.012f * nt : 0.0f) + crowd +
-                                   0.012f * std::min(ctas, 150);
+                auto round = [&](const float (&t)[3]) {
+                    const float step = std::max(t[0], t[1] + t[2] * nt) + (unit_parts(nt, half) == 1 ? C.unpaired : 0.0f);
+                    return C.round[half] + C.round_nt[half] * nt + steps * step;
+                };
+                float cost;
+                if (half) {                                          // rounds that share SMs; the last one may not need to
+                    const long long rounds = clusters / (2 * fit), rest = clusters - rounds * 2 * fit;
+                    cost = C.narrow + rounds * round(C.shared) + (rest == 0 ? 0.0f : round(rest <= fit ? C.alone : C.shared));
+                } else {
+                    cost = (clusters + fit - 1) / fit * round(C.own);
+                }
+                cost += C.split[l] + (l > 0 ? C.split_nt * nt : 0.0f) + C.cta * std::min(ctas, 150LL);
+                if (2 * ctas > static_cast<long long>(sms) * (1 + half)) cost += C.crowd;
                 if (cost < best_cost) {
                     best_cost = cost;
                     best = {nt, s, half != 0};
@@ -993,12 +1029,12 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms) {
 }
 
 // The last plans of this thread: a call's host side is a few microseconds, ranking the candidates is one of them.
-W4gPlan plan_cached(int tiles, int M, int k_blocks, int sms) {
-    struct Entry { int tiles, M, k_blocks, sms; W4gPlan plan; };
+W4gPlan plan_cached(int tiles, int M, int k_blocks, int sms, int fmt) {
+    struct Entry { int tiles, M, k_blocks, sms, fmt; W4gPlan plan; };
     static thread_local Entry cache[32] = {};
     Entry& e = cache[(static_cast<unsigned>(tiles) * 31u + static_cast<unsigned>(M) * 7u + static_cast<unsigned>(k_blocks)) % 32u];
-    if (e.tiles != tiles || e.M != M || e.k_blocks != k_blocks || e.sms != sms) {
-        e = {tiles, M, k_blocks, sms, plan_w4_gemm(tiles, M, k_blocks, sms)};
+    if (e.tiles != tiles || e.M != M || e.k_blocks != k_blocks || e.sms != sms || e.fmt != fmt) {
+        e = {tiles, M, k_blocks, sms, fmt, plan_w4_gemm(tiles, M, k_blocks, sms, fmt)};
     }
     return e.plan;
 }
@@ -1013,9 +1049,7 @@ W4gRing ring_of(const W4gPlan& plan, int k_blocks, int k_steps) {
     r.a_col = (plan.nt + 31) / 32 * 32;
     const int blocks_per = (k_blocks + plan.splits - 1) / plan.splits, steps_per = std::min(blocks_per * 4, k_steps);
     const int budget = (plan.half ? 112 : 225) * 1024 - 1024;
-    // Two parts a unit where four such units (one per group of warps) fit the step ring: what a unit costs beside its
-    // arithmetic (barriers, positions, phases) is ~100 instructions of a loop that is bound by their issue.
-    r.parts = plan.nt <= (plan.half ? 64 : 144) ? 2 : 1;
+    r.parts = unit_parts(plan.nt, plan.half);
     r.groups = plan.half ? 2 : 4;
     // A group takes every `stride`-th weight block.  A parity wait tells a phase from the one before it only, so a group
     // must have waited for EVERY earlier block of a slot it comes to: with more blocks than slots, the number of slots is
@@ -1130,7 +1164,7 @@ int w4_gemm_launch(const tpb200_w4_gemm_args* a, cudaStream_t stream, bool trans
     P.img_kblocks = P.k_blocks;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const W4gPlan plan = plan_cached(tiles, M, P.k_blocks, sms);
+    const W4gPlan plan = plan_cached(tiles, M, P.k_blocks, sms, fmt);
     P.nt = plan.nt;
     P.splits = plan.splits;
     bool ok = make_tensor_map_2d(&P.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a->x, K, M, static_cast<uint64_t>(a->ldx) * 2, 64,
@@ -1239,7 +1273,7 @@ extern "C" int tpb200_w4_gemm_plan(int M, int N, int K, int sms, tpb200_w4_gemm_
     TPB_REQUIRE(info != nullptr, TPB200_ERR_NULL);
     TPB_REQUIRE(M >= 1 && M <= 65535 * 256 && N >= 8 && K >= 16 && sms >= 1, TPB200_ERR_SHAPE);
     const int k_blocks = (K + tpb::kBlkK - 1) / tpb::kBlkK, k_steps = (K + tpb::kPartK - 1) / tpb::kPartK;
-    const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms);
+    const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms, tpb::kFmtNvfp4);
     const tpb::W4gRing r = tpb::ring_of(plan, k_blocks, k_steps);
     *info = {plan.nt, plan.splits, plan.half ? 2 : 1, r.groups, r.parts, r.n_w, r.n_s * r.merge, k_blocks, k_steps};
     return TPB200_OK;
@@ -1250,7 +1284,8 @@ extern "C" int tpb200_w4_gemm_describe(int M, int N, int K, int format, int flag
     TPB_REQUIRE(M >= 1 && M <= 65535 * 256 && N >= 8 && K >= 16 && sms >= 1, TPB200_ERR_SHAPE);
     TPB_REQUIRE(format >= TPB200_W4_NVFP4_ROWMAJOR && format <= TPB200_W4_INT4_PLUGIN && (flags & ~TPB200_FLAG_PDL) == 0, TPB200_ERR_ENUM);
     const int k_blocks = (K + tpb::kBlkK - 1) / tpb::kBlkK, k_steps = (K + tpb::kPartK - 1) / tpb::kPartK;
-    const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms);
+    const tpb::W4gPlan plan = tpb::plan_w4_gemm((N + tpb::kRows - 1) / tpb::kRows, M, k_blocks, sms,
+                                               format >= TPB200_W4_INT4_KBLOCK ? tpb::kFmtKblock : tpb::kFmtNvfp4);
     const tpb::W4gRing r = tpb::ring_of(plan, k_blocks, k_steps);
     *info = {plan.nt, plan.splits, plan.half ? 2 : 1, r.groups, r.parts, r.merge, r.n_w, r.n_s, k_blocks, k_steps, r.tmem_cols,
              tpb::smem_of(plan, r, plan.splits == 1)};
