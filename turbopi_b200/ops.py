@@ -64,13 +64,6 @@ def _run_on(device, fn, *args):
     return fn(*args, _raw_stream(i))
 
 
-def registered(module, table, name):
-    """module.<name>, without the module's attribute search (a third of a microsecond) where it is a registered parameter or
-    buffer; replicas, pruned and parametrised modules hold it elsewhere."""
-    held = module.__dict__[table]
-    return held[name] if name in held else getattr(module, name)
-
-
 def _result(done, what):
     """What a call of csrc/calls.cpp returned: its result, or an int, the status it failed with."""
     if type(done) is int:

@@ -153,8 +153,11 @@ class W4A16Linear(nn.Module):
         return dequantize_kblock(self.weight_packed, self.scales)
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
-        packed, scales = ops.registered(self, "_buffers", "weight_packed"), ops.registered(self, "_buffers", "scales")
-        bias = ops.registered(self, "_parameters", "bias")
+        try:                                          # without the module's attribute search (a third of a microsecond each)
+            held = self._buffers
+            packed, scales, bias = held["weight_packed"], held["scales"], self._parameters["bias"]
+        except KeyError:                              # replicas, pruned and parametrised modules hold them elsewhere
+            packed, scales, bias = self.weight_packed, self.scales, self.bias
         done = (_lib._native or _lib.native()).w4a16_linear(input, packed, scales, bias, self.out_features, ops._flags.value)
         if done is not None:
             return ops._result(done, "W4A16Linear")
