@@ -961,11 +961,11 @@ constexpr int unit_parts(int nt, bool half) { return nt <= (half ? 64 : 144) ? 2
 // to itself (16 warps).
 struct W4gPlan { int nt, splits; bool half; };
 
-// What a launch takes, about in microseconds on a B200; it only has to rank the candidates.  One per weight form, fitted to 485 shapes
+// What a launch takes, about in microseconds on a B200; it only has to rank the candidates.  One per weight form, fitted to 665 shapes
 // (1 to 1000 tokens, 512 to 32768 rows, K 512 to 16384) with every candidate measured as a plain launch and in a chain of
 // programmatic dependent ones.  A shape has one plan for both (a launch flag does not change a result's bits): NVFP4 weighs the chains
 // of the modules and the pipeline more, INT4 plain calls; the transposed form is fitted to plain launches alone.  Off the best
-// candidate on average, plain / in a chain: INT4 2.4 / 1.2 %, NVFP4 3.3 / 1.2, transposed 0.7.  One model for all forms was 10 / 6, 7 /
+// candidate on average, plain / in a chain: INT4 2.0 / 1.6 %, NVFP4 2.3 / 1.2, transposed 0.7.  One model for all forms was 10 / 6, 7 /
 // 4 and 9 % off, 86 % at worst: it had 0.33 us per 64 K for two CTAs that share an SM, which take 0.62 with INT4 codes, as
 // long as one after the other (712 x 2048 x 16384: 89 us, 49 as planned now).
 struct W4gCost {
@@ -977,17 +977,18 @@ struct W4gCost {
     float narrow;                                    // a launch of narrow CTAs
     float split[4], split_nt;                        // 1, 2, 4, 8 K ranges: barrier and sums; NT x 512 bytes per CTA move
     float cta;                                       // each of up to 150
-    float crowd;                                     // a grid of more than half the room: the next launch of a chain cannot start
+    float crowd[2];                                  // a grid of more than half the room leaves the next launch of a chain less to
+                                                     // start in: [0] from a share [1] beyond the half on, in proportion before
 };
-constexpr W4gCost kCostNvfp4 = {{0.0751f, 0.0396f, 0.000391f}, {0.278f, 0.0011f, 0.00152f}, {0.0263f, 0.107f, 0.00137f},
-    -0.00485f, {4.0f, 2.97f}, {0.0109f, 0.0123f}, 0.373f,
-    {0.0f, 0.0402f, 0.00588f, 0.119f}, 0.00461f, 0.0111f, 0.573f};
-constexpr W4gCost kCostInt4 = {{0.0152f, 0.0929f, 0.000222f}, {0.694f, 0.0332f, 0.00325f}, {0.787f, 0.0718f, 0.0357f},
-    0.0143f, {4.05f, 1.1f}, {0.0112f, 0.0149f}, -0.0602f,
-    {0.0f, -0.0167f, 0.0528f, 0.794f}, 0.00374f, 0.0116f, 0.686f};
+constexpr W4gCost kCostNvfp4 = {{0.0723f, 0.0677f, 0.000111f}, {0.247f, 0.0499f, 0.000327f}, {0.00406f, 0.119f, 0.00163f},
+    0.00399f, {3.93f, 2.74f}, {0.014f, 0.0149f}, 0.32f,
+    {0.0f, 0.112f, 0.0622f, 0.0429f}, 0.00508f, 0.00958f, {0.638f, 0.214f}};
+constexpr W4gCost kCostInt4 = {{0.00801f, 0.13f, 0.000399f}, {0.431f, 0.0927f, 0.000306f}, {0.303f, 0.139f, 0.00361f},
+    0.0027f, {2.09f, 0.0589f}, {0.0176f, 0.033f}, -0.11f,
+    {0.0f, 0.02f, 0.0365f, 0.0585f}, 0.00405f, 0.0133f, {1.34f, 0.0866f}};
 constexpr W4gCost kCostTransposed = {{0.308f, 0.0662f, 0.00107f}, {0.744f, 0.332f, 0.00168f}, {0.347f, 0.0999f, 0.00141f},
     0.0599f, {5.9f, 6.86f}, {0.0382f, 0.0202f}, 0.574f,
-    {0.0f, 0.361f, 0.131f, -0.147f}, 0.00485f, 0.0121f, 0.0f};
+    {0.0f, 0.361f, 0.131f, -0.147f}, 0.00485f, 0.0121f, {0.0f, 1.0f}};
 
 // Clusters of 1, 2, 4 and 8 CTAs that run at once with an SM each (GPCs of 16 to 20 SMs hold whole clusters only), as
 // cudaOccupancyMaxActiveClusters has it for every one of these kernels.  Two narrow CTAs do share an SM: times step where
@@ -1019,7 +1020,8 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms, int fmt) {
                     cost = (clusters + fit - 1) / fit * round(C.own);
                 }
                 cost += C.split[l] + (l > 0 ? C.split_nt * nt : 0.0f) + C.cta * std::min(ctas, 150LL);
-                if (2 * ctas > static_cast<long long>(sms) * (1 + half)) cost += C.crowd;
+                const float over = 2.0f * ctas / (sms * (1 + half)) - 1.0f;
+                cost += C.crowd[0] * std::min(1.0f, std::max(0.0f, over / C.crowd[1]));
                 if (cost < best_cost) {
                     best_cost = cost;
                     best = {nt, s, half != 0};
