@@ -463,22 +463,6 @@ struct ClusterControl {
     float weight[kRows / 2][9];                 // of the rows this CTA finishes: 2^(m_p - max) per key tile, 1 / sum
 };
 
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-    return v;
-}
-
 // kTiles: the most key tiles (4 or 8)
 template <int kTiles>
 __global__ void __launch_bounds__(kThreadsAttn, 1) attention_cluster_kernel(const __grid_constant__ AttnParams P) {
