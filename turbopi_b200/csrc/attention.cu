@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kThreadsAttn, 1) attention_partial_kernel(cons
 // against 12.6 with a merge kernel) is the size of the exchange: loads from a peer bring ~15 bytes a nanosecond.  So head_dim is
 // cut as well: CTA (key tile, row tile, piece of head_dim) repeats S = Q K^T and the softmax -- there are SMs to spare -- and
 // computes dv_part columns of O; with 64 columns it stages 32 KB and reads 28 KB.  Chains of dependent launches (B200): 400 rows
-// on 762 keys 11.3 -> 7.7 us, 2744 rows on 343 keys 12.0 -> 9.5.  Of the 7.7: loads of Q and K 1.7, softmax 1.3, O 0.5,
+// on 762 keys 11.3 -> 7.5 us, 2744 rows on 343 keys 12.0 -> 9.2.  Of the first: loads of Q and K 1.7, softmax 1.3, O 0.5,
 // staging and cluster barrier 0.9, merge 1.9.  (The rows sent as bulk copies into the peers' K: 8.0.)
 struct ClusterControl {
     uint64_t bar_qk[4];                         // per 64-column block of head_dim: Q and K have landed

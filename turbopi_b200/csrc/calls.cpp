@@ -2,8 +2,8 @@
 // C ABI's entry point in one step.  The Python forms of the same calls (turbopi_b200/ops.py and the modules) stay the
 // reference for what is accepted: whatever a function here does not recognise as its plain case (a CPU tensor, another
 // device, a dtype or a stride that needs a conversion) returns None and takes the Python form, which converts or refuses.
-// A non-zero status of the C ABI comes back as an int.  Host time per call (us, Python form -> here): one-token INT4 linear
-// 13.4 -> 7.9, 50-token MLP 37 -> 20, attention 20 -> 11, W4A4 linear 27 -> 17, FP8 quantiser + W4A8 launcher 30 -> 23.
+// A non-zero status of the C ABI comes back as an int.  Time to issue a call (us, Python form -> here): one-token INT4 linear
+// 13.1 -> 7.1, 50-token MLP 31.2 -> 17.4, attention 18.2 -> 8.2, W4A4 linear 21.7 -> 12.4, FP8 quantiser + W4A8 launcher 24.4 -> 18.1.
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>

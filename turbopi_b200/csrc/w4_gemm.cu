@@ -19,10 +19,12 @@
 // What bounds it: four 128 x NT x 16 MMAs with A in tensor memory take exactly 2 NT cycles (measured, NT 32..256), the
 // dequantisation of their 128 x 64 weights 250 (NVFP4) to 340 (INT4) cycles of an SM's instruction issue, ~350 to 450 with the
 // loop around it (470-530 before a unit was two parts and the positions were counted), and the token tiles are re-read once
-// per 128 weight rows (434 MB through the L2 at 712 x 16384 x 2048).  B200, in a chain of programmatic dependent launches: INT4
-// 712 x 16384 x 2048 47 us (85 us with weights dequantised through shared memory), 397 x 2048 x 16384 28 us with K split (265
-// without).  Pairs of CTAs sharing the token tile (cta_group::2) halve those reads but were slower (147 against 103 us at 712 x
-// 32768 x 2048): the barrier round trips between the two SMs sit on the issuing warp's path.
+// per 128 weight rows (434 MB through the L2 at 712 x 16384 x 2048).  Counters of that launch and of 712 x 2048 x 16384: issue
+// slots used in 53 and 66 % of the active cycles, tensor pipe 52 and 61 %; the rest is fill, hand-over and epilogue.  B200, in a
+// chain of programmatic dependent launches: INT4 712 x 16384 x 2048 47 us (85 us with weights dequantised through shared
+// memory), 712 x 2048 x 16384 45 and 397 x 2048 x 16384 29 us with K split (265 without).  Pairs of CTAs sharing the token tile
+// (cta_group::2) halve those reads but were slower (147 against 103 us at 712 x 32768 x 2048): the barrier round trips
+// between the two SMs sit on the issuing warp's path.
 //
 // Roles: warp 0 activation tiles (TMA), warp 1 tensor memory + MMA issue, warp 2 weight blocks (256 K values of 128 rows:
 // 16 KB of codes + scales), then 16 warps (8 where two CTAs share an SM) of dequantisation and epilogue.  Weight blocks are
