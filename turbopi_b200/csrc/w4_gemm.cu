@@ -952,16 +952,19 @@ struct W4gPlan { int nt, splits; bool half; };
 
 // What a launch takes, about in microseconds on a B200; it only has to rank the candidates.  One per weight form, fitted to 665 shapes
 // (1 to 1000 tokens, 512 to 32768 rows, K 512 to 16384) with every candidate measured as a plain launch and in a chain of
-// programmatic dependent ones.  A shape has one plan for both (a launch flag does not change a result's bits): NVFP4 weighs the chains
-// of the modules and the pipeline more, INT4 plain calls; the transposed form is fitted to plain launches alone.  Off the best
-// candidate on average, plain / in a chain: INT4 2.0 / 1.6 %, NVFP4 2.3 / 1.2, transposed 0.7.  One model for all forms was 10 / 6, 7 /
-// 4 and 9 % off, 86 % at worst: it had 0.33 us per 64 K for two CTAs that share an SM, which take 0.62 with INT4 codes, as
-// long as one after the other (712 x 2048 x 16384: 89 us, 49 as planned now).
+// programmatic dependent ones.  A shape has one plan for both (a launch flag does not change a result's bits): NVFP4 weighs the
+// chains of the modules and the pipeline more, INT4 plain calls; the transposed form is fitted to plain launches alone.  How many K
+// ranges NVFP4 weights get is ranked by a cost of its own: it decides in which order a result's sums are added, and the
+// pipeline hands on fp32 actions that follow every rounding before them, so it differs from what it was only where it was far off
+// (CTAs of more than 64 tokens that share SMs).  Off the best candidate on average, plain / in a chain: INT4 2.0 / 1.6 %, NVFP4 5.0 /
+// 2.0 (2.3 / 1.2 with free ranges), transposed 0.7.  One model for all forms was 10 / 6, 7 / 4 and 9 % off, 86 % at worst: it
+// had 0.33 us per 64 K for two CTAs that share an SM, which take 0.62 with INT4 codes, as long as one after the other (712 x
+// 2048 x 16384: 89 us, 48 as planned now).
 struct W4gCost {
     // 64 K values: max(a, b + c NT), for a CTA with an SM of its own, two that share one, and the narrow form of a CTA
     // where it has the SM to itself
     float own[3], shared[3], alone[3];
-    float unpaired;                                  // more where a unit is one part only (ring_of)
+    float unpaired[2];                               // more where a unit is one part only (ring_of), whole and narrow
     float round[2], round_nt[2];                     // per round of CTAs, whole and narrow, and its NT x ...
     float narrow;                                    // a launch of narrow CTAs
     float split[4], split_nt;                        // 1, 2, 4, 8 K ranges: barrier and sums; NT x 512 bytes per CTA move
@@ -969,14 +972,17 @@ struct W4gCost {
     float crowd[2];                                  // a grid of more than half the room leaves the next launch of a chain less to
                                                      // start in: [0] from a share [1] beyond the half on, in proportion before
 };
+constexpr W4gCost kCostNvfp4Ranges = {{0.18f, 0.05f, 0.0014f}, {0.34f, 0.0f, 0.0f}, {0.30f, 0.13f, 0.0025f},
+    {0.0f, 0.11f}, {1.85f, 1.85f}, {0.007f, 0.006f}, 0.5f,
+    {0.0f, 0.43f, 1.3f, 2.45f}, 0.012f, 0.012f, {1.8f, 1e-6f}};
 constexpr W4gCost kCostNvfp4 = {{0.0723f, 0.0677f, 0.000111f}, {0.247f, 0.0499f, 0.000327f}, {0.00406f, 0.119f, 0.00163f},
-    0.00399f, {3.93f, 2.74f}, {0.014f, 0.0149f}, 0.32f,
+    {0.00399f, 0.00399f}, {3.93f, 2.74f}, {0.014f, 0.0149f}, 0.32f,
     {0.0f, 0.112f, 0.0622f, 0.0429f}, 0.00508f, 0.00958f, {0.638f, 0.214f}};
 constexpr W4gCost kCostInt4 = {{0.00801f, 0.13f, 0.000399f}, {0.431f, 0.0927f, 0.000306f}, {0.303f, 0.139f, 0.00361f},
-    0.0027f, {2.09f, 0.0589f}, {0.0176f, 0.033f}, -0.11f,
+    {0.0027f, 0.0027f}, {2.09f, 0.0589f}, {0.0176f, 0.033f}, -0.11f,
     {0.0f, 0.02f, 0.0365f, 0.0585f}, 0.00405f, 0.0133f, {1.34f, 0.0866f}};
 constexpr W4gCost kCostTransposed = {{0.308f, 0.0662f, 0.00107f}, {0.744f, 0.332f, 0.00168f}, {0.347f, 0.0999f, 0.00141f},
-    0.0599f, {5.9f, 6.86f}, {0.0382f, 0.0202f}, 0.574f,
+    {0.0599f, 0.0599f}, {5.9f, 6.86f}, {0.0382f, 0.0202f}, 0.574f,
     {0.0f, 0.361f, 0.131f, -0.147f}, 0.00485f, 0.0121f, {0.0f, 1.0f}};
 
 // Clusters of 1, 2, 4 and 8 CTAs that run at once with an SM each (GPCs of 16 to 20 SMs hold whole clusters only), as
@@ -985,8 +991,8 @@ constexpr W4gCost kCostTransposed = {{0.308f, 0.0662f, 0.00107f}, {0.744f, 0.332
 // a kernel that allocates tensor memory one CTA per SM.
 constexpr int kFit[4] = {148, 74, 33, 15};
 
-W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms, int fmt) {
-    const W4gCost& C = fmt == kFmtNvfp4 ? kCostNvfp4 : fmt == kFmtNvfp4T ? kCostTransposed : kCostInt4;
+// The cheapest plan, of `ranges` K ranges where that is not 0
+W4gPlan cheapest_plan(const W4gCost& C, int tiles, int M, int k_blocks, int sms, int ranges) {
     W4gPlan best{256, 1, false};
     float best_cost = 1e30f;
     for (int nt = 16; nt <= 256; nt += 16) {
@@ -994,11 +1000,12 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms, int fmt) {
         if (tt > 65535 || (nt > 16 && (M + nt - 17) / (nt - 16) == tt)) continue;      // a narrower tile does the same
         const long long clusters = static_cast<long long>(tiles) * tt;
         for (int s = 1, l = 0; s <= 8 && s <= k_blocks; s *= 2, ++l) {
+            if (ranges != 0 && s != ranges) continue;
             const long long ctas = clusters * s, fit = std::max(1, kFit[l] * sms / 148);
             const int steps = (k_blocks + s - 1) / s * 4;            // parts of 64 K values
             for (int half = 0; half <= (nt <= 128 ? 1 : 0); ++half) {
                 auto round = [&](const float (&t)[3]) {
-                    const float step = std::max(t[0], t[1] + t[2] * nt) + (unit_parts(nt, half) == 1 ? C.unpaired : 0.0f);
+                    const float step = std::max(t[0], t[1] + t[2] * nt) + (unit_parts(nt, half) == 1 ? C.unpaired[half] : 0.0f);
                     return C.round[half] + C.round_nt[half] * nt + steps * step;
                 };
                 float cost;
@@ -1019,6 +1026,12 @@ W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms, int fmt) {
         }
     }
     return best;
+}
+
+W4gPlan plan_w4_gemm(int tiles, int M, int k_blocks, int sms, int fmt) {
+    if (fmt != kFmtNvfp4) return cheapest_plan(fmt == kFmtNvfp4T ? kCostTransposed : kCostInt4, tiles, M, k_blocks, sms, 0);
+    const int ranges = cheapest_plan(kCostNvfp4Ranges, tiles, M, k_blocks, sms, 0).splits;
+    return cheapest_plan(kCostNvfp4, tiles, M, k_blocks, sms, ranges);
 }
 
 // The last plans of this thread: a call's host side is a few microseconds, ranking the candidates is one of them.
