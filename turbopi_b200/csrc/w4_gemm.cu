@@ -954,12 +954,12 @@ struct W4gPlan { int nt, splits; bool half; };
 // (1 to 1000 tokens, 512 to 32768 rows, K 512 to 16384) with every candidate measured as a plain launch and in a chain of
 // programmatic dependent ones.  A shape has one plan for both (a launch flag does not change a result's bits): NVFP4 weighs the
 // chains of the modules and the pipeline more, INT4 plain calls; the transposed form is fitted to plain launches alone.  How many K
-// ranges NVFP4 weights get is ranked by a cost of its own: it decides in which order a result's sums are added, and the
-// pipeline hands on fp32 actions that follow every rounding before them, so it differs from what it was only where it was far off
-// (CTAs of more than 64 tokens that share SMs).  Off the best candidate on average, plain / in a chain: INT4 2.0 / 1.6 %, NVFP4 5.0 /
-// 2.0 (2.3 / 1.2 with free ranges), transposed 0.7.  One model for all forms was 10 / 6, 7 / 4 and 9 % off, 86 % at worst: it
-// had 0.33 us per 64 K for two CTAs that share an SM, which take 0.62 with INT4 codes, as long as one after the other (712 x
-// 2048 x 16384: 89 us, 48 as planned now).
+// ranges NVFP4 weights get is ranked by a cost of its own, good for nothing but that: it decides in which order a result's sums
+// are added, and the pipeline hands on fp32 actions that follow every rounding before them, so it is fitted with the condition
+// that no linear of the pipeline changes its ranges.  Off the best candidate on average, plain / in a chain: INT4 2.0 / 1.6 %, NVFP4
+// 2.3 / 1.8, transposed 0.7.  One model for all forms was 10 / 6, 7 / 4 and 9 % off, 86 % at worst: it had 0.33 us per 64 K for
+// two CTAs that share an SM, which take 0.62 with INT4 codes, as long as one after the other (712 x 2048 x 16384: 89 us, 48 as
+// planned now).
 struct W4gCost {
     // 64 K values: max(a, b + c NT), for a CTA with an SM of its own, two that share one, and the narrow form of a CTA
     // where it has the SM to itself
@@ -972,9 +972,9 @@ struct W4gCost {
     float crowd[2];                                  // a grid of more than half the room leaves the next launch of a chain less to
                                                      // start in: [0] from a share [1] beyond the half on, in proportion before
 };
-constexpr W4gCost kCostNvfp4Ranges = {{0.18f, 0.05f, 0.0014f}, {0.34f, 0.0f, 0.0f}, {0.30f, 0.13f, 0.0025f},
-    {0.0f, 0.11f}, {1.85f, 1.85f}, {0.007f, 0.006f}, 0.5f,
-    {0.0f, 0.43f, 1.3f, 2.45f}, 0.012f, 0.012f, {1.8f, 1e-6f}};
+constexpr W4gCost kCostNvfp4Ranges = {{0.246f, 0.0f, 0.0012f}, {1.96f, 0.0f, 0.0f}, {0.303f, 0.0283f, 0.00875f},
+    {0.0f, 0.133f}, {6.66f, 1.95f}, {0.0138f, 0.0384f}, 1.9f,
+    {0.0f, 0.7f, 1.89f, 1.87f}, 0.0295f, 0.0203f, {1.28f, 0.516f}};
 constexpr W4gCost kCostNvfp4 = {{0.0723f, 0.0677f, 0.000111f}, {0.247f, 0.0499f, 0.000327f}, {0.00406f, 0.119f, 0.00163f},
     {0.00399f, 0.00399f}, {3.93f, 2.74f}, {0.014f, 0.0149f}, 0.32f,
     {0.0f, 0.112f, 0.0622f, 0.0429f}, 0.00508f, 0.00958f, {0.638f, 0.214f}};
